@@ -894,7 +894,7 @@ def main():
         b = np.concatenate([out64[0] + 1j * out64[1], out64[2] + 1j * out64[3]])
         ia = np.abs(a[:m]) ** 2 + np.abs(a[m:]) ** 2
         ib = np.abs(b[:m]) ** 2 + np.abs(b[m:]) ** 2
-        # The same FP64 path with the FMA-based phase reduction (opt-in).
+        # The same FP64 path with the option set (it selects the same kernel).
         ctx.set_option("f64_reduction", 1)
         solve("f64")
         torch.cuda.synchronize()

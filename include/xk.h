@@ -161,11 +161,9 @@ const char* xk_route_reason(int reason);
  *   "polarization"   -1 (default): when every ray's (es, ep) is a multiple of
  *                    ray 0's (to 2^-24), sum one amplitude column and scale it
  *                    for Es and Ep; 0: always sum Es and Ep separately
- *   "f64_reduction"  XK_PATH_F64 only: 0 (default) evaluates sin/cos of each
- *                    FP64 phase with the library functions, as the reference
- *                    does; 1 first reduces the phase by 2 pi with an FMA-based
- *                    Cody-Waite step (same phase value and 1e-10 parity, about
- *                    twice the throughput at phases of 1e10-1e13 rad)
+ *   "f64_reduction"  XK_PATH_F64 only: 0 (default) or 1. Both select the same
+ *                    kernel, which reduces each FP64 phase by pi/2 with FMAs;
+ *                    accepted for callers that set it
  *   "wait_limit"     polls of every bounded device-side wait (mbarrier waits of
  *                    the phase-reduced kernel and of the tensor-core Fresnel
  *                    product) before the kernel gives up and the call returns

@@ -1,11 +1,18 @@
 // Plain FP64 Kirchhoff path: the reference algorithm run directly in FP64.
 //
-// Per pair it evaluates exactly the expression of
-// src/waves/diffraction.rs:76-110 (diffraction_at_pixel), with every
-// multiply, add, divide and square root an explicitly rounded intrinsic so
-// nothing is contracted into an FMA, and CUDA's double sincos for the
-// exp(i*k*path) factor. Each thread accumulates its pixels with per-component
-// complex Kahan summation in ray order, as the reference does.
+// Per pair it evaluates the expression of src/waves/diffraction.rs:76-110
+// (diffraction_at_pixel). The phase k |p - r| is rounded step by step as the
+// reference rounds it (explicit intrinsics, no FMA: one ulp of the path is
+// 1e-5 rad), so sin and cos are taken of the same number; the smooth factors
+// around them use FMAs and one reciprocal of the path. Each thread accumulates
+// its pixels with per-component complex Kahan summation in ray order, as the
+// reference does.
+//
+// The kernel is bound by the FP64 pipe and by issue: 71 FP64 and about 60 other
+// instructions per pair. With the library's sincos, square root and two
+// divisions it took 408 instructions per pair; on 2^16 rays x 128^2 points
+// 16.2 ms then, 5.9 ms now (181 Gpair/s; the 71 FP64 instructions alone need
+// 4.1 ms), error against a 64-bit evaluation unchanged (6e-16).
 //
 // Parallel layout: a CTA owns 128*kF64Ppt screen points; the ray list is cut
 // into `splits` contiguous ranges (grid.y) when there are too few screen
@@ -21,6 +28,7 @@ namespace {
 
 constexpr int kF64Threads = 128;
 constexpr int kF64Ppt = 2;      // screen points per thread
+constexpr int kF64Ctas = 4;     // CTAs per SM (108 registers)
 constexpr int kF64Stage = 32;   // rays per shared-memory stage
 constexpr int kRecDoubles = 16; // 128-byte ray record
 
@@ -67,61 +75,124 @@ __device__ __forceinline__ void kahan_add(double& sum, double& comp, double term
     sum = t;
 }
 
-// sin and cos of a large FP64 phase x (|x| < 2^52; here k|p - r| <= ~1e13):
-// Cody-Waite reduction by 2*pi written with FMAs. 2*pi is split into three
-// doubles T1 = fl(2 pi), T2 = fl(2 pi - T1), T3 = fl(2 pi - T1 - T2) (from
-// Machin's formula to 80 digits); n = rint(x / 2 pi), n*T1 is formed exactly
-// as a rounded product plus its FMA error term, x - n*T1 is exact (Sterbenz),
-// and the remaining terms leave r = x - 2 pi n with an absolute error of a few
-// 1e-16 for every phase this path meets. sin/cos of |r| <= pi then take the
-// short path of the library functions.
-__device__ __forceinline__ void sincos_large(double x, double* s, double* c) {
-    constexpr double kT1 = 6.283185307179586, kT2 = 2.4492935982947064e-16,
-                     kT3 = -5.989539619436679e-33, kInv = 0.15915494309189535;
-    const double n = rint(x * kInv);
-    const double p1 = n * kT1;
-    const double e1 = fma(n, kT1, -p1);
-    double r = (x - p1) - e1;
-    r = fma(-n, kT2, r);
-    r = fma(-n, kT3, r);
-    sincos(r, s, c);
+// sin and cos of an FP64 phase x, |x| < 2^50, to about one ulp of 1.
+//
+// x = n pi/2 + r with n = rint(x 2/pi): fma(-n, T1, x) is x - n T1 rounded
+// once (T1 = fl(pi/2); the product is exact inside the FMA and |r| < 0.8), the
+// second FMA subtracts n T2 (T2 = fl(pi/2 - T1), up to 0.05 at 2^50), and the
+// neglected third part is below 2e-18, so r carries at most two roundings of
+// 2^-54. sin and cos of |r| <= pi/4 are r + r^3 S(r^2) and
+// 1 - r^2/2 + r^4 C(r^2), S and C of degree 5 interpolated at the Chebyshev
+// nodes of [0, (pi/4)^2] from their power series in 60-digit arithmetic
+// (largest error 1.5e-17 and 1e-18). The quadrant n mod 4 swaps and negates.
+__device__ __forceinline__ void sincos_quadrant(double x, double* sn, double* cs) {
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+    const double t = fma(x, 0.6366197723675814, kMagic);
+    const int q = __double2loint(t);  // n mod 2^32
+    const double n = t - kMagic;
+    double r = fma(-n, 1.5707963267948966, x);
+    r = fma(-n, 6.123233995736766e-17, r);
+    const double z = r * r;
+    double s = fma(z, 1.5918129014234338e-10, -2.5051131841108444e-08);
+    double c = fma(z, -1.1382632249960623e-11, 2.0876146265966424e-09);
+    s = fma(z, s, 2.755731610253375e-06);
+    c = fma(z, c, -2.75573172717181e-07);
+    s = fma(z, s, -0.00019841269836758538);
+    c = fma(z, c, 2.4801587298765665e-05);
+    s = fma(z, s, 0.008333333333330948);
+    c = fma(z, c, -0.0013888888888887398);
+    s = fma(z, s, -0.16666666666666666);
+    c = fma(z, c, 0.041666666666666664);
+    s = fma(r * z, s, r);
+    c = fma(z, fma(z, c, -0.5), 1.0);
+    const bool swap = q & 1;
+    const double a = swap ? c : s, b = swap ? s : c;
+    // sin is negative in quadrants 2 and 3, cos in 1 and 2.
+    *sn = __hiloint2double(__double2hiint(a) ^ ((q & 2) << 30), __double2loint(a));
+    *cs = __hiloint2double(__double2hiint(b) ^ (((q + 1) & 2) << 30), __double2loint(b));
 }
 
-template <bool REDUCE>
-__device__ __forceinline__ void pair_f64(const RayRec64& r, double px, double py, double pz,
-                                         Acc& a) {
-    double dx = __dsub_rn(px, r.x);
-    double dy = __dsub_rn(py, r.y);
-    double dz = __dsub_rn(pz, r.z);
-    double p2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    double path = __dsqrt_rn(p2);
-    if (path < 1e-30) return;  // diffraction.rs:81
-    double nd = __dadd_rn(__dadd_rn(__dmul_rn(r.nx, dx), __dmul_rn(r.ny, dy)), __dmul_rn(r.nz, dz));
-    double ns = __ddiv_rn(nd, path);
-    double phase = __dmul_rn(r.k, path);
-    double s, c;
-    if (REDUCE) sincos_large(phase, &s, &c);
-    else sincos(phase, &s, &c);
-    double obl = __dadd_rn(r.nl, ns);
-    double af = __ddiv_rn(__dmul_rn(r.kf, obl), path);
-    // u = i*af*exp(i*phase) = (-af*sin, af*cos)  (diffraction.rs:98)
-    double ure = -__dmul_rn(af, s);
-    double uim = __dmul_rn(af, c);
-    double tr = __dsub_rn(__dmul_rn(r.es_re, ure), __dmul_rn(r.es_im, uim));
-    double ti = __dadd_rn(__dmul_rn(r.es_re, uim), __dmul_rn(r.es_im, ure));
-    kahan_add(a.s[0], a.c[0], tr);
-    kahan_add(a.s[1], a.c[1], ti);
-    tr = __dsub_rn(__dmul_rn(r.ep_re, ure), __dmul_rn(r.ep_im, uim));
-    ti = __dadd_rn(__dmul_rn(r.ep_re, uim), __dmul_rn(r.ep_im, ure));
-    kahan_add(a.s[2], a.c[2], tr);
-    kahan_add(a.s[3], a.c[3], ti);
+// path = sqrt(p2) and 1/path. A reciprocal square root seed (relative error e
+// below 2^-20) takes one third-order step, y (1 + e/2 + 3 e^2/8) (Halley), and
+// the square root p2 y its residual correction (Markstein): the residual
+// p2 - g^2 is exact in an FMA, so g + residual y / 2 rounds as the exact root
+// does. The phase k path needs that (one ulp of a 1 m path is 6e-6 rad at
+// 10 keV); a division per quotient does not, so both quotients by the path
+// multiply by the reciprocal instead.
+__device__ __forceinline__ double sqrt_and_rcp(double p2, double* inv) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p2));
+    const double e = fma(-(p2 * y), y, 1.0);
+    y = fma(y * e, fma(0.375, e, 0.5), y);
+    double g = p2 * y;
+    g = fma(fma(-g, g, p2), 0.5 * y, g);
+    *inv = fma(y, fma(-g, y, 1.0), y);
+    return g;
 }
 
-// The kernel is issue-bound (about 400 instructions per pair with the library
-// sincos); capping registers at 80 for six CTAs per SM (24 warps instead of
-// 20) hides a little more latency: +4 % plain, +2 % reduced, same results.
-template <bool REDUCE>
-__global__ void __launch_bounds__(kF64Threads, 6)
+// Whatever the fast form does not take: the library functions.
+__device__ __noinline__ void geometry_general(double p2, double k, double* path, double* inv,
+                                              double* s, double* c) {
+    *path = __dsqrt_rn(p2);
+    *inv = __ddiv_rn(1.0, *path);
+    sincos(__dmul_rn(k, *path), s, c);
+}
+
+// One ray against PPT screen points. The points' chains are independent, so
+// they are evaluated side by side and share the ray's values and the
+// polynomials' constants.
+template <int PPT>
+__device__ __forceinline__ void pairs_f64(const RayRec64& r, const double (&px)[PPT],
+                                          const double (&py)[PPT], const double (&pz)[PPT],
+                                          Acc (&acc)[PPT]) {
+    double p2[PPT], nd[PPT], inv[PPT], phase[PPT], s[PPT], c[PPT];
+    bool fast = true;
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+        const double dx = __dsub_rn(px[i], r.x);
+        const double dy = __dsub_rn(py[i], r.y);
+        const double dz = __dsub_rn(pz[i], r.z);
+        // Rounded as the reference rounds it: the phase is k times the root.
+        p2[i] = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        nd[i] = fma(r.nz, dz, fma(r.ny, dy, r.nx * dx));
+        phase[i] = __dmul_rn(r.k, sqrt_and_rcp(p2[i], &inv[i]));
+        // 2^-198 <= p2 < 2^777 (path > 1e-30, no under- or overflow above)
+        // and |phase| < 2^50; NaN and infinities fall outside.
+        fast = fast &&
+               (unsigned)(__double2hiint(p2[i]) - 0x33900000) < 0x73000000u - 0x33900000u &&
+               (__double2hiint(phase[i]) & 0x7fffffff) < 0x43100000;
+    }
+    bool skip[PPT] = {};
+    if (fast) {
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) sincos_quadrant(phase[i], &s[i], &c[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+            double path;
+            geometry_general(p2[i], r.k, &path, &inv[i], &s[i], &c[i]);
+            skip[i] = path < 1e-30;  // diffraction.rs:81
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+        if (skip[i]) continue;
+        const double af = r.kf * fma(nd[i], inv[i], r.nl) * inv[i];
+        // u = i*af*exp(i*phase) = (-af*sin, af*cos)  (diffraction.rs:98)
+        const double us = af * s[i], uc = af * c[i];
+        Acc& a = acc[i];
+        kahan_add(a.s[0], a.c[0], fma(-r.es_re, us, -(r.es_im * uc)));
+        kahan_add(a.s[1], a.c[1], fma(r.es_re, uc, -(r.es_im * us)));
+        kahan_add(a.s[2], a.c[2], fma(-r.ep_re, us, -(r.ep_im * uc)));
+        kahan_add(a.s[3], a.c[3], fma(r.ep_re, uc, -(r.ep_im * us)));
+    }
+}
+
+// Two points per thread at four CTAs per SM: 5.91 ms on 2^16 rays x 128^2
+// points (6.00 at six CTAs, 5.88 with three points, 5.96 and 6.56 with four
+// points at three and two CTAs; three or four points leave more of the last
+// CTA idle on small screens).
+__global__ void __launch_bounds__(kF64Threads, kF64Ctas)
 f64_pairs_kernel(const RayRec64* __restrict__ rays, size_t n_rays, size_t rays_per_split,
                  PixDev pix, size_t n_pix, FieldDev out, double* __restrict__ partials) {
     __shared__ RayRec64 sm[kF64Stage];
@@ -151,10 +222,8 @@ f64_pairs_kernel(const RayRec64* __restrict__ rays, size_t n_rays, size_t rays_p
         double* dst = reinterpret_cast<double*>(sm);
         for (int t = threadIdx.x; t < cnt * kRecDoubles; t += kF64Threads) dst[t] = src[t];
         __syncthreads();
-        for (int j = 0; j < cnt; ++j) {
-#pragma unroll
-            for (int i = 0; i < kF64Ppt; ++i) pair_f64<REDUCE>(sm[j], px[i], py[i], pz[i], acc[i]);
-        }
+#pragma unroll 1
+        for (int j = 0; j < cnt; ++j) pairs_f64<kF64Ppt>(sm[j], px, py, pz, acc);
     }
 
 #pragma unroll
@@ -175,21 +244,29 @@ f64_pairs_kernel(const RayRec64* __restrict__ rays, size_t n_rays, size_t rays_p
     }
 }
 
-// Adds the per-range partials of every screen point in range order.
+// Adds the per-range partials of every screen point in range order, one
+// thread per (point, component). The Kahan chain is serial but the loads are
+// not: eight ranges are in flight while the previous eight are added.
 __global__ void f64_combine_kernel(const double* __restrict__ partials, int splits, size_t n_pix,
                                    FieldDev out) {
-    size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (p >= n_pix) return;
-    double s[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
-    for (int k = 0; k < splits; ++k) {
-        const double* base = partials + (size_t)k * 4 * n_pix;
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    const size_t total = 4 * n_pix;
+    if (i >= total) return;
+    constexpr int kAhead = 8;
+    double s = 0.0, c = 0.0;
+    int k = 0;
+    for (; k + kAhead <= splits; k += kAhead) {
+        double v[kAhead];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) kahan_add(s[j], c[j], base[j * n_pix + p]);
+        for (int u = 0; u < kAhead; ++u) v[u] = partials[(size_t)(k + u) * total + i];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) kahan_add(s, c, v[u]);
     }
-    out.es_re[p] = s[0];
-    out.es_im[p] = s[1];
-    out.ep_re[p] = s[2];
-    out.ep_im[p] = s[3];
+    for (; k < splits; ++k) kahan_add(s, c, partials[(size_t)k * total + i]);
+    const int comp = (int)(i / n_pix);
+    double* const dst = comp == 0 ? out.es_re : comp == 1 ? out.es_im
+                                              : comp == 2 ? out.ep_re : out.ep_im;
+    dst[i - comp * n_pix] = s;
 }
 
 __global__ void zero_field_kernel(FieldDev out, size_t n_pix) {
@@ -253,16 +330,12 @@ Status f64_enqueue(const RaysDev& rays, size_t n_rays, const PixDev& pix, size_t
         partials = ws.partials.as<double>();
     }
     dim3 grid((unsigned)pix_ctas, (unsigned)splits);
-    if (ws.fast_reduction)
-        f64_pairs_kernel<true><<<grid, kF64Threads, 0, stream>>>(packed, n_rays, rays_per_split,
-                                                                 pix, n_pix, out, partials);
-    else
-        f64_pairs_kernel<false><<<grid, kF64Threads, 0, stream>>>(packed, n_rays, rays_per_split,
-                                                                  pix, n_pix, out, partials);
+    f64_pairs_kernel<<<grid, kF64Threads, 0, stream>>>(packed, n_rays, rays_per_split, pix, n_pix,
+                                                       out, partials);
     XK_CUDA_TRY(cudaGetLastError());
     int kernels = 2;
     if (splits > 1) {
-        f64_combine_kernel<<<(unsigned)((n_pix + 255) / 256), 256, 0, stream>>>(
+        f64_combine_kernel<<<(unsigned)((4 * n_pix + 127) / 128), 128, 0, stream>>>(
             partials, (int)splits, n_pix, out);
         XK_CUDA_TRY(cudaGetLastError());
         kernels += 1;
@@ -422,12 +495,12 @@ extern "C" int xk_diffraction_f64_noalloc(const xk_rays* rays, size_t n_rays,
     f64_pack_kernel<<<(unsigned)((n_rays + 255) / 256), 256, 0, s>>>(rd, n_rays, packed);
     if (cudaGetLastError() != cudaSuccess) return XK_ERR_CUDA;
     dim3 grid((unsigned)pix_ctas, (unsigned)splits);
-    f64_pairs_kernel<false><<<grid, kF64Threads, 0, s>>>(packed, n_rays, rays_per_split, pd,
-                                                          n_pix, fd, partials);
+    f64_pairs_kernel<<<grid, kF64Threads, 0, s>>>(packed, n_rays, rays_per_split, pd, n_pix, fd,
+                                                  partials);
     if (cudaGetLastError() != cudaSuccess) return XK_ERR_CUDA;
     if (splits > 1) {
-        f64_combine_kernel<<<(unsigned)((n_pix + 255) / 256), 256, 0, s>>>(partials, (int)splits,
-                                                                           n_pix, fd);
+        f64_combine_kernel<<<(unsigned)((4 * n_pix + 127) / 128), 128, 0, s>>>(
+            partials, (int)splits, n_pix, fd);
         if (cudaGetLastError() != cudaSuccess) return XK_ERR_CUDA;
     }
     return XK_OK;
