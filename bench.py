@@ -464,6 +464,21 @@ def run_sweep(args):
     return 0
 
 
+def tensor_peak():
+    """Dense f16/bf16 tensor rate [TFLOP/s] the rooflines divide by, and where it is from."""
+    peaks = {}
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            peaks = json.load(f)
+    except OSError:
+        pass
+    if "bf16_tflops" in peaks:
+        return (float(peaks["bf16_tflops"]),
+                "MEASURED_PEAKS.json bf16_tflops (burst; f16 runs at the bf16 rate)")
+    return 1590.0, ("fallback: 1590 TFLOP/s, an earlier burst cuBLAS bf16 measurement on "
+                    "this pool (MEASURED_PEAKS.json absent; f16 runs at the bf16 rate)")
+
+
 def run_fresnel(args):
     """2-D Fresnel propagation (src/waves/fresnel.rs:53-106): the aperture's
     2^20 rays (x, z) with complex amplitudes onto a 512x512 screen of
@@ -504,19 +519,7 @@ def run_fresnel(args):
     # Tensor work: per pair one complex multiply-add (8 real flops) in each of
     # the three f16 partial products.
     algo_flops = 24.0 * pairs
-    peaks = {}
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            peaks = json.load(f)
-    except OSError:
-        pass
-    if "bf16_tflops" in peaks:
-        peak = float(peaks["bf16_tflops"])
-        peak_source = "MEASURED_PEAKS.json bf16_tflops (burst; f16 runs at the bf16 rate)"
-    else:
-        peak = 1590.0
-        peak_source = ("fallback: 1590 TFLOP/s, an earlier burst cuBLAS bf16 measurement on "
-                       "this pool (MEASURED_PEAKS.json absent; f16 runs at the bf16 rate)")
+    peak, peak_source = tensor_peak()
     gemm = float(np.mean(gemm_ms))
     achieved = algo_flops / (gemm / 1e3) / 1e12
     # Screens of more than 128 rows run on CTA pairs (stats sweep = 1).
@@ -965,6 +968,21 @@ def main():
                     "fma_pipe_ops_per_pair": fma_ops, "sfu_ops_per_pair": SFU_OPS_PER_PAIR,
                     "peak": algo_peak, "ratio": achieved / algo_peak}}
 
+    if stats["sweep"] == 3:
+        # The rectangular screen as a tensor-core product: four f16 products
+        # (three of the split phasors, the first-order coupling) of one complex
+        # multiply-add per pair and amplitude column.
+        flops = 32.0 * pairs * (1 if one_col else 2)
+        peak, peak_source = tensor_peak()
+        achieved_tf = flops / (kms / 1e3) / 1e12
+        roofline = {"bound": "tensor", "achieved": achieved_tf, "peak": peak, "unit": "TFLOP/s",
+                    "frac": achieved_tf / peak, "traffic": None, "kernel": "grid_product_kernel",
+                    "kernel_ms": kms, "peak_source": peak_source,
+                    "flops_per_pair": 32 * (1 if one_col else 2),
+                    "sum_own_flops": {"flops_per_pair": 8 * (1 if one_col else 2),
+                                      "achieved": achieved_tf / 4.0,
+                                      "frac": achieved_tf / 4.0 / peak}}
+
     cpu = None
     if rank == 0 and not args.no_cpu:
         cpu = cpu_baseline(rays, screen, args.cpu_seconds)
@@ -1004,7 +1022,7 @@ def main():
                    "l2": "flushed between steps (256 MiB write)",
                    "path": "f32pr", "phase_bound_rad": stats["phase_bound_rad"],
                    "n_tiles": stats["n_tiles"], "n_chunks": stats["n_chunks"],
-                   "groups": stats["groups"], "sweep": ["sfu_rcp", "packed_f32x2", "packed_f32x2_linear_series"][stats["sweep"]],
+                   "groups": stats["groups"], "sweep": ["sfu_rcp", "packed_f32x2", "packed_f32x2_linear_series", "tensor_core_product"][stats["sweep"]],
                    "amplitude_columns": 1 if stats["one_polarization"] else 2},
         "e2e": e2e, "fp64_plain": fp64, "two_amplitude_columns": two_col,
         "roofline": roofline, "cpu_baseline": cpu, "serve": serve,

@@ -19,7 +19,9 @@
  *   XK_PATH_F32PR  FP32 phase-reduced form: per (screen tile, ray chunk)
  *                  item the phase is split into FP64 per-pixel and per-ray
  *                  parts and an FP32 residual, compensated two-float
- *                  accumulation, FP64 cross-chunk reduction. Solves it cannot
+ *                  accumulation, FP64 cross-chunk reduction; rectangular
+ *                  screens as a product of split f16 phasors on the tensor
+ *                  cores (option "grid_product"). Solves it cannot
  *                  bound (mixed energies within a chunk, rays touching the
  *                  screen) are routed to XK_PATH_F64 and reported in stats.
  *
@@ -108,7 +110,9 @@ typedef struct xk_stats {
     int groups;              /* ray groups per tile (F32PR) */
     int routed_reason;       /* 0 = not routed; see xk_route_reason() */
     int sweep;               /* F32PR sweep used: 0 SFU reciprocal, 1 packed + quadratic series,
-                                2 packed + linear series; XK_PATH_SEPARABLE (Fresnel): 1 CTA-pair
+                                2 packed + linear series, 3 rectangular screen as a tensor-core
+                                product (n_tiles, groups and n_chunks: its 256 x 128 tiles, ray
+                                splits and 32-ray blocks); XK_PATH_SEPARABLE (Fresnel): 1 CTA-pair
                                 tiles, 0 one CTA per tile; -1 none */
     int one_polarization;    /* F32PR: 1 if every ray had ray 0's polarization, so the kernel
                                 summed one amplitude column and Ep = (ep_0 / es_0) Es */
@@ -161,6 +165,12 @@ const char* xk_route_reason(int reason);
  *   "polarization"   -1 (default): when every ray's (es, ep) is a multiple of
  *                    ray 0's (to 2^-24), sum one amplitude column and scale it
  *                    for Es and Ep; 0: always sum Es and Ep separately
+ *   "grid_product"   1 (default): a rectangular screen (points outer x inner along
+ *                    two coordinates, the third constant, bit for bit) far enough
+ *                    from the rays runs as a tensor-core product, to the same
+ *                    tolerance; 0: always the general kernel. A set "sweep" or
+ *                    "groups", or a tolerance under 6e-5, also takes the general
+ *                    kernel
  *   "f64_reduction"  XK_PATH_F64 only: 0 (default) or 1. Both select the same
  *                    kernel, which reduces each FP64 phase by pi/2 with FMAs;
  *                    accepted for callers that set it

@@ -128,7 +128,7 @@ xk::Status run_solve(xk_ctx* ctx, const xk::RaysDev& rays, size_t n_rays, const 
             stats->groups = P.groups;
             stats->routed_reason = P.routed ? P.route_reason : 0;
             stats->main_kernel_ms = er.main_kernel_ms;
-            stats->sweep = P.routed ? -1 : (P.fast ? (P.lin ? 2 : 1) : 0);
+            stats->sweep = P.routed ? -1 : P.grid ? 3 : (P.fast ? (P.lin ? 2 : 1) : 0);
             stats->one_polarization = !P.routed && P.one_pol;
         }
     } else {
@@ -342,6 +342,9 @@ int xk_set_option(xk_ctx* ctx, const char* name, double value) {
     } else if (n == "items_per_warp") {
         if (value < 1.0 || value > 4096.0) return fail(ctx, XK_ERR_INVALID, "items_per_warp out of range");
         ctx->pr_opts.items_per_warp = (long long)value;
+    } else if (n == "grid_product") {
+        if (value != 0.0 && value != 1.0) return fail(ctx, XK_ERR_INVALID, "grid_product is 0 or 1");
+        ctx->pr_opts.grid = value != 0.0;
     } else if (n == "use_tuned") {
         if (value != 0.0 && value != 1.0) return fail(ctx, XK_ERR_INVALID, "use_tuned is 0 or 1");
         ctx->tune.use = value != 0.0;

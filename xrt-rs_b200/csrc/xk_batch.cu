@@ -181,6 +181,8 @@ xk::Status create_batch(xk_ctx* ctx, const xk_solve* solves, size_t n, int path,
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 
     XK_TRY(xk::pr_reserve_exec(b->ws, (int)n, ctx->num_sms));
+    for (const xk::PrPlan& P : b->plans)
+        if (!P.routed && P.grid) XK_TRY(xk::grid_reserve(P.grid_plan, b->ws.grid));
     if ((flags & XK_BATCH_NO_GRAPH) == 0) {
         XK_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         xk::Status st = enqueue_batch(b);
@@ -300,7 +302,7 @@ int xk_batch_solve_plan(const xk_batch* batch, size_t i, xk_solve_plan* out) {
     out->groups = P.groups;
     out->phase_bound_rad = P.phase_bound;
     out->tuned = P.tuned ? 1 : 0;
-    out->sweep = P.routed ? -1 : (P.fast ? (P.lin ? 2 : 1) : 0);
+    out->sweep = P.routed ? -1 : P.grid ? 3 : (P.fast ? (P.lin ? 2 : 1) : 0);
     out->one_polarization = !P.routed && P.one_pol;
     return XK_OK;
 }

@@ -1,0 +1,912 @@
+// Phase-reduced Kirchhoff sum on a rectangular screen as a tensor-core product.
+//
+// On a screen whose points are (a_i, b_l, c) the squared distance to a ray is a
+// sum of a row part and a column part, and only the square root couples them.
+// For a tile with reference point p0 = (a0, b0, c), u = a_i - a0, v = b_l - b0,
+// A = a0 - r_a, B = b0 - r_b, D = |p0 - r|:
+//     |p - r|^2 = D^2 + dS + dT,  dS = u (u + 2A),  dT = v (v + 2B),
+//     |p - r|   = D + (sqrt(D^2 + dS) - D) + (sqrt(D^2 + dT) - D) + E/k,
+//     E         = -k dS dT / (4 D^3) (1 + O((dS + dT) / D^2)).
+// The first three terms make a phase that is a row phase plus a column phase,
+// so the tile is a complex matrix product over the rays, and
+// exp(i E) = 1 + i E + O(E^2) adds one more product with the same ray index as
+// contraction, because E is a row factor dS times a column factor dT. The
+// planner takes the product only where the dropped terms stay far below the
+// requested tolerance (grid_plan). The amplitude (nl + n.(p - r)/|p - r|) /
+// |p - r| varies along a tile by 1e-7 to 1e-2; its ray part at p0 goes to the
+// columns, its first-order change to each side as a factor.
+//
+//   * grid_records_kernel: per (tile, ray) 64 bytes: k D in turns, reduced in
+//     double-double (k D reaches 1e12 rad), the linear phase coefficients as
+//     hi + lo floats, the amplitude at p0.
+//   * grid_product_kernel: CTA pairs (tcgen05 cta_group::2, 256 rows x 128
+//     columns), the structure of fresnel_pair_kernel: producer warps turn rays
+//     into f16 hi + lo phasor tiles in shared memory, one thread issues
+//     A_hi B_hi + A_hi B_lo + A_lo B_hi + A_1 B_1 per block of 32 rays, four
+//     epilogue warps drain the f32 accumulator every `seg` blocks.
+//   * grid_reduce_kernel: adds the ray splits in FP64, in split order, applies
+//     i k / (4 pi) and the polarization.
+//
+// Row and column phases are evaluated as in the Fresnel product: sqrt(D^2 + dS)
+// - D = dS / (2D) - dS^2 / (8 D^3), where dS / (2D) = u^2 h + u (2 h A), h =
+// 1 / (2D): u^2 h0 is reduced in FP64 per row, u (2 h A) is an exact FP32
+// product of hi + lo parts, u^2 (h - h0) and the second-order term are small.
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "xk_dd.cuh"
+#include "xk_grid.cuh"
+#include "xk_phasor.cuh"
+
+namespace xk {
+namespace {
+
+using namespace phasor;
+
+constexpr int kTileM = 256, kTileN = 128;
+constexpr uint32_t kGA = 128 * 128;      // one operand tile: 128 rows x 128 B (A or this CTA's B half)
+constexpr uint32_t kGStage = 6 * kGA;    // A_hi | A_lo | B_hi | B_lo | A_1 | B_1
+constexpr int kGStages = 2;
+constexpr int kGProdThreads = 384;       // warps 5..16
+constexpr int kGThreads = 32 + kFEpiThreads + kGProdThreads + 32;
+constexpr uint32_t kGRayBytes = kFRays * 64;
+constexpr size_t kGSmem =
+    1024 + (size_t)kGStages * kGStage + kFRayBufs * kGRayBytes + kFEpiBytes + 256;
+static_assert(kGSmem <= 227 * 1024, "shared memory");
+constexpr double kSmallSpread = 16.0;    // [rad] mean residual phase of the whole ray set
+constexpr double kGridScale = 1024.0;    // largest |W|: lo parts stay normal f16 numbers
+constexpr size_t kGridRecBytes = (size_t)512 << 20;  // ray records of one launch
+constexpr size_t kGridMaxTiles = 4096;               // at least 2048 rays per launch fit then
+
+// ---- order of the screen points -------------------------------------------------
+
+__device__ __forceinline__ const double* coord(const PixDev& p, int c) {
+    return c == 0 ? p.x : (c == 1 ? p.y : p.z);
+}
+
+__global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
+                                                         const double* __restrict__ len_part,
+                                                         int parts, int stride,
+                                                         GridProbe* __restrict__ out) {
+    __shared__ double s_len[256];
+    double v = INFINITY;
+    for (int i = threadIdx.x; i < parts; i += 256) v = fmin(v, len_part[(size_t)i * stride]);
+    s_len[threadIdx.x] = v;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) s_len[threadIdx.x] = fmin(s_len[threadIdx.x], s_len[threadIdx.x + o]);
+        __syncthreads();
+    }
+    const double lend = s_len[0];
+    if (!(lend >= 2.0 && lend <= 0.5 * m)) return;  // len stays 0
+    const int len = (int)lend;
+    if (m % len != 0) return;
+    const int inner = p.x[1] != p.x[0] ? 0 : (p.y[1] != p.y[0] ? 1 : 2);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        out->len = len;
+        out->inner = inner;
+    }
+    const int t0 = blockIdx.x * 256 + threadIdx.x, step = gridDim.x * 256;
+    int bad = 0, mask = 0;
+    for (int q = t0; q < m; q += step) {
+        const int i = q / len, l = q - i * len;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double* a = coord(p, c);
+            const double w = a[q];
+            bad |= w != a[c == inner ? l : i * len];
+            if (c != inner) mask |= (w != a[0]) << c;
+        }
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    mask = __reduce_or_sync(0xffffffffu, (unsigned)mask);
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        if (bad) atomicOr(&out->bad, 1);
+        if (mask) atomicOr(&out->outer_mask, mask);
+    }
+    // Tile extents, one warp per tile.
+    const int warp = t0 >> 5, warps = step >> 5;
+    for (int axis = 0; axis < 2; ++axis)
+        for (int k = 0; k < 2; ++k) {
+            const int count = axis ? len : m / len, size = 128 << k;
+            for (int t = warp; t * size < count; t += warps) {
+                double half = 0.0;
+                for (int c = 0; c < 3; ++c) {
+                    if ((c == inner) != (axis == 1)) continue;
+                    const double* a = coord(p, c);
+                    double lo = INFINITY, hi = -INFINITY;
+                    for (int q = t * size + lane; q < min(count, (t + 1) * size); q += 32) {
+                        const double w = a[axis ? q : q * len];
+                        lo = fmin(lo, w);
+                        hi = fmax(hi, w);
+                    }
+                    for (int o = 16; o > 0; o >>= 1) {
+                        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+                    }
+                    half = fmax(half, 0.5 * (hi - lo));
+                }
+                if (lane == 0)
+                    atomicMax(&out->extent[axis][k], (unsigned long long)__double_as_longlong(half));
+            }
+        }
+}
+
+// One block per tile: the axis coordinates of its points and their mid-range.
+__global__ void __launch_bounds__(kTileM) grid_axes_kernel(const double* __restrict__ src_m,
+                                                           size_t stride_m, int nm, int m_tiles,
+                                                           const double* __restrict__ src_n,
+                                                           size_t stride_n, int nn,
+                                                           double* __restrict__ axes) {
+    const bool is_m = (int)blockIdx.x < m_tiles;
+    const int t = is_m ? blockIdx.x : blockIdx.x - m_tiles;
+    const int size = is_m ? kTileM : kTileN, count = is_m ? nm : nn;
+    const int q = t * size + threadIdx.x;
+    double lo = INFINITY, hi = -INFINITY;
+    if ((int)threadIdx.x < size && q < count) {
+        const double w = is_m ? src_m[q * stride_m] : src_n[q * stride_n];
+        axes[is_m ? q : nm + q] = w;
+        lo = hi = w;
+    }
+    __shared__ double s[8][2];
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s[threadIdx.x >> 5][0] = lo;
+        s[threadIdx.x >> 5][1] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            lo = fmin(lo, s[w][0]);
+            hi = fmax(hi, s[w][1]);
+        }
+        axes[nm + nn + blockIdx.x] = 0.5 * (lo + hi);
+    }
+}
+
+// ---- ray records ------------------------------------------------------------------
+
+// Per ray and tile (64 bytes; a / b: row / column axis):
+//   {La hi, Lb hi, La lo, Lb lo}   L = 2 h A turns / mm
+//   {2A, 2B, h - h0, -q}           q = turns of the second-order term per dS^2
+//   {R, W re, W im, -m}            R = frac(k D), W = amplitude at p0, scaled
+//   {sa, sb, W2 re, W2 im}         amplitude slopes; second column
+struct RecordArgs {
+    const double *ra, *rb, *rc, *na, *nb, *nc, *nl;
+    const double *w_re, *w_im, *w2_re, *w2_im;
+    const double* refs;  // tile references: m_tiles, then n_tiles
+    int m_tiles, n_tiles;
+    size_t n, pad;       // rays of this launch, rounded up to whole blocks
+    double c0, h0, kt, kt_lo, scale;
+};
+
+__global__ void __launch_bounds__(256) grid_records_kernel(RecordArgs g, float4* __restrict__ out) {
+    const size_t j = blockIdx.x * (size_t)256 + threadIdx.x;
+    if (j >= g.pad) return;
+    const int tile = blockIdx.y, mt = tile / g.n_tiles, nt = tile - mt * g.n_tiles;
+    float4* o = out + ((size_t)tile * g.pad + j) * 4;
+    if (j >= g.n) {
+        for (int i = 0; i < 4; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    double al, bl, cl;
+    const double a = dd_diff(g.refs[mt], g.ra[j], &al), b = dd_diff(g.refs[g.m_tiles + nt], g.rb[j], &bl),
+                 c = dd_diff(g.c0, g.rc[j], &cl);
+    double d, unused;
+    const double turns = dd_turns<true>(g.kt, g.kt_lo, a, b, c, &d, &unused,
+                                        2.0 * (a * al + b * bl + c * cl));
+    const double inv = 1.0 / d, h = 0.5 * g.kt * inv;
+    const double na = g.na[j], nb = g.nb[j], nc = g.nc[j];
+    const double nu = (na * a + nb * b + nc * c) * inv;
+    const double obl = g.nl[j] + nu;
+    const double w = obl * inv * g.scale;
+    const double la = 2.0 * h * a, lb = 2.0 * h * b;
+    const float lah = (float)la, lbh = (float)lb;
+    o[0] = make_float4(lah, lbh, (float)(la - (double)lah), (float)(lb - (double)lbh));
+    o[1] = make_float4((float)(2.0 * a), (float)(2.0 * b), (float)(h - g.h0),
+                       (float)(-0.25 * h * inv * inv));
+    o[2] = make_float4((float)(turns - rint(turns)), (float)(g.w_re[j] * w), (float)(g.w_im[j] * w),
+                       (float)(-0.5 * (1.0 + nu / obl) * inv * inv));
+    float4 e = make_float4((float)(na * inv / obl), (float)(nb * inv / obl), 0.f, 0.f);
+    if (g.w2_re) {
+        e.z = (float)(g.w2_re[j] * w);
+        e.w = (float)(g.w2_im[j] * w);
+    }
+    o[3] = e;
+}
+
+// ---- the product --------------------------------------------------------------------
+
+struct ProductArgs {
+    const float4* recs;
+    size_t pad;
+    int ray_blocks, splits, seg;
+    int m_tiles, n_tiles;
+    const double *cm, *cn, *refs;
+    size_t nm, nn;
+    double h0;
+    float* partial;  // [splits][m_pad][n_pad]
+    int m_pad, n_pad;
+    bool first;      // the splits' first segments store
+    int* err;
+    uint32_t wait_limit, stall;
+};
+
+__device__ __forceinline__ uint32_t neg2(uint32_t v) { return v ^ 0x80008000u; }
+
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+    const __half2 r = __hmul2(*reinterpret_cast<const __half2*>(&a),
+                              *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// Producer warps of a CTA of the pair, the work split of fresnel_pair_kernel:
+// warps 0..7 (ZZ = false) fill 16-byte chunk c0 (four rays) of the A rows l,
+// l + 32 and of the B rows of points l, l + 32; warps 8..11 (ZZ = true) chunks
+// c0, c0 + 1 of the A rows 64 + l, 96 + l. Inside a chunk the contraction runs
+// (re j, re j+1, im j, im j+1) over ray pairs, in both operands, so that the
+// real-part and imaginary-part rows of B hold the same words in another order
+// (and one sign). Rows and columns past the screen's edge hold the phasors of
+// the tile's reference point: they only reach accumulators nobody reads. AMP:
+// the amplitude varies along the tile.
+template <bool ZZ, bool AMP>
+__device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int r, int mt, int nt,
+                                              int col, uint32_t half, int nrb, unsigned char* tiles,
+                                              uint32_t full_lead, uint64_t* empty,
+                                              uint64_t* ray_full, uint64_t* ray_empty,
+                                              unsigned char* rays_smem, volatile int* flag) {
+    using namespace sm100;
+    constexpr int NE = ZZ ? 1 : 2;   // pair-rows per thread
+    constexpr int NCH = ZZ ? 2 : 1;  // chunks per thread
+    float2 kh2[NE], khn2[NE], kl2[NE], pp2[NE], sq2[NE];
+    const double ref_m = g.refs[mt >> 1], ref_n = g.refs[g.m_tiles + nt];
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+        const size_t im = (size_t)mt * 128 + (ZZ ? 64 + r : r + 32 * e);
+        const double ux = im < g.nm ? g.cm[im] - ref_m : 0.0;
+        double uy;
+        if (ZZ) {
+            const size_t iy = (size_t)mt * 128 + 96 + r;
+            uy = iy < g.nm ? g.cm[iy] - ref_m : 0.0;
+        } else {
+            const size_t in = (size_t)nt * 128 + 64 * half + r + 32 * e;
+            uy = in < g.nn ? g.cn[in] - ref_n : 0.0;
+        }
+        float hx, lx, hy, ly, fx, fy;
+        split_coord(ux, g.h0, &hx, &lx, &fx);
+        split_coord(uy, g.h0, &hy, &ly, &fy);
+        kh2[e] = make_float2(hx, hy);
+        khn2[e] = make_float2(-hx, -hy);
+        kl2[e] = make_float2(lx, ly);
+        pp2[e] = make_float2(fx, fy);
+        sq2[e] = make_float2((float)(ux * ux), (float)(uy * uy));
+    }
+    for (int i = 0; i < nrb; ++i) {
+        const int s = i % kGStages, rb = i % kFRayBufs;
+        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kFRayBufs) & 1u, g.wait_limit);
+        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kGStages) & 1u) ^ 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *flag = 1;
+            return;
+        }
+        unsigned char* base = tiles + (size_t)s * kGStage;
+        const float4* sr = reinterpret_cast<const float4*>(rays_smem + rb * kGRayBytes);
+#pragma unroll
+        for (int ch = 0; ch < NCH; ++ch) {
+            const int c = c0 + ch;
+            // A rows of .x and (ZZ) of .y; B points of .y: four words per tile.
+            uint32_t ah[2][4], al[2][4], ae[2][4], bh[2][4], bl[2][4], be[2][4];
+#pragma unroll
+            for (int pr = 0; pr < 2; ++pr) {
+                float cx[2][2], sx[2][2], cy[2][2], sy[2][2], ex[2][2], ey[2][2];  // [e][ray]
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float4* rec = sr + 4 * (4 * c + 2 * pr + u);
+                    const float4 v0 = rec[0], v1 = rec[1], v2 = rec[2];
+                    float4 v3 = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (AMP || (!ZZ && col)) v3 = rec[3];
+                    const float2 rh = ZZ ? f2(v0.x) : make_float2(v0.x, v0.y);
+                    const float2 rl = ZZ ? f2(v0.z) : make_float2(v0.z, v0.w);
+                    const float2 ab = ZZ ? f2(v1.x) : make_float2(v1.x, v1.y);
+                    const float wr0 = col ? v3.z : v2.y, wi0 = col ? v3.w : v2.z;
+#pragma unroll
+                    for (int e = 0; e < NE; ++e) {
+                        const float2 ds = __ffma2_rn(kh2[e], ab, sq2[e]);  // dS, dT
+                        const float2 qd = __fmul2_rn(f2(v1.w), ds);        // -q dS, -q dT
+                        const float2 small = __ffma2_rn(qd, ds, __fmul2_rn(f2(v1.z), sq2[e]));
+                        float2 p0 = __fadd2_rn(pp2[e], small);
+                        if (!ZZ) p0 = __fadd2_rn(p0, make_float2(0.f, v2.x));
+                        const float2 t = pair_turns2(kh2[e], khn2[e], kl2[e], p0, rh, rl);
+                        const float2 th = __fmul2_rn(t, f2(6.28318530717958647692f));
+                        __sincosf(th.x, &sx[e][u], &cx[e][u]);
+                        __sincosf(th.y, &sy[e][u], &cy[e][u]);
+                        ex[e][u] = ds.x;
+                        ey[e][u] = ZZ ? ds.y : qd.y * 12.566370614359172f;
+                        float2 f = f2(1.f);
+                        if (AMP) {
+                            const float2 sl = ZZ ? f2(v3.x) : make_float2(v3.x, v3.y);
+                            f = __ffma2_rn(kh2[e], sl, __ffma2_rn(f2(v2.w), ds, f2(1.f)));
+                            cx[e][u] *= f.x;
+                            sx[e][u] *= f.x;
+                        }
+                        if (ZZ) {
+                            if (AMP) {
+                                cy[e][u] *= f.y;
+                                sy[e][u] *= f.y;
+                            }
+                        } else {
+                            const float ar = AMP ? wr0 * f.y : wr0, ai = AMP ? wi0 * f.y : wi0;
+                            const float co = cy[e][u], si = sy[e][u];
+                            cy[e][u] = cmul_re(ar, ai, co, si);  // W
+                            sy[e][u] = cmul_im(ar, ai, co, si);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < NE; ++e) {
+                    const int k = 2 * pr;
+                    split16x2(cx[e][0], cx[e][1], &ah[e][k], &al[e][k]);
+                    split16x2(sx[e][0], sx[e][1], &ah[e][k + 1], &al[e][k + 1]);
+                    const uint32_t fx = pack16x2(ex[e][0], ex[e][1]);
+                    const uint32_t fy = pack16x2(ey[e][0], ey[e][1]);
+                    ae[e][k] = mul2(ah[e][k], fx);
+                    ae[e][k + 1] = mul2(ah[e][k + 1], fx);
+                    uint32_t(&h)[4] = ZZ ? ah[1] : bh[e];
+                    uint32_t(&l)[4] = ZZ ? al[1] : bl[e];
+                    uint32_t(&o)[4] = ZZ ? ae[1] : be[e];
+                    split16x2(cy[e][0], cy[e][1], &h[k], &l[k]);
+                    split16x2(sy[e][0], sy[e][1], &h[k + 1], &l[k + 1]);
+                    o[k] = mul2(h[k], fy);
+                    o[k + 1] = mul2(h[k + 1], fy);
+                }
+            }
+            auto put = [&](uint32_t tile, uint32_t row, uint32_t a, uint32_t b, uint32_t d,
+                           uint32_t e) {
+                *reinterpret_cast<uint4*>(base + tile * kGA + sw128(row, c)) = make_uint4(a, b, d, e);
+            };
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t row = (uint32_t)(ZZ ? 64 + r + 32 * k : r + 32 * k);
+                put(0, row, ah[k][0], ah[k][1], ah[k][2], ah[k][3]);
+                put(1, row, al[k][0], al[k][1], al[k][2], al[k][3]);
+                put(4, row, ae[k][0], ae[k][1], ae[k][2], ae[k][3]);
+            }
+            if (!ZZ) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    // Point r + 32 k: (Re W, -Im W) in row r + 32 k, (Im W,
+                    // Re W) in row 64 + r + 32 k; and the same of i E W, whose
+                    // real part is -E Im W (be holds E Re W, E Im W).
+                    const uint32_t row = (uint32_t)(r + 32 * k);
+                    const uint32_t(&h)[4] = bh[k], (&l)[4] = bl[k], (&o)[4] = be[k];
+                    put(2, row, h[0], neg2(h[1]), h[2], neg2(h[3]));
+                    put(2, 64 + row, h[1], h[0], h[3], h[2]);
+                    put(3, row, l[0], neg2(l[1]), l[2], neg2(l[3]));
+                    put(3, 64 + row, l[1], l[0], l[3], l[2]);
+                    const uint32_t n1 = neg2(o[1]), n3 = neg2(o[3]);
+                    put(5, row, n1, neg2(o[0]), n3, neg2(o[2]));
+                    put(5, 64 + row, o[0], n1, o[2], n3);
+                }
+            }
+        }
+        // Make the generic-proxy stores visible to the tensor cores, then one
+        // arrival per warp on the even CTA's stage barrier.
+        fence_proxy_async();
+        __syncwarp();
+        if (r == 0) {
+            mbar_arrive_cluster(full_lead + 8u * (uint32_t)s);
+            mbar_arrive(&ray_empty[rb]);
+        }
+    }
+}
+
+// Epilogue role (warps 1..4): adds each finished accumulator segment to this
+// CTA's 128 rows of the split's partial. Lane l of warp w owns row
+// 32 (w % 4) + l: 32 columns at a time go from TMEM to the lane's 128-byte
+// staging row and from there to a bulk copy, a store for the split's first
+// segment and an FP32 add at the memory side (round to nearest) for the others.
+// A segment's operations complete before the next segment's start, so the
+// partial is s0 + s1 + ... in segment order.
+__device__ __forceinline__ void grid_drain(const ProductArgs& g, int warp, int lane, int mt, int nt,
+                                           int sp, int nseg, uint32_t tmem, uint64_t* acc_full,
+                                           uint32_t acc_empty_lead, unsigned char* stage,
+                                           volatile int* flag) {
+    using namespace sm100;
+    const int qd = warp & 3;
+    float* row = g.partial + ((size_t)sp * g.m_pad + (size_t)mt * 128 + qd * 32 + lane) * g.n_pad +
+                 (size_t)nt * kFN;
+    if (nseg == 0) {
+        for (int c = 0; g.first && c < kFN; ++c) row[c] = 0.f;
+        return;
+    }
+    unsigned char* srow = stage + lane * kFEpiRow;
+    const uint32_t s_addr = smem_u32(srow);
+    for (int q = 0; q < nseg; ++q) {
+        const int b = q & 1;
+        const bool ok = mbar_wait(&acc_full[b], (uint32_t)(q >> 1) & 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *flag = 1;
+            break;
+        }
+        tc_fence_after();
+        bulk_wait_all();  // the previous segment's writes to this row are performed
+#pragma unroll 1
+        for (int c = 0; c < kFN / 32; ++c) {
+            float v[32];
+            tmem_ld_32cols(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(b * kFN + c * 32), v);
+            bulk_wait_read();  // the staging row is free again
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                reinterpret_cast<float4*>(srow)[k] =
+                    make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            fence_proxy_async();
+            if (q == 0 && g.first)
+                bulk_s2g(row + c * 32, s_addr, 128);
+            else
+                bulk_add_s2g_f32(row + c * 32, s_addr, 128);
+            bulk_commit();
+        }
+        tc_fence_before();
+        mbar_arrive_cluster(acc_empty_lead + 8u * (uint32_t)b);
+    }
+    bulk_wait_all();
+}
+
+template <bool AMP>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
+    grid_product_kernel(ProductArgs g) {
+    using namespace sm100;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* rays_smem = tiles + kGStages * kGStage;
+    unsigned char* epi_smem = rays_smem + kFRayBufs * kGRayBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(epi_smem + kFEpiBytes);
+    uint64_t* empty = full + kGStages;
+    uint64_t* acc_full = empty + kGStages;
+    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* ray_full = acc_empty + 2;
+    uint64_t* ray_empty = ray_full + kFRayBufs;
+    uint64_t* mma_done = ray_empty + kFRayBufs;  // every issued MMA has completed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
+    volatile int* flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int mt = blockIdx.x, sp = blockIdx.z;
+    const int col = blockIdx.y / g.n_tiles, nt = blockIdx.y - col * g.n_tiles;
+    const uint32_t half = cluster_ctarank(), peer = half ^ 1u;
+    const bool leader = half == 0;
+    const int rb0 = (int)((long long)g.ray_blocks * sp / g.splits);
+    const int rb1 = (int)((long long)g.ray_blocks * (sp + 1) / g.splits);
+    const int nrb = rb1 - rb0;
+    const int nseg = (nrb + g.seg - 1) / g.seg;
+
+    if (threadIdx.x == 0) {
+        // full and acc_empty are used in the even CTA only: they collect the
+        // arrivals of both CTAs' producer and epilogue warps.
+        for (int s = 0; s < kGStages; ++s) {
+            mbar_init(&full[s], 2 * kGProdThreads / 32 + (s == 0 ? g.stall : 0u));
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 2 * kFEpiThreads);
+        }
+        for (int b = 0; b < kFRayBufs; ++b) {
+            mbar_init(&ray_full[b], 1);
+            mbar_init(&ray_empty[b], kGProdThreads / 32);
+        }
+        mbar_init(mma_done, 1);
+        mbar_init_fence();
+        *flag = 0;
+    }
+    if (warp == 0) tmem_alloc_pair(tmem_slot, 2 * kFN);
+    tc_fence_before();
+    cluster_sync();  // both CTAs' barriers initialised, TMEM allocated in both
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (leader && lane == 0) {
+            // Pair MMA issuer: per ray block the three products of the split
+            // phasors and the first-order one, four 256x256x16 steps each;
+            // segment q accumulates into buffer q & 1 of both CTAs' TMEM.
+            constexpr uint32_t idesc = idesc_f16_f32(256, kFN);
+            bool good = true;
+            for (int q = 0; q < nseg && good; ++q) {
+                const int b = q & 1, use = q >> 1;
+                if (use >= 1 &&
+                    !mbar_wait_cluster(&acc_empty[b], (uint32_t)(use - 1) & 1u, g.wait_limit)) {
+                    *flag = 1;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d = tmem + (uint32_t)(b * kFN);
+                const int i0 = q * g.seg, i1 = min(nrb, i0 + g.seg);
+                for (int i = i0; i < i1; ++i) {
+                    const int s = i % kGStages;
+                    if (!mbar_wait_cluster(&full[s], (uint32_t)(i / kGStages) & 1u, g.wait_limit)) {
+                        *flag = 1;
+                        good = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t t0 = smem_u32(tiles + (size_t)s * kGStage);
+                    const uint32_t as[4] = {t0 + 4 * kGA, t0, t0, t0 + kGA};
+                    const uint32_t bs[4] = {t0 + 5 * kGA, t0 + 2 * kGA, t0 + 3 * kGA, t0 + 2 * kGA};
+#pragma unroll
+                    for (int p = 0; p < 4; ++p)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            umma_f16_pair(d, desc_kmajor_sw128(as[p] + 32u * k),
+                                          desc_kmajor_sw128(bs[p] + 32u * k), idesc,
+                                          (uint32_t)((i - i0) | p | k));
+                    umma_commit_pair(smem_u32(&empty[s]));
+                    umma_commit_pair(mapa_shared(&empty[s], peer));
+                }
+                umma_commit_pair(smem_u32(&acc_full[b]));
+                umma_commit_pair(mapa_shared(&acc_full[b], peer));
+            }
+            // A loop that gave up on a wait may leave MMAs in flight: wait
+            // (bounded) for them before either CTA frees its accumulators.
+            umma_commit_pair(smem_u32(mma_done));
+            if (!mbar_wait(mma_done, 0, max(g.wait_limit, kMmaDrainPolls))) *flag = 1;
+        }
+        __syncwarp();
+    } else if (warp <= 4) {
+        grid_drain(g, warp, lane, mt, (int)blockIdx.y, sp, nseg, tmem, acc_full,
+                   mapa_shared(acc_empty, 0), epi_smem + (warp - 1) * 32 * kFEpiRow, flag);
+    } else if (warp < 5 + kGProdThreads / 32) {
+        const int w = warp - 5;
+        const uint32_t full_lead = mapa_shared(full, 0);
+        if (w < 8)
+            grid_producer<false, AMP>(g, w, lane, mt, nt, col, half, nrb, tiles, full_lead, empty,
+                                      ray_full, ray_empty, rays_smem, flag);
+        else
+            grid_producer<true, AMP>(g, 2 * (w - 8), lane, mt, nt, col, half, nrb, tiles, full_lead,
+                                     empty, ray_full, ray_empty, rays_smem, flag);
+    } else if (lane == 0) {
+        // Ray stager: one bulk copy of 32 records per block.
+        const float4* src =
+            g.recs + ((size_t)((mt >> 1) * g.n_tiles + nt) * g.pad + (size_t)rb0 * kFRays) * 4;
+        int i = 0;
+        for (; i < nrb; ++i) {
+            const int rb = i % kFRayBufs;
+            if (i >= kFRayBufs &&
+                !mbar_wait(&ray_empty[rb], (uint32_t)(i / kFRayBufs - 1) & 1u, g.wait_limit)) {
+                *flag = 1;
+                break;
+            }
+            mbar_arrive_expect_tx(&ray_full[rb], kGRayBytes);
+            bulk_g2s(rays_smem + rb * kGRayBytes, src + (size_t)i * kFRays * 4, kGRayBytes,
+                     &ray_full[rb]);
+        }
+        // No copy may still be writing into this CTA's shared memory when it
+        // exits: the last ones land whether or not a producer waits for them.
+        for (int k = max(0, i - kFRayBufs); k < i; ++k)
+            if (!mbar_wait(&ray_full[k % kFRayBufs], (uint32_t)(k / kFRayBufs) & 1u,
+                           max(g.wait_limit, kMmaDrainPolls)))
+                *flag = 1;
+    }
+    __syncthreads();
+    if (*flag != 0 && threadIdx.x == 0) atomicExch(g.err, 1);
+    tc_fence_before();
+    cluster_sync();  // the pair MMAs and all cross-CTA arrivals are done
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_free_pair(tmem, 2 * kFN);
+    }
+}
+
+// Field of every screen point: the splits' sums in split order, times `scale`
+// (i k / (4 pi) over the f16 scaling). One column: (Es, Ep) = (pes, pep) A.
+// Threads run along the columns, which are consecutive in the partials.
+__global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restrict__ partial,
+                                                          int splits, int m_pad, int n_pad,
+                                                          int n_tiles, int columns, size_t nm,
+                                                          size_t nn, bool rows_outer, double scale,
+                                                          double2 pes, double2 pep, FieldDev out) {
+    const size_t idx = blockIdx.x * (size_t)256 + threadIdx.x;
+    if (idx >= nm * nn) return;
+    const size_t im = idx / nn, in = idx - im * nn;
+    const size_t loc = in & 127, at = (in >> 7) * kFN + 128 * (loc >> 6) + (loc & 63);
+    double re[2] = {0.0, 0.0}, ie[2] = {0.0, 0.0};
+    for (int c = 0; c < columns; ++c)
+        for (int s = 0; s < splits; ++s) {
+            const float* row =
+                partial + ((size_t)s * m_pad + im) * n_pad + (size_t)c * n_tiles * kFN + at;
+            re[c] += row[0];
+            ie[c] += row[64];
+        }
+    // times i
+    for (int c = 0; c < 2; ++c) {
+        const double t = re[c];
+        re[c] = -ie[c] * scale;
+        ie[c] = t * scale;
+    }
+    const size_t o = rows_outer ? idx : in * nm + im;
+    if (columns == 1) {
+        out.es_re[o] = pes.x * re[0] - pes.y * ie[0];
+        out.es_im[o] = pes.x * ie[0] + pes.y * re[0];
+        out.ep_re[o] = pep.x * re[0] - pep.y * ie[0];
+        out.ep_im[o] = pep.x * ie[0] + pep.y * re[0];
+    } else {
+        out.es_re[o] = re[0];
+        out.es_im[o] = ie[0];
+        out.ep_re[o] = re[1];
+        out.ep_im[o] = ie[1];
+    }
+}
+
+// ---- host ------------------------------------------------------------------------------
+
+struct Range {
+    double lo, hi;
+};
+Range mul(Range a, Range b) {
+    const double v[4] = {a.lo * b.lo, a.lo * b.hi, a.hi * b.lo, a.hi * b.hi};
+    return {*std::min_element(v, v + 4), *std::max_element(v, v + 4)};
+}
+
+double largest(Range a) { return std::max(std::fabs(a.lo), std::fabs(a.hi)); }
+
+size_t blocks_of(size_t n, size_t size) { return (n + size - 1) / size; }
+
+const double* coord_host(const PixDev& p, int c) { return c == 0 ? p.x : (c == 1 ? p.y : p.z); }
+
+double bits_to_double(unsigned long long b) {
+    double d;
+    std::memcpy(&d, &b, sizeof(d));
+    return d;
+}
+
+}  // namespace
+
+Status grid_probe_enqueue(const PixDev& pix, int m, const double* len_part, int parts, int stride,
+                          GridProbe* probe, cudaStream_t stream) {
+    const int blocks = (int)std::min<size_t>(blocks_of((size_t)m, 1024), 296);
+    grid_probe_kernel<<<blocks, 256, 0, stream>>>(pix, m, len_part, parts, stride, probe);
+    XK_CUDA_TRY(cudaGetLastError());
+    return Status::Ok();
+}
+
+bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, int columns,
+               double tolerance, int num_sms, GridPlan* g) {
+    if (probe.len < 2 || probe.bad || !(r.max_amp > 0.0)) return false;
+    const int inner = probe.inner;
+    const int mask = probe.outer_mask;
+    if (mask != 1 && mask != 2 && mask != 4) return false;
+    const int outer = mask == 1 ? 0 : (mask == 2 ? 1 : 2);
+    const size_t len = (size_t)probe.len, rows = m / len;
+
+    // Ray-to-point ranges: |p - r| between the boxes, components of p - r.
+    Range del[3];
+    double d2lo = 0.0, d2hi = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        del[c] = {r.plo[c] - r.rhi[c], r.phi[c] - r.rlo[c]};
+        const double gap = std::max(0.0, std::max(del[c].lo, -del[c].hi));
+        d2lo += gap * gap;
+        d2hi += largest(del[c]) * largest(del[c]);
+    }
+    const double dlo = std::sqrt(d2lo), dhi = std::sqrt(d2hi);
+    if (!(dlo > 0.0)) return false;
+    const double kt = r.k / (2.0 * 3.14159265358979323846);
+    // Obliquity factor nl + n.(p - r)/|p - r|.
+    Range nd{0.0, 0.0};
+    for (int c = 0; c < 3; ++c) {
+        const Range u = mul(del[c], {1.0 / dhi, 1.0 / dlo});
+        const Range t = mul({r.nlo[c], r.nhi[c]}, {std::max(u.lo, -1.0), std::min(u.hi, 1.0)});
+        nd.lo += t.lo;
+        nd.hi += t.hi;
+    }
+    const Range obl{r.nl_lo + nd.lo, r.nl_hi + nd.hi};
+    if (!(obl.lo > 0.0 || obl.hi < 0.0)) return false;
+    const double omin = std::min(std::fabs(obl.lo), std::fabs(obl.hi)), omax = largest(obl);
+
+    // Rows along the outer or the inner axis, whichever pads less (then
+    // whichever leaves the smaller first-order phase).
+    bool found = false;
+    double best_area = 0.0, best_e = 0.0;
+    for (int swap = 0; swap < 2; ++swap) {
+        const int am = swap ? inner : outer, an = swap ? outer : inner;
+        const size_t nm = swap ? len : rows, nn = swap ? rows : len;
+        const double em = bits_to_double(probe.extent[swap ? 1 : 0][1]);  // 256-point tiles
+        const double en = bits_to_double(probe.extent[swap ? 0 : 1][0]);  // 128-point tiles
+        // |dS| = |u| |(p - r) + (p0 - r)| with |p0 - r| <= |p - r|max - |u|max
+        // when the tile lies inside the screen's range.
+        const double pm = largest(del[am]), pn = largest(del[an]);
+        const double ds = em * (2.0 * pm - em), dt = en * (2.0 * pn - en);
+        const double e = r.k * ds * dt / (4.0 * dlo * dlo * dlo);
+        const double big = std::max(ds, dt);
+        // The first-order factors dS and 4 pi q dT are f16 numbers.
+        if (!(big <= 3e4)) continue;
+        // Second-order part of exp(iE): E^2/2 at the far corner of a tile and
+        // of the ray box; its mean over the pairs is some fifty times smaller.
+        if (!(0.5 * e * e <= 2.0 * tolerance)) continue;
+        if (!(big / (dlo * dlo) <= 1e-2)) continue;
+        // Linear phase: an exact FP32 product up to 2^21 turns.
+        if (!(kt / dlo * std::max(em * pm, en * pn) < 1.9e6)) continue;
+        // FP32 terms: u^2 (h - h0) and the dropped third order of the root.
+        if (!(0.5 * kt * (1.0 / dlo - 1.0 / dhi) * std::max(em * em, en * en) <= 8.0)) continue;
+        if (!(kt * big * big * big / (16.0 * std::pow(dlo, 5)) <= 1e-7)) continue;
+        // Amplitude: first order along each axis, mixed terms dropped.
+        const double sm = largest({r.nlo[am], r.nhi[am]}) * em / (dlo * omin);
+        const double sn = largest({r.nlo[an], r.nhi[an]}) * en / (dlo * omin);
+        const double mq = 0.5 * (1.0 + largest(nd) / omin) * big / (dlo * dlo);
+        if (!(sm <= 0.25 && sn <= 0.25 && sm * sn <= 1e-6 && (sm + sn) * mq <= 1e-6 &&
+              mq * mq <= 1e-7))
+            continue;
+        const size_t mt = blocks_of(nm, kTileM), nt = blocks_of(nn, kTileN);
+        if (mt * nt > kGridMaxTiles) continue;
+        const double area = (double)mt * kTileM * (double)nt * kTileN;
+        if (found && !(area < best_area || (area == best_area && e < best_e))) continue;
+        found = true;
+        best_area = area;
+        best_e = e;
+        g->m_axis = am;
+        g->n_axis = an;
+        g->c_axis = 3 - am - an;
+        g->rows_outer = swap == 0;
+        g->nm = nm;
+        g->nn = nn;
+        g->m_tiles = (int)mt;
+        g->n_tiles = (int)nt;
+        g->e_bound = e;
+        // Below 2^-22 the change of the amplitude along a tile is lost in the
+        // split phasors' own rounding.
+        g->amp = std::max(sm, sn) + mq > 2.384185791015625e-7;
+    }
+    if (!found) return false;
+    // Measured rates: the product 36e12 pairs/s of the padded screen (2^20 rays
+    // x 512^2 points, one column), the general path 1.6e12 pairs/s (1.2e12 with
+    // two columns) after 0.2 ms of sorting tiles and rays that the product does
+    // without (0.34 ms in all against 0.10 on 1024 rays x 40 x 51 points).
+    const double t_product = best_area * columns * (double)n / 36e12;
+    const double t_general = 2e-4 + (double)m * (double)n / (columns == 1 ? 1.6e12 : 1.2e12);
+    if (t_product > t_general) return false;
+    const double d0 = std::sqrt((r.pc[0] - r.rc[0]) * (r.pc[0] - r.rc[0]) +
+                                (r.pc[1] - r.rc[1]) * (r.pc[1] - r.rc[1]) +
+                                (r.pc[2] - r.rc[2]) * (r.pc[2] - r.rc[2]));
+    const long double kt_ld =
+        (long double)r.k / (2.0L * 3.14159265358979323846264338327950288L);
+    g->k = r.k;
+    g->kt = (double)kt_ld;
+    g->kt_lo = (double)(kt_ld - (long double)g->kt);
+    g->h0 = g->kt / (2.0 * d0);
+    g->c0 = r.plo[g->c_axis];
+    g->inner_len = len;
+    g->columns = columns;
+    g->n = n;
+    g->inv_scale = kGridScale / (1.4142135623730951 * r.max_amp * omax / dlo);
+    if (!std::isfinite(g->inv_scale) || !std::isfinite(g->h0)) return false;
+    const size_t tiles = (size_t)g->m_tiles * g->n_tiles;
+    const size_t fit = std::max<size_t>(kGridRecBytes / (tiles * 64) / kFRays, 64) * kFRays;
+    g->chunk_rays = std::min(blocks_of(n, kFRays) * kFRays, fit);
+    g->ray_blocks = (int)blocks_of(n, kFRays);
+    // Ray splits: whole waves of CTA pairs, a split at least ten blocks long.
+    const size_t units = std::max(1, num_sms / 2), work = tiles * columns;
+    const size_t most = std::max<size_t>(1, g->chunk_rays / kFRays / 10);
+    size_t s = work >= units ? 1 : units / work;
+    if (work > units) {
+        double best = 1e300;
+        for (size_t t = 1; t <= 8; ++t) {
+            const double cost = (double)blocks_of(work * t, units) / t + 0.01 * t;
+            if (cost < best) {
+                best = cost;
+                s = t;
+            }
+        }
+    }
+    g->splits = (int)std::max<size_t>(1, std::min(s, most));
+    // The tensor cores truncate when they accumulate: 1.3e-8 of the field per
+    // MMA, 16 per block, 2.0e-6 at ten blocks per segment (7.6 ms on 2^20 rays
+    // x 512^2 points; 7.4 ms and 4.1e-6 at twenty, 8.4 ms and 1.1e-6 at five,
+    // 12.5 ms and 0.7e-6 at three). The persistent kernel's own error comes
+    // from its FP32 residual phases, 5e-6 to 1.6e-5 where those are tens of
+    // radians; where the whole ray set spans fewer it stays below 1e-6, and so
+    // does the product with short segments.
+    const double spread = r.k * r.spread2 / (2.0 * d0);
+    g->seg = spread < kSmallSpread ? 3 : 10;
+    return true;
+}
+
+Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream) {
+    const size_t sm = g.rows_outer ? g.inner_len : 1, sn = g.rows_outer ? 1 : g.inner_len;
+    grid_axes_kernel<<<g.m_tiles + g.n_tiles, kTileM, 0, stream>>>(
+        coord_host(g.pix, g.m_axis), sm, (int)g.nm, g.m_tiles, coord_host(g.pix, g.n_axis), sn,
+        (int)g.nn, g.axes);
+    XK_CUDA_TRY(cudaGetLastError());
+    return Status::Ok();
+}
+
+Status grid_reserve(const GridPlan& g, GridWorkspace& ws) {
+    const size_t tiles = (size_t)g.m_tiles * g.n_tiles;
+    XK_TRY(ws.recs.ensure(tiles * g.chunk_rays * 64));
+    XK_TRY(ws.partial.ensure((size_t)g.splits * g.m_tiles * kTileM * g.n_tiles * g.columns * kFN *
+                             sizeof(float)));
+    return Status::Ok();
+}
+
+Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* d_err, uint32_t wait_limit,
+                    bool stall, cudaStream_t stream, int* kernels) {
+    XK_TRY(grid_reserve(g, ws));
+    const double* rays[12];
+    std::memcpy(rays, &g.rays, sizeof(rays));
+    const double* axes_m = g.axes;
+    ProductArgs p{};
+    p.recs = ws.recs.as<float4>();
+    p.splits = g.splits;
+    p.seg = g.seg;
+    p.m_tiles = g.m_tiles;
+    p.n_tiles = g.n_tiles;
+    p.cm = axes_m;
+    p.cn = axes_m + g.nm;
+    p.refs = axes_m + g.nm + g.nn;
+    p.nm = g.nm;
+    p.nn = g.nn;
+    p.h0 = g.h0;
+    p.partial = ws.partial.as<float>();
+    p.m_pad = g.m_tiles * kTileM;
+    p.n_pad = g.n_tiles * g.columns * kFN;
+    p.err = d_err;
+    p.wait_limit = wait_limit;
+    p.stall = stall ? 1 : 0;
+    const auto kern = g.amp ? grid_product_kernel<true> : grid_product_kernel<false>;
+    // Set on every call: the attribute belongs to the current device's context.
+    XK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem));
+    const dim3 grid((unsigned)(2 * g.m_tiles), (unsigned)(g.n_tiles * g.columns),
+                    (unsigned)g.splits);
+    for (size_t j0 = 0; j0 < g.n; j0 += g.chunk_rays) {
+        const size_t cnt = std::min(g.chunk_rays, g.n - j0), pad = blocks_of(cnt, kFRays) * kFRays;
+        RecordArgs a{};
+        a.ra = rays[g.m_axis] + j0;
+        a.rb = rays[g.n_axis] + j0;
+        a.rc = rays[g.c_axis] + j0;
+        a.na = rays[3 + g.m_axis] + j0;
+        a.nb = rays[3 + g.n_axis] + j0;
+        a.nc = rays[3 + g.c_axis] + j0;
+        a.nl = g.rays.nl + j0;
+        a.w_re = g.amps[0][0] + j0;
+        a.w_im = g.amps[0][1] + j0;
+        if (g.columns == 2) {
+            a.w2_re = g.amps[1][0] + j0;
+            a.w2_im = g.amps[1][1] + j0;
+        }
+        a.refs = p.refs;
+        a.m_tiles = g.m_tiles;
+        a.n_tiles = g.n_tiles;
+        a.n = cnt;
+        a.pad = pad;
+        a.c0 = g.c0;
+        a.h0 = g.h0;
+        a.kt = g.kt;
+        a.kt_lo = g.kt_lo;
+        a.scale = g.inv_scale;
+        grid_records_kernel<<<dim3((unsigned)blocks_of(pad, 256),
+                                   (unsigned)(g.m_tiles * g.n_tiles)), 256, 0, stream>>>(
+            a, ws.recs.as<float4>());
+        XK_CUDA_TRY(cudaGetLastError());
+        p.pad = pad;
+        p.ray_blocks = (int)(pad / kFRays);
+        p.first = j0 == 0;
+        kern<<<grid, kGThreads, kGSmem, stream>>>(p);
+        XK_CUDA_TRY(cudaGetLastError());
+        p.stall = 0;
+        *kernels += 2;
+    }
+    grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
+        p.partial, g.splits, p.m_pad, p.n_pad, g.n_tiles, g.columns, g.nm, g.nn, g.rows_outer,
+        g.k / (4.0 * 3.14159265358979323846) / g.inv_scale, make_double2(g.pes[0], g.pes[1]),
+        make_double2(g.pep[0], g.pep[1]), g.out);
+    XK_CUDA_TRY(cudaGetLastError());
+    *kernels += 1;
+    return Status::Ok();
+}
+
+}  // namespace xk

@@ -1,0 +1,86 @@
+// Phase-reduced Kirchhoff sum on a rectangular screen as a tensor-core
+// product (xk_grid.cu).
+#pragma once
+
+#include "xk_internal.cuh"
+
+namespace xk {
+
+// What the device finds out about the order of a solve's screen points: point
+// i * len + l has one coordinate that depends on l alone (the inner axis), at
+// most one that depends on i alone (the outer axis), the rest constant, bit
+// for bit. extent[axis][k]: largest half-extent of a tile of 128 << k
+// consecutive points of the axis (0 outer, 1 inner), as the bits of a double.
+struct GridProbe {
+    int len;         // inner length; 0 if there is no such order
+    int bad;         // a point breaks the order
+    int inner;       // coordinate index (0 x, 1 y, 2 z) of the inner axis
+    int outer_mask;  // coordinates that vary with i
+    unsigned long long extent[2][2];
+};
+
+// Ranges of a solve's inputs (from the planner's summary).
+struct GridRanges {
+    double rlo[3], rhi[3];  // rays
+    double plo[3], phi[3];  // screen
+    double nlo[3], nhi[3];  // normals
+    double nl_lo, nl_hi;
+    double rc[3], pc[3];    // centroids
+    double spread2;         // mean squared ray distance from the centroid
+    double max_amp;         // largest amplitude component
+    double k;
+};
+
+// Everything the product of one solve needs besides the workspace.
+struct GridPlan {
+    int m_axis = 0, n_axis = 0, c_axis = 0;  // coordinates of the product's rows, columns, the rest
+    bool rows_outer = true;                  // rows are the outer screen axis
+    size_t nm = 0, nn = 0;                   // rows, columns (screen points along the axes)
+    size_t inner_len = 0;
+    int m_tiles = 0, n_tiles = 0, columns = 1;  // 256-row tiles, 128-point tiles, amplitude columns
+    int ray_blocks = 0, splits = 1, seg = 0;
+    size_t n = 0, chunk_rays = 0;            // rays, rays per product launch
+    bool amp = false;                        // amplitude varies along a tile
+    double c0 = 0.0, h0 = 0.0, k = 0.0, kt = 0.0, kt_lo = 0.0;
+    double inv_scale = 0.0, e_bound = 0.0;
+    RaysDev rays{};
+    PixDev pix{};
+    FieldDev out{};
+    const double* amps[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [column][re, im]
+    double pes[2] = {1.0, 0.0}, pep[2] = {0.0, 0.0};  // one column: (Es, Ep) = (pes, pep) A
+    double* axes = nullptr;  // nm + nn coordinates, then m_tiles + n_tiles tile references
+};
+
+struct GridWorkspace {
+    DevBuf recs, partial;
+};
+
+// Below these the general kernel's whole solve is a few tens of microseconds
+// of work; a screen of at most 1024 points fills four of its tiles.
+constexpr size_t kGridMinRays = 1024, kGridMinPoints = 1025;
+
+// Doubles `axes` of a plan for m screen points may need.
+inline size_t grid_axes_doubles(size_t m) { return 2 * (m + 2) + 4; }
+
+// Checks the screen's order; `len_part` holds `parts` candidates for the inner
+// length (stride `stride` doubles, the smallest counts). `probe` is zeroed by
+// an earlier kernel on the stream.
+Status grid_probe_enqueue(const PixDev& pix, int m, const double* len_part, int parts, int stride,
+                          GridProbe* probe, cudaStream_t stream);
+
+// Decides whether the product takes the solve and fills `g` (without device
+// pointers); `columns` amplitude columns; `tolerance` as requested.
+bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, int columns,
+               double tolerance, int num_sms, GridPlan* g);
+
+// Gathers the axes into g.axes.
+Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream);
+
+Status grid_reserve(const GridPlan& g, GridWorkspace& ws);
+
+// Enqueues the product (allocates nothing beyond grid_reserve). `stall`: test
+// hook, the first stage never completes.
+Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* d_err, uint32_t wait_limit,
+                    bool stall, cudaStream_t stream, int* kernels);
+
+}  // namespace xk

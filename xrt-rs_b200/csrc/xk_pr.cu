@@ -48,6 +48,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "xk_dd.cuh"
 #include "xk_pr.cuh"
 #include "xk_sm100.cuh"
 
@@ -55,7 +56,7 @@ namespace xk {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kSumFields = 33;
+constexpr int kSumFields = 40;
 // Stages of FP32 partial sums per fold into the two-float accumulators.
 constexpr int kFoldStages = 1;
 // |e| bound under which the packed sweep's series reciprocal is used.
@@ -81,19 +82,29 @@ constexpr double kF32AmpMax = 1e30, kF32AmpMin = 1e-30;
 // ---------------------------------------------------------------------------
 
 enum : int { OP_SUM = 0, OP_MIN = 1, OP_MAX = 2 };
-__constant__ int c_sum_ops[kSumFields] = {
-    OP_SUM, OP_SUM, OP_SUM,                          // ray position sums
-    OP_MIN, OP_MIN, OP_MIN, OP_MAX, OP_MAX, OP_MAX,  // ray bbox
-    OP_MIN, OP_MAX,                                  // energy range
-    OP_MIN, OP_MIN, OP_MIN, OP_MAX, OP_MAX, OP_MAX,  // normal range
-    OP_SUM, OP_SUM, OP_SUM,                          // screen position sums
-    OP_MIN, OP_MIN, OP_MIN, OP_MAX, OP_MAX, OP_MAX,  // screen bbox
-    OP_SUM,                                          // non-finite probe
-    OP_MAX,                                          // polarization deviation
-    OP_SUM, OP_SUM, OP_SUM, OP_SUM,                  // ray 0's es, ep
-    OP_MAX};                                         // largest amplitude component
-const int h_sum_ops[kSumFields] = {0, 0, 0, 1, 1, 1, 2, 2, 2, 1, 2, 1, 1, 1, 2, 2, 2,
-                                   0, 0, 0, 1, 1, 1, 2, 2, 2, 0, 2, 0, 0, 0, 0, 2};
+// How field i of a solve's summary combines.
+__host__ __device__ constexpr int sum_op(int i) {
+    switch (i) {
+        case 3: case 4: case 5:        // ray bbox
+        case 9:                        // energy range
+        case 11: case 12: case 13:     // normal range
+        case 20: case 21: case 22:     // screen bbox
+        case 33:                       // inner length of a rectangular screen
+        case 34:                       // nl range
+            return OP_MIN;
+        case 6: case 7: case 8:
+        case 10:
+        case 14: case 15: case 16:
+        case 23: case 24: case 25:
+        case 27:                       // polarization deviation
+        case 32:                       // largest amplitude component
+        case 35:
+            return OP_MAX;
+        default:  // 0-2 ray and 17-19 screen position sums, 26 non-finite probe, 28-31
+                  // ray 0's es and ep, 36 squared distances from ray 0, 37-39 its position
+            return OP_SUM;
+    }
+}
 
 __device__ __forceinline__ double op_combine(int op, double a, double b) {
     return op == OP_SUM ? a + b : (op == OP_MIN ? fmin(a, b) : fmax(a, b));
@@ -104,15 +115,26 @@ __device__ __forceinline__ double op_combine(int op, double a, double b) {
 // (fmin / fmax skip NaN, so the boxes alone would not show it). Fields 27-31
 // test whether all rays share ray 0's polarization: the largest relative
 // |es_j ep_0 - ep_j es_0|, and ray 0's (es, ep); field 32 is the largest
-// amplitude component.
+// amplitude component. Field 33 is the first point at which a coordinate that
+// points 0 and 1 share changes: the inner length if the screen is rectangular
+// (infinite if points 0 and 1 differ in none or several coordinates). Clears
+// `probe` for the check of that order.
 __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p, int m,
-                                                     double* __restrict__ block_out) {
+                                                     double* __restrict__ block_out,
+                                                     GridProbe* __restrict__ probe) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *probe = GridProbe{};
     double f[kSumFields];
+#pragma unroll
     for (int i = 0; i < kSumFields; ++i)
-        f[i] = c_sum_ops[i] == OP_SUM ? 0.0 : (c_sum_ops[i] == OP_MIN ? INFINITY : -INFINITY);
+        f[i] = sum_op(i) == OP_SUM ? 0.0 : (sum_op(i) == OP_MIN ? INFINITY : -INFINITY);
     const int stride = gridDim.x * blockDim.x;
     const double a0r = r.es_re[0], a0i = r.es_im[0], b0r = r.ep_re[0], b0i = r.ep_im[0];
     const double a0n = sqrt(a0r * a0r + a0i * a0i), b0n = sqrt(b0r * b0r + b0i * b0i);
+    const double x0 = r.x[0], y0 = r.y[0], z0 = r.z[0];
+    const double q0 = p.x[0], q1 = p.y[0], q2 = p.z[0];
+    const int one = m > 1 ? 1 : 0;
+    const bool in0 = p.x[one] != q0, in1 = p.y[one] != q1, in2 = p.z[one] != q2;
+    const bool ordered = (int)in0 + (int)in1 + (int)in2 == 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         double x = r.x[i], y = r.y[i], z = r.z[i], e = r.energy[i];
         double a = r.nx[i], b = r.ny[i], c = r.nz[i];
@@ -123,7 +145,12 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
         f[11] = fmin(f[11], a); f[12] = fmin(f[12], b); f[13] = fmin(f[13], c);
         f[14] = fmax(f[14], a); f[15] = fmax(f[15], b); f[16] = fmax(f[16], c);
         const double ar = r.es_re[i], ai = r.es_im[i], br = r.ep_re[i], bi = r.ep_im[i];
-        f[26] += (x + y + z + e + a + b + c + r.nl[i] + ar + ai + br + bi) * 0.0;
+        const double nl = r.nl[i];
+        f[34] = fmin(f[34], nl);
+        f[35] = fmax(f[35], nl);
+        const double ux = x - x0, uy = y - y0, uz = z - z0;
+        f[36] += ux * ux + uy * uy + uz * uz;
+        f[26] += (x + y + z + e + a + b + c + nl + ar + ai + br + bi) * 0.0;
         const double dr = (ar * b0r - ai * b0i) - (br * a0r - bi * a0i);
         const double di = (ar * b0i + ai * b0r) - (br * a0i + bi * a0r);
         const double nrm = sqrt(ar * ar + ai * ai) * b0n + sqrt(br * br + bi * bi) * a0n;
@@ -135,6 +162,9 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
             f[29] += ai;
             f[30] += br;
             f[31] += bi;
+            f[37] += x;
+            f[38] += y;
+            f[39] += z;
         }
     }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride) {
@@ -143,19 +173,24 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
         f[20] = fmin(f[20], x); f[21] = fmin(f[21], y); f[22] = fmin(f[22], z);
         f[23] = fmax(f[23], x); f[24] = fmax(f[24], y); f[25] = fmax(f[25], z);
         f[26] += (x + y + z) * 0.0;
+        if (ordered && ((!in0 && x != q0) || (!in1 && y != q1) || (!in2 && z != q2)))
+            f[33] = fmin(f[33], (double)i);
     }
     __shared__ double sm[8][kSumFields];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
     for (int i = 0; i < kSumFields; ++i) {
         double v = f[i];
-        for (int o = 16; o > 0; o >>= 1) v = op_combine(c_sum_ops[i], v, __shfl_xor_sync(kFull, v, o));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = op_combine(sum_op(i), v, __shfl_xor_sync(kFull, v, o));
         if (lane == 0) sm[warp][i] = v;
     }
     __syncthreads();
     if (threadIdx.x < kSumFields) {
         int i = threadIdx.x;
         double v = sm[0][i];
-        for (int w = 1; w < 8; ++w) v = op_combine(c_sum_ops[i], v, sm[w][i]);
+        const int op = sum_op(i);
+        for (int w = 1; w < 8; ++w) v = op_combine(op, v, sm[w][i]);
         block_out[blockIdx.x * kSumFields + i] = v;
     }
 }
@@ -522,37 +557,6 @@ struct PackedState {
     float2 phi[kPrPpl / 2];  // base phase k|q| mod 2 pi
     float2 acc[kPrPpl / 2][4];
 };
-
-// Fractional part of (kt_hi + kt_lo) * |q| in turns, |q| = sqrt(qx^2+qy^2+qz^2),
-// evaluated in double-double arithmetic (error-free products by FMA, TwoSum,
-// one Newton correction of the square root).
-__device__ __forceinline__ double dd_turns(double kt_hi, double kt_lo, double qx, double qy,
-                                           double qz, double* qn, double* inv2q) {
-    const double p0 = qx * qx, p1 = qy * qy, p2 = qz * qz;
-    const double e0 = fma(qx, qx, -p0), e1 = fma(qy, qy, -p1), e2 = fma(qz, qz, -p2);
-    double s1 = p0 + p1;
-    double b1 = s1 - p0;
-    double t1 = (p0 - (s1 - b1)) + (p1 - b1);
-    double s2 = s1 + p2;
-    double b2 = s2 - s1;
-    double t2 = (s1 - (s2 - b2)) + (p2 - b2);
-    double lo = t1 + t2 + e0 + e1 + e2;
-    double hi = s2 + lo;
-    lo -= hi - s2;
-    const double r = sqrt(hi);
-    *qn = r;
-    // 1/(2r): f32 reciprocal seed and one FP64 Newton step (~1e-14 relative);
-    // it scales the square root's low-order correction and is the sweep's
-    // 1/(2|q|).
-    const double d2 = 2.0 * r;
-    const double y0 = (double)__frcp_rn((float)d2);
-    const double y = fma(y0, fma(-d2, y0, 1.0), y0);
-    *inv2q = y;
-    const double rl = (fma(-r, r, hi) + lo) * y;
-    const double ph = kt_hi * r;
-    const double pe = fma(kt_hi, r, -ph) + (kt_hi * rl + kt_lo * r);
-    return (ph - rint(ph)) + pe;
-}
 
 // Per chunk: FP64 geometry of the lane's points, written into the sweep
 // state, and the per-point base phase k|q|: folded into the sweep state
@@ -1160,6 +1164,8 @@ double phase_bound(double k, double a, double b, double d) {
 // Per-solve planning scratch carved from the arena.
 struct SolveBufs {
     double* sum;
+    GridProbe* probe;
+    double* axes;  // of a rectangular screen (xk_grid.cuh)
     uint64_t *pk_in, *pk_out;
     int *pi_in, *pi_out;
     int* tile_perm;
@@ -1178,6 +1184,8 @@ struct SolveBufs {
 void carve(Arena& a, SolveBufs& b, int n, int m, int n_tiles, int groups, int sum_blocks) {
     const size_t slots = (size_t)n_tiles * kPrTile;
     b.sum = a.take<double>((size_t)sum_blocks * kSumFields);
+    b.probe = a.take<GridProbe>(1);
+    b.axes = a.take<double>(grid_axes_doubles((size_t)m));
     b.pk_in = a.take<uint64_t>(m);
     b.pk_out = a.take<uint64_t>(m);
     b.pi_in = a.take<int>(m);
@@ -1208,10 +1216,10 @@ struct HostSolveInfo {
     Frame fr{};
 };
 
-// Pinned host area layout: [per-solve summaries][per-solve amax][per-solve
+// Pinned host area layout: [per-solve summaries][per-solve screen probes][per-solve amax][per-solve
 // n_chunks][error word][solve tables].
 struct HostLayout {
-    size_t sum_off, amax_off, nch_off, err_off, tab_off, total;
+    size_t sum_off, probe_off, amax_off, nch_off, err_off, tab_off, total;
 };
 
 HostLayout host_layout(int count, int sum_blocks) {
@@ -1219,6 +1227,8 @@ HostLayout host_layout(int count, int sum_blocks) {
     size_t off = 0;
     L.sum_off = off;
     off = align_up(off + (size_t)count * sum_blocks * kSumFields * sizeof(double), 256);
+    L.probe_off = off;
+    off = align_up(off + (size_t)count * sizeof(GridProbe), 256);
     L.amax_off = off;
     off = align_up(off + (size_t)count * sizeof(double), 256);
     L.nch_off = off;
@@ -1229,6 +1239,23 @@ HostLayout host_layout(int count, int sum_blocks) {
     off = align_up(off + (size_t)count * sizeof(PrSolve), 256);
     L.total = off;
     return L;
+}
+
+// Whether a solve's screen is looked at for the tensor-core product
+// (xk_grid.cuh): not where the caller set this kernel's own knobs, nor where the
+// requested error is near the product's (up to 6e-6; 165 rad of budget stand
+// for a tolerance of 6e-5).
+bool grid_candidate(const PrOptions& o, size_t n, size_t m) {
+    return o.grid && o.sweep < 0 && o.groups == 0 && effective_phase_budget(o) >= 165.0 &&
+           n >= kGridMinRays && m >= kGridMinPoints;
+}
+
+// Blocks of a solve's summary: at least four elements per thread, because below
+// that the reduction of the fields and the host's pass over the blocks' results
+// cost more than reading the inputs (10^4 rays: 18 us and 95 KB with 296
+// blocks).
+int sum_parts(size_t n, size_t m, int sum_blocks) {
+    return (int)std::min<size_t>(sum_blocks, std::max<size_t>(1, (std::max(n, m) + 1023) / 1024));
 }
 
 int sum_blocks_for(int num_sms) { return std::min(512, std::max(1, 2 * num_sms)); }
@@ -1322,6 +1349,8 @@ void PrWorkspace::release() {
     cub_tmp.release();
     solves.release();
     ctrl.release();
+    grid.recs.release();
+    grid.partial.release();
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);
     ev[0] = ev[1] = nullptr;
@@ -1344,6 +1373,71 @@ size_t pr_plan_bytes(size_t n, size_t m, int num_sms, const PrOptions& opt) {
     // a few bytes per item; 16 per item plus 1 MiB bounds them.
     return a.off + 16 * std::max(n, m) + (1u << 20) + (2u << 20);
 }
+
+namespace {
+
+// Plans the solve as a tensor-core product if its screen and ranges allow.
+Status try_grid(const PrSolveIn& in, const GridProbe& probe, const HostSolveInfo& I,
+                const PrOptions& opt, const SolveBufs& B, int num_sms, cudaStream_t stream,
+                PrPlan* P, int* kernels) {
+    PrOptions o = opt;
+    bool tuned = false;
+    if (opt.tune && opt.tune->use) {
+        PrTuned t;
+        if (opt.tune->find(P->energy_ev, P->dist_mm, in.n, in.m, &t)) {
+            o.phase_budget = std::min(t.phase_budget, opt.phase_budget);
+            o.sweep = t.sweep;
+            tuned = true;
+        }
+    }
+    if (!grid_candidate(o, in.n, in.m)) return Status::Ok();
+    const double* f = I.f;
+    GridRanges r{};
+    double off2 = 0.0;
+    for (int a = 0; a < 3; ++a) {
+        r.rlo[a] = I.rlo[a];
+        r.rhi[a] = I.rhi[a];
+        r.plo[a] = I.plo[a];
+        r.phi[a] = I.phi[a];
+        r.nlo[a] = f[11 + a];
+        r.nhi[a] = f[14 + a];
+        r.rc[a] = I.rc[a];
+        r.pc[a] = I.pc[a];
+        off2 += (I.rc[a] - f[37 + a]) * (I.rc[a] - f[37 + a]);
+    }
+    r.spread2 = std::max(0.0, f[36] / (double)in.n - off2);
+    r.nl_lo = f[34];
+    r.nl_hi = f[35];
+    r.max_amp = f[32];
+    r.k = I.k;
+    GridPlan& g = P->grid_plan;
+    if (!grid_plan(probe, r, in.n, in.m, P->one_pol ? 1 : 2, o.tolerance, num_sms, &g))
+        return Status::Ok();
+    g.rays = in.rays;
+    g.pix = in.pix;
+    g.out = in.out;
+    const double* amps[2][2] = {{in.rays.es_re, in.rays.es_im}, {in.rays.ep_re, in.rays.ep_im}};
+    const int first = P->one_pol && P->dev.amp_src ? 1 : 0;
+    for (int c = 0; c < g.columns; ++c)
+        for (int k = 0; k < 2; ++k) g.amps[c][k] = amps[first + c][k];
+    for (int k = 0; k < 2; ++k) {
+        g.pes[k] = P->pol_es[k];
+        g.pep[k] = P->pol_ep[k];
+    }
+    g.axes = B.axes;
+    XK_TRY(grid_axes_enqueue(g, stream));
+    ++*kernels;
+    P->grid = true;
+    P->tuned = tuned;
+    P->fast = P->lin = P->fold = false;
+    P->n_tiles = g.m_tiles * g.n_tiles;
+    P->groups = g.splits;
+    P->n_chunks = g.ray_blocks;
+    P->phase_bound = 3.14159265358979323846;
+    return Status::Ok();
+}
+
+}  // namespace
 
 Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t stream, int num_sms,
                const PrOptions& opt, std::vector<PrPlan>& plans, int* kernels,
@@ -1390,6 +1484,7 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
     XK_TRY(ws.ensure_host(HL.total));
     char* hbase = static_cast<char*>(ws.host);
     double* h_sum = reinterpret_cast<double*>(hbase + HL.sum_off);
+    GridProbe* h_probe = reinterpret_cast<GridProbe*>(hbase + HL.probe_off);
     double* h_amax = reinterpret_cast<double*>(hbase + HL.amax_off);
     int* h_nch = reinterpret_cast<int*>(hbase + HL.nch_off);
 
@@ -1409,11 +1504,19 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
     for (int s = 0; s < count; ++s) {
         if (plans[s].routed) continue;
         any = true;
-        summary_kernel<<<sum_blocks, 256, 0, stream>>>(in[s].rays, (int)in[s].n, in[s].pix,
-                                                        (int)in[s].m, bufs[s].sum);
+        const int parts = sum_parts(in[s].n, in[s].m, sum_blocks);
+        summary_kernel<<<parts, 256, 0, stream>>>(in[s].rays, (int)in[s].n, in[s].pix,
+                                                        (int)in[s].m, bufs[s].sum, bufs[s].probe);
         XK_CUDA_TRY(cudaGetLastError());
+        if (grid_candidate(opt, in[s].n, in[s].m)) {
+            XK_TRY(grid_probe_enqueue(in[s].pix, (int)in[s].m, bufs[s].sum + 33, parts,
+                                      kSumFields, bufs[s].probe, stream));
+            XK_CUDA_TRY(cudaMemcpyAsync(h_probe + s, bufs[s].probe, sizeof(GridProbe),
+                                        cudaMemcpyDeviceToHost, stream));
+            ++nk;
+        }
         XK_CUDA_TRY(cudaMemcpyAsync(h_sum + (size_t)s * sum_blocks * kSumFields, bufs[s].sum,
-                                    (size_t)sum_blocks * kSumFields * sizeof(double),
+                                    (size_t)parts * kSumFields * sizeof(double),
                                     cudaMemcpyDeviceToHost, stream));
         ++nk;
     }
@@ -1429,11 +1532,12 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         if (P.routed) continue;
         HostSolveInfo& I = info[s];
         const double* hs = h_sum + (size_t)s * sum_blocks * kSumFields;
+        const int parts = sum_parts(in[s].n, in[s].m, sum_blocks);
         for (int i = 0; i < kSumFields; ++i) {
             double v = hs[i];
-            for (int bk = 1; bk < sum_blocks; ++bk) {
+            for (int bk = 1; bk < parts; ++bk) {
                 double w = hs[bk * kSumFields + i];
-                v = h_sum_ops[i] == 0 ? v + w : (h_sum_ops[i] == 1 ? std::min(v, w) : std::max(v, w));
+                v = sum_op(i) == OP_SUM ? v + w : (sum_op(i) == OP_MIN ? std::min(v, w) : std::max(v, w));
             }
             I.f[i] = v;
         }
@@ -1523,13 +1627,14 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             I.fr.e2[i] = e2[i];
             I.fr.u0[i] = u0[i];
         }
+        if (grid_candidate(opt, in[s].n, in[s].m)) XK_TRY(try_grid(in[s], h_probe[s], I, opt, bufs[s], num_sms, stream, &P, &nk));
     }
 
     // --- B. screen tiles ----------------------------------------------------
     any = false;
     for (int s = 0; s < count; ++s) {
         PrPlan& P = plans[s];
-        if (P.routed) continue;
+        if (P.routed || P.grid) continue;
         any = true;
         HostSolveInfo& I = info[s];
         SolveBufs& B = bufs[s];
@@ -1565,7 +1670,7 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
     // --- C. ray chunks ------------------------------------------------------
     for (int s = 0; s < count; ++s) {
         PrPlan& P = plans[s];
-        if (P.routed) continue;
+        if (P.routed || P.grid) continue;
         HostSolveInfo& I = info[s];
         SolveBufs& B = bufs[s];
         const int n = (int)in[s].n;
@@ -1807,7 +1912,7 @@ Status pr_execute_enqueue(std::vector<PrPlan>& plans, PrWorkspace& ws, cudaStrea
         Launch L{tab, 0, 0, variant};
         for (int s = 0; s < count; ++s) {
             PrPlan& P = plans[s];
-            if (P.routed || P.variant() != variant) continue;
+            if (P.routed || P.grid || P.variant() != variant) continue;
             P.dev.item_begin = L.items;
             h_tab[tab++] = P.dev;
             L.items += P.dev.n_items;
@@ -1816,9 +1921,12 @@ Status pr_execute_enqueue(std::vector<PrPlan>& plans, PrWorkspace& ws, cudaStrea
         }
         if (L.count) launches.push_back(L);
     }
-    if (tab == 0) return Status::Ok();
-    XK_CUDA_TRY(cudaMemcpyAsync(ws.solves.ptr, h_tab, (size_t)tab * sizeof(PrSolve),
-                                cudaMemcpyHostToDevice, stream));
+    bool any_grid = false;
+    for (const PrPlan& P : plans) any_grid |= !P.routed && P.grid;
+    if (tab == 0 && !any_grid) return Status::Ok();
+    if (tab)
+        XK_CUDA_TRY(cudaMemcpyAsync(ws.solves.ptr, h_tab, (size_t)tab * sizeof(PrSolve),
+                                    cudaMemcpyHostToDevice, stream));
     if (time_kernels) XK_CUDA_TRY(cudaEventRecord(ws.ev[0], stream));
     int li = 0;
     PrCtl ctl = ws.ctl;
@@ -1831,10 +1939,17 @@ Status pr_execute_enqueue(std::vector<PrPlan>& plans, PrWorkspace& ws, cudaStrea
         R.n_items += L.items;
         ++li;
     }
+    for (const PrPlan& P : plans) {
+        if (P.routed || !P.grid) continue;
+        XK_TRY(grid_enqueue(P.grid_plan, ws.grid, d_err, ctl.wait_limit, ctl.stall_bytes != 0,
+                            stream, &R.kernels));
+        ctl.stall_bytes = 0;
+        R.n_items += (long long)P.n_tiles * P.groups;
+    }
     if (time_kernels) XK_CUDA_TRY(cudaEventRecord(ws.ev[1], stream));
     for (int s = 0; s < count; ++s) {
         PrPlan& P = plans[s];
-        if (P.routed) continue;
+        if (P.routed || P.grid) continue;
         XK_TRY(pr_finalize(P, stream));
         XK_CUDA_TRY(cudaMemcpyAsync(h_nch + s, P.dev.n_chunks_dev, sizeof(int),
                                     cudaMemcpyDeviceToHost, stream));
@@ -1850,9 +1965,9 @@ Status pr_execute_finish(std::vector<PrPlan>& plans, PrWorkspace& ws, PrExecRepo
         if (cudaEventElapsedTime(&ms, ws.ev[0], ws.ev[1]) == cudaSuccess) rep->main_kernel_ms = ms;
     }
     for (auto& P : plans)
-        if (!P.routed && P.n_chunks_host) P.n_chunks = *P.n_chunks_host;
+        if (!P.routed && !P.grid && P.n_chunks_host) P.n_chunks = *P.n_chunks_host;
     if (ws.host_err && *ws.host_err != 0)
-        return Status::Err(XK_ERR_TIMEOUT, "persistent kernel: a bounded wait for a ray stage ran out");
+        return Status::Err(XK_ERR_TIMEOUT, "phase-reduced kernel: a bounded wait for a ray stage ran out");
     return Status::Ok();
 }
 

@@ -5,6 +5,7 @@
 #include <mutex>
 #include <vector>
 
+#include "xk_grid.cuh"
 #include "xk_internal.cuh"
 
 namespace xk {
@@ -52,6 +53,7 @@ struct PrOptions {
                                   // series reciprocal, 2 packed + linear series
     long long items_per_warp = 16;  // target items per resident warp (automatic groups)
     int polarization = -1;        // -1 automatic, 0 always sum Es and Ep separately
+    bool grid = true;             // rectangular screens may run as a tensor-core product
     PrTuneCache* tune = nullptr;  // per-bucket settings that override the above, or null
 };
 
@@ -156,6 +158,8 @@ struct PrPlan {
     int m = 0;
     FieldDev out{};
     int* n_chunks_host = nullptr;    // filled after execution
+    bool grid = false;               // runs as a tensor-core product instead (xk_grid.cuh)
+    GridPlan grid_plan;
 };
 
 struct PrExecReport {
@@ -169,6 +173,7 @@ struct PrWorkspace {
     DevBuf cub_tmp;
     DevBuf solves;  // PrSolve tables for the persistent launches
     DevBuf ctrl;    // item counters + error flag
+    GridWorkspace grid;  // shared by the workspace's products, which run one after another
     cudaEvent_t ev[2] = {nullptr, nullptr};  // bracket the pair kernels
     void* host = nullptr;  // pinned readback / upload area
     size_t host_bytes = 0;
@@ -179,6 +184,7 @@ struct PrWorkspace {
     void release();
     // Stream-ordered allocation for every device buffer of this workspace.
     void set_async(cudaStream_t s) {
+        grid.recs.async_stream = grid.partial.async_stream = s;
         arena.async_stream = cub_tmp.async_stream = solves.async_stream = ctrl.async_stream = s;
     }
 };

@@ -675,6 +675,7 @@ xk::Status create_server(xk_ctx* ctx, const xk_server_opts* opts, xk_server** ou
     if (s->opts.aging_ms <= 0) s->opts.aging_ms = 1000.0;
     s->opts.reserve_sms = std::min(s->opts.reserve_sms, s->num_sms - 1);
     s->pr_opts = ctx->pr_opts;
+    s->pr_opts.grid = false;  // epochs are cut from the persistent kernel's items
     // Keep freed stream-ordered memory in the pool instead of returning it to
     // the driver at every synchronisation.
     XK_TRY(xk::keep_pool_memory(ctx->device));

@@ -182,7 +182,7 @@ __device__ __forceinline__ void tmem_ld_16cols(uint32_t taddr, float* v) {
 // ---- bulk shared-to-global stores and FP64 reduce-adds (one thread each) ----
 // Both addresses 16-byte aligned, size a multiple of 16.
 
-__device__ __forceinline__ void bulk_s2g(double* dst, uint32_t src, uint32_t bytes) {
+__device__ __forceinline__ void bulk_s2g(void* dst, uint32_t src, uint32_t bytes) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src),
                  "r"(bytes)
                  : "memory");
@@ -191,6 +191,14 @@ __device__ __forceinline__ void bulk_s2g(double* dst, uint32_t src, uint32_t byt
 // dst[i] += src[i] in FP64, performed at the memory side.
 __device__ __forceinline__ void bulk_add_s2g_f64(double* dst, uint32_t src, uint32_t bytes) {
     asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(
+                     dst),
+                 "r"(src), "r"(bytes)
+                 : "memory");
+}
+
+// dst[i] += src[i] in FP32 (round to nearest), performed at the memory side.
+__device__ __forceinline__ void bulk_add_s2g_f32(float* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(
                      dst),
                  "r"(src), "r"(bytes)
                  : "memory");
