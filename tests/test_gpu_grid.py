@@ -163,12 +163,22 @@ def test_amplitude_range(grid_ctx, scale):
     assert cases.rel_l2(out, [b * scale for b in base]) < 1e-6
 
 
-@pytest.mark.parametrize("energy,dist,sigma", [(1000.0, 20000.0, 0.1), (1000.0, 8000.0, 0.05),
+@pytest.mark.parametrize("energy,dist,sigma", [(1000.0, 8400.0, 0.1), (1000.0, 4200.0, 0.1),
                                                 (30000.0, 20000.0, 0.2), (30000.0, 4000.0, 0.1)])
 def test_energy_distance_corners(grid_ctx, oracle, energy, dist, sigma):
+    """At 1 keV the residual phases of the whole ray set are 14 and 27 rad."""
     rays = synth.gaussian_aperture(20000, sigma, energy, 3e4, seed=11)
-    check(grid_ctx, oracle, rays, synth.grid_screen(65, 65, 1.0, dist),
-          tol=1e-6 if energy == 1000.0 else TOL)
+    check(grid_ctx, oracle, rays, synth.grid_screen(99, 99, 1.0, dist))
+
+
+@pytest.mark.parametrize("dist,sweep", [(20000.0, 2), (14000.0, 3), (8400.0, 3)])
+def test_small_residual_phases(grid_ctx, oracle, dist, sweep):
+    """Where the general kernel's residual phases are a few radians its error
+    is below 1e-6: the product has to be as good (short segments), or is not
+    taken. 48 truncations of 2^-24 at most, and 3.5e-7 without any."""
+    rays = synth.gaussian_aperture(20000, 0.1, 1000.0, 3e4, seed=11)
+    check(grid_ctx, oracle, rays, synth.grid_screen(99, 99, 1.0, dist), want=sweep,
+          tol=48 * 2.0 ** -24 * 2 / 3 + 3.5e-7)
 
 
 @pytest.mark.parametrize("form", ["rotated", "one_point_off", "swapped_points", "short", "line",

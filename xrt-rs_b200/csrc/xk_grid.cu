@@ -55,7 +55,6 @@ constexpr uint32_t kGRayBytes = kFRays * 64;
 constexpr size_t kGSmem =
     1024 + (size_t)kGStages * kGStage + kFRayBufs * kGRayBytes + kFEpiBytes + 256;
 static_assert(kGSmem <= 227 * 1024, "shared memory");
-constexpr double kSmallSpread = 16.0;    // [rad] mean residual phase of the whole ray set
 constexpr double kGridScale = 1024.0;    // largest |W|: lo parts stay normal f16 numbers
 constexpr size_t kGridRecBytes = (size_t)512 << 20;  // ray records of one launch
 constexpr size_t kGridMaxTiles = 4096;               // at least 2048 rays per launch fit then
@@ -804,15 +803,22 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         }
     }
     g->splits = (int)std::max<size_t>(1, std::min(s, most));
-    // The tensor cores truncate when they accumulate: 1.3e-8 of the field per
-    // MMA, 16 per block, 2.0e-6 at ten blocks per segment (7.6 ms on 2^20 rays
-    // x 512^2 points; 7.4 ms and 4.1e-6 at twenty, 8.4 ms and 1.1e-6 at five,
-    // 12.5 ms and 0.7e-6 at three). The persistent kernel's own error comes
-    // from its FP32 residual phases, 5e-6 to 1.6e-5 where those are tens of
-    // radians; where the whole ray set spans fewer it stays below 1e-6, and so
-    // does the product with short segments.
-    const double spread = r.k * r.spread2 / (2.0 * d0);
-    g->seg = spread < kSmallSpread ? 3 : 10;
+    // Blocks per segment. The tensor cores truncate when they accumulate, 16 MMAs
+    // per block: on top of 3.5e-7 (sine and cosine of both factors) the error
+    // against 64 bits is 4.7e-7, 6.5e-7, 8.3e-7 and 2.4e-6 of the field at 1, 2,
+    // 3 and 10 blocks (32.8, 17.6, 12.5 and 7.6 ms on 2^20 rays x 512^2 points).
+    // The persistent kernel's error grows with its FP32 residual phases, whose
+    // mean over the whole ray set is about
+    //     phase = k (rho^2 + 2 v rho) / (2 d),
+    // rho the rays' spread and v the radius of its 256-point tiles: measured
+    // 3e-7, 5.3e-7, 1.2e-6, 1.6e-6 and 6e-6 at 5, 7, 14, 18 and from 27 rad on.
+    // Below 7 rad the product would be the less exact of the two.
+    const double side = 16.0 * std::sqrt((r.phi[g->m_axis] - r.plo[g->m_axis]) *
+                                         (r.phi[g->n_axis] - r.plo[g->n_axis]) / (double)m);
+    const double phase =
+        r.k * (r.spread2 + 0.6 * side * std::sqrt(r.spread2)) / (2.0 * d0);
+    if (phase < 7.0) return false;
+    g->seg = phase < 12.0 ? 1 : phase < 24.0 ? 3 : 10;
     return true;
 }
 
