@@ -458,35 +458,44 @@ __global__ void __launch_bounds__(1024) group_order_kernel(const int* __restrict
     for (int i = threadIdx.x; i < groups; i += blockDim.x) order[i] = (int)(key[i] & 0xffffffffu);
 }
 
-// Adds the groups' slots of every tile slot in order and scatters the sum to
-// the screen point's original index.
-// One-polarization solves hold A in components 0 and 1; the field is
-// (pes * A, pep * A).
-__global__ void finalize_kernel(const double* __restrict__ partial, const int* __restrict__ tile_perm,
-                                int groups, int slots, FieldDev out, int one_pol, double2 pes,
-                                double2 pep) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= slots) return;
-    int id = tile_perm[s];
-    if (id < 0) return;
-    if (one_pol) {
-        double ar = 0.0, ai = 0.0;
-        for (int g = 0; g < groups; ++g) {
-            const double* b = partial + (size_t)g * 4 * slots;
-            ar += b[s];
-            ai += b[(size_t)slots + s];
-        }
-        out.es_re[id] = pes.x * ar - pes.y * ai;
-        out.es_im[id] = pes.x * ai + pes.y * ar;
-        out.ep_re[id] = pep.x * ar - pep.y * ai;
-        out.ep_im[id] = pep.x * ai + pep.y * ar;
-        return;
-    }
+// Adds the groups' slots of every tile slot and scatters the sum to the screen
+// point's original index: a block takes kFinSlots slots, its kFinLanes rows of
+// threads every kFinLanes-th group each (with one row a line of 256 points and
+// 44 groups took 31 us, one dependent load after the other), and row 0 adds the
+// rows in order. One-polarization solves hold A in components 0 and 1; the
+// field is (pes * A, pep * A).
+constexpr int kFinSlots = 32, kFinLanes = 16;
+
+__global__ void __launch_bounds__(kFinSlots * kFinLanes)
+finalize_kernel(const double* __restrict__ partial, const int* __restrict__ tile_perm, int groups,
+                int slots, FieldDev out, int one_pol, double2 pes, double2 pep) {
+    __shared__ double sm[kFinLanes][4][kFinSlots];
+    const int x = threadIdx.x % kFinSlots, y = threadIdx.x / kFinSlots;
+    const int s = blockIdx.x * kFinSlots + x;  // slots is a multiple of 256
+    const int nc = one_pol ? 2 : 4;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int g = 0; g < groups; ++g) {
+#pragma unroll 4
+    for (int g = y; g < groups; g += kFinLanes) {
         const double* b = partial + (size_t)g * 4 * slots;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[c] += b[(size_t)c * slots + s];
+        for (int c = 0; c < 4; ++c)
+            if (c < nc) acc[c] += b[(size_t)c * slots + s];
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sm[y][c][x] = acc[c];
+    __syncthreads();
+    if (y != 0) return;
+    const int id = tile_perm[s];
+    if (id < 0) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        for (int w = 1; w < kFinLanes; ++w) acc[c] += sm[w][c][x];
+    if (one_pol) {
+        out.es_re[id] = pes.x * acc[0] - pes.y * acc[1];
+        out.es_im[id] = pes.x * acc[1] + pes.y * acc[0];
+        out.ep_re[id] = pep.x * acc[0] - pep.y * acc[1];
+        out.ep_im[id] = pep.x * acc[1] + pep.y * acc[0];
+        return;
     }
     out.es_re[id] = acc[0];
     out.es_im[id] = acc[1];
@@ -925,7 +934,8 @@ __device__ bool process_item(const PrSolve& sv, long long local, WarpPipe& wp,
     // groups * n_tiles consecutive items of a solve).
     const int t = (int)(local % sv.n_tiles);
     const long long rest = local / sv.n_tiles;
-    const int g = sv.group_order[(int)(rest % sv.groups)];
+    const int rank = (int)(rest % sv.groups);
+    const int g = sv.group_order ? sv.group_order[rank] : rank;
     const int sub = (int)(rest / sv.groups);
     const long long n = sv.n_rays;
     const long long g0 = (long long)g * n / sv.groups;
@@ -1262,7 +1272,7 @@ int sum_blocks_for(int num_sms) { return std::min(512, std::max(1, 2 * num_sms))
 
 // Ray groups per tile: enough items to keep every resident warp busy, at
 // least four stages of rays per item, partial slots within 1 GiB.
-int plan_groups(int n, int m, int n_tiles, int num_sms, const PrOptions& opt) {
+int plan_groups_large(int n, int m, int n_tiles, int num_sms, const PrOptions& opt) {
     if (opt.groups > 0) return std::min(opt.groups, kMaxGroups);
     long long ipw = opt.items_per_warp;
     if (opt.tune && opt.tune->use) opt.tune->find_ipw((size_t)n, (size_t)m, &ipw);
@@ -1272,6 +1282,32 @@ int plan_groups(int n, int m, int n_tiles, int num_sms, const PrOptions& opt) {
     long long cap = (1LL << 30) / (32LL * n_tiles * kPrTile);
     g = (int)std::max<long long>(1, std::min<long long>(g, cap));
     return std::min(g, kMaxGroups);
+}
+
+// The same, and where that leaves less than four items per resident warp (a
+// line of 256 points is one tile: 44 items on 1776 warps with 10^4 rays), the
+// count that minimises rounds of items x (rays per item + the item's fixed
+// cost), items as small as kPrMinItem rays.
+int plan_groups(int n, int m, int n_tiles, int num_sms, const PrOptions& opt) {
+    const int base = plan_groups_large(n, m, n_tiles, num_sms, opt);
+    const long long warps = (long long)num_sms * 12;
+    if (opt.groups > 0 || (long long)base * n_tiles >= 4 * warps) return base;
+    constexpr double kItemCost = 60.0;  // set-up, flush and pipeline fill of an item, in rays
+    const long long cap = (1LL << 30) / (32LL * n_tiles * kPrTile);
+    const int most = (int)std::min<long long>(std::min(n / kPrMinItem, kMaxGroups), cap);
+    int best = base;
+    double best_cost = 1e300;
+    for (int waves = 1; waves <= 8; ++waves)
+        for (int g : {(int)std::min<long long>(waves * warps / n_tiles, most), base}) {
+            if (g < 1) continue;
+            const long long rounds = ((long long)g * n_tiles + warps - 1) / warps;
+            const double cost = rounds * ((double)n / g + kItemCost);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = g;
+            }
+        }
+    return best;
 }
 
 }  // namespace
@@ -1654,8 +1690,10 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         pixel_keys_kernel<<<(m + 255) / 256, 256, 0, stream>>>(in[s].pix, m, pf, B.pk_in, B.pi_in);
         XK_CUDA_TRY(cudaGetLastError());
         size_t tmp = ws.cub_tmp.bytes;
+        // A screen without depth has zeros in the keys' low 21 bits.
         XK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws.cub_tmp.ptr, tmp, B.pk_in, B.pk_out, B.pi_in,
-                                                    B.pi_out, m, 0, 53, stream));
+                                                    B.pi_out, m, pf.scale[2] > 0.0 ? 0 : 21, 53,
+                                                    stream));
         XK_CUDA_TRY(cudaMemsetAsync(B.amax, 0, sizeof(unsigned long long), stream));
         tile_kernel<<<(n_tiles[s] * 32 + 255) / 256, 256, 0, stream>>>(
             in[s].pix, m, n_tiles[s], B.pi_out, B.tile_perm, B.tpx, B.tpy, B.tpz, B.tile_center,
@@ -1770,15 +1808,21 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             double cells = 1.0;
             for (int ax = 0; ax < 3; ++ax) cells *= (double)cg.n[ax];
             const double est_chunks = std::min(cells, (double)n);
-            P.fold = est_chunks >= kFoldChunksPerGroup * (double)groups[s] &&
+            const int base = plan_groups_large(n, (int)in[s].m, n_tiles[s], num_sms, opt);
+            P.fold = est_chunks >= kFoldChunksPerGroup * (double)base &&
                      (double)n < kFoldRaysPerChunk * est_chunks;
         }
 
         ray_keys_kernel<<<(n + 255) / 256, 256, 0, stream>>>(in[s].rays, n, cg, B.rk_in, B.ri_in);
         XK_CUDA_TRY(cudaGetLastError());
         size_t tmp = ws.cub_tmp.bytes;
+        // Cell indices: as many key bits as there are cells (a sort pass takes
+        // eight bits and 9 us however few the rays).
+        double cells = 1.0;
+        for (int ax = 0; ax < 3; ++ax) cells *= (double)cg.n[ax];
+        const int key_bits = std::min(63, std::max(1, std::ilogb(cells) + 1));
         XK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws.cub_tmp.ptr, tmp, B.rk_in, B.rk_out, B.ri_in,
-                                                    B.ri_out, n, 0, 63, stream));
+                                                    B.ri_out, n, 0, key_bits, stream));
         head_flags_kernel<<<(n + 255) / 256, 256, 0, stream>>>(B.rk_out, n, B.flags);
         XK_CUDA_TRY(cudaGetLastError());
         tmp = ws.cub_tmp.bytes;
@@ -1790,10 +1834,15 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         records_kernel<<<(n + 255) / 256, 256, 0, stream>>>(in[s].rays, n, B.ri_out, B.run,
                                                              B.chunk_center, B.recs);
         XK_CUDA_TRY(cudaGetLastError());
-        group_order_kernel<<<1, 1024, 0, stream>>>(B.chunk_begin, B.n_chunks, n, groups[s],
-                                                   B.group_order);
-        XK_CUDA_TRY(cudaGetLastError());
-        nk += 6;
+        nk += 5;
+        // Items that all start at once need no order.
+        const bool ordered = (long long)groups[s] * n_tiles[s] > (long long)num_sms * 12;
+        if (ordered) {
+            group_order_kernel<<<1, 1024, 0, stream>>>(B.chunk_begin, B.n_chunks, n, groups[s],
+                                                       B.group_order);
+            XK_CUDA_TRY(cudaGetLastError());
+            ++nk;
+        }
 
         PrSolve& D = P.dev;
         D.recs = B.recs;
@@ -1804,7 +1853,7 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         D.tpy = B.tpy;
         D.tpz = B.tpz;
         D.tile_center = B.tile_center;
-        D.group_order = B.group_order;
+        D.group_order = ordered ? B.group_order : nullptr;
         D.partial = B.partial;
         D.item_begin = 0;
         D.item_offset = 0;
@@ -1863,7 +1912,7 @@ Status pr_launch(const PrSolve* d_table, int n_solves, long long n_items, int va
 
 Status pr_finalize(const PrPlan& P, cudaStream_t stream) {
     const int slots = P.n_tiles * kPrTile;
-    finalize_kernel<<<(slots + 255) / 256, 256, 0, stream>>>(
+    finalize_kernel<<<slots / kFinSlots, kFinSlots * kFinLanes, 0, stream>>>(
         P.dev.partial, P.tile_perm, P.groups, slots, P.out, P.one_pol ? 1 : 0,
         make_double2(P.pol_es[0], P.pol_es[1]), make_double2(P.pol_ep[0], P.pol_ep[1]));
     XK_CUDA_TRY(cudaGetLastError());

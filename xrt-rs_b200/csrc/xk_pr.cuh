@@ -13,6 +13,7 @@ namespace xk {
 // Geometry of the work decomposition.
 constexpr int kPrWarpsPerCta = 4;
 constexpr int kPrStage = 56;          // rays per shared-memory stage
+constexpr int kPrMinItem = 16;        // fewest rays of an automatic item
 constexpr int kPrPpl = 8;             // screen points per lane
 constexpr int kPrTile = 32 * kPrPpl;  // screen points per tile (one warp)
 
@@ -107,7 +108,7 @@ struct PrSolve {
     const int* n_chunks_dev;      // scalar
     const double *tpx, *tpy, *tpz;  // screen points in tile-slot order (padding = tile centre)
     const double* tile_center;    // [3 * n_tiles]
-    const int* group_order;       // [groups] ray groups by decreasing estimated cost
+    const int* group_order;       // [groups] ray groups by decreasing estimated cost, or null
     double* partial;              // [groups][4][n_tiles * kPrTile], tile-slot order
     long long item_begin;         // first global item of this solve in its launch
     long long item_offset;        // first of the solve's own items covered by the launch
