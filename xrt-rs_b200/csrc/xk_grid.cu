@@ -732,7 +732,7 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         // Linear phase: an exact FP32 product up to 2^21 turns.
         if (!(kt / dlo * std::max(em * pm, en * pn) < 1.9e6)) continue;
         // FP32 terms: u^2 (h - h0) and the dropped third order of the root.
-        if (!(0.5 * kt * (1.0 / dlo - 1.0 / dhi) * std::max(em * em, en * en) <= 8.0)) continue;
+        if (!(0.5 * kt * (1.0 / dlo - 1.0 / dhi) * std::max(em * em, en * en) <= 24.0)) continue;
         if (!(kt * big * big * big / (16.0 * std::pow(dlo, 5)) <= 1e-7)) continue;
         // Amplitude: first order along each axis, mixed terms dropped.
         const double sm = largest({r.nlo[am], r.nhi[am]}) * em / (dlo * omin);

@@ -252,8 +252,10 @@ __global__ void pixel_keys_kernel(PixDev p, int m, Frame fr, uint64_t* __restric
 }
 
 // One warp per tile: slot table, slot-ordered coordinates, bounding-box
-// centre, radius.
-__global__ void tile_kernel(PixDev p, int m, int n_tiles, const int* __restrict__ sorted_idx,
+// centre; the largest radius of any tile, its largest extents across and along
+// the frame's long axis u0 (amax_bits[0..2]) and the sum of the tiles' extents
+// across (amax_bits[3], a double).
+__global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, const int* __restrict__ sorted_idx,
                             int* __restrict__ tile_perm, double* __restrict__ tpx,
                             double* __restrict__ tpy, double* __restrict__ tpz,
                             double* __restrict__ tile_center,
@@ -280,7 +282,7 @@ __global__ void tile_kernel(PixDev p, int m, int n_tiles, const int* __restrict_
             hi[a] = fmax(hi[a], __shfl_xor_sync(kFull, hi[a], o));
         }
     double c[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
-    double rad = 0.0;
+    double rad = 0.0, across = 0.0, along = 0.0;
     for (int i = 0; i < kPrPpl; ++i) {
         long long s = (long long)t * kPrTile + lane + 32 * i;
         int id = s < m ? sorted_idx[s] : -1;
@@ -291,17 +293,28 @@ __global__ void tile_kernel(PixDev p, int m, int n_tiles, const int* __restrict_
             z = p.z[id];
             double dx = x - c[0], dy = y - c[1], dz = z - c[2];
             rad = fmax(rad, sqrt(dx * dx + dy * dy + dz * dz));
+            const double f1 = dx * fr.e1[0] + dy * fr.e1[1] + dz * fr.e1[2];
+            const double f2 = dx * fr.e2[0] + dy * fr.e2[1] + dz * fr.e2[2];
+            across = fmax(across, sqrt(f1 * f1 + f2 * f2));
+            along = fmax(along, fabs(dx * fr.u0[0] + dy * fr.u0[1] + dz * fr.u0[2]));
         }
         tpx[s] = x;
         tpy[s] = y;
         tpz[s] = z;
     }
-    for (int o = 16; o > 0; o >>= 1) rad = fmax(rad, __shfl_xor_sync(kFull, rad, o));
+    for (int o = 16; o > 0; o >>= 1) {
+        rad = fmax(rad, __shfl_xor_sync(kFull, rad, o));
+        across = fmax(across, __shfl_xor_sync(kFull, across, o));
+        along = fmax(along, __shfl_xor_sync(kFull, along, o));
+    }
     if (lane == 0) {
         tile_center[3 * t + 0] = c[0];
         tile_center[3 * t + 1] = c[1];
         tile_center[3 * t + 2] = c[2];
         atomicMax(amax_bits, (unsigned long long)__double_as_longlong(rad));
+        atomicMax(amax_bits + 1, (unsigned long long)__double_as_longlong(across));
+        atomicMax(amax_bits + 2, (unsigned long long)__double_as_longlong(along));
+        atomicAdd(reinterpret_cast<double*>(amax_bits + 3), across);
     }
 }
 
@@ -1171,6 +1184,82 @@ double phase_bound(double k, double a, double b, double d) {
     return k * (b * b + 2.0 * a * b) / (2.0 * den);
 }
 
+// Ray cells of their own length along the beam. The bound above takes tiles and
+// cells as balls, but lengths along the line of sight hardly enter the
+// residual phase: with A and B the extents across u (for a tile and a cell that
+// reach a and b along u0, u within the angle g of u0, A = a_across + a g, B =
+// b_across + b g) and v.rho = q_perp.rho_perp + O(|q_perp|^2 / |q|) (u.rho),
+//     |k Delta| <= k (B^2 + 2 A B + 2 A^2 b / d) / (2 (d - 2 (B + b))).
+// On a mirror lit at grazing incidence, 60 mm along the beam and 1 mm across,
+// the ball bound leaves about one ray per cell.
+struct DepthCells {
+    double cell[3];
+    long long n[3];
+    double bound, rcp;
+};
+
+// Residual phase bounds [rad] such cells are sized for. The ball bound kept the
+// true phases of these solves, and so their errors, below what the budget
+// allows; these bounds keep the errors where they were. Deep tiles: 6 rad in the
+// mean tile, 60 in the widest (mirror to mirror, 6e4 rays x 5e4 points: 35.8 ms
+// and 2.9e-7 with the ball bound, 9.7 ms and 3.5e-7 so, 7.4 ms and 4.3e-7 at 10
+// and 100, 6.3 ms and 4.9e-7 at 20 and 100). Flat tiles: a share of the budget.
+constexpr double kDeepTileBudget = 6.0, kDeepWideBudget = 60.0;
+constexpr double kDepthShare = 0.3;
+
+// Fills `c` and returns true where such cells are clearly fewer than the n[]
+// cells of the ball bound. `a_across`, `a_mean`: largest and mean extent of
+// the tiles across u0, `a_along`: largest along it, `a_max`: largest radius.
+bool depth_cells(double k, double d, double g, double a_across, double a_mean, double a_along,
+                 double a_max, const double ext[3], double budget, double tolerance,
+                 const long long n[3], DepthCells* c) {
+    const double wide = a_across + a_along * g, mean = a_mean + a_along * g;
+    const bool deep = a_max > 1.25 * wide;
+    // Along the beam: the linear series' argument (b / d)^2 budget within a
+    // tenth of the tolerance, with a margin.
+    const double b_most = 0.9 * d * std::sqrt(0.1 * tolerance / budget);
+    auto eval = [&](double h) -> double {  // <= 1: fits
+        double sq = 0.0;
+        for (int ax = 0; ax < 2; ++ax) {
+            c->cell[ax] = std::min(ext[ax], h);
+            sq += 0.25 * c->cell[ax] * c->cell[ax];
+        }
+        const double across = std::sqrt(sq);
+        const double along =
+            std::min(0.5 * ext[2], std::min(b_most - across * g, 0.3 * across / std::max(g, 1e-9)));
+        if (!(along >= 0.0)) return INFINITY;
+        c->cell[2] = 2.0 * along;
+        const double b = across + along * g, den = d - 2.0 * (b + along);
+        if (!(den > 0.0)) return INFINITY;
+        auto bound = [&](double a) {
+            return k * (b * b + 2.0 * a * b + 2.0 * a * a * along / d) / (2.0 * den);
+        };
+        c->rcp = (along + across * g) / std::max(d - along - across, 1e-300);
+        c->bound = bound(wide);
+        return deep ? std::max(c->bound / std::min(budget, kDeepWideBudget),
+                               bound(mean) / kDeepTileBudget)
+                    : c->bound / (kDepthShare * budget);
+    };
+    double lo = 0.0, hi = 2.0 * std::max(ext[0], ext[1]);
+    if (!(hi > 0.0)) return false;
+    for (int it = 0; it < 100; ++it) {
+        const double h = 0.5 * (lo + hi);
+        if (eval(h) <= 1.0) lo = h;
+        else hi = h;
+    }
+    if (!(lo > 0.0)) return false;
+    eval(lo);
+    double cells = 1.0, before = 1.0;
+    for (int ax = 0; ax < 3; ++ax) {
+        const double cnt = c->cell[ax] > 0 ? std::floor(ext[ax] / c->cell[ax]) + 1.0 : 1.0;
+        if (!(cnt <= 2097151.0)) return false;
+        c->n[ax] = (long long)cnt;
+        cells *= cnt;
+        before *= (double)n[ax];
+    }
+    return cells < 0.5 * before;
+}
+
 // Per-solve planning scratch carved from the arena.
 struct SolveBufs {
     double* sum;
@@ -1205,7 +1294,7 @@ void carve(Arena& a, SolveBufs& b, int n, int m, int n_tiles, int groups, int su
     b.tpy = a.take<double>(slots);
     b.tpz = a.take<double>(slots);
     b.tile_center = a.take<double>(3 * (size_t)n_tiles);
-    b.amax = a.take<unsigned long long>(1);
+    b.amax = a.take<unsigned long long>(4);
     b.rk_in = a.take<uint64_t>(n);
     b.rk_out = a.take<uint64_t>(n);
     b.ri_in = a.take<int>(n);
@@ -1240,7 +1329,7 @@ HostLayout host_layout(int count, int sum_blocks) {
     L.probe_off = off;
     off = align_up(off + (size_t)count * sizeof(GridProbe), 256);
     L.amax_off = off;
-    off = align_up(off + (size_t)count * sizeof(double), 256);
+    off = align_up(off + 4 * (size_t)count * sizeof(double), 256);
     L.nch_off = off;
     off = align_up(off + (size_t)count * sizeof(int), 256);
     L.err_off = off;
@@ -1687,6 +1776,13 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             pf.lo[ax] = mn;
             pf.scale[ax] = (mx > mn) ? qmax[ax] / (mx - mn) : 0.0;
         }
+        // A screen deeper than it is wide, such as a second mirror seen end-on
+        // (2 mm wide, 1 um high): one scale for both transverse axes, so that
+        // tiles are as wide as they are high. Separate scales made every tile
+        // of that mirror fourteen times wider than it need be.
+        const double deep = qmax[2] / pf.scale[2], wide = qmax[0] / std::min(pf.scale[0], pf.scale[1]);
+        if (pf.scale[0] > 0.0 && pf.scale[1] > 0.0 && pf.scale[2] > 0.0 && deep > wide)
+            pf.scale[0] = pf.scale[1] = std::min(pf.scale[0], pf.scale[1]);
         pixel_keys_kernel<<<(m + 255) / 256, 256, 0, stream>>>(in[s].pix, m, pf, B.pk_in, B.pi_in);
         XK_CUDA_TRY(cudaGetLastError());
         size_t tmp = ws.cub_tmp.bytes;
@@ -1694,13 +1790,13 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         XK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws.cub_tmp.ptr, tmp, B.pk_in, B.pk_out, B.pi_in,
                                                     B.pi_out, m, pf.scale[2] > 0.0 ? 0 : 21, 53,
                                                     stream));
-        XK_CUDA_TRY(cudaMemsetAsync(B.amax, 0, sizeof(unsigned long long), stream));
+        XK_CUDA_TRY(cudaMemsetAsync(B.amax, 0, 4 * sizeof(unsigned long long), stream));
         tile_kernel<<<(n_tiles[s] * 32 + 255) / 256, 256, 0, stream>>>(
-            in[s].pix, m, n_tiles[s], B.pi_out, B.tile_perm, B.tpx, B.tpy, B.tpz, B.tile_center,
+            in[s].pix, m, n_tiles[s], pf, B.pi_out, B.tile_perm, B.tpx, B.tpy, B.tpz, B.tile_center,
             B.amax);
         XK_CUDA_TRY(cudaGetLastError());
-        XK_CUDA_TRY(cudaMemcpyAsync(h_amax + s, B.amax, sizeof(double), cudaMemcpyDeviceToHost,
-                                    stream));
+        XK_CUDA_TRY(cudaMemcpyAsync(h_amax + 4 * s, B.amax, 4 * sizeof(double),
+                                    cudaMemcpyDeviceToHost, stream));
         nk += 2;
     }
     if (any) XK_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1712,7 +1808,7 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         HostSolveInfo& I = info[s];
         SolveBufs& B = bufs[s];
         const int n = (int)in[s].n;
-        const double a_max = h_amax[s] * 1.001;
+        const double a_max = h_amax[4 * s] * 1.001;
         const double k = I.k;
         // Autotuned settings of this solve's bucket, if any.
         PrOptions o = opt;
@@ -1792,6 +1888,27 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         // |e| = |u.rho| / |q| <= b / (d_lo - b): the series reciprocal's
         // argument.
         P.rcp_bound = b_max / std::max(I.d_lo - b_max, 1e-300);
+        {
+            // Largest transverse distance between a ray and a screen point.
+            double side2 = 0.0;
+            for (int ax = 0; ax < 2; ++ax) {
+                double mn, mx;
+                project_box(I.plo, I.phi, I.rc, axes[ax], &mn, &mx);
+                const double gap = std::max(mx - cg.fr.lo[ax], cg.fr.lo[ax] + ext[ax] - mn);
+                side2 += gap * gap;
+            }
+            DepthCells dc;
+            if (depth_cells(k, I.d_lo, std::sqrt(side2) / I.d_lo, h_amax[4 * s + 1] * 1.001,
+                            h_amax[4 * s + 3] / n_tiles[s], h_amax[4 * s + 2] * 1.001, a_max, ext,
+                            budget, o.tolerance, cg.n, &dc)) {
+                for (int ax = 0; ax < 3; ++ax) {
+                    cg.cell[ax] = dc.cell[ax];
+                    cg.n[ax] = dc.n[ax];
+                }
+                P.phase_bound = dc.bound;
+                P.rcp_bound = dc.rcp;
+            }
+        }
         P.fast = o.sweep >= 1 || (o.sweep < 0 && P.rcp_bound <= kSeriesRcpBound);
         // The linear series drops r0 e^2: a relative error of at most e^2 in
         // the reciprocal, |residual phase| e^2 in the phase (a bias shared by
