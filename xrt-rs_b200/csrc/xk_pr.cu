@@ -57,8 +57,6 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kSumFields = 40;
-// Stages of FP32 partial sums per fold into the two-float accumulators.
-constexpr int kFoldStages = 1;
 // |e| bound under which the packed sweep's series reciprocal is used.
 constexpr double kSeriesRcpBound = 2e-3;
 // Fold the base phase when the estimated chunks per ray group reach this.
@@ -255,8 +253,14 @@ __global__ void pixel_keys_kernel(PixDev p, int m, Frame fr, uint64_t* __restric
 // centre; the largest radius of any tile, its largest extents across and along
 // the frame's long axis u0 (amax_bits[0..2]) and the sum of the tiles' extents
 // across (amax_bits[3], a double).
-__global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, const int* __restrict__ sorted_idx,
-                            int* __restrict__ tile_perm, double* __restrict__ tpx,
+// Centres are snapped to multiples of `quantum` as the chunk centres are, so
+// that differences between points, tile and chunk centres are exact. rel, ns:
+// each slot's offset from the centre (PrSolve::tile_rel); n2 = 2 n for solves
+// of one normal.
+__global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, double quantum,
+                            double inv_quantum, double3 n2,
+                            const int* __restrict__ sorted_idx, double4* __restrict__ rel,
+                            float* __restrict__ ns, int* __restrict__ tile_perm, double* __restrict__ tpx,
                             double* __restrict__ tpy, double* __restrict__ tpz,
                             double* __restrict__ tile_center,
                             unsigned long long* __restrict__ amax_bits) {
@@ -281,7 +285,8 @@ __global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, const int* _
             lo[a] = fmin(lo[a], __shfl_xor_sync(kFull, lo[a], o));
             hi[a] = fmax(hi[a], __shfl_xor_sync(kFull, hi[a], o));
         }
-    double c[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
+    double c[3];
+    for (int a = 0; a < 3; ++a) c[a] = rint(0.5 * (lo[a] + hi[a]) * inv_quantum) * quantum;
     double rad = 0.0, across = 0.0, along = 0.0;
     for (int i = 0; i < kPrPpl; ++i) {
         long long s = (long long)t * kPrTile + lane + 32 * i;
@@ -301,6 +306,9 @@ __global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, const int* _
         tpx[s] = x;
         tpy[s] = y;
         tpz[s] = z;
+        const double sx = x - c[0], sy = y - c[1], sz = z - c[2];
+        rel[s] = make_double4(sx, sy, sz, sx * sx + sy * sy + sz * sz);
+        ns[s] = (float)(n2.x * sx + n2.y * sy + n2.z * sz);
     }
     for (int o = 16; o > 0; o >>= 1) {
         rad = fmax(rad, __shfl_xor_sync(kFull, rad, o));
@@ -549,14 +557,27 @@ __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 // Per-warp shared state besides the two ray buffers. NC components per point:
 // 4 (Es, Ep) or 2 (the one-polarization kernels' single column), which is
 // what lets those kernels fit four CTAs per SM.
-template <int NC>
-struct WarpSharedT {
+template <bool FOLD>
+struct ChunkGeometry {        // unfolded: of the current chunk
+    float2 ph[kPrPpl][32];    // (k/2pi) i exp(i k |q|)
+    double ux, uy, uz;        // item direction
+    double r0x, r0y, r0z;     // chunk centre
+};
+// Folded kernels switch chunks every few dozen rays: lane l prepares chunk
+// first + l of the next 32 at once. Q = tile centre - chunk centre, D = |Q|.
+//   dir   u = Q / D
+//   geo   flat tiles: 1 / (2 D), 2 / D, frac(k D / 2 pi); others: chunk centre
+//   geof  flat tiles: 1 / D, 1 / (2 D) or 2 D (SFU sweep) as hi + lo, 2 n.Q, Q
+template <>
+struct ChunkGeometry<true> {
+    double dir[3][32], geo[3][32];
+    float geof[7][32];
+};
+template <int NC, bool FOLD>
+struct WarpSharedT : ChunkGeometry<FOLD> {
     static constexpr int kNC = NC;
     float hi[kPrPpl * NC][32];  // two-float accumulators, [point*NC + component][lane]
     float lo[kPrPpl * NC][32];
-    float2 ph[kPrPpl][32];      // (k/2pi) i exp(i k |q|) of the current chunk (unfolded variants)
-    double ux, uy, uz;          // item direction for the current chunk
-    double r0x, r0y, r0z;       // chunk centre
     uint64_t bar[2];            // mbarriers of the two ray buffers
 };
 
@@ -585,9 +606,8 @@ struct PackedState {
 // (FOLD) or as the chunk phasor (k/2pi) i exp(i k|q|) into shared memory.
 template <bool UNIFORM, bool FAST, bool FOLD, class State, class WS>
 __device__ __forceinline__ void setup_points(const PrSolve& sv, int t, int lane, WS& ws,
-                                             State& st) {
-    const double ux = ws.ux, uy = ws.uy, uz = ws.uz;
-    const double r0x = ws.r0x, r0y = ws.r0y, r0z = ws.r0z;
+                                             State& st, double ux, double uy, double uz,
+                                             double r0x, double r0y, double r0z) {
     const double k = sv.k;
     float* vxp = reinterpret_cast<float*>(st.vx);
     float* vyp = reinterpret_cast<float*>(st.vy);
@@ -627,7 +647,101 @@ __device__ __forceinline__ void setup_points(const PrSolve& sv, int t, int lane,
             const float kt = (float)sv.kt;
             float sp, cp;
             __sincosf(6.28318530717958647692f * fr, &sp, &cp);
-            ws.ph[i][lane] = make_float2(-kt * sp, kt * cp);
+            if constexpr (!FOLD) ws.ph[i][lane] = make_float2(-kt * sp, kt * cp);
+        }
+    }
+}
+
+// Folded kernels: geometry of chunks first .. first + 31 (clamped to the last).
+template <bool UNIFORM, bool FAST, class WS>
+__device__ __forceinline__ void chunk_geometry(const PrSolve& sv, int t, int first, int n_chunks,
+                                               int lane, WS& ws) {
+    const int c = min(first + lane, n_chunks - 1);
+    const double rx = sv.chunk_center[3 * c], ry = sv.chunk_center[3 * c + 1],
+                 rz = sv.chunk_center[3 * c + 2];
+    const double qx = sv.tile_center[3 * t] - rx, qy = sv.tile_center[3 * t + 1] - ry,
+                 qz = sv.tile_center[3 * t + 2] - rz;
+    if (!sv.flat) {
+        const double inv = 1.0 / sqrt(qx * qx + qy * qy + qz * qz);
+        ws.dir[0][lane] = qx * inv;
+        ws.dir[1][lane] = qy * inv;
+        ws.dir[2][lane] = qz * inv;
+        ws.geo[0][lane] = rx;
+        ws.geo[1][lane] = ry;
+        ws.geo[2][lane] = rz;
+        return;
+    }
+    double d, unused;
+    const double turns = dd_turns(sv.kt, sv.kt_lo, qx, qy, qz, &d, &unused);
+    const double inv = 1.0 / d, ux = qx * inv, uy = qy * inv, uz = qz * inv;
+    ws.dir[0][lane] = ux;
+    ws.dir[1][lane] = uy;
+    ws.dir[2][lane] = uz;
+    ws.geo[0][lane] = 0.5 * inv;
+    ws.geo[1][lane] = 2.0 * inv;
+    ws.geo[2][lane] = turns - rint(turns);
+    ws.geof[0][lane] = (float)inv;
+    const double base = FAST ? 0.5 * inv : 2.0 * d;
+    ws.geof[1][lane] = (float)base;
+    ws.geof[2][lane] = (float)(base - (double)(float)base);
+    if (UNIFORM)
+        ws.geof[3][lane] =
+            (float)(2.0 * ((double)sv.unx * qx + (double)sv.uny * qy + (double)sv.unz * qz));
+    ws.geof[4][lane] = (float)qx;
+    ws.geof[5][lane] = (float)qy;
+    ws.geof[6][lane] = (float)qz;
+}
+
+// The set-up of a flat tile's points: |q| expanded about the tile centre.
+// With s = p - tile centre, h = u.s + s^2 / (2D) and e = 2 h / D,
+//     |q| - D = h (1 - e/4 + e^2/8 - 5 e^3/64 + 7 e^4/128 - ...),
+// whose product with k / 2 pi (1e4 turns) needs FP64 but no double-double, and
+// v = s - (|q| - D) u. 14 FP64 operations per point instead of 55.
+template <bool UNIFORM, bool FAST, class State, class WS>
+__device__ __forceinline__ void setup_points_flat(const PrSolve& sv, int t, int lane, const WS& ws,
+                                                  int g, State& st) {
+    float* vxp = reinterpret_cast<float*>(st.vx);
+    float* vyp = reinterpret_cast<float*>(st.vy);
+    float* vzp = reinterpret_cast<float*>(st.vz);
+    float* q2p = reinterpret_cast<float*>(st.q2);
+    float* nqp = reinterpret_cast<float*>(st.nq);
+    float* qxp = reinterpret_cast<float*>(st.qx);
+    float* qyp = reinterpret_cast<float*>(st.qy);
+    float* qzp = reinterpret_cast<float*>(st.qz);
+    float* php = reinterpret_cast<float*>(st.phi);
+    const double ux = ws.dir[0][g], uy = ws.dir[1][g], uz = ws.dir[2][g];
+    const double half_inv = ws.geo[0][g], two_inv = ws.geo[1][g], turn0 = ws.geo[2][g];
+    const float inv = ws.geof[0][g], base = ws.geof[1][g], base_lo = ws.geof[2][g];
+    const double kt = sv.kt, m2k = -2.0 * sv.k;
+    constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
+#pragma unroll
+    for (int i = 0; i < kPrPpl; ++i) {
+        const size_t s = (size_t)t * kPrTile + lane + 32 * i;
+        const double4 r = sv.tile_rel[s];
+        const double h = fma(r.w, half_inv, fma(uz, r.z, fma(uy, r.y, ux * r.x)));
+        const double e = h * two_inv;
+        double p = fma(e, 7.0 / 128.0, -5.0 / 64.0);
+        p = fma(e, p, 0.125);
+        p = fma(e, p, -0.25);
+        const double d = fma(h * e, p, h);
+        const double w = fma(kt, d, turn0);
+        php[i] = 6.28318530717958647692f * (float)(w - ((w + kRound) - kRound));
+        const float df = (float)d;
+        // In FP64: with FP32 offsets the error of the near-field screen rose from
+        // 7.6e-6 to 8.1e-6, and tenfold on tiles that reach along u.
+        vxp[i] = (float)(m2k * fma(-d, ux, r.x));
+        vyp[i] = (float)(m2k * fma(-d, uy, r.y));
+        vzp[i] = (float)(m2k * fma(-d, uz, r.z));
+        const float x = df * inv;
+        // One rounding, as (float)(1 / (2 |q|)) has: an error here is shared by
+        // every pair of the point and the chunk.
+        q2p[i] = base + (FAST ? fmaf(base, x * (x - 1.f), base_lo) : fmaf(2.f, df, base_lo));
+        if (UNIFORM) {
+            nqp[i] = ws.geof[3][g] + sv.tile_ns[s];
+        } else {
+            qxp[i] = ws.geof[4][g] + (float)r.x;
+            qyp[i] = ws.geof[5][g] + (float)r.y;
+            qzp[i] = ws.geof[6][g] + (float)r.z;
         }
     }
 }
@@ -699,10 +813,9 @@ __device__ __forceinline__ void flush_item(const PrSolve& sv, int t, int g, int 
 // one multiply and two FMAs on the sums instead of a complex multiply-add.
 // (In the folded kernels the same form measured 3x the field error and no
 // faster; they keep the Cartesian amplitude.)
-template <bool POL, bool POLAR, class WS>
+template <bool POL, bool POLAR>
 __device__ __forceinline__ void prep_stage(PrRawRay* buf, int len, int lane, const PrSolve& sv,
-                                           const WS& ws) {
-    const double ux = ws.ux, uy = ws.uy, uz = ws.uz;
+                                           double ux, double uy, double uz) {
     for (int j = lane; j < len; j += 32) {
         const PrRawRay r = buf[j];
         double ur = ux * r.rx + uy * r.ry + uz * r.rz;
@@ -739,7 +852,7 @@ __device__ __forceinline__ void prep_stage(PrRawRay* buf, int len, int lane, con
 }
 
 // Adds the lane's FP32 partials into its two-float accumulators and clears
-// them (every kFoldStages stages and at chunk and item ends).
+// them (at most kPrStage rays apart, and at item ends).
 // One-polarization kernels (POL) carry components 0 and 1 only.
 template <bool POL, bool UNIFORM, class WS>
 __device__ __forceinline__ void fold_acc(ScalarState<UNIFORM>& ls, WS& ws, int lane) {
@@ -939,7 +1052,7 @@ __device__ __forceinline__ int chunk_of(const int* __restrict__ begin, int n_chu
 // Processes one (tile, ray-range) item; false if a bounded wait ran out.
 template <bool UNIFORM, bool FAST, bool FOLD, bool POL, bool LIN>
 __device__ bool process_item(const PrSolve& sv, long long local, WarpPipe& wp,
-                             WarpSharedT<POL ? 2 : 4>& ws,
+                             WarpSharedT<POL ? 2 : 4, FOLD>& ws,
                              int lane, uint32_t wait_limit, uint32_t stall_bytes) {
     // local = (sub * groups + g) * n_tiles + t: sub-range `sub` of ray group g
     // against tile t. Sub-items of one (g, t) add into the same slots, so a
@@ -965,8 +1078,9 @@ __device__ bool process_item(const PrSolve& sv, long long local, WarpPipe& wp,
     using State = typename std::conditional<FAST, PackedState<UNIFORM>, ScalarState<UNIFORM>>::type;
     State st;
     clear_acc(st);
-    int since_fold = 0;
+    int since_fold = 0;  // rays summed in FP32 since the last fold
     int cur_chunk = -1;
+    int geo_first = -64;  // FOLD: first of the 32 chunks whose geometry is in `ws`
     int pos = r0;
     int c = chunk_of(cb, n_chunks, pos);
     int len = min(kPrStage, min(cb[c + 1], r1) - pos);
@@ -999,31 +1113,56 @@ __device__ bool process_item(const PrSolve& sv, long long local, WarpPipe& wp,
             return false;
         }
         if (c != cur_chunk) {
-            if (!FOLD && cur_chunk >= 0) flush_chunk<POL>(sv, t, g, lane, ws);
-            __syncwarp();
-            if (lane == 0) {
-                const double p0x = sv.tile_center[3 * t], p0y = sv.tile_center[3 * t + 1],
-                             p0z = sv.tile_center[3 * t + 2];
-                const double r0x = sv.chunk_center[3 * c], r0y = sv.chunk_center[3 * c + 1],
-                             r0z = sv.chunk_center[3 * c + 2];
-                const double dx = p0x - r0x, dy = p0y - r0y, dz = p0z - r0z;
-                const double inv = 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
-                ws.ux = dx * inv;
-                ws.uy = dy * inv;
-                ws.uz = dz * inv;
-                ws.r0x = r0x;
-                ws.r0y = r0y;
-                ws.r0z = r0z;
+            if constexpr (FOLD) {
+                if (c - geo_first >= 32) {
+                    geo_first = c;
+                    __syncwarp();
+                    chunk_geometry<UNIFORM, FAST>(sv, t, c, n_chunks, lane, ws);
+                    __syncwarp();
+                }
+                const int gi = c - geo_first;
+                if (sv.flat)
+                    setup_points_flat<UNIFORM, FAST>(sv, t, lane, ws, gi, st);
+                else
+                    setup_points<UNIFORM, FAST, FOLD>(sv, t, lane, ws, st, ws.dir[0][gi],
+                                                      ws.dir[1][gi], ws.dir[2][gi], ws.geo[0][gi],
+                                                      ws.geo[1][gi], ws.geo[2][gi]);
+            } else {
+                if (cur_chunk >= 0) flush_chunk<POL>(sv, t, g, lane, ws);
+                __syncwarp();
+                if (lane == 0) {
+                    const double p0x = sv.tile_center[3 * t], p0y = sv.tile_center[3 * t + 1],
+                                 p0z = sv.tile_center[3 * t + 2];
+                    const double r0x = sv.chunk_center[3 * c], r0y = sv.chunk_center[3 * c + 1],
+                                 r0z = sv.chunk_center[3 * c + 2];
+                    const double dx = p0x - r0x, dy = p0y - r0y, dz = p0z - r0z;
+                    const double inv = 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
+                    ws.ux = dx * inv;
+                    ws.uy = dy * inv;
+                    ws.uz = dz * inv;
+                    ws.r0x = r0x;
+                    ws.r0y = r0y;
+                    ws.r0z = r0z;
+                }
+                __syncwarp();
+                setup_points<UNIFORM, FAST, FOLD>(sv, t, lane, ws, st, ws.ux, ws.uy, ws.uz, ws.r0x,
+                                                  ws.r0y, ws.r0z);
             }
-            __syncwarp();
-            setup_points<UNIFORM, FAST, FOLD>(sv, t, lane, ws, st);
             cur_chunk = c;
         }
-        prep_stage<POL, POL && !FOLD>(wp.buf[b], len, lane, sv, ws);
+        if constexpr (FOLD) {
+            const int gi = c - geo_first;
+            prep_stage<POL, false>(wp.buf[b], len, lane, sv, ws.dir[0][gi], ws.dir[1][gi],
+                                   ws.dir[2][gi]);
+        } else {
+            prep_stage<POL, POL>(wp.buf[b], len, lane, sv, ws.ux, ws.uy, ws.uz);
+        }
         __syncwarp();
         sweep_stage<UNIFORM, FOLD, POL, LIN>(wp.buf[b], len, lane, st, ws);
-        // FP32 partials run over at most kFoldStages stages of one chunk.
-        if (++since_fold == kFoldStages || nlen == 0 || nc != c) {
+        // FP32 partials run over at most one full stage of rays, of one chunk or
+        // (folded) of several short ones.
+        since_fold += len;
+        if (since_fold + nlen > kPrStage || nlen == 0 || (!FOLD && nc != c)) {
             fold_acc<POL>(st, ws, lane);
             since_fold = 0;
         }
@@ -1037,7 +1176,7 @@ __device__ bool process_item(const PrSolve& sv, long long local, WarpPipe& wp,
         len = nlen;
         b ^= 1;
     }
-    if (FOLD) flush_item<POL>(sv, t, g, lane, ws);
+    if constexpr (FOLD) flush_item<POL>(sv, t, g, lane, ws);
     else flush_chunk<POL>(sv, t, g, lane, ws);
     __syncwarp();
     return true;
@@ -1054,7 +1193,7 @@ pr_persistent_kernel(const PrSolve* __restrict__ solves, int n_solves, long long
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     PrRawRay* bufs = reinterpret_cast<PrRawRay*>(smem) + warp * 2 * kPrStage;
-    using WS = WarpSharedT<POL ? 2 : 4>;
+    using WS = WarpSharedT<POL ? 2 : 4, FOLD>;
     WS* wsh = reinterpret_cast<WS*>(smem + kPrWarpsPerCta * 2 * kPrStage * sizeof(PrRawRay)) + warp;
     WarpPipe wp;
     wp.buf[0] = bufs;
@@ -1092,9 +1231,11 @@ pr_persistent_kernel(const PrSolve* __restrict__ solves, int n_solves, long long
 }
 
 // Dynamic shared memory of a launch: the warps' ray buffers and their state.
-constexpr size_t pr_smem_bytes(bool pol) {
-    return (size_t)kPrWarpsPerCta * 2 * kPrStage * sizeof(PrRawRay) +
-           (size_t)kPrWarpsPerCta * (pol ? sizeof(WarpSharedT<2>) : sizeof(WarpSharedT<4>));
+constexpr size_t pr_smem_bytes(int variant) {
+    const size_t state =
+        (variant & 8) ? ((variant & 4) ? sizeof(WarpSharedT<2, true>) : sizeof(WarpSharedT<2, false>))
+                      : ((variant & 4) ? sizeof(WarpSharedT<4, true>) : sizeof(WarpSharedT<4, false>));
+    return (size_t)kPrWarpsPerCta * (2 * kPrStage * sizeof(PrRawRay) + state);
 }
 
 using PrKernel = void (*)(const PrSolve*, int, long long, unsigned long long*, int*, PrCtl);
@@ -1269,6 +1410,8 @@ struct SolveBufs {
     int *pi_in, *pi_out;
     int* tile_perm;
     double *tpx, *tpy, *tpz, *tile_center;
+    double4* rel;
+    float* ns;
     unsigned long long* amax;
     uint64_t *rk_in, *rk_out;
     int *ri_in, *ri_out, *flags, *run;
@@ -1294,6 +1437,8 @@ void carve(Arena& a, SolveBufs& b, int n, int m, int n_tiles, int groups, int su
     b.tpy = a.take<double>(slots);
     b.tpz = a.take<double>(slots);
     b.tile_center = a.take<double>(3 * (size_t)n_tiles);
+    b.rel = a.take<double4>(slots);
+    b.ns = a.take<float>(slots);
     b.amax = a.take<unsigned long long>(4);
     b.rk_in = a.take<uint64_t>(n);
     b.rk_out = a.take<uint64_t>(n);
@@ -1311,7 +1456,7 @@ void carve(Arena& a, SolveBufs& b, int n, int m, int n_tiles, int groups, int su
 
 struct HostSolveInfo {
     double f[kSumFields];
-    double k = 0, d_lo = 0, rc[3], pc[3], rlo[3], rhi[3], plo[3], phi[3];
+    double k = 0, d_lo = 0, quantum = 0, rc[3], pc[3], rlo[3], rhi[3], plo[3], phi[3];
     Frame fr{};
 };
 
@@ -1728,6 +1873,16 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             I.pc[a] = f[17 + a] / (double)in[s].m;
         }
         I.d_lo = box_distance(I.rlo, I.rhi, I.plo, I.phi);
+        {
+            // 2^E bounds every screen and ray coordinate; multiples of 2^(E-52)
+            // then subtract from any screen coordinate exactly.
+            double amax = 0.0;
+            for (int a = 0; a < 3; ++a)
+                amax = std::max(amax, std::max(std::max(std::fabs(I.plo[a]), std::fabs(I.phi[a])),
+                                               std::max(std::fabs(I.rlo[a]), std::fabs(I.rhi[a]))));
+            const int e = amax > 0 ? std::ilogb(amax) + 2 : -960;
+            I.quantum = std::ldexp(1.0, e - 52);
+        }
         P.energy_ev = f[9];
         P.dist_mm = std::sqrt((I.pc[0] - I.rc[0]) * (I.pc[0] - I.rc[0]) +
                               (I.pc[1] - I.rc[1]) * (I.pc[1] - I.rc[1]) +
@@ -1792,7 +1947,9 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
                                                     stream));
         XK_CUDA_TRY(cudaMemsetAsync(B.amax, 0, 4 * sizeof(unsigned long long), stream));
         tile_kernel<<<(n_tiles[s] * 32 + 255) / 256, 256, 0, stream>>>(
-            in[s].pix, m, n_tiles[s], pf, B.pi_out, B.tile_perm, B.tpx, B.tpy, B.tpz, B.tile_center,
+            in[s].pix, m, n_tiles[s], pf, I.quantum, 1.0 / I.quantum,
+            make_double3(2.0 * I.f[11], 2.0 * I.f[12], 2.0 * I.f[13]), B.pi_out, B.rel, B.ns,
+            B.tile_perm, B.tpx, B.tpy, B.tpz, B.tile_center,
             B.amax);
         XK_CUDA_TRY(cudaGetLastError());
         XK_CUDA_TRY(cudaMemcpyAsync(h_amax + 4 * s, B.amax, 4 * sizeof(double),
@@ -1873,23 +2030,15 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             P.route_reason = 6;
             continue;
         }
-        {
-            // 2^E bounds every screen and ray coordinate; multiples of 2^(E-52)
-            // then subtract from any screen coordinate exactly.
-            double amax = 0.0;
-            for (int a = 0; a < 3; ++a)
-                amax = std::max(amax, std::max(std::max(std::fabs(I.plo[a]), std::fabs(I.phi[a])),
-                                               std::max(std::fabs(I.rlo[a]), std::fabs(I.rhi[a]))));
-            const int e = amax > 0 ? std::ilogb(amax) + 2 : -1000;
-            cg.quantum = std::ldexp(1.0, e - 52);
-            cg.inv_quantum = std::ldexp(1.0, 52 - e);
-        }
+        cg.quantum = I.quantum;
+        cg.inv_quantum = 1.0 / I.quantum;
         P.phase_bound = phase_bound(k, a_max, b_max, I.d_lo);
         // |e| = |u.rho| / |q| <= b / (d_lo - b): the series reciprocal's
         // argument.
         P.rcp_bound = b_max / std::max(I.d_lo - b_max, 1e-300);
+        // Largest angle between a ray-to-point line and u0, and longest line.
+        double tilt = 0.0, d_hi = 0.0;
         {
-            // Largest transverse distance between a ray and a screen point.
             double side2 = 0.0;
             for (int ax = 0; ax < 2; ++ax) {
                 double mn, mx;
@@ -1897,8 +2046,14 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
                 const double gap = std::max(mx - cg.fr.lo[ax], cg.fr.lo[ax] + ext[ax] - mn);
                 side2 += gap * gap;
             }
+            tilt = std::sqrt(side2) / I.d_lo;
+            for (int a = 0; a < 3; ++a) {
+                const double gap = std::max(I.phi[a] - I.rlo[a], I.rhi[a] - I.plo[a]);
+                d_hi += gap * gap;
+            }
+            d_hi = std::sqrt(d_hi);
             DepthCells dc;
-            if (depth_cells(k, I.d_lo, std::sqrt(side2) / I.d_lo, h_amax[4 * s + 1] * 1.001,
+            if (depth_cells(k, I.d_lo, tilt, h_amax[4 * s + 1] * 1.001,
                             h_amax[4 * s + 3] / n_tiles[s], h_amax[4 * s + 2] * 1.001, a_max, ext,
                             budget, o.tolerance, cg.n, &dc)) {
                 for (int ax = 0; ax < 3; ++ax) {
@@ -1970,6 +2125,17 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         D.tpy = B.tpy;
         D.tpz = B.tpz;
         D.tile_center = B.tile_center;
+        D.tile_rel = B.rel;
+        D.tile_ns = B.ns;
+        {
+            // Flat tiles: the first dropped term of the expansion of |q|,
+            // 21/1024 e^6 D, below 1e-8 turn. |e| <= (2 |u.s| + s^2 / D) / D,
+            // u.s at most the tile's extent along u0 plus its extent across
+            // times the angle between u and u0.
+            const double us = h_amax[4 * s + 2] + h_amax[4 * s + 1] * tilt;
+            const double e = (2.0 * us + a_max * a_max / I.d_lo) * 1.01 / I.d_lo;
+            D.flat = k / 6.28 * d_hi * 0.0206 * std::pow(e, 6.0) < 1e-8;
+        }
         D.group_order = ordered ? B.group_order : nullptr;
         D.partial = B.partial;
         D.item_begin = 0;
@@ -2012,7 +2178,7 @@ Status pr_launch(const PrSolve* d_table, int n_solves, long long n_items, int va
                  int max_ctas_per_sm, const PrCtl& ctl) {
     if (n_items <= 0) return Status::Ok();
     PrKernel kern = pr_kernel(variant);
-    const size_t smem = pr_smem_bytes((variant & 8) != 0);
+    const size_t smem = pr_smem_bytes(variant);
     XK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     XK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPrWarpsPerCta * 32,

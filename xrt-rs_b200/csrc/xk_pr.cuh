@@ -107,7 +107,12 @@ struct PrSolve {
     const double* chunk_center;   // [3 * n_chunks]
     const int* n_chunks_dev;      // scalar
     const double *tpx, *tpy, *tpz;  // screen points in tile-slot order (padding = tile centre)
-    const double* tile_center;    // [3 * n_tiles]
+    const double* tile_center;    // [3 * n_tiles], multiples of the chunk centres' quantum
+    // Flat tiles (folded kernels), tile-slot order: s = p - tile centre and
+    // |s|^2; 2 n.s.
+    const double4* tile_rel;
+    const float* tile_ns;
+    int flat;                     // the points' set-up may expand |q| about the tile centre
     const int* group_order;       // [groups] ray groups by decreasing estimated cost, or null
     double* partial;              // [groups][4][n_tiles * kPrTile], tile-slot order
     long long item_begin;         // first global item of this solve in its launch
