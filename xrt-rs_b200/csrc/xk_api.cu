@@ -14,6 +14,61 @@
 
 #include "xk_ctx.cuh"
 
+namespace xk {
+
+namespace {
+
+bool is_pinned(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeUnregistered;
+}
+
+}  // namespace
+
+Status stage_in(xk_ctx* ctx, const double* const* src, int cols, double* dst, size_t n, size_t at,
+                cudaStream_t s) {
+    if (n == 0) return Status::Ok();
+    const size_t bytes = n * sizeof(double), end = at * sizeof(double) + cols * bytes;
+    if (end > kStageBytes || is_pinned(src[0])) {
+        for (int c = 0; c < cols; ++c)
+            XK_CUDA_TRY(cudaMemcpyAsync(dst + c * n, src[c], bytes, cudaMemcpyHostToDevice, s));
+        return Status::Ok();
+    }
+    XK_TRY(ctx->stage_up.ensure(kStageBytes));
+    double* p = ctx->stage_up.as<double>() + at;
+    for (int c = 0; c < cols; ++c) std::memcpy(p + c * n, src[c], bytes);
+    XK_CUDA_TRY(cudaMemcpyAsync(dst, p, cols * bytes, cudaMemcpyHostToDevice, s));
+    return Status::Ok();
+}
+
+Status stage_out(xk_ctx* ctx, double* const* dst, int cols, const double* src, size_t n, size_t at,
+                 cudaStream_t s) {
+    if (n == 0) return Status::Ok();
+    const size_t bytes = n * sizeof(double), end = at * sizeof(double) + cols * bytes;
+    if (end > kStageBytes || is_pinned(dst[0])) {
+        for (int c = 0; c < cols; ++c)
+            XK_CUDA_TRY(cudaMemcpyAsync(dst[c], src + c * n, bytes, cudaMemcpyDeviceToHost, s));
+        return Status::Ok();
+    }
+    XK_TRY(ctx->stage_down.ensure(kStageBytes));
+    XK_CUDA_TRY(cudaMemcpyAsync(ctx->stage_down.as<double>() + at, src, cols * bytes,
+                                cudaMemcpyDeviceToHost, s));
+    for (int c = 0; c < cols; ++c) ctx->pending.push_back({dst[c], at + c * n, n});
+    return Status::Ok();
+}
+
+void unstage(xk_ctx* ctx) {
+    for (const xk_ctx::Pending& p : ctx->pending)
+        std::memcpy(p.dst, ctx->stage_down.as<double>() + p.at, p.n * sizeof(double));
+    ctx->pending.clear();
+}
+
+}  // namespace xk
+
 namespace {
 
 const char* kVersion = "xk 0.1.0 (sm_100a)";
@@ -70,6 +125,11 @@ void destroy_ctx(xk_ctx* ctx) {
     ctx->fresnel.coords.release();
     ctx->fresnel.partial.release();
     ctx->fresnel.ctrl.release();
+    ctx->fresnel.host.release();
+    for (auto& e : ctx->fresnel.ev)
+        if (e) cudaEventDestroy(e);
+    ctx->stage_up.release();
+    ctx->stage_down.release();
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -156,6 +216,7 @@ xk::Status finish_stats(xk_ctx* ctx, xk_stats* stats, int used_path, size_t n_ra
 xk::Status solve_host(xk_ctx* ctx, const xk_rays* rays, size_t n_rays, const xk_pixels* pixels,
                       size_t n_pix, xk_field* out, int path, xk_stats* stats) {
     cudaStream_t s = ctx->stream;
+    ctx->pending.clear();  // of a call that failed
     const size_t nb = n_rays * sizeof(double), mb = n_pix * sizeof(double);
     XK_TRY(ctx->in_rays.ensure(12 * nb > 0 ? 12 * nb : 8));
     XK_TRY(ctx->in_pix.ensure(3 * mb));
@@ -164,12 +225,10 @@ xk::Status solve_host(xk_ctx* ctx, const xk_rays* rays, size_t n_rays, const xk_
     const double* hsrc[12] = {rays->x, rays->y, rays->z, rays->nx, rays->ny, rays->nz,
                               rays->nl, rays->es_re, rays->es_im, rays->ep_re, rays->ep_im,
                               rays->energy};
-    for (int i = 0; i < 12 && n_rays; ++i)
-        XK_CUDA_TRY(cudaMemcpyAsync(dr + i * n_rays, hsrc[i], nb, cudaMemcpyHostToDevice, s));
+    XK_TRY(xk::stage_in(ctx, hsrc, 12, dr, n_rays, 0, s));
     double* dp = ctx->in_pix.as<double>();
-    XK_CUDA_TRY(cudaMemcpyAsync(dp, pixels->x, mb, cudaMemcpyHostToDevice, s));
-    XK_CUDA_TRY(cudaMemcpyAsync(dp + n_pix, pixels->y, mb, cudaMemcpyHostToDevice, s));
-    XK_CUDA_TRY(cudaMemcpyAsync(dp + 2 * n_pix, pixels->z, mb, cudaMemcpyHostToDevice, s));
+    const double* psrc[3] = {pixels->x, pixels->y, pixels->z};
+    XK_TRY(xk::stage_in(ctx, psrc, 3, dp, n_pix, 12 * n_rays, s));
     xk::RaysDev rd;
     const double** f = reinterpret_cast<const double**>(&rd);
     for (int i = 0; i < 12; ++i) f[i] = dr + i * n_rays;
@@ -179,9 +238,9 @@ xk::Status solve_host(xk_ctx* ctx, const xk_rays* rays, size_t n_rays, const xk_
     int used = path;
     XK_TRY(run_solve(ctx, rd, n_rays, pd, n_pix, fd, path, s, stats, &used));
     double* hdst[4] = {out->es_re, out->es_im, out->ep_re, out->ep_im};
-    for (int i = 0; i < 4; ++i)
-        XK_CUDA_TRY(cudaMemcpyAsync(hdst[i], dout + i * n_pix, mb, cudaMemcpyDeviceToHost, s));
+    XK_TRY(xk::stage_out(ctx, hdst, 4, dout, n_pix, 0, s));
     XK_CUDA_TRY(cudaStreamSynchronize(s));
+    xk::unstage(ctx);
     if (stats) {
         stats->h2d_bytes = 12.0 * nb + 3.0 * mb;
         stats->d2h_bytes = 4.0 * mb;
@@ -215,8 +274,9 @@ xk::WaveGrid to_grid(const xk_wave_params* p) {
 xk::Status upload_beam(xk_ctx* ctx, const xk_beam* beam, size_t n_beam, const double* normals,
                        const size_t* good, size_t n_good, cudaStream_t s, xk::BeamDev* bd,
                        const uint64_t** d_good, double* h2d) {
-    for (size_t i = 0; i < n_good; ++i)
-        if (good[i] >= n_beam) return xk::Status::Err(XK_ERR_INVALID, "good index out of range");
+    bool outside = false;  // no early exit: the loop vectorises
+    for (size_t i = 0; i < n_good; ++i) outside |= good[i] >= n_beam;
+    if (outside) return xk::Status::Err(XK_ERR_INVALID, "good index out of range");
     const bool amps = beam->es_re != nullptr;
     const int cols = amps ? 11 : 7;
     const size_t nb = n_beam * sizeof(double);
@@ -502,6 +562,7 @@ int xk_kirchhoff_gpu(xk_ctx* ctx, const xk_gpu_ray* rays, size_t n_rays,
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
+    ctx->pending.clear();
     // The f32 records go to the device as they are (48 + 16 bytes each) and
     // are widened to f64 SoA there (exact, as the reference's host side
     // promotes them for the base-phase restore, kirchhoff.rs:96-104); the
@@ -536,9 +597,9 @@ int xk_kirchhoff_gpu(xk_ctx* ctx, const xk_gpu_ray* rays, size_t n_rays,
     int used = XK_PATH_F32PR;
     if (st.ok()) st = run_solve(ctx, rd, n_rays, pd, n_pix, fd, XK_PATH_F32PR, s, nullptr, &used);
     if (st.ok()) st = xk::interleave_field_enqueue(fd, n_pix, d_out, s);
-    if (st.ok()) st = xk::Status::FromCuda(cudaMemcpyAsync(out, d_out, 4 * n_pix * sizeof(double),
-                                                           cudaMemcpyDeviceToHost, s));
+    if (st.ok()) st = xk::stage_out(ctx, &out, 1, d_out, 4 * n_pix, 0, s);
     if (st.ok()) st = xk::Status::FromCuda(cudaStreamSynchronize(s));
+    if (st.ok()) xk::unstage(ctx);
     return st.ok() ? XK_OK : fail(ctx, st);
 }
 
@@ -632,6 +693,7 @@ int xk_diffraction_beam(xk_ctx* ctx, const xk_beam* beam, size_t n_beam, const d
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
+    ctx->pending.clear();
     xk::BeamDev bd;
     const uint64_t* d_good = nullptr;
     double h2d = 0.0;
@@ -652,12 +714,10 @@ int xk_diffraction_beam(xk_ctx* ctx, const xk_beam* beam, size_t n_beam, const d
     int used = path;
     if (st.ok()) st = run_solve(ctx, rd, n_good, pd, m, fd, path, s, stats, &used);
     double* hdst[4] = {out->es_re, out->es_im, out->ep_re, out->ep_im};
-    for (int i = 0; i < 4 && st.ok(); ++i)
-        if (cudaMemcpyAsync(hdst[i], dout + i * m, m * sizeof(double), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess)
-            st = xk::Status::Err(XK_ERR_CUDA, "device-to-host copy failed");
+    if (st.ok()) st = xk::stage_out(ctx, hdst, 4, dout, m, 0, s);
     if (st.ok() && cudaStreamSynchronize(s) != cudaSuccess)
         st = xk::Status::Err(XK_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+    if (st.ok()) xk::unstage(ctx);
     if (st.ok()) st = finish_stats(ctx, stats, used, n_good, m);
     if (!st.ok()) return fail(ctx, st);
     if (stats) {

@@ -204,6 +204,7 @@ xk::Status run_batch(xk_batch* b, xk_batch_stats* stats) {
     auto t0 = std::chrono::steady_clock::now();
     XK_CUDA_TRY(cudaEventRecord(b->ev0, b->stream));
     if (b->exec) {
+        if (b->ws.host_err) *b->ws.host_err = 0;  // written by the replayed kernels
         XK_CUDA_TRY(cudaGraphLaunch(b->exec, b->stream));
     } else {
         XK_TRY(enqueue_batch(b));

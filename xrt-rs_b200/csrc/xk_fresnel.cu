@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kFThreads, 1) fresnel_fused_kernel(FusedArgs g
         stage_rays_role(g, lane, rb0, nrb, rays_smem, ray_full, ray_empty, flag);
     }
     __syncthreads();
-    if (*flag != 0 && threadIdx.x == 0) atomicExch(g.err, 1);
+    if (*flag != 0 && threadIdx.x == 0) *static_cast<volatile int*>(g.err) = 1;
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -718,7 +718,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
         stage_rays_role(g, lane, rb0, nrb, rays_smem, ray_full, ray_empty, flag);
     }
     __syncthreads();
-    if (*flag != 0 && threadIdx.x == 0) atomicExch(g.err, 1);
+    if (*flag != 0 && threadIdx.x == 0) *static_cast<volatile int*>(g.err) = 1;
     tc_fence_before();
     cluster_sync();  // the pair MMAs and all cross-CTA arrivals are done
     if (warp == 0) {
@@ -733,14 +733,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
 // |es_im| (the f16 scaling), max |x - ox| and |z - oz| (the cross-term bound),
 // and whether every value is finite. The maxima of non-negative doubles are
 // taken on their bit patterns, which order like the values; fmax skips NaN,
-// which the finiteness flag reports instead.
+// which the finiteness flag reports instead. The last block writes the three
+// maxima and the flag to pinned host memory.
 __global__ void __launch_bounds__(256) ray_bounds_kernel(const double* __restrict__ rx,
                                                          const double* __restrict__ rz,
                                                          const double* __restrict__ er,
                                                          const double* __restrict__ ei, size_t n,
                                                          double ox, double oz,
                                                          unsigned long long* __restrict__ max_bits,
-                                                         int* __restrict__ nonfinite) {
+                                                         int* __restrict__ nonfinite,
+                                                         unsigned* __restrict__ ticket,
+                                                         unsigned long long* __restrict__ host_out) {
     double m[3] = {0.0, 0.0, 0.0};
     bool bad = false;
     for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < n;
@@ -766,6 +769,9 @@ __global__ void __launch_bounds__(256) ray_bounds_kernel(const double* __restric
         for (int w = 1; w < 8; ++w) v = fmax(v, sm[w][threadIdx.x]);
         atomicMax(max_bits + threadIdx.x, (unsigned long long)__double_as_longlong(v));
     }
+    if (!last_block(ticket)) return;
+    if (threadIdx.x < 3) host_out[threadIdx.x] = __ldcg(max_bits + threadIdx.x);
+    if (threadIdx.x == 3) host_out[3] = (unsigned long long)__ldcg(nonfinite);
 }
 
 // `group`: x points per real / imaginary column group of a 128-point block
@@ -797,6 +803,9 @@ __global__ void reduce_kernel(const double* __restrict__ partial, int splits, in
 // ---- host --------------------------------------------------------------------
 
 size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// Words of FresnelWorkspace::host: ray bounds (4 x 8 bytes), then the error word.
+constexpr int kFresnelErrWord = 16;
 
 unsigned grid_1d(size_t n, unsigned threads) { return (unsigned)((n + threads - 1) / threads); }
 
@@ -854,7 +863,6 @@ Status fresnel_enqueue(const FresnelIn& in, FresnelWorkspace& ws, cudaStream_t s
     }
     const FresnelShape sh = fresnel_shape(n, nx, nz, num_sms, ws.allow_pair);
     XK_TRY(ws.partial.ensure((size_t)sh.splits * sh.m_pad * sh.n_pad * sizeof(double)));
-    XK_TRY(ws.ctrl.ensure(256));
     // Set on every call: the attribute belongs to the current device's
     // context, and a process may use several devices.
     if (sh.pair)
@@ -863,8 +871,8 @@ Status fresnel_enqueue(const FresnelIn& in, FresnelWorkspace& ws, cudaStream_t s
     else
         XK_CUDA_TRY(cudaFuncSetAttribute(fresnel_fused_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmem));
-    int* d_err = ws.ctrl.as<int>();
-    XK_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
+    int* err = ws.host.as<int>() + kFresnelErrWord;
+    *err = 0;
     FusedArgs fa;
     fa.rx = in.rx;
     fa.rz = in.rz;
@@ -884,7 +892,7 @@ Status fresnel_enqueue(const FresnelIn& in, FresnelWorkspace& ws, cudaStream_t s
     fa.partial = ws.partial.as<double>();
     fa.m_pad = (int)sh.m_pad;
     fa.n_pad = (int)sh.n_pad;
-    fa.err = d_err;
+    fa.err = err;
     fa.wait_limit = ws.wait_limit;
     fa.stall = ws.stall_once;
     ws.stall_once = 0;  // armed for one execution
@@ -903,14 +911,8 @@ Status fresnel_enqueue(const FresnelIn& in, FresnelWorkspace& ws, cudaStream_t s
                                                         in.max_amp, in.out_re, in.out_im, 1);
     XK_CUDA_TRY(cudaGetLastError());
     rep->kernels += 2;
-    if (timed) {
-        XK_CUDA_TRY(cudaEventSynchronize(rep->ev_gemm[1]));
-        float ms = 0.f;
-        XK_CUDA_TRY(cudaEventElapsedTime(&ms, rep->ev_gemm[0], rep->ev_gemm[1]));
-        rep->gemm_ms += ms;
-    }
     rep->shape = sh;
-    rep->d_err = d_err;
+    rep->err = err;
     return Status::Ok();
 }
 
@@ -930,47 +932,44 @@ xk::Status fresnel_host(xk_ctx* ctx, const double* rx, const double* rz, const d
                         const xk_fresnel_screen* sc, double* amp_re, double* amp_im,
                         double* x_pixels, double* z_pixels, int path, xk_stats* stats) {
     cudaStream_t s = ctx->stream;
+    ctx->pending.clear();
     xk::FresnelWorkspace& ws = ctx->fresnel;
     const size_t nx = sc->nx, nz = sc->nz, m = nx * nz;
     const size_t nb = n * sizeof(double);
     XK_TRY(ctx->in_rays.ensure(std::max<size_t>(4 * nb, 8)));
     XK_TRY(ws.coords.ensure((std::max<size_t>(nx, 1) + std::max<size_t>(nz, 1)) * sizeof(double)));
     XK_TRY(ctx->out_field.ensure(std::max<size_t>(2 * m * sizeof(double), 8)));
+    XK_TRY(ws.host.ensure(256));
     double* d = ctx->in_rays.as<double>();
     const double* src[4] = {rx, rz, er, ei};
-    for (int f = 0; f < 4 && n; ++f)
-        XK_CUDA_TRY(cudaMemcpyAsync(d + f * n, src[f], nb, cudaMemcpyHostToDevice, s));
+    XK_TRY(xk::stage_in(ctx, src, 4, d, n, 0, s));
     double max_amp = 0.0, max_rx = 0.0, max_rz = 0.0;
     const double ox = 0.5 * (sc->x_min + sc->x_max), oz = 0.5 * (sc->z_min + sc->z_max);
     bool finite = true;
     int bounds_kernels = 0;
     if (n) {
         // The bounds come from the uploaded columns on the device (a host
-        // loop over 2^20 rays takes milliseconds); one small read-back.
+        // loop over 2^20 rays takes milliseconds), which writes them here.
         XK_TRY(ws.ctrl.ensure(256));
-        unsigned long long* d_max = reinterpret_cast<unsigned long long*>(ws.ctrl.as<char>() + 64);
+        unsigned long long* d_max = ws.ctrl.as<unsigned long long>();
         int* d_bad = reinterpret_cast<int*>(d_max + 3);
-        XK_CUDA_TRY(cudaMemsetAsync(d_max, 0, 3 * sizeof(unsigned long long) + sizeof(int), s));
+        unsigned* ticket = reinterpret_cast<unsigned*>(d_max + 4);
+        XK_CUDA_TRY(cudaMemsetAsync(d_max, 0, 5 * sizeof(unsigned long long), s));
         const unsigned blocks =
             (unsigned)std::min<size_t>((n + 255) / 256, (size_t)std::max(ctx->num_sms, 1) * 4);
+        unsigned long long* h = ws.host.as<unsigned long long>();
         xk::ray_bounds_kernel<<<blocks, 256, 0, s>>>(d, d + n, d + 2 * n, d + 3 * n, n, ox, oz,
-                                                     d_max, d_bad);
+                                                     d_max, d_bad, ticket, h);
         XK_CUDA_TRY(cudaGetLastError());
         bounds_kernels = 1;
-        struct {
-            unsigned long long m[3];
-            int bad;
-        } h{};
-        XK_CUDA_TRY(cudaMemcpyAsync(&h, d_max, sizeof(h.m) + sizeof(int),
-                                    cudaMemcpyDeviceToHost, s));
         XK_CUDA_TRY(cudaStreamSynchronize(s));
         double v[3];
-        std::memcpy(v, h.m, sizeof(v));
+        std::memcpy(v, h, sizeof(v));
         // An upper bound of |es_j| is all the f16 scaling needs.
         max_amp = v[0];
         max_rx = v[1];
         max_rz = v[2];
-        finite = h.bad == 0;
+        finite = h[3] == 0;
     }
     max_amp *= 1.4142135623730951;
     double* out = ctx->out_field.as<double>();
@@ -978,40 +977,32 @@ xk::Status fresnel_host(xk_ctx* ctx, const double* rx, const double* rz, const d
                      sc->x_min, sc->x_max, sc->z_min, sc->z_max, nx, nz, max_amp, max_rx, max_rz,
                      out, out + m, finite};
     xk::FresnelReport rep;
-    cudaEvent_t g0 = nullptr, g1 = nullptr;
-    if (stats && path == XK_PATH_SEPARABLE) {
-        XK_CUDA_TRY(cudaEventCreate(&g0));
-        XK_CUDA_TRY(cudaEventCreate(&g1));
-        rep.ev_gemm[0] = g0;
-        rep.ev_gemm[1] = g1;
+    const bool timed = stats && path == XK_PATH_SEPARABLE;
+    if (timed) {
+        for (auto& e : ws.ev)
+            if (!e) XK_CUDA_TRY(cudaEventCreate(&e));
+        rep.ev_gemm[0] = ws.ev[0];
+        rep.ev_gemm[1] = ws.ev[1];
     }
     XK_CUDA_TRY(cudaEventRecord(ctx->ev0, s));
     xk::Status st = xk::fresnel_enqueue(in, ws, s, ctx->num_sms, path, &rep);
     if (st.ok()) st = xk::Status::FromCuda(cudaEventRecord(ctx->ev1, s));
-    int h_err = 0;
-    if (st.ok() && rep.d_err)
-        st = xk::Status::FromCuda(cudaMemcpyAsync(&h_err, rep.d_err, sizeof(int),
-                                                  cudaMemcpyDeviceToHost, s));
-    if (st.ok()) {
-        st = xk::Status::FromCuda(cudaMemcpyAsync(amp_re, out, m * sizeof(double),
-                                                  cudaMemcpyDeviceToHost, s));
-        if (st.ok())
-            st = xk::Status::FromCuda(cudaMemcpyAsync(amp_im, out + m, m * sizeof(double),
-                                                      cudaMemcpyDeviceToHost, s));
-        const double* xp = ws.coords.as<double>();
-        if (st.ok() && x_pixels && nx)
-            st = xk::Status::FromCuda(cudaMemcpyAsync(x_pixels, xp, nx * sizeof(double),
-                                                      cudaMemcpyDeviceToHost, s));
-        if (st.ok() && z_pixels && nz)
-            st = xk::Status::FromCuda(cudaMemcpyAsync(z_pixels, xp + std::max<size_t>(nx, 1),
-                                                      nz * sizeof(double),
-                                                      cudaMemcpyDeviceToHost, s));
-    }
+    double* const fields[2] = {amp_re, amp_im};
+    if (st.ok()) st = xk::stage_out(ctx, fields, 2, out, m, 0, s);
+    const double* xp = ws.coords.as<double>();
+    if (st.ok() && x_pixels && nx) st = xk::stage_out(ctx, &x_pixels, 1, xp, nx, 2 * m, s);
+    if (st.ok() && z_pixels && nz)
+        st = xk::stage_out(ctx, &z_pixels, 1, xp + std::max<size_t>(nx, 1), nz, 2 * m + nx, s);
     if (st.ok()) st = xk::Status::FromCuda(cudaStreamSynchronize(s));
-    if (g0) cudaEventDestroy(g0);
-    if (g1) cudaEventDestroy(g1);
     XK_TRY(st);
-    if (h_err) return xk::Status::Err(XK_ERR_TIMEOUT, "tensor-core product: a bounded wait ran out");
+    if (rep.err && *rep.err)
+        return xk::Status::Err(XK_ERR_TIMEOUT, "tensor-core product: a bounded wait ran out");
+    xk::unstage(ctx);
+    if (timed && rep.used_path == XK_PATH_SEPARABLE && rep.err) {
+        float ms = 0.f;
+        XK_CUDA_TRY(cudaEventElapsedTime(&ms, ws.ev[0], ws.ev[1]));
+        rep.gemm_ms = ms;
+    }
     if (stats) {
         float ms = 0.f;
         XK_CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));

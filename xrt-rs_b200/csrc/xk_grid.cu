@@ -66,19 +66,11 @@ __device__ __forceinline__ const double* coord(const PixDev& p, int c) {
 }
 
 __global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
-                                                         const double* __restrict__ len_part,
-                                                         int parts, int stride,
-                                                         GridProbe* __restrict__ out) {
-    __shared__ double s_len[256];
-    double v = INFINITY;
-    for (int i = threadIdx.x; i < parts; i += 256) v = fmin(v, len_part[(size_t)i * stride]);
-    s_len[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s_len[threadIdx.x] = fmin(s_len[threadIdx.x], s_len[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const double lend = s_len[0];
+                                                         const double* __restrict__ first_change,
+                                                         GridProbe* __restrict__ out,
+                                                         unsigned* __restrict__ ticket,
+                                                         GridProbe* __restrict__ host_out) {
+    const double lend = *first_change;
     if (!(lend >= 2.0 && lend <= 0.5 * m)) return;  // len stays 0
     const int len = (int)lend;
     if (m % len != 0) return;
@@ -132,6 +124,10 @@ __global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
                     atomicMax(&out->extent[axis][k], (unsigned long long)__double_as_longlong(half));
             }
         }
+    static_assert(sizeof(GridProbe) % 8 == 0, "copied by 8-byte words");
+    if (last_block(ticket) && threadIdx.x < sizeof(GridProbe) / 8)
+        reinterpret_cast<unsigned long long*>(host_out)[threadIdx.x] =
+            __ldcg(reinterpret_cast<const unsigned long long*>(out) + threadIdx.x);
 }
 
 // One block per tile: the axis coordinates of its points and their mid-range.
@@ -594,7 +590,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
                 *flag = 1;
     }
     __syncthreads();
-    if (*flag != 0 && threadIdx.x == 0) atomicExch(g.err, 1);
+    if (*flag != 0 && threadIdx.x == 0) *static_cast<volatile int*>(g.err) = 1;
     tc_fence_before();
     cluster_sync();  // the pair MMAs and all cross-CTA arrivals are done
     if (warp == 0) {
@@ -667,10 +663,10 @@ double bits_to_double(unsigned long long b) {
 
 }  // namespace
 
-Status grid_probe_enqueue(const PixDev& pix, int m, const double* len_part, int parts, int stride,
-                          GridProbe* probe, cudaStream_t stream) {
+Status grid_probe_enqueue(const PixDev& pix, int m, const double* first_change, GridProbe* probe,
+                          unsigned* ticket, GridProbe* host_probe, cudaStream_t stream) {
     const int blocks = (int)std::min<size_t>(blocks_of((size_t)m, 1024), 296);
-    grid_probe_kernel<<<blocks, 256, 0, stream>>>(pix, m, len_part, parts, stride, probe);
+    grid_probe_kernel<<<blocks, 256, 0, stream>>>(pix, m, first_change, probe, ticket, host_probe);
     XK_CUDA_TRY(cudaGetLastError());
     return Status::Ok();
 }
@@ -839,7 +835,7 @@ Status grid_reserve(const GridPlan& g, GridWorkspace& ws) {
     return Status::Ok();
 }
 
-Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* d_err, uint32_t wait_limit,
+Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wait_limit,
                     bool stall, cudaStream_t stream, int* kernels) {
     XK_TRY(grid_reserve(g, ws));
     const double* rays[12];
@@ -860,7 +856,7 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* d_err, uint32_t w
     p.partial = ws.partial.as<float>();
     p.m_pad = g.m_tiles * kTileM;
     p.n_pad = g.n_tiles * g.columns * kFN;
-    p.err = d_err;
+    p.err = err;
     p.wait_limit = wait_limit;
     p.stall = stall ? 1 : 0;
     const auto kern = g.amp ? grid_product_kernel<true> : grid_product_kernel<false>;

@@ -62,11 +62,11 @@ constexpr size_t kGridMinRays = 1024, kGridMinPoints = 1025;
 // Doubles `axes` of a plan for m screen points may need.
 inline size_t grid_axes_doubles(size_t m) { return 2 * (m + 2) + 4; }
 
-// Checks the screen's order; `len_part` holds `parts` candidates for the inner
-// length (stride `stride` doubles, the smallest counts). `probe` is zeroed by
-// an earlier kernel on the stream.
-Status grid_probe_enqueue(const PixDev& pix, int m, const double* len_part, int parts, int stride,
-                          GridProbe* probe, cudaStream_t stream);
+// Checks the screen's order. `first_change`: the candidate for the inner length
+// (device). `probe` is zeroed by an earlier kernel on the stream, `host_probe`
+// (pinned) by the caller; the kernel writes both. `ticket`: see last_block.
+Status grid_probe_enqueue(const PixDev& pix, int m, const double* first_change, GridProbe* probe,
+                          unsigned* ticket, GridProbe* host_probe, cudaStream_t stream);
 
 // Decides whether the product takes the solve and fills `g` (without device
 // pointers); `columns` amplitude columns; `tolerance` as requested.
@@ -78,9 +78,10 @@ Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream);
 
 Status grid_reserve(const GridPlan& g, GridWorkspace& ws);
 
-// Enqueues the product (allocates nothing beyond grid_reserve). `stall`: test
-// hook, the first stage never completes.
-Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* d_err, uint32_t wait_limit,
+// Enqueues the product (allocates nothing beyond grid_reserve). `err`: error
+// word the kernels can write (device or pinned). `stall`: test hook, the first
+// stage never completes.
+Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wait_limit,
                     bool stall, cudaStream_t stream, int* kernels);
 
 }  // namespace xk

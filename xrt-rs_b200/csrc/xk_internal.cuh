@@ -98,6 +98,44 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(ptr); }
 };
 
+// A growable pinned host buffer.
+struct HostBuf {
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    Status ensure(size_t want) {
+        if (want <= bytes) return Status::Ok();
+        release();
+        XK_CUDA_TRY(cudaMallocHost(&ptr, want));
+        bytes = want;
+        return Status::Ok();
+    }
+    void release() {
+        if (ptr) cudaFreeHost(ptr);
+        ptr = nullptr;
+        bytes = 0;
+    }
+    template <class T>
+    T* as() const { return static_cast<T*>(ptr); }
+};
+
+#ifdef __CUDACC__
+// Whole block: true in the block that arrives last. What the blocks wrote
+// before is visible to it (read it with __ldcg). `ticket` starts at zero and is
+// left at zero, so it needs clearing only once.
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0;
+    }
+    __syncthreads();
+    __threadfence();
+    return last;
+}
+#endif
+
 // Device-pointer views used by the launchers.
 struct RaysDev {
     const double *x, *y, *z, *nx, *ny, *nz, *nl, *es_re, *es_im, *ep_re, *ep_im, *energy;
@@ -174,6 +212,8 @@ struct FresnelShape {
 
 struct FresnelWorkspace {
     DevBuf coords, partial, ctrl;
+    HostBuf host;                    // error word and ray bounds, written by the kernels
+    cudaEvent_t ev[2] = {nullptr, nullptr};  // bracket the product
     uint32_t wait_limit = 1u << 24;  // polls of every bounded wait of the tensor-core product
     bool allow_pair = true;          // CTA-pair product on screens of more than 128 rows
     uint32_t stall_once = 0;         // test hook: the next product's first stage never completes
@@ -182,9 +222,9 @@ struct FresnelWorkspace {
 struct FresnelReport {
     int kernels = 0;
     double gemm_ms = 0.0;                       // device time of the tensor-core products
-    cudaEvent_t ev_gemm[2] = {nullptr, nullptr};  // set to time the products (synchronises per chunk)
+    cudaEvent_t ev_gemm[2] = {nullptr, nullptr};  // recorded around the product if set
     FresnelShape shape;
-    int* d_err = nullptr;                       // device error word of the products
+    int* err = nullptr;                         // error word of the product (pinned host)
     int used_path = 0;                          // XK_PATH_* that ran
 };
 

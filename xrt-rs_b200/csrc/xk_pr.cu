@@ -116,10 +116,14 @@ __device__ __forceinline__ double op_combine(int op, double a, double b) {
 // amplitude component. Field 33 is the first point at which a coordinate that
 // points 0 and 1 share changes: the inner length if the screen is rectangular
 // (infinite if points 0 and 1 differ in none or several coordinates). Clears
-// `probe` for the check of that order.
+// `probe` for the check of that order. The last block combines the rows into row
+// gridDim.x and into pinned host memory, which the host reads after its next
+// synchronisation (a copy of a few hundred bytes costs more than the kernel).
 __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p, int m,
                                                      double* __restrict__ block_out,
-                                                     GridProbe* __restrict__ probe) {
+                                                     GridProbe* __restrict__ probe,
+                                                     unsigned* __restrict__ ticket,
+                                                     double* __restrict__ host_out) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *probe = GridProbe{};
     double f[kSumFields];
 #pragma unroll
@@ -191,6 +195,25 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
         for (int w = 1; w < 8; ++w) v = op_combine(op, v, sm[w][i]);
         block_out[blockIdx.x * kSumFields + i] = v;
     }
+    if (!last_block(ticket)) return;
+    constexpr int kParts = 6;  // threads per field
+    __shared__ double sp[kParts][kSumFields];
+    const int rows = gridDim.x, i = threadIdx.x % kSumFields, part = threadIdx.x / kSumFields;
+    const int op = sum_op(i);
+    if (part < kParts) {
+        double v = op == OP_SUM ? 0.0 : (op == OP_MIN ? INFINITY : -INFINITY);
+#pragma unroll 4
+        for (int b = part; b < rows; b += kParts)
+            v = op_combine(op, v, __ldcg(block_out + b * kSumFields + i));
+        sp[part][i] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < kSumFields) {
+        double v = sp[0][i];
+        for (int w = 1; w < kParts; ++w) v = op_combine(op, v, sp[w][i]);
+        block_out[rows * kSumFields + i] = v;
+        host_out[i] = v;
+    }
 }
 
 struct Frame {
@@ -236,9 +259,12 @@ __device__ __forceinline__ uint32_t hilbert16(uint32_t x, uint32_t y) {
 
 // Hilbert key of every screen point over its two transverse frame axes, the
 // longitudinal coordinate as tie-break.
+// Clears the tile extents for the next kernel.
 __global__ void pixel_keys_kernel(PixDev p, int m, Frame fr, uint64_t* __restrict__ keys,
-                                  int* __restrict__ idx) {
+                                  int* __restrict__ idx,
+                                  unsigned long long* __restrict__ amax_bits) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 4) amax_bits[i] = 0;
     if (i >= m) return;
     double c[3];
     to_frame(fr, p.x[i], p.y[i], p.z[i], c);
@@ -252,7 +278,8 @@ __global__ void pixel_keys_kernel(PixDev p, int m, Frame fr, uint64_t* __restric
 // One warp per tile: slot table, slot-ordered coordinates, bounding-box
 // centre; the largest radius of any tile, its largest extents across and along
 // the frame's long axis u0 (amax_bits[0..2]) and the sum of the tiles' extents
-// across (amax_bits[3], a double).
+// across (amax_bits[3], a double), which the last block writes to pinned host
+// memory.
 // Centres are snapped to multiples of `quantum` as the chunk centres are, so
 // that differences between points, tile and chunk centres are exact. rel, ns:
 // each slot's offset from the centre (PrSolve::tile_rel); n2 = 2 n for solves
@@ -263,67 +290,72 @@ __global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, double quant
                             float* __restrict__ ns, int* __restrict__ tile_perm, double* __restrict__ tpx,
                             double* __restrict__ tpy, double* __restrict__ tpz,
                             double* __restrict__ tile_center,
-                            unsigned long long* __restrict__ amax_bits) {
+                            unsigned long long* __restrict__ amax_bits,
+                            unsigned* __restrict__ ticket, double* __restrict__ host_out) {
     int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
-    if (t >= n_tiles) return;
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = 0; i < kPrPpl; ++i) {
-        long long s = (long long)t * kPrTile + lane + 32 * i;
-        int id = s < m ? sorted_idx[s] : -1;
-        tile_perm[s] = id;
-        if (id >= 0) {
-            double v[3] = {p.x[id], p.y[id], p.z[id]};
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = fmin(lo[a], v[a]);
-                hi[a] = fmax(hi[a], v[a]);
+    if (t < n_tiles) {
+        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        for (int i = 0; i < kPrPpl; ++i) {
+            long long s = (long long)t * kPrTile + lane + 32 * i;
+            int id = s < m ? sorted_idx[s] : -1;
+            tile_perm[s] = id;
+            if (id >= 0) {
+                double v[3] = {p.x[id], p.y[id], p.z[id]};
+                for (int a = 0; a < 3; ++a) {
+                    lo[a] = fmin(lo[a], v[a]);
+                    hi[a] = fmax(hi[a], v[a]);
+                }
             }
         }
-    }
-    for (int a = 0; a < 3; ++a)
+        for (int a = 0; a < 3; ++a)
+            for (int o = 16; o > 0; o >>= 1) {
+                lo[a] = fmin(lo[a], __shfl_xor_sync(kFull, lo[a], o));
+                hi[a] = fmax(hi[a], __shfl_xor_sync(kFull, hi[a], o));
+            }
+        double c[3];
+        for (int a = 0; a < 3; ++a) c[a] = rint(0.5 * (lo[a] + hi[a]) * inv_quantum) * quantum;
+        double rad = 0.0, across = 0.0, along = 0.0;
+        for (int i = 0; i < kPrPpl; ++i) {
+            long long s = (long long)t * kPrTile + lane + 32 * i;
+            int id = s < m ? sorted_idx[s] : -1;
+            double x = c[0], y = c[1], z = c[2];
+            if (id >= 0) {
+                x = p.x[id];
+                y = p.y[id];
+                z = p.z[id];
+                double dx = x - c[0], dy = y - c[1], dz = z - c[2];
+                rad = fmax(rad, sqrt(dx * dx + dy * dy + dz * dz));
+                const double f1 = dx * fr.e1[0] + dy * fr.e1[1] + dz * fr.e1[2];
+                const double f2 = dx * fr.e2[0] + dy * fr.e2[1] + dz * fr.e2[2];
+                across = fmax(across, sqrt(f1 * f1 + f2 * f2));
+                along = fmax(along, fabs(dx * fr.u0[0] + dy * fr.u0[1] + dz * fr.u0[2]));
+            }
+            tpx[s] = x;
+            tpy[s] = y;
+            tpz[s] = z;
+            const double sx = x - c[0], sy = y - c[1], sz = z - c[2];
+            rel[s] = make_double4(sx, sy, sz, sx * sx + sy * sy + sz * sz);
+            ns[s] = (float)(n2.x * sx + n2.y * sy + n2.z * sz);
+        }
         for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = fmin(lo[a], __shfl_xor_sync(kFull, lo[a], o));
-            hi[a] = fmax(hi[a], __shfl_xor_sync(kFull, hi[a], o));
+            rad = fmax(rad, __shfl_xor_sync(kFull, rad, o));
+            across = fmax(across, __shfl_xor_sync(kFull, across, o));
+            along = fmax(along, __shfl_xor_sync(kFull, along, o));
         }
-    double c[3];
-    for (int a = 0; a < 3; ++a) c[a] = rint(0.5 * (lo[a] + hi[a]) * inv_quantum) * quantum;
-    double rad = 0.0, across = 0.0, along = 0.0;
-    for (int i = 0; i < kPrPpl; ++i) {
-        long long s = (long long)t * kPrTile + lane + 32 * i;
-        int id = s < m ? sorted_idx[s] : -1;
-        double x = c[0], y = c[1], z = c[2];
-        if (id >= 0) {
-            x = p.x[id];
-            y = p.y[id];
-            z = p.z[id];
-            double dx = x - c[0], dy = y - c[1], dz = z - c[2];
-            rad = fmax(rad, sqrt(dx * dx + dy * dy + dz * dz));
-            const double f1 = dx * fr.e1[0] + dy * fr.e1[1] + dz * fr.e1[2];
-            const double f2 = dx * fr.e2[0] + dy * fr.e2[1] + dz * fr.e2[2];
-            across = fmax(across, sqrt(f1 * f1 + f2 * f2));
-            along = fmax(along, fabs(dx * fr.u0[0] + dy * fr.u0[1] + dz * fr.u0[2]));
+        if (lane == 0) {
+            tile_center[3 * t + 0] = c[0];
+            tile_center[3 * t + 1] = c[1];
+            tile_center[3 * t + 2] = c[2];
+            atomicMax(amax_bits, (unsigned long long)__double_as_longlong(rad));
+            atomicMax(amax_bits + 1, (unsigned long long)__double_as_longlong(across));
+            atomicMax(amax_bits + 2, (unsigned long long)__double_as_longlong(along));
+            atomicAdd(reinterpret_cast<double*>(amax_bits + 3), across);
         }
-        tpx[s] = x;
-        tpy[s] = y;
-        tpz[s] = z;
-        const double sx = x - c[0], sy = y - c[1], sz = z - c[2];
-        rel[s] = make_double4(sx, sy, sz, sx * sx + sy * sy + sz * sz);
-        ns[s] = (float)(n2.x * sx + n2.y * sy + n2.z * sz);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        rad = fmax(rad, __shfl_xor_sync(kFull, rad, o));
-        across = fmax(across, __shfl_xor_sync(kFull, across, o));
-        along = fmax(along, __shfl_xor_sync(kFull, along, o));
-    }
-    if (lane == 0) {
-        tile_center[3 * t + 0] = c[0];
-        tile_center[3 * t + 1] = c[1];
-        tile_center[3 * t + 2] = c[2];
-        atomicMax(amax_bits, (unsigned long long)__double_as_longlong(rad));
-        atomicMax(amax_bits + 1, (unsigned long long)__double_as_longlong(across));
-        atomicMax(amax_bits + 2, (unsigned long long)__double_as_longlong(along));
-        atomicAdd(reinterpret_cast<double*>(amax_bits + 3), across);
-    }
+    if (last_block(ticket) && threadIdx.x < 4)
+        host_out[threadIdx.x] =
+            __longlong_as_double((long long)__ldcg(amax_bits + threadIdx.x));
 }
 
 struct CellGrid {
@@ -364,7 +396,7 @@ __global__ void head_flags_kernel(const uint64_t* __restrict__ keys, int n, int*
 __global__ void chunk_table_kernel(const uint64_t* __restrict__ keys, const int* __restrict__ flags,
                                    const int* __restrict__ run_id, int n, CellGrid g,
                                    int* __restrict__ chunk_begin, double* __restrict__ chunk_center,
-                                   int* __restrict__ n_chunks) {
+                                   int* __restrict__ n_chunks, int* __restrict__ host_chunks) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (flags[i]) {
@@ -391,6 +423,7 @@ __global__ void chunk_table_kernel(const uint64_t* __restrict__ keys, const int*
     if (i == n - 1) {
         int nc = run_id[i];
         *n_chunks = nc;
+        *host_chunks = nc;
         chunk_begin[nc] = n;
     }
 }
@@ -1224,7 +1257,7 @@ pr_persistent_kernel(const PrSolve* __restrict__ solves, int n_solves, long long
         const bool ok = process_item<UNIFORM, FAST, FOLD, POL, LIN>(
             sv, local, wp, *wsh, lane, ctl.wait_limit, item == 0 ? ctl.stall_bytes : 0u);
         if (!ok) {
-            if (lane == 0) atomicExch(err, 1);
+            if (lane == 0) *static_cast<volatile int*>(err) = 1;
             break;
         }
     }
@@ -1425,7 +1458,7 @@ struct SolveBufs {
 
 void carve(Arena& a, SolveBufs& b, int n, int m, int n_tiles, int groups, int sum_blocks) {
     const size_t slots = (size_t)n_tiles * kPrTile;
-    b.sum = a.take<double>((size_t)sum_blocks * kSumFields);
+    b.sum = a.take<double>((size_t)(sum_blocks + 1) * kSumFields);
     b.probe = a.take<GridProbe>(1);
     b.axes = a.take<double>(grid_axes_doubles((size_t)m));
     b.pk_in = a.take<uint64_t>(m);
@@ -1466,11 +1499,11 @@ struct HostLayout {
     size_t sum_off, probe_off, amax_off, nch_off, err_off, tab_off, total;
 };
 
-HostLayout host_layout(int count, int sum_blocks) {
+HostLayout host_layout(int count) {
     HostLayout L;
     size_t off = 0;
     L.sum_off = off;
-    off = align_up(off + (size_t)count * sum_blocks * kSumFields * sizeof(double), 256);
+    off = align_up(off + (size_t)count * kSumFields * sizeof(double), 256);
     L.probe_off = off;
     off = align_up(off + (size_t)count * sizeof(GridProbe), 256);
     L.amax_off = off;
@@ -1614,7 +1647,15 @@ Status PrWorkspace::ensure_host(size_t bytes) {
     return Status::Ok();
 }
 
+Status PrWorkspace::ensure_tickets(int count, cudaStream_t stream) {
+    const size_t had = tickets.bytes;
+    XK_TRY(tickets.ensure(std::max(count, 1) * 4 * sizeof(unsigned)));
+    if (tickets.bytes != had) XK_CUDA_TRY(cudaMemsetAsync(tickets.ptr, 0, tickets.bytes, stream));
+    return Status::Ok();
+}
+
 void PrWorkspace::release() {
+    tickets.release();
     arena.release();
     cub_tmp.release();
     solves.release();
@@ -1750,13 +1791,15 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
     }
     XK_TRY(ws.cub_tmp.ensure(cub_need + 256));
     if (!arenas) XK_TRY(ws.arena.ensure(need + 256));
-    const HostLayout HL = host_layout(count, sum_blocks);
+    const HostLayout HL = host_layout(count);
     XK_TRY(ws.ensure_host(HL.total));
     char* hbase = static_cast<char*>(ws.host);
     double* h_sum = reinterpret_cast<double*>(hbase + HL.sum_off);
     GridProbe* h_probe = reinterpret_cast<GridProbe*>(hbase + HL.probe_off);
     double* h_amax = reinterpret_cast<double*>(hbase + HL.amax_off);
     int* h_nch = reinterpret_cast<int*>(hbase + HL.nch_off);
+    XK_TRY(ws.ensure_tickets(count, stream));
+    unsigned* tickets = ws.tickets.as<unsigned>();
 
     std::vector<SolveBufs> bufs(count);
     {
@@ -1776,18 +1819,15 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         any = true;
         const int parts = sum_parts(in[s].n, in[s].m, sum_blocks);
         summary_kernel<<<parts, 256, 0, stream>>>(in[s].rays, (int)in[s].n, in[s].pix,
-                                                        (int)in[s].m, bufs[s].sum, bufs[s].probe);
+                                                  (int)in[s].m, bufs[s].sum, bufs[s].probe,
+                                                  tickets + 4 * s, h_sum + s * kSumFields);
         XK_CUDA_TRY(cudaGetLastError());
         if (grid_candidate(opt, in[s].n, in[s].m)) {
-            XK_TRY(grid_probe_enqueue(in[s].pix, (int)in[s].m, bufs[s].sum + 33, parts,
-                                      kSumFields, bufs[s].probe, stream));
-            XK_CUDA_TRY(cudaMemcpyAsync(h_probe + s, bufs[s].probe, sizeof(GridProbe),
-                                        cudaMemcpyDeviceToHost, stream));
+            h_probe[s] = GridProbe{};
+            XK_TRY(grid_probe_enqueue(in[s].pix, (int)in[s].m, bufs[s].sum + parts * kSumFields + 33,
+                                      bufs[s].probe, tickets + 4 * s + 1, h_probe + s, stream));
             ++nk;
         }
-        XK_CUDA_TRY(cudaMemcpyAsync(h_sum + (size_t)s * sum_blocks * kSumFields, bufs[s].sum,
-                                    (size_t)parts * kSumFields * sizeof(double),
-                                    cudaMemcpyDeviceToHost, stream));
         ++nk;
     }
     if (!any) {
@@ -1801,16 +1841,7 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         PrPlan& P = plans[s];
         if (P.routed) continue;
         HostSolveInfo& I = info[s];
-        const double* hs = h_sum + (size_t)s * sum_blocks * kSumFields;
-        const int parts = sum_parts(in[s].n, in[s].m, sum_blocks);
-        for (int i = 0; i < kSumFields; ++i) {
-            double v = hs[i];
-            for (int bk = 1; bk < parts; ++bk) {
-                double w = hs[bk * kSumFields + i];
-                v = sum_op(i) == OP_SUM ? v + w : (sum_op(i) == OP_MIN ? std::min(v, w) : std::max(v, w));
-            }
-            I.f[i] = v;
-        }
+        std::memcpy(I.f, h_sum + s * kSumFields, sizeof(I.f));
         const double* f = I.f;
         if (!(f[26] == 0.0)) {
             // NaN or infinite inputs: the FP64 sum propagates them the way
@@ -1907,7 +1938,8 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             I.fr.e2[i] = e2[i];
             I.fr.u0[i] = u0[i];
         }
-        if (grid_candidate(opt, in[s].n, in[s].m)) XK_TRY(try_grid(in[s], h_probe[s], I, opt, bufs[s], num_sms, stream, &P, &nk));
+        if (grid_candidate(opt, in[s].n, in[s].m))
+            XK_TRY(try_grid(in[s], h_probe[s], I, opt, bufs[s], num_sms, stream, &P, &nk));
     }
 
     // --- B. screen tiles ----------------------------------------------------
@@ -1938,22 +1970,20 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         const double deep = qmax[2] / pf.scale[2], wide = qmax[0] / std::min(pf.scale[0], pf.scale[1]);
         if (pf.scale[0] > 0.0 && pf.scale[1] > 0.0 && pf.scale[2] > 0.0 && deep > wide)
             pf.scale[0] = pf.scale[1] = std::min(pf.scale[0], pf.scale[1]);
-        pixel_keys_kernel<<<(m + 255) / 256, 256, 0, stream>>>(in[s].pix, m, pf, B.pk_in, B.pi_in);
+        pixel_keys_kernel<<<(m + 255) / 256, 256, 0, stream>>>(in[s].pix, m, pf, B.pk_in, B.pi_in,
+                                                                B.amax);
         XK_CUDA_TRY(cudaGetLastError());
         size_t tmp = ws.cub_tmp.bytes;
         // A screen without depth has zeros in the keys' low 21 bits.
         XK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws.cub_tmp.ptr, tmp, B.pk_in, B.pk_out, B.pi_in,
                                                     B.pi_out, m, pf.scale[2] > 0.0 ? 0 : 21, 53,
                                                     stream));
-        XK_CUDA_TRY(cudaMemsetAsync(B.amax, 0, 4 * sizeof(unsigned long long), stream));
         tile_kernel<<<(n_tiles[s] * 32 + 255) / 256, 256, 0, stream>>>(
             in[s].pix, m, n_tiles[s], pf, I.quantum, 1.0 / I.quantum,
             make_double3(2.0 * I.f[11], 2.0 * I.f[12], 2.0 * I.f[13]), B.pi_out, B.rel, B.ns,
             B.tile_perm, B.tpx, B.tpy, B.tpz, B.tile_center,
-            B.amax);
+            B.amax, tickets + 4 * s + 2, h_amax + 4 * s);
         XK_CUDA_TRY(cudaGetLastError());
-        XK_CUDA_TRY(cudaMemcpyAsync(h_amax + 4 * s, B.amax, 4 * sizeof(double),
-                                    cudaMemcpyDeviceToHost, stream));
         nk += 2;
     }
     if (any) XK_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -2101,7 +2131,7 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         XK_CUDA_TRY(cub::DeviceScan::InclusiveSum(ws.cub_tmp.ptr, tmp, B.flags, B.run, n, stream));
         chunk_table_kernel<<<(n + 255) / 256, 256, 0, stream>>>(B.rk_out, B.flags, B.run, n, cg,
                                                                  B.chunk_begin, B.chunk_center,
-                                                                 B.n_chunks);
+                                                                 B.n_chunks, h_nch + s);
         XK_CUDA_TRY(cudaGetLastError());
         records_kernel<<<(n + 255) / 256, 256, 0, stream>>>(in[s].rays, n, B.ri_out, B.run,
                                                              B.chunk_center, B.recs);
@@ -2160,7 +2190,6 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         P.n_tiles = n_tiles[s];
         P.groups = groups[s];
         P.n_chunks_host = h_nch + s;
-        *P.n_chunks_host = 0;
     }
     if (kernels) *kernels += nk;
     return Status::Ok();
@@ -2203,11 +2232,11 @@ Status pr_finalize(const PrPlan& P, cudaStream_t stream) {
 }
 
 Status pr_reserve_plan_host(PrWorkspace& ws, int count, int num_sms) {
-    return ws.ensure_host(host_layout(count, sum_blocks_for(num_sms)).total);
+    return ws.ensure_host(host_layout(count).total);
 }
 
 Status pr_reserve_exec(PrWorkspace& ws, int count, int num_sms) {
-    const HostLayout HL = host_layout(count, sum_blocks_for(num_sms));
+    const HostLayout HL = host_layout(count);
     XK_TRY(ws.ensure_host(HL.total));
     XK_TRY(ws.solves.ensure(std::max<size_t>(1, count) * sizeof(PrSolve)));
     XK_TRY(ws.ctrl.ensure(kPrCtrlBytes));
@@ -2221,16 +2250,13 @@ Status pr_execute_enqueue(std::vector<PrPlan>& plans, PrWorkspace& ws, cudaStrea
     PrExecReport local;
     PrExecReport& R = rep ? *rep : local;
     const int count = (int)plans.size();
-    const HostLayout HL = host_layout(count, sum_blocks_for(num_sms));
+    const HostLayout HL = host_layout(count);
     XK_TRY(pr_reserve_exec(ws, count, num_sms));
     char* hbase = static_cast<char*>(ws.host);
     PrSolve* h_tab = reinterpret_cast<PrSolve*>(hbase + HL.tab_off);
-    int* h_nch = reinterpret_cast<int*>(hbase + HL.nch_off);
     ws.host_err = reinterpret_cast<int*>(hbase + HL.err_off);
     *ws.host_err = 0;
     unsigned long long* d_counters = reinterpret_cast<unsigned long long*>(ws.ctrl.ptr);
-    int* d_err = reinterpret_cast<int*>(static_cast<char*>(ws.ctrl.ptr) + kPrCtrlErrOffset);
-    XK_CUDA_TRY(cudaMemsetAsync(ws.ctrl.ptr, 0, kPrCtrlBytes, stream));
 
     // Group the planned solves by kernel variant into contiguous tables.
     struct Launch {
@@ -2256,16 +2282,18 @@ Status pr_execute_enqueue(std::vector<PrPlan>& plans, PrWorkspace& ws, cudaStrea
     bool any_grid = false;
     for (const PrPlan& P : plans) any_grid |= !P.routed && P.grid;
     if (tab == 0 && !any_grid) return Status::Ok();
-    if (tab)
+    if (tab) {
+        XK_CUDA_TRY(cudaMemsetAsync(ws.ctrl.ptr, 0, kPrCtrlBytes, stream));
         XK_CUDA_TRY(cudaMemcpyAsync(ws.solves.ptr, h_tab, (size_t)tab * sizeof(PrSolve),
                                     cudaMemcpyHostToDevice, stream));
+    }
     if (time_kernels) XK_CUDA_TRY(cudaEventRecord(ws.ev[0], stream));
     int li = 0;
     PrCtl ctl = ws.ctl;
     ws.ctl.stall_bytes = 0;  // the stall test hook arms one execution only
     for (const Launch& L : launches) {
         XK_TRY(pr_launch(reinterpret_cast<const PrSolve*>(ws.solves.ptr) + L.first, L.count,
-                         L.items, L.variant, d_counters + li, d_err, stream, num_sms, 0, ctl));
+                         L.items, L.variant, d_counters + li, ws.host_err, stream, num_sms, 0, ctl));
         ctl.stall_bytes = 0;
         R.kernels += 1;
         R.n_items += L.items;
@@ -2273,7 +2301,7 @@ Status pr_execute_enqueue(std::vector<PrPlan>& plans, PrWorkspace& ws, cudaStrea
     }
     for (const PrPlan& P : plans) {
         if (P.routed || !P.grid) continue;
-        XK_TRY(grid_enqueue(P.grid_plan, ws.grid, d_err, ctl.wait_limit, ctl.stall_bytes != 0,
+        XK_TRY(grid_enqueue(P.grid_plan, ws.grid, ws.host_err, ctl.wait_limit, ctl.stall_bytes != 0,
                             stream, &R.kernels));
         ctl.stall_bytes = 0;
         R.n_items += (long long)P.n_tiles * P.groups;
@@ -2283,11 +2311,8 @@ Status pr_execute_enqueue(std::vector<PrPlan>& plans, PrWorkspace& ws, cudaStrea
         PrPlan& P = plans[s];
         if (P.routed || P.grid) continue;
         XK_TRY(pr_finalize(P, stream));
-        XK_CUDA_TRY(cudaMemcpyAsync(h_nch + s, P.dev.n_chunks_dev, sizeof(int),
-                                    cudaMemcpyDeviceToHost, stream));
         R.kernels += 1;
     }
-    XK_CUDA_TRY(cudaMemcpyAsync(ws.host_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
     return Status::Ok();
 }
 

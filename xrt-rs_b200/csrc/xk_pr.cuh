@@ -183,14 +183,16 @@ struct PrWorkspace {
     cudaEvent_t ev[2] = {nullptr, nullptr};  // bracket the pair kernels
     void* host = nullptr;  // pinned readback / upload area
     size_t host_bytes = 0;
-    int* host_err = nullptr;  // error word copied back by the last execution
+    int* host_err = nullptr;  // error word (in `host`), written by the kernels
+    DevBuf tickets;           // last-block counters of the planner kernels, zero between uses
+    Status ensure_tickets(int count, cudaStream_t stream);
     bool host_borrowed = false;  // `host` belongs to the caller: never freed here
     PrCtl ctl;                   // wait limit; stall_bytes is cleared after one execution
     Status ensure_host(size_t bytes);
     void release();
     // Stream-ordered allocation for every device buffer of this workspace.
     void set_async(cudaStream_t s) {
-        grid.recs.async_stream = grid.partial.async_stream = s;
+        grid.recs.async_stream = grid.partial.async_stream = tickets.async_stream = s;
         arena.async_stream = cub_tmp.async_stream = solves.async_stream = ctrl.async_stream = s;
     }
 };

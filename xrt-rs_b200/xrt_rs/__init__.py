@@ -17,6 +17,7 @@ no CUDA device every compute call raises XkError (code XK_ERR_NO_DEVICE).
 from __future__ import annotations
 
 import ctypes
+import struct
 
 import numpy as np
 
@@ -125,6 +126,15 @@ def _ptr(a):
     return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
+def _columns(cls, arrays):
+    """A struct of pointers to the arrays (numpy arrays or device tensors), filled
+    in one step: one ctypes cast per column costs more than a small launch."""
+    ptrs = [int(a.data_ptr()) if hasattr(a, "data_ptr") else a.ctypes.data for a in arrays]
+    if ctypes.sizeof(cls) != 8 * len(ptrs):
+        raise ValueError(f"expected {ctypes.sizeof(cls) // 8} arrays, got {len(ptrs)}")
+    return cls.from_buffer_copy(struct.pack(f"{len(ptrs)}Q", *ptrs))
+
+
 def _check_lengths(pairs):
     # Same message shape as check_equal_lengths (crates/xrt-python/src/lib.rs:31-45).
     if len(pairs) < 2:
@@ -158,9 +168,9 @@ def diffraction_integral(rays, pixels, path="f64", ctx=None, return_stats=False)
     out = [np.zeros(m, dtype=np.float64) for _ in range(4)]
     ctx = _require_ctx(ctx)
     lib = _lib.load()
-    xr = _lib.XkRays(*[_ptr(a) for a in r])
-    xp = _lib.XkPixels(*[_ptr(a) for a in p])
-    xf = _lib.XkField(*[_ptr(a) for a in out])
+    xr = _columns(_lib.XkRays, r)
+    xp = _columns(_lib.XkPixels, p)
+    xf = _columns(_lib.XkField, out)
     st = _lib.XkStats()
     rc = lib.xk_diffraction_integral(ctx.handle, ctypes.byref(xr), n, ctypes.byref(xp), m,
                                      ctypes.byref(xf), path_code, ctypes.byref(st))
@@ -191,11 +201,6 @@ def diffraction_integral_device(rays, pixels, out, path="f32pr", ctx=None, strea
     (e.g. a contiguous float64 CUDA tensor). Returns the stats dict."""
     ctx = _require_ctx(ctx)
     lib = _lib.load()
-    dp = ctypes.POINTER(ctypes.c_double)
-
-    def cast(t):
-        return ctypes.cast(ctypes.c_void_p(int(t.data_ptr())), dp)
-
     if isinstance(rays, dict):
         rays = [rays[k] for k in RAY_FIELDS]
     if isinstance(pixels, dict):
@@ -204,9 +209,9 @@ def diffraction_integral_device(rays, pixels, out, path="f32pr", ctx=None, strea
         out = [out[k] for k in FIELD_FIELDS]
     n = int(rays[0].numel()) if hasattr(rays[0], "numel") else len(rays[0])
     m = int(pixels[0].numel()) if hasattr(pixels[0], "numel") else len(pixels[0])
-    xr = _lib.XkRays(*[cast(a) for a in rays])
-    xp = _lib.XkPixels(*[cast(a) for a in pixels])
-    xf = _lib.XkField(*[cast(a) for a in out])
+    xr = _columns(_lib.XkRays, rays)
+    xp = _columns(_lib.XkPixels, pixels)
+    xf = _columns(_lib.XkField, out)
     st = _lib.XkStats()
     s = ctypes.c_void_p(int(stream)) if stream is not None else None
     rc = lib.xk_diffraction_integral_device(ctx.handle, ctypes.byref(xr), n, ctypes.byref(xp), m,
