@@ -81,6 +81,24 @@ def test_tile_edges(grid_ctx, oracle, n_outer, n_inner):
     check(grid_ctx, oracle, rays, pix)
 
 
+# Tiles of 256 x 256 points: the smallest (129 columns), last tiles of one, of
+# half and of half and one columns in either orientation; accumulators drained in
+# turn after one block, after an odd number of blocks and with an empty split.
+@pytest.mark.parametrize("n_outer,n_inner,n,pol", [(256, 129, 1024, 1), (129, 256, 4000, 2),
+                                                    (200, 257, 1055, 2), (384, 250, 3333, 1),
+                                                    (385, 131, 30011, 1), (512, 255, 1100, 2)])
+@pytest.mark.parametrize("dist", [700.0, 3000.0])
+def test_wide_tiles(grid_ctx, oracle, n_outer, n_inner, n, pol, dist):
+    rays = synth.gaussian_aperture(n, 0.1, 12000.0, 2e4, seed=21)
+    if pol == 2:
+        rng = np.random.default_rng(n)
+        rays.update(ep_re=rng.normal(0, 1, n), ep_im=rng.normal(0, 1, n))
+    pix = grid(np.linspace(-0.5, 0.5, n_outer), np.linspace(-0.4, 0.4, n_inner), dist, "xyz")
+    out, st = check(grid_ctx, oracle, rays, pix, want=3 if dist > 1000 else run(
+        grid_ctx, rays, pix)[1]["sweep"])
+    assert st["one_polarization"] == (pol == 1)
+
+
 def test_mostly_padding_takes_the_general_kernel(grid_ctx, oracle):
     """A screen that fills a 32nd of its tile, with many rays."""
     rays = synth.gaussian_aperture(1_500_000, 0.1, 10000.0, 3e4, seed=14)

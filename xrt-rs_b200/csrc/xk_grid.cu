@@ -19,8 +19,8 @@
 //   * grid_records_kernel: per (tile, ray) 64 bytes: k D in turns, reduced in
 //     double-double (k D reaches 1e12 rad), the linear phase coefficients as
 //     hi + lo floats, the amplitude at p0.
-//   * grid_product_kernel: CTA pairs (tcgen05 cta_group::2, 256 rows x 128
-//     columns), the structure of fresnel_pair_kernel: producer warps turn rays
+//   * grid_product_kernel: CTA pairs (tcgen05 cta_group::2, 256 rows x 128 or
+//     256 columns), the structure of fresnel_pair_kernel: producer warps turn rays
 //     into f16 hi + lo phasor tiles in shared memory, one thread issues
 //     A_hi B_hi + A_hi B_lo + A_lo B_hi + A_1 B_1 per block of 32 rays, four
 //     epilogue warps drain the f32 accumulator every `seg` blocks.
@@ -45,17 +45,39 @@ namespace {
 
 using namespace phasor;
 
-constexpr int kTileM = 256, kTileN = 128;
-constexpr uint32_t kGA = 128 * 128;      // one operand tile: 128 rows x 128 B (A or this CTA's B half)
-constexpr uint32_t kGStage = 6 * kGA;    // A_hi | A_lo | B_hi | B_lo | A_1 | B_1
+constexpr int kTileM = 256;
+constexpr uint32_t kGA = 128 * 128;  // 128 rows x 128 B: one f16 tile of a CTA
 constexpr int kGStages = 2;
-constexpr int kGProdThreads = 384;       // warps 5..16
-constexpr int kGThreads = 32 + kFEpiThreads + kGProdThreads + 32;
+constexpr uint32_t kGStage = 6 * kGA;  // hi, lo, first order of A (128 rows) and of B (128 rows)
 constexpr uint32_t kGRayBytes = kFRays * 64;
-constexpr size_t kGSmem =
-    1024 + (size_t)kGStages * kGStage + kFRayBufs * kGRayBytes + kFEpiBytes + 256;
+constexpr int kGRayBufs = 3;
+constexpr int kGEpiBufs = 3;  // staging buffers per epilogue warp
+constexpr uint32_t kDrainBytes = 32 * 16 * 4;  // 32 rows x 16 columns of a partial
+constexpr size_t kGSmem = 1024 + (size_t)kGStages * kGStage + kGRayBufs * kGRayBytes +
+                          4 * kGEpiBufs * kDrainBytes + 256;
 static_assert(kGSmem <= 227 * 1024, "shared memory");
-constexpr double kGridScale = 1024.0;    // largest |W|: lo parts stay normal f16 numbers
+
+// The product's two forms, the same bytes per stage of 32 rays.
+// Narrow: 128 columns per tile. A row of either operand holds its rays' (re, im)
+// words, and B has a real-part and an imaginary-part row per column; the two
+// accumulators of 256 TMEM columns alternate between segments.
+// Wide: 256 columns. A row holds 32 real parts, then 32 imaginary parts, so that
+// one B row per column serves both parts of the field (Ar Br - Ai Bi and Ar Bi +
+// Ai Br, the sign a bit of the instruction): half the phasor stores per column,
+// and the A phasors serve twice the columns. One accumulator each for the real
+// and the imaginary part; a part is drained while the other's products run.
+// 2^20 rays x 512^2 points: 7.5 ms narrow, 6.3 ms wide (first calls; 8.5 and
+// 7.1 ms in a row, the chip at its power limit and 1.55 GHz). In the wide form
+// the tensor pipe is busy 72 % of the time (narrow 43 %) and shared memory 77 %
+// (products 35, record loads 24, stores 18 %).
+template <bool WIDE>
+struct Form {
+    static constexpr int kTileN = WIDE ? 256 : 128;
+    static constexpr int kAcc = WIDE ? 2 : 1;       // accumulators of a segment
+    static constexpr int kProdWarps = WIDE ? 8 : 12;
+    static constexpr int kThreads = 32 + kFEpiThreads + 32 * kProdWarps + 32;
+};
+constexpr double kGridScale = 1024.0;  // largest |W|: lo parts stay normal f16 numbers
 constexpr size_t kGridRecBytes = (size_t)512 << 20;  // ray records of one launch
 constexpr size_t kGridMaxTiles = 4096;               // at least 2048 rays per launch fit then
 
@@ -134,11 +156,11 @@ __global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
 __global__ void __launch_bounds__(kTileM) grid_axes_kernel(const double* __restrict__ src_m,
                                                            size_t stride_m, int nm, int m_tiles,
                                                            const double* __restrict__ src_n,
-                                                           size_t stride_n, int nn,
+                                                           size_t stride_n, int nn, int tile_n,
                                                            double* __restrict__ axes) {
     const bool is_m = (int)blockIdx.x < m_tiles;
     const int t = is_m ? blockIdx.x : blockIdx.x - m_tiles;
-    const int size = is_m ? kTileM : kTileN, count = is_m ? nm : nn;
+    const int size = is_m ? kTileM : tile_n, count = is_m ? nm : nn;
     const int q = t * size + threadIdx.x;
     double lo = INFINITY, hi = -INFINITY;
     if ((int)threadIdx.x < size && q < count) {
@@ -226,7 +248,7 @@ struct ProductArgs {
     const double *cm, *cn, *refs;
     size_t nm, nn;
     double h0;
-    float* partial;  // [splits][m_pad][n_pad]
+    float* partial;  // [splits][m_pad][n_pad], in the order of partial_at
     int m_pad, n_pad;
     bool first;      // the splits' first segments store
     int* err;
@@ -241,25 +263,93 @@ __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
     return *reinterpret_cast<const uint32_t*>(&r);
 }
 
-// Producer warps of a CTA of the pair, the work split of fresnel_pair_kernel:
-// warps 0..7 (ZZ = false) fill 16-byte chunk c0 (four rays) of the A rows l,
-// l + 32 and of the B rows of points l, l + 32; warps 8..11 (ZZ = true) chunks
-// c0, c0 + 1 of the A rows 64 + l, 96 + l. Inside a chunk the contraction runs
-// (re j, re j+1, im j, im j+1) over ray pairs, in both operands, so that the
-// real-part and imaginary-part rows of B hold the same words in another order
-// (and one sign). Rows and columns past the screen's edge hold the phasors of
-// the tile's reference point: they only reach accumulators nobody reads. AMP:
-// the amplitude varies along the tile.
+// A pair-row: a row of A (.x) and a row of B (.y), or two rows of A (ZZ),
+// evaluated together in packed instructions.
+struct PairRow {
+    float2 kh, khn, kl, pp, sq;
+    __device__ __forceinline__ void set(double ux, double uy, double h0) {
+        float hx, lx, hy, ly, fx, fy;
+        split_coord(ux, h0, &hx, &lx, &fx);
+        split_coord(uy, h0, &hy, &ly, &fy);
+        kh = make_float2(hx, hy);
+        khn = make_float2(-hx, -hy);
+        kl = make_float2(lx, ly);
+        pp = make_float2(fx, fy);
+        sq = make_float2((float)(ux * ux), (float)(uy * uy));
+    }
+    // Phasors (c, s) of one ray record and the first-order factors ex, ey. The
+    // B row's phasor is W; ZZ: a second A phasor. AMP: the amplitude varies
+    // along the tile.
+    template <bool ZZ, bool AMP>
+    __device__ __forceinline__ void ray(float4 v0, float4 v1, float4 v2, float4 v3, bool col,
+                                        float& cx, float& sx, float& cy, float& sy, float& ex,
+                                        float& ey) const {
+        const float2 rh = ZZ ? f2(v0.x) : make_float2(v0.x, v0.y);
+        const float2 rl = ZZ ? f2(v0.z) : make_float2(v0.z, v0.w);
+        const float2 ab = ZZ ? f2(v1.x) : make_float2(v1.x, v1.y);
+        const float2 ds = __ffma2_rn(kh, ab, sq);    // dS, dT
+        const float2 qd = __fmul2_rn(f2(v1.w), ds);  // -q dS, -q dT
+        const float2 small = __ffma2_rn(qd, ds, __fmul2_rn(f2(v1.z), sq));
+        float2 p0 = __fadd2_rn(pp, small);
+        if (!ZZ) p0 = __fadd2_rn(p0, make_float2(0.f, v2.x));
+        const float2 t = pair_turns2(kh, khn, kl, p0, rh, rl);
+        const float2 th = __fmul2_rn(t, f2(6.28318530717958647692f));
+        __sincosf(th.x, &sx, &cx);
+        __sincosf(th.y, &sy, &cy);
+        ex = ds.x;
+        ey = ZZ ? ds.y : qd.y * 12.566370614359172f;
+        float2 f = f2(1.f);
+        if (AMP) {
+            const float2 sl = ZZ ? f2(v3.x) : make_float2(v3.x, v3.y);
+            f = __ffma2_rn(kh, sl, __ffma2_rn(f2(v2.w), ds, f2(1.f)));
+            cx *= f.x;
+            sx *= f.x;
+        }
+        if (ZZ) {
+            if (AMP) {
+                cy *= f.y;
+                sy *= f.y;
+            }
+        } else {
+            const float wr0 = col ? v3.z : v2.y, wi0 = col ? v3.w : v2.z;
+            const float ar = AMP ? wr0 * f.y : wr0, ai = AMP ? wi0 * f.y : wi0;
+            const float co = cy, si = sy;
+            cy = cmul_re(ar, ai, co, si);  // W
+            sy = cmul_im(ar, ai, co, si);
+        }
+    }
+};
+
+// (c, s) of two rays -> f16 hi, lo and hi times the factors (e0, e1).
+__device__ __forceinline__ void split_pair(const float (&c)[2], const float (&s)[2], float e0,
+                                           float e1, uint32_t* h, uint32_t* l, uint32_t* e,
+                                           int re, int im) {
+    split16x2(c[0], c[1], &h[re], &l[re]);
+    split16x2(s[0], s[1], &h[im], &l[im]);
+    const uint32_t f = pack16x2(e0, e1);
+    e[re] = mul2(h[re], f);
+    e[im] = mul2(h[im], f);
+}
+
+// Producer warps of a CTA of the pair, narrow form. A warp fills 16-byte chunks
+// (four rays) of pair-rows: warp w < 8 chunk w of the pair-rows 0..63 (A rows with
+// the CTA's 64 columns), warps 8..11 (ZZ) two chunks each of the pair-rows
+// (64 + r, 96 + r) of A alone. Inside a chunk the contraction runs (re j, re j+1,
+// im j, im j+1) over ray pairs, in both operands, so that the real-part and
+// imaginary-part rows of B hold the same words in another order (and one sign).
+// Rows and columns past the screen's edge hold the phasors of the tile's
+// reference point: they only reach accumulators nobody reads.
 template <bool ZZ, bool AMP>
 __device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int r, int mt, int nt,
-                                              int col, uint32_t half, int nrb, unsigned char* tiles,
-                                              uint32_t full_lead, uint64_t* empty,
-                                              uint64_t* ray_full, uint64_t* ray_empty,
-                                              unsigned char* rays_smem, volatile int* flag) {
+                                              int col, uint32_t half, int nrb,
+                                              unsigned char* tiles, uint32_t full_lead,
+                                              uint64_t* empty, uint64_t* ray_full,
+                                              uint64_t* ray_empty, unsigned char* rays_smem,
+                                              volatile int* flag) {
     using namespace sm100;
     constexpr int NE = ZZ ? 1 : 2;   // pair-rows per thread
     constexpr int NCH = ZZ ? 2 : 1;  // chunks per thread
-    float2 kh2[NE], khn2[NE], kl2[NE], pp2[NE], sq2[NE];
+    PairRow row[NE];
     const double ref_m = g.refs[mt >> 1], ref_n = g.refs[g.m_tiles + nt];
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
@@ -273,18 +363,11 @@ __device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int 
             const size_t in = (size_t)nt * 128 + 64 * half + r + 32 * e;
             uy = in < g.nn ? g.cn[in] - ref_n : 0.0;
         }
-        float hx, lx, hy, ly, fx, fy;
-        split_coord(ux, g.h0, &hx, &lx, &fx);
-        split_coord(uy, g.h0, &hy, &ly, &fy);
-        kh2[e] = make_float2(hx, hy);
-        khn2[e] = make_float2(-hx, -hy);
-        kl2[e] = make_float2(lx, ly);
-        pp2[e] = make_float2(fx, fy);
-        sq2[e] = make_float2((float)(ux * ux), (float)(uy * uy));
+        row[e].set(ux, uy, g.h0);
     }
     for (int i = 0; i < nrb; ++i) {
-        const int s = i % kGStages, rb = i % kFRayBufs;
-        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kFRayBufs) & 1u, g.wait_limit);
+        const int s = i % kGStages, rb = i % kGRayBufs;
+        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kGRayBufs) & 1u, g.wait_limit);
         ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kGStages) & 1u) ^ 1u, g.wait_limit);
         if (!__all_sync(0xffffffffu, ok)) {
             *flag = 1;
@@ -306,84 +389,42 @@ __device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int 
                     const float4 v0 = rec[0], v1 = rec[1], v2 = rec[2];
                     float4 v3 = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (AMP || (!ZZ && col)) v3 = rec[3];
-                    const float2 rh = ZZ ? f2(v0.x) : make_float2(v0.x, v0.y);
-                    const float2 rl = ZZ ? f2(v0.z) : make_float2(v0.z, v0.w);
-                    const float2 ab = ZZ ? f2(v1.x) : make_float2(v1.x, v1.y);
-                    const float wr0 = col ? v3.z : v2.y, wi0 = col ? v3.w : v2.z;
 #pragma unroll
-                    for (int e = 0; e < NE; ++e) {
-                        const float2 ds = __ffma2_rn(kh2[e], ab, sq2[e]);  // dS, dT
-                        const float2 qd = __fmul2_rn(f2(v1.w), ds);        // -q dS, -q dT
-                        const float2 small = __ffma2_rn(qd, ds, __fmul2_rn(f2(v1.z), sq2[e]));
-                        float2 p0 = __fadd2_rn(pp2[e], small);
-                        if (!ZZ) p0 = __fadd2_rn(p0, make_float2(0.f, v2.x));
-                        const float2 t = pair_turns2(kh2[e], khn2[e], kl2[e], p0, rh, rl);
-                        const float2 th = __fmul2_rn(t, f2(6.28318530717958647692f));
-                        __sincosf(th.x, &sx[e][u], &cx[e][u]);
-                        __sincosf(th.y, &sy[e][u], &cy[e][u]);
-                        ex[e][u] = ds.x;
-                        ey[e][u] = ZZ ? ds.y : qd.y * 12.566370614359172f;
-                        float2 f = f2(1.f);
-                        if (AMP) {
-                            const float2 sl = ZZ ? f2(v3.x) : make_float2(v3.x, v3.y);
-                            f = __ffma2_rn(kh2[e], sl, __ffma2_rn(f2(v2.w), ds, f2(1.f)));
-                            cx[e][u] *= f.x;
-                            sx[e][u] *= f.x;
-                        }
-                        if (ZZ) {
-                            if (AMP) {
-                                cy[e][u] *= f.y;
-                                sy[e][u] *= f.y;
-                            }
-                        } else {
-                            const float ar = AMP ? wr0 * f.y : wr0, ai = AMP ? wi0 * f.y : wi0;
-                            const float co = cy[e][u], si = sy[e][u];
-                            cy[e][u] = cmul_re(ar, ai, co, si);  // W
-                            sy[e][u] = cmul_im(ar, ai, co, si);
-                        }
-                    }
+                    for (int e = 0; e < NE; ++e)
+                        row[e].template ray<ZZ, AMP>(v0, v1, v2, v3, col, cx[e][u], sx[e][u],
+                                                     cy[e][u], sy[e][u], ex[e][u], ey[e][u]);
                 }
 #pragma unroll
                 for (int e = 0; e < NE; ++e) {
                     const int k = 2 * pr;
-                    split16x2(cx[e][0], cx[e][1], &ah[e][k], &al[e][k]);
-                    split16x2(sx[e][0], sx[e][1], &ah[e][k + 1], &al[e][k + 1]);
-                    const uint32_t fx = pack16x2(ex[e][0], ex[e][1]);
-                    const uint32_t fy = pack16x2(ey[e][0], ey[e][1]);
-                    ae[e][k] = mul2(ah[e][k], fx);
-                    ae[e][k + 1] = mul2(ah[e][k + 1], fx);
-                    uint32_t(&h)[4] = ZZ ? ah[1] : bh[e];
-                    uint32_t(&l)[4] = ZZ ? al[1] : bl[e];
-                    uint32_t(&o)[4] = ZZ ? ae[1] : be[e];
-                    split16x2(cy[e][0], cy[e][1], &h[k], &l[k]);
-                    split16x2(sy[e][0], sy[e][1], &h[k + 1], &l[k + 1]);
-                    o[k] = mul2(h[k], fy);
-                    o[k + 1] = mul2(h[k + 1], fy);
+                    split_pair(cx[e], sx[e], ex[e][0], ex[e][1], ah[e], al[e], ae[e], k, k + 1);
+                    split_pair(cy[e], sy[e], ey[e][0], ey[e][1], ZZ ? ah[1] : bh[e],
+                               ZZ ? al[1] : bl[e], ZZ ? ae[1] : be[e], k, k + 1);
                 }
             }
-            auto put = [&](uint32_t tile, uint32_t row, uint32_t a, uint32_t b, uint32_t d,
-                           uint32_t e) {
-                *reinterpret_cast<uint4*>(base + tile * kGA + sw128(row, c)) = make_uint4(a, b, d, e);
+            auto put = [&](int tile, uint32_t row, uint32_t a, uint32_t b, uint32_t d, uint32_t e) {
+                *reinterpret_cast<uint4*>(base + tile * kGA + sw128(row, c)) =
+                    make_uint4(a, b, d, e);
             };
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const uint32_t row = (uint32_t)(ZZ ? 64 + r + 32 * k : r + 32 * k);
+                const uint32_t row = (uint32_t)((ZZ ? 64 : 0) + r + 32 * k);
                 put(0, row, ah[k][0], ah[k][1], ah[k][2], ah[k][3]);
                 put(1, row, al[k][0], al[k][1], al[k][2], al[k][3]);
-                put(4, row, ae[k][0], ae[k][1], ae[k][2], ae[k][3]);
+                put(2, row, ae[k][0], ae[k][1], ae[k][2], ae[k][3]);
             }
             if (!ZZ) {
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    // Point r + 32 k: (Re W, -Im W) in row r + 32 k, (Im W,
-                    // Re W) in row 64 + r + 32 k; and the same of i E W, whose
-                    // real part is -E Im W (be holds E Re W, E Im W).
+                    // Point j: (Re W, -Im W) in row j, (Im W, Re W) in row 64 + j;
+                    // and the same of i E W, whose real part is -E Im W (be
+                    // holds E Re W, E Im W).
                     const uint32_t row = (uint32_t)(r + 32 * k);
                     const uint32_t(&h)[4] = bh[k], (&l)[4] = bl[k], (&o)[4] = be[k];
-                    put(2, row, h[0], neg2(h[1]), h[2], neg2(h[3]));
-                    put(2, 64 + row, h[1], h[0], h[3], h[2]);
-                    put(3, row, l[0], neg2(l[1]), l[2], neg2(l[3]));
-                    put(3, 64 + row, l[1], l[0], l[3], l[2]);
+                    put(3, row, h[0], neg2(h[1]), h[2], neg2(h[3]));
+                    put(3, 64 + row, h[1], h[0], h[3], h[2]);
+                    put(4, row, l[0], neg2(l[1]), l[2], neg2(l[3]));
+                    put(4, 64 + row, l[1], l[0], l[3], l[2]);
                     const uint32_t n1 = neg2(o[1]), n3 = neg2(o[3]);
                     put(5, row, n1, neg2(o[0]), n3, neg2(o[2]));
                     put(5, 64 + row, o[0], n1, o[2], n3);
@@ -401,74 +442,195 @@ __device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int 
     }
 }
 
+// Producer warps of the wide form: warp w takes rays 8 (w % 4) .. + 7 of the
+// stage for the pair-rows 64 (w / 4) .. + 63 (A row and column of the same
+// number). Lanes r and r + 8 hold the same pair-row and four rays each, so that
+// 16 lanes' 8-byte stores cover eight rows' 16-byte words: no bank conflicts, and
+// a record is read once for eight rays x 16 lanes.
+template <bool AMP>
+__device__ __forceinline__ void grid_producer_wide(const ProductArgs& g, int w, int lane, int mt,
+                                                   int nt, int col, uint32_t half, int nrb,
+                                                   unsigned char* tiles, uint32_t full_lead,
+                                                   uint64_t* empty, uint64_t* ray_full,
+                                                   uint64_t* ray_empty, unsigned char* rays_smem,
+                                                   volatile int* flag) {
+    using namespace sm100;
+    constexpr int NE = 2;  // pair-rows at a time (1: 6.68, 2: 6.50, 4: 7.85 ms)
+    const int sub = (lane >> 3) & 1, oct = w & 3;
+    const int row0 = 64 * (w >> 2) + (lane & 7) + ((lane & 16) >> 1);  // + 16 e
+    PairRow row[4];
+    const double ref_m = g.refs[mt >> 1], ref_n = g.refs[g.m_tiles + nt];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const size_t im = (size_t)mt * 128 + row0 + 16 * e;
+        const size_t in = (size_t)nt * 256 + 128 * half + row0 + 16 * e;
+        row[e].set(im < g.nm ? g.cm[im] - ref_m : 0.0, in < g.nn ? g.cn[in] - ref_n : 0.0, g.h0);
+    }
+    // This thread's 8 bytes of the real and the imaginary 16-byte word of row 0.
+    const uint32_t at_re = sw128(row0, oct) + 8 * sub, at_im = sw128(row0, 4 + oct) + 8 * sub;
+    for (int i = 0; i < nrb; ++i) {
+        const int s = i % kGStages, rb = i % kGRayBufs;
+        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kGRayBufs) & 1u, g.wait_limit);
+        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kGStages) & 1u) ^ 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *flag = 1;
+            return;
+        }
+        unsigned char* base = tiles + (size_t)s * kGStage;
+        const float4* sr =
+            reinterpret_cast<const float4*>(rays_smem + rb * kGRayBytes) + 4 * (8 * oct + 4 * sub);
+#pragma unroll
+        for (int e0 = 0; e0 < 4; e0 += NE) {
+            uint32_t ah[NE][4], al[NE][4], ae[NE][4];  // re, re, im, im
+            uint32_t bh[NE][4], bl[NE][4], be[NE][4];
+#pragma unroll
+            for (int pr = 0; pr < 2; ++pr) {
+                float cx[NE][2], sx[NE][2], cy[NE][2], sy[NE][2], ex[NE][2], ey[NE][2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float4* rec = sr + 4 * (2 * pr + u);
+                    const float4 v0 = rec[0], v1 = rec[1], v2 = rec[2];
+                    float4 v3 = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (AMP || col) v3 = rec[3];
+#pragma unroll
+                    for (int e = 0; e < NE; ++e)
+                        row[e0 + e].template ray<false, AMP>(v0, v1, v2, v3, col, cx[e][u],
+                                                             sx[e][u], cy[e][u], sy[e][u],
+                                                             ex[e][u], ey[e][u]);
+                }
+#pragma unroll
+                for (int e = 0; e < NE; ++e) {
+                    split_pair(cx[e], sx[e], ex[e][0], ex[e][1], ah[e], al[e], ae[e], pr, 2 + pr);
+                    split_pair(cy[e], sy[e], ey[e][0], ey[e][1], bh[e], bl[e], be[e], pr, 2 + pr);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+                auto put = [&](int tile, const uint32_t(&v)[4]) {
+                    unsigned char* o = base + tile * kGA + 16 * 128 * (e0 + e);
+                    *reinterpret_cast<uint2*>(o + at_re) = make_uint2(v[0], v[1]);
+                    *reinterpret_cast<uint2*>(o + at_im) = make_uint2(v[2], v[3]);
+                };
+                put(0, ah[e]);
+                put(1, al[e]);
+                put(2, ae[e]);
+                put(3, bh[e]);
+                put(4, bl[e]);
+                put(5, be[e]);
+            }
+        }
+        // Make the generic-proxy stores visible to the tensor cores, then one
+        // arrival per warp on the even CTA's stage barrier.
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive_cluster(full_lead + 8u * (uint32_t)s);
+            mbar_arrive(&ray_empty[rb]);
+        }
+    }
+}
+
 // Epilogue role (warps 1..4): adds each finished accumulator segment to this
-// CTA's 128 rows of the split's partial. Lane l of warp w owns row
-// 32 (w % 4) + l: 32 columns at a time go from TMEM to the lane's 128-byte
-// staging row and from there to a bulk copy, a store for the split's first
-// segment and an FP32 add at the memory side (round to nearest) for the others.
-// A segment's operations complete before the next segment's start, so the
+// CTA's 128 rows of the split's partial. The partial is stored in contiguous
+// blocks of 32 rows x 16 columns (partial_at), so that 16 columns of a warp's 32
+// rows go from TMEM through 2 KB of staging to ONE bulk operation, a store for
+// the split's first segment and an FP32 add at the memory side (round to nearest)
+// for the others. (A 128-byte operation per row kept the bulk unit busy longer
+// than a short segment's products: 2^20 rays x 512^2 points took 32.8 ms with
+// segments of one block and 7.8 ms with ten, now 16.8 and 7.5 ms, narrow form.)
+// Each block's operations complete before its next segment's start, so the
 // partial is s0 + s1 + ... in segment order.
-__device__ __forceinline__ void grid_drain(const ProductArgs& g, int warp, int lane, int mt, int nt,
-                                           int sp, int nseg, uint32_t tmem, uint64_t* acc_full,
+template <bool WIDE>
+__device__ __forceinline__ void grid_drain(const ProductArgs& g, int warp, int lane, int mt,
+                                           int sp, int nrb, uint32_t tmem, uint64_t* acc_full,
                                            uint32_t acc_empty_lead, unsigned char* stage,
                                            volatile int* flag) {
     using namespace sm100;
+    using F = Form<WIDE>;
+    constexpr int kBlocks = kFN / 16, kBlock = 512;  // blocks per accumulator, floats
     const int qd = warp & 3;
-    float* row = g.partial + ((size_t)sp * g.m_pad + (size_t)mt * 128 + qd * 32 + lane) * g.n_pad +
-                 (size_t)nt * kFN;
-    if (nseg == 0) {
-        for (int c = 0; g.first && c < kFN; ++c) row[c] = 0.f;
+    float* row = g.partial + (((size_t)sp * (g.m_pad / 32) + (size_t)mt * 4 + qd) * (g.n_pad / 16) +
+                              (size_t)blockIdx.y * F::kAcc * kBlocks) * kBlock;
+    // Segments of the accumulators, as the MMA issuer counts them.
+    int drains = (nrb + g.seg - 1) / g.seg;
+    if (WIDE) drains += 1 + (max(0, nrb - max(1, g.seg / 2)) + g.seg - 1) / g.seg;
+    if (nrb == 0) {
+        for (int c = lane; g.first && c < F::kAcc * kBlocks * kBlock; c += 32) row[c] = 0.f;
         return;
     }
-    unsigned char* srow = stage + lane * kFEpiRow;
-    const uint32_t s_addr = smem_u32(srow);
-    for (int q = 0; q < nseg; ++q) {
-        const int b = q & 1;
+    int buf = 0;
+    for (int q = 0; q < drains; ++q) {
+        // Accumulator b's next segment; wide: the second one's ends first.
+        const int b = (q & 1) ^ (WIDE ? 1 : 0), seg = q / F::kAcc;
         const bool ok = mbar_wait(&acc_full[b], (uint32_t)(q >> 1) & 1u, g.wait_limit);
         if (!__all_sync(0xffffffffu, ok)) {
             *flag = 1;
             break;
         }
         tc_fence_after();
-        bulk_wait_all();  // the previous segment's writes to this row are performed
+        float* dst = row + (WIDE ? b * kBlocks * kBlock : 0);
 #pragma unroll 1
-        for (int c = 0; c < kFN / 32; ++c) {
+        for (int c = 0; c < kBlocks; c += 2) {
             float v[32];
-            tmem_ld_32cols(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(b * kFN + c * 32), v);
-            bulk_wait_read();  // the staging row is free again
+            tmem_ld_32cols(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(b * kFN + c * 16), v);
+            if (c == kBlocks - 2) {  // the accumulator is free again
+                tc_fence_before();
+                mbar_arrive_cluster(acc_empty_lead + 8u * (uint32_t)b);
+            }
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                reinterpret_cast<float4*>(srow)[k] =
-                    make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-            fence_proxy_async();
-            if (q == 0 && g.first)
-                bulk_s2g(row + c * 32, s_addr, 128);
-            else
-                bulk_add_s2g_f32(row + c * 32, s_addr, 128);
-            bulk_commit();
+            for (int h = 0; h < 2; ++h) {
+                if (lane == 0) bulk_wait_read_but<kGEpiBufs - 1>();  // the buffer is free again
+                __syncwarp();
+                unsigned char* sb = stage + buf * kDrainBytes;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float* w = v + 16 * h + 4 * k;
+                    reinterpret_cast<float4*>(sb + lane * 64)[k ^ ((lane >> 1) & 3)] =
+                        make_float4(w[0], w[1], w[2], w[3]);
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    // The previous segment's operation on this block is performed.
+                    bulk_wait_but<F::kAcc * kBlocks - 1>();
+                    float* to = dst + (c + h) * kBlock;
+                    if (seg == 0 && g.first)
+                        bulk_s2g(to, smem_u32(sb), kDrainBytes);
+                    else
+                        bulk_add_s2g_f32(to, smem_u32(sb), kDrainBytes);
+                    bulk_commit();
+                }
+                buf = buf + 1 == kGEpiBufs ? 0 : buf + 1;
+            }
         }
-        tc_fence_before();
-        mbar_arrive_cluster(acc_empty_lead + 8u * (uint32_t)b);
     }
     bulk_wait_all();
 }
 
-template <bool AMP>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
+// Element (row, column) of a split's partial: blocks of 32 x 16, the 16-byte
+// words of a block's row permuted by the row (conflict-free staging writes).
+__device__ __forceinline__ size_t partial_at(size_t im, size_t x, int n_pad) {
+    const size_t r = im & 31, k = (x & 15) ^ (((r >> 1) & 3) << 2);
+    return ((im >> 5) * (size_t)(n_pad >> 4) + (x >> 4)) * 512 + r * 16 + k;
+}
+
+template <bool AMP, bool WIDE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads, 1)
     grid_product_kernel(ProductArgs g) {
     using namespace sm100;
+    using F = Form<WIDE>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     unsigned char* rays_smem = tiles + kGStages * kGStage;
-    unsigned char* epi_smem = rays_smem + kFRayBufs * kGRayBytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(epi_smem + kFEpiBytes);
+    unsigned char* epi_smem = rays_smem + kGRayBufs * kGRayBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(epi_smem + 4 * kGEpiBufs * kDrainBytes);
     uint64_t* empty = full + kGStages;
     uint64_t* acc_full = empty + kGStages;
     uint64_t* acc_empty = acc_full + 2;
     uint64_t* ray_full = acc_empty + 2;
-    uint64_t* ray_empty = ray_full + kFRayBufs;
-    uint64_t* mma_done = ray_empty + kFRayBufs;  // every issued MMA has completed
+    uint64_t* ray_empty = ray_full + kGRayBufs;
+    uint64_t* mma_done = ray_empty + kGRayBufs;  // every issued MMA has completed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
     volatile int* flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -480,22 +642,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
     const int rb0 = (int)((long long)g.ray_blocks * sp / g.splits);
     const int rb1 = (int)((long long)g.ray_blocks * (sp + 1) / g.splits);
     const int nrb = rb1 - rb0;
-    const int nseg = (nrb + g.seg - 1) / g.seg;
 
     if (threadIdx.x == 0) {
         // full and acc_empty are used in the even CTA only: they collect the
         // arrivals of both CTAs' producer and epilogue warps.
         for (int s = 0; s < kGStages; ++s) {
-            mbar_init(&full[s], 2 * kGProdThreads / 32 + (s == 0 ? g.stall : 0u));
+            mbar_init(&full[s], 2 * F::kProdWarps + (s == 0 ? g.stall : 0u));
             mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 2 * kFEpiThreads);
         }
-        for (int b = 0; b < kFRayBufs; ++b) {
+        for (int b = 0; b < kGRayBufs; ++b) {
             mbar_init(&ray_full[b], 1);
-            mbar_init(&ray_empty[b], kGProdThreads / 32);
+            mbar_init(&ray_empty[b], F::kProdWarps);
         }
         mbar_init(mma_done, 1);
         mbar_init_fence();
@@ -509,44 +670,70 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
 
     if (warp == 0) {
         if (leader && lane == 0) {
-            // Pair MMA issuer: per ray block the three products of the split
-            // phasors and the first-order one, four 256x256x16 steps each;
-            // segment q accumulates into buffer q & 1 of both CTAs' TMEM.
+            // Pair MMA issuer: per stage the first-order product and the three
+            // of the split phasors, 256x256x16 steps, in two parts of a segment
+            // (wide: h = 0 the real, 1 the imaginary part of the field).
             constexpr uint32_t idesc = idesc_f16_f32(256, kFN);
             bool good = true;
-            for (int q = 0; q < nseg && good; ++q) {
-                const int b = q & 1, use = q >> 1;
+            auto wait_acc = [&](int b, int use) {  // use: earlier segments of buffer b
                 if (use >= 1 &&
                     !mbar_wait_cluster(&acc_empty[b], (uint32_t)(use - 1) & 1u, g.wait_limit)) {
+                    *flag = 1;
+                    good = false;
+                }
+                tc_fence_after();
+            };
+            // Ends of the accumulators' segments; a wide tile's second one ends its
+            // own half a segment earlier. A part is issued first in its segment's
+            // last stage and last in the next stage, so that the other part's
+            // products of both stages run while it is drained.
+            int end0 = min(nrb, g.seg), end1 = min(nrb, max(1, g.seg / 2)), q0 = 0, q1 = 0;
+            bool new0 = true, new1 = true;
+            for (int i = 0; i < nrb && good; ++i) {
+                const int s = i % kGStages;
+                if (!mbar_wait_cluster(&full[s], (uint32_t)(i / kGStages) & 1u, g.wait_limit)) {
                     *flag = 1;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(b * kFN);
-                const int i0 = q * g.seg, i1 = min(nrb, i0 + g.seg);
-                for (int i = i0; i < i1; ++i) {
-                    const int s = i % kGStages;
-                    if (!mbar_wait_cluster(&full[s], (uint32_t)(i / kGStages) & 1u, g.wait_limit)) {
-                        *flag = 1;
-                        good = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t t0 = smem_u32(tiles + (size_t)s * kGStage);
-                    const uint32_t as[4] = {t0 + 4 * kGA, t0, t0, t0 + kGA};
-                    const uint32_t bs[4] = {t0 + 5 * kGA, t0 + 2 * kGA, t0 + 3 * kGA, t0 + 2 * kGA};
+                const uint32_t t0 = smem_u32(tiles) + (uint32_t)s * kGStage;
+                const uint32_t as[4] = {t0 + 2 * kGA, t0, t0, t0 + kGA};
+                const uint32_t bs[4] = {t0 + 5 * kGA, t0 + 3 * kGA, t0 + 4 * kGA, t0 + 3 * kGA};
+                const int first = WIDE && ((new0 && i > 0) || i + 1 == end1);
+                for (int h = first, t = 0; t < F::kAcc; ++t, h ^= 1) {
+                    const bool fresh = h ? new1 : new0;
+                    const int q = h ? q1 : q0, b = WIDE ? h : (q & 1);
+                    if (fresh) wait_acc(b, WIDE ? q : q >> 1);
+                    if (!good) break;
+                    const uint32_t d = tmem + (uint32_t)(b * kFN);
 #pragma unroll
                     for (int p = 0; p < 4; ++p)
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)
+                        for (int k = 0; k < 4; ++k) {
+                            // Wide: A's real (k < 2) or imaginary parts meet B's
+                            // of the same kind, subtracted for the imaginary
+                            // ones, or (h) of the other kind; of i E W (p == 0),
+                            // stored as E W, the other way round.
+                            const int x = k >> 1;
+                            const bool swap = WIDE && (h ^ (p == 0));
+                            const bool neg =
+                                WIDE && (p == 0 ? (h == 0 || x == 1) : (h == 0 && x == 1));
                             umma_f16_pair(d, desc_kmajor_sw128(as[p] + 32u * k),
-                                          desc_kmajor_sw128(bs[p] + 32u * k), idesc,
-                                          (uint32_t)((i - i0) | p | k));
-                    umma_commit_pair(smem_u32(&empty[s]));
-                    umma_commit_pair(mapa_shared(&empty[s], peer));
+                                          desc_kmajor_sw128(bs[p] + 32u * (swap ? k ^ 2 : k)),
+                                          neg ? idesc | kNegateB : idesc,
+                                          (uint32_t)(!fresh | p | k));
+                        }
+                    const bool last = i + 1 == (h ? end1 : end0);
+                    if (last) {
+                        umma_commit_pair(smem_u32(&acc_full[b]));
+                        umma_commit_pair(mapa_shared(&acc_full[b], peer));
+                    }
+                    (h ? new1 : new0) = last;
+                    (h ? q1 : q0) += last;
+                    (h ? end1 : end0) = last ? min(nrb, i + 1 + g.seg) : (h ? end1 : end0);
                 }
-                umma_commit_pair(smem_u32(&acc_full[b]));
-                umma_commit_pair(mapa_shared(&acc_full[b], peer));
+                umma_commit_pair(smem_u32(&empty[s]));
+                umma_commit_pair(mapa_shared(&empty[s], peer));
             }
             // A loop that gave up on a wait may leave MMAs in flight: wait
             // (bounded) for them before either CTA frees its accumulators.
@@ -555,26 +742,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
         }
         __syncwarp();
     } else if (warp <= 4) {
-        grid_drain(g, warp, lane, mt, (int)blockIdx.y, sp, nseg, tmem, acc_full,
-                   mapa_shared(acc_empty, 0), epi_smem + (warp - 1) * 32 * kFEpiRow, flag);
-    } else if (warp < 5 + kGProdThreads / 32) {
+        grid_drain<WIDE>(g, warp, lane, mt, sp, nrb, tmem, acc_full, mapa_shared(acc_empty, 0),
+                         epi_smem + (warp - 1) * kGEpiBufs * kDrainBytes, flag);
+    } else if (warp < 5 + F::kProdWarps) {
         const int w = warp - 5;
         const uint32_t full_lead = mapa_shared(full, 0);
-        if (w < 8)
+        if constexpr (WIDE)
+            grid_producer_wide<AMP>(g, w, lane, mt, nt, col, half, nrb, tiles, full_lead, empty,
+                                    ray_full, ray_empty, rays_smem, flag);
+        else if (w < 8)
             grid_producer<false, AMP>(g, w, lane, mt, nt, col, half, nrb, tiles, full_lead, empty,
                                       ray_full, ray_empty, rays_smem, flag);
         else
             grid_producer<true, AMP>(g, 2 * (w - 8), lane, mt, nt, col, half, nrb, tiles, full_lead,
                                      empty, ray_full, ray_empty, rays_smem, flag);
     } else if (lane == 0) {
-        // Ray stager: one bulk copy of 32 records per block.
+        // Ray stager: one bulk copy of a stage's records.
         const float4* src =
             g.recs + ((size_t)((mt >> 1) * g.n_tiles + nt) * g.pad + (size_t)rb0 * kFRays) * 4;
         int i = 0;
         for (; i < nrb; ++i) {
-            const int rb = i % kFRayBufs;
-            if (i >= kFRayBufs &&
-                !mbar_wait(&ray_empty[rb], (uint32_t)(i / kFRayBufs - 1) & 1u, g.wait_limit)) {
+            const int rb = i % kGRayBufs;
+            if (i >= kGRayBufs &&
+                !mbar_wait(&ray_empty[rb], (uint32_t)(i / kGRayBufs - 1) & 1u, g.wait_limit)) {
                 *flag = 1;
                 break;
             }
@@ -584,8 +774,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
         }
         // No copy may still be writing into this CTA's shared memory when it
         // exits: the last ones land whether or not a producer waits for them.
-        for (int k = max(0, i - kFRayBufs); k < i; ++k)
-            if (!mbar_wait(&ray_full[k % kFRayBufs], (uint32_t)(k / kFRayBufs) & 1u,
+        for (int k = max(0, i - kGRayBufs); k < i; ++k)
+            if (!mbar_wait(&ray_full[k % kGRayBufs], (uint32_t)(k / kGRayBufs) & 1u,
                            max(g.wait_limit, kMmaDrainPolls)))
                 *flag = 1;
     }
@@ -604,20 +794,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGThreads, 1)
 // Threads run along the columns, which are consecutive in the partials.
 __global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restrict__ partial,
                                                           int splits, int m_pad, int n_pad,
-                                                          int n_tiles, int columns, size_t nm,
+                                                          int columns, bool wide, size_t nm,
                                                           size_t nn, bool rows_outer, double scale,
                                                           double2 pes, double2 pep, FieldDev out) {
     const size_t idx = blockIdx.x * (size_t)256 + threadIdx.x;
     if (idx >= nm * nn) return;
     const size_t im = idx / nn, in = idx - im * nn;
-    const size_t loc = in & 127, at = (in >> 7) * kFN + 128 * (loc >> 6) + (loc & 63);
+    // Column of the real part; the imaginary part's is 256 (wide) or 64 further.
+    const size_t at = wide ? (in >> 8) * 512 + (in & 255)
+                           : (in >> 7) * 256 + 128 * ((in >> 6) & 1) + (in & 63);
+    const int im_off = (wide ? 256 : 64) / 16 * 512;
     double re[2] = {0.0, 0.0}, ie[2] = {0.0, 0.0};
     for (int c = 0; c < columns; ++c)
         for (int s = 0; s < splits; ++s) {
-            const float* row =
-                partial + ((size_t)s * m_pad + im) * n_pad + (size_t)c * n_tiles * kFN + at;
-            re[c] += row[0];
-            ie[c] += row[64];
+            const float* e = partial + partial_at((size_t)s * m_pad + im,
+                                                  (size_t)c * (n_pad / columns) + at, n_pad);
+            re[c] += e[0];
+            ie[c] += e[im_off];
         }
     // times i
     for (int c = 0; c < 2; ++c) {
@@ -704,15 +897,16 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     if (!(obl.lo > 0.0 || obl.hi < 0.0)) return false;
     const double omin = std::min(std::fabs(obl.lo), std::fabs(obl.hi)), omax = largest(obl);
 
-    // Rows along the outer or the inner axis, whichever pads less (then
-    // whichever leaves the smaller first-order phase).
+    // Form, and rows along the outer or the inner axis: whichever costs less
+    // (then whichever leaves the smaller first-order phase).
     bool found = false;
     double best_area = 0.0, best_e = 0.0;
-    for (int swap = 0; swap < 2; ++swap) {
+    for (int form = 0; form < 4; ++form) {
+        const bool swap = form & 1, wide = form & 2;
         const int am = swap ? inner : outer, an = swap ? outer : inner;
         const size_t nm = swap ? len : rows, nn = swap ? rows : len;
         const double em = bits_to_double(probe.extent[swap ? 1 : 0][1]);  // 256-point tiles
-        const double en = bits_to_double(probe.extent[swap ? 0 : 1][0]);  // 128-point tiles
+        const double en = bits_to_double(probe.extent[swap ? 0 : 1][wide]);  // 128 or 256
         // |dS| = |u| |(p - r) + (p0 - r)| with |p0 - r| <= |p - r|max - |u|max
         // when the tile lies inside the screen's range.
         const double pm = largest(del[am]), pn = largest(del[an]);
@@ -737,9 +931,12 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         if (!(sm <= 0.25 && sn <= 0.25 && sm * sn <= 1e-6 && (sm + sn) * mq <= 1e-6 &&
               mq * mq <= 1e-7))
             continue;
-        const size_t mt = blocks_of(nm, kTileM), nt = blocks_of(nn, kTileN);
+        const int tile_n = wide ? Form<true>::kTileN : Form<false>::kTileN;
+        const size_t mt = blocks_of(nm, kTileM), nt = blocks_of(nn, tile_n);
         if (mt * nt > kGridMaxTiles) continue;
-        const double area = (double)mt * kTileM * (double)nt * kTileN;
+        // Cost: the padded area, at 0.85 for the wide form (6.3 to 7.5 ms on 512 x
+        // 512 points, 0.48 to 0.55 on 256 x 256): it is taken unless it pads more.
+        const double area = (double)mt * kTileM * (double)nt * tile_n * (wide ? 0.85 : 1.0);
         if (found && !(area < best_area || (area == best_area && e < best_e))) continue;
         found = true;
         best_area = area;
@@ -750,6 +947,7 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         g->rows_outer = swap == 0;
         g->nm = nm;
         g->nn = nn;
+        g->wide = wide;
         g->m_tiles = (int)mt;
         g->n_tiles = (int)nt;
         g->e_bound = e;
@@ -802,7 +1000,7 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     // Blocks per segment. The tensor cores truncate when they accumulate, 16 MMAs
     // per block: on top of 3.5e-7 (sine and cosine of both factors) the error
     // against 64 bits is 4.7e-7, 6.5e-7, 8.3e-7 and 2.4e-6 of the field at 1, 2,
-    // 3 and 10 blocks (32.8, 17.6, 12.5 and 7.6 ms on 2^20 rays x 512^2 points).
+    // 3 and 10 blocks (14.9, 8.6, 7.7 and 6.3 ms on 2^20 rays x 512^2 points).
     // The persistent kernel's error grows with its FP32 residual phases, whose
     // mean over the whole ray set is about
     //     phase = k (rho^2 + 2 v rho) / (2 d),
@@ -822,7 +1020,7 @@ Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream) {
     const size_t sm = g.rows_outer ? g.inner_len : 1, sn = g.rows_outer ? 1 : g.inner_len;
     grid_axes_kernel<<<g.m_tiles + g.n_tiles, kTileM, 0, stream>>>(
         coord_host(g.pix, g.m_axis), sm, (int)g.nm, g.m_tiles, coord_host(g.pix, g.n_axis), sn,
-        (int)g.nn, g.axes);
+        (int)g.nn, g.wide ? 256 : 128, g.axes);
     XK_CUDA_TRY(cudaGetLastError());
     return Status::Ok();
 }
@@ -830,8 +1028,8 @@ Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream) {
 Status grid_reserve(const GridPlan& g, GridWorkspace& ws) {
     const size_t tiles = (size_t)g.m_tiles * g.n_tiles;
     XK_TRY(ws.recs.ensure(tiles * g.chunk_rays * 64));
-    XK_TRY(ws.partial.ensure((size_t)g.splits * g.m_tiles * kTileM * g.n_tiles * g.columns * kFN *
-                             sizeof(float)));
+    XK_TRY(ws.partial.ensure((size_t)g.splits * g.m_tiles * kTileM * g.n_tiles * g.columns *
+                             (g.wide ? 2 : 1) * kFN * sizeof(float)));
     return Status::Ok();
 }
 
@@ -855,11 +1053,15 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
     p.h0 = g.h0;
     p.partial = ws.partial.as<float>();
     p.m_pad = g.m_tiles * kTileM;
-    p.n_pad = g.n_tiles * g.columns * kFN;
+    p.n_pad = g.n_tiles * g.columns * (g.wide ? 2 : 1) * kFN;
     p.err = err;
     p.wait_limit = wait_limit;
     p.stall = stall ? 1 : 0;
-    const auto kern = g.amp ? grid_product_kernel<true> : grid_product_kernel<false>;
+    const auto kern = g.wide ? (g.amp ? grid_product_kernel<true, true>
+                                      : grid_product_kernel<false, true>)
+                             : (g.amp ? grid_product_kernel<true, false>
+                                      : grid_product_kernel<false, false>);
+    const int threads = g.wide ? Form<true>::kThreads : Form<false>::kThreads;
     // Set on every call: the attribute belongs to the current device's context.
     XK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem));
     const dim3 grid((unsigned)(2 * g.m_tiles), (unsigned)(g.n_tiles * g.columns),
@@ -897,13 +1099,13 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         p.pad = pad;
         p.ray_blocks = (int)(pad / kFRays);
         p.first = j0 == 0;
-        kern<<<grid, kGThreads, kGSmem, stream>>>(p);
+        kern<<<grid, threads, kGSmem, stream>>>(p);
         XK_CUDA_TRY(cudaGetLastError());
         p.stall = 0;
         *kernels += 2;
     }
     grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
-        p.partial, g.splits, p.m_pad, p.n_pad, g.n_tiles, g.columns, g.nm, g.nn, g.rows_outer,
+        p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.nm, g.nn, g.rows_outer,
         g.k / (4.0 * 3.14159265358979323846) / g.inv_scale, make_double2(g.pes[0], g.pes[1]),
         make_double2(g.pep[0], g.pep[1]), g.out);
     XK_CUDA_TRY(cudaGetLastError());

@@ -37,7 +37,8 @@ struct GridPlan {
     bool rows_outer = true;                  // rows are the outer screen axis
     size_t nm = 0, nn = 0;                   // rows, columns (screen points along the axes)
     size_t inner_len = 0;
-    int m_tiles = 0, n_tiles = 0, columns = 1;  // 256-row tiles, 128-point tiles, amplitude columns
+    bool wide = false;                       // 256 columns per tile instead of 128
+    int m_tiles = 0, n_tiles = 0, columns = 1;  // tiles of 256 rows and 128 or 256 columns; amplitude columns
     int ray_blocks = 0, splits = 1, seg = 0;
     size_t n = 0, chunk_rays = 0;            // rays, rays per product launch
     bool amp = false;                        // amplitude varies along a tile

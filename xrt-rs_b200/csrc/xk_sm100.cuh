@@ -123,6 +123,8 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int m, int n) {
            | ((uint32_t)(m >> 4) << 24);// M / 16
 }
 
+constexpr uint32_t kNegateB = 1u << 14;  // instruction descriptor: -B in place of B
+
 // One thread: D[tmem] (+)= A[adesc] * B[bdesc]^T.
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, uint32_t accumulate) {
@@ -211,6 +213,16 @@ __device__ __forceinline__ void bulk_commit() {
 // This thread's committed bulk operations have read their shared-memory source.
 __device__ __forceinline__ void bulk_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
+// The same, or completed, for all but this thread's N latest groups.
+template <int N>
+__device__ __forceinline__ void bulk_wait_read_but() {
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_but() {
+    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // This thread's committed bulk operations have completed (their global writes
