@@ -727,8 +727,332 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
     }
 }
 
-// acc[iz*nx + ix] (+)= scale * sum over splits of C[iz][n(ix, c)], in FP64 and
-// split order.
+// ---- CTA pairs on 256 x points --------------------------------------------------
+//
+// The wide form of the pair product, 256 z rows x 256 x points per cluster. A row
+// of either operand holds a block's 32 real parts, then its 32 imaginary parts, so
+// that one B row per x point serves both parts of the field (Re Z Re W - Im Z Im W
+// and Re Z Im W + Im Z Re W, the sign a bit of the instruction): half the stores
+// per point, and the A phasors serve twice the points. TMEM holds one accumulator
+// of 256 columns for the real and one for the imaginary part; a part is drained
+// while the other's products run. 2^20
+// rays x 512^2 points: 5.30 ms in the form above, 4.78 in this one, of which 0.5 are
+// waits for drains (4.28 with segments of 400 blocks; with four epilogue warps 5.16)
+// and 3.6 the tensor cores at the 1.55 GHz that the power limit leaves.
+constexpr int kWStages = 2;
+constexpr uint32_t kWStage = 4 * kPA;  // A_hi | A_lo | B_hi | B_lo, 128 rows each
+constexpr int kWEpiWarps = 8;          // warps 1..8, two per quarter of the TMEM lanes
+constexpr int kWProdWarps = 8;         // warps 9..16
+constexpr int kWThreads = 32 * (1 + kWEpiWarps + kWProdWarps + 1);
+constexpr int kWEpiBufs = 4;           // staging buffers per epilogue warp
+constexpr uint32_t kWDrainBytes = 32 * 8 * 8;  // 32 rows x 8 columns of the partial
+constexpr size_t kWSmem = 1024 + (size_t)kWStages * kWStage + kFRayBufs * kFRayBytes +
+                          kWEpiWarps * kWEpiBufs * kWDrainBytes + 256;
+static_assert(kWSmem <= 227 * 1024, "wide pair kernel shared memory");
+
+// Element (row, column) of the partials, stored in contiguous blocks of 32 rows x
+// 8 columns: one bulk operation drains a block. The 16-byte words of a block's row
+// are permuted by the row (conflict-free staging writes).
+__device__ __forceinline__ size_t wide_at(size_t row, size_t col, int n_pad) {
+    const size_t r = row & 31, c = (col & 7) ^ (((r >> 1) & 3) << 1);
+    return ((row >> 5) * (size_t)(n_pad >> 3) + (col >> 3)) * 256 + r * 8 + c;
+}
+
+// Producer warp w: rays 8 (w % 4) .. + 7 of the block for the z rows and x points
+// 64 (w / 4) .. + 63 (a row and a point of the same number in packed instructions).
+// Lanes r and r + 8 hold the same pair and four rays each, so that 16 lanes' 8-byte
+// stores cover eight rows' 16-byte words (no bank conflicts). Rows and points past
+// the screen's edge hold the phasors of its centre: they only reach accumulators
+// nobody reads.
+__device__ __forceinline__ void wide_producer(const FusedArgs& g, int w, int lane, int mt, int nt,
+                                              uint32_t half, int nrb, unsigned char* tiles,
+                                              uint32_t full_lead, uint64_t* empty,
+                                              uint64_t* ray_full, uint64_t* ray_empty,
+                                              unsigned char* rays_smem, volatile int* flag) {
+    using namespace sm100;
+    constexpr int NE = 2;  // pairs at a time
+    const int sub = (lane >> 3) & 1, oct = w & 3;
+    const int row0 = 64 * (w >> 2) + (lane & 7) + ((lane & 16) >> 1);  // + 16 e
+    float2 kh2[4], khn2[4], kl2[4], pp2[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const size_t iz = (size_t)mt * 128 + row0 + 16 * e;
+        const size_t ix = (size_t)nt * 256 + 128 * half + row0 + 16 * e;
+        const double uz = iz < g.nz ? g.zp[iz] - g.oz : 0.0;
+        const double ux = ix < g.nx ? g.xp[ix] - g.ox : 0.0;
+        float hz, lz, hx, lx, fz, fx, unused, h0, l0;
+        split_coord(-2.0 * g.a_turns * uz, 0.0, &hz, &lz, &unused);
+        split_coord(-2.0 * g.a_turns * ux, 0.0, &hx, &lx, &unused);
+        split_coord(uz, g.a_turns, &h0, &l0, &fz);
+        split_coord(ux, g.a_turns, &h0, &l0, &fx);
+        kh2[e] = make_float2(hz, hx);
+        khn2[e] = make_float2(-hz, -hx);
+        kl2[e] = make_float2(lz, lx);
+        pp2[e] = make_float2(fz, fx);
+    }
+    // This thread's 8 bytes of the real and the imaginary 16-byte word of row 0.
+    const uint32_t at_re = sw128(row0, oct) + 8 * sub, at_im = sw128(row0, 4 + oct) + 8 * sub;
+    for (int i = 0; i < nrb; ++i) {
+        const int s = i % kWStages, rb = i % kFRayBufs;
+        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kFRayBufs) & 1u, g.wait_limit);
+        ok = mbar_wait(&empty[s], ((uint32_t)(i / kWStages) & 1u) ^ 1u, g.wait_limit) && ok;
+        if (!ok) *flag = 1;
+        unsigned char* base = tiles + (size_t)s * kWStage;
+        const float4* sr =
+            reinterpret_cast<const float4*>(rays_smem + rb * kFRayBytes) + 2 * (8 * oct + 4 * sub);
+#pragma unroll
+        for (int e0 = 0; e0 < 4; e0 += NE) {
+            uint32_t ah[NE][4], al[NE][4], bh[NE][4], bl[NE][4];  // re, re, im, im
+#pragma unroll
+            for (int pr = 0; pr < 2; ++pr) {
+                float cz[NE][2], sz[NE][2], wr[NE][2], wi[NE][2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float4 v0 = sr[2 * (2 * pr + u)], v1 = sr[2 * (2 * pr + u) + 1];
+#pragma unroll
+                    for (int e = 0; e < NE; ++e) {
+                        const float2 t = pair_turns2(
+                            kh2[e0 + e], khn2[e0 + e], kl2[e0 + e],
+                            __fadd2_rn(pp2[e0 + e], make_float2(v1.x, v1.y)),
+                            make_float2(v0.x, v0.y), make_float2(v0.z, v0.w));
+                        const float2 th = __fmul2_rn(t, f2(6.28318530717958647692f));
+                        float sx, cx;
+                        __sincosf(th.x, &sz[e][u], &cz[e][u]);
+                        __sincosf(th.y, &sx, &cx);
+                        wr[e][u] = cmul_re(v1.z, v1.w, cx, sx);
+                        wi[e][u] = cmul_im(v1.z, v1.w, cx, sx);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < NE; ++e) {
+                    split16x2(cz[e][0], cz[e][1], &ah[e][pr], &al[e][pr]);
+                    split16x2(sz[e][0], sz[e][1], &ah[e][2 + pr], &al[e][2 + pr]);
+                    split16x2(wr[e][0], wr[e][1], &bh[e][pr], &bl[e][pr]);
+                    split16x2(wi[e][0], wi[e][1], &bh[e][2 + pr], &bl[e][2 + pr]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+                auto put = [&](int tile, const uint32_t(&v)[4]) {
+                    unsigned char* o = base + tile * kPA + 16 * 128 * (e0 + e);
+                    *reinterpret_cast<uint2*>(o + at_re) = make_uint2(v[0], v[1]);
+                    *reinterpret_cast<uint2*>(o + at_im) = make_uint2(v[2], v[3]);
+                };
+                put(0, ah[e]);
+                put(1, al[e]);
+                put(2, bh[e]);
+                put(3, bl[e]);
+            }
+        }
+        // Make the generic-proxy stores visible to the tensor cores, then one
+        // arrival per warp on the even CTA's stage barrier.
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive_cluster(full_lead + 8u * (uint32_t)s);
+            mbar_arrive(&ray_empty[rb]);
+        }
+    }
+}
+
+// The accumulators' segments (0 real, 1 imaginary) are kFSeg blocks, the imaginary
+// part's shifted by half a segment.
+constexpr int kWShift = kFSeg / 2;
+
+// Epilogue role (warps 1..8) of the wide form: as drain_role, in blocks of 32 rows
+// x 8 columns, the accumulators in turn (the imaginary part's segment ends first).
+__device__ __forceinline__ void wide_drain(const FusedArgs& g, int warp, int lane, int mt, int nt,
+                                           int sp, int nrb, uint32_t tmem, uint64_t* acc_full,
+                                           uint32_t acc_empty_lead, unsigned char* stage,
+                                           volatile int* flag) {
+    using namespace sm100;
+    // Blocks per accumulator and warp, doubles per block.
+    constexpr int kBlocks = kFN / 8 / (kWEpiWarps / 4), kBlock = 256;
+    const int col0 = (warp - 1) / 4 * (kBlocks * 8);
+    const int qd = warp & 3;
+    double* row = g.partial + (((size_t)sp * (g.m_pad / 32) + (size_t)mt * 4 + qd) * (g.n_pad / 8) +
+                               (size_t)nt * 2 * (kFN / 8) + col0 / 8) * kBlock;
+    if (nrb == 0) {
+        for (int c = lane; c < kBlocks * kBlock; c += 32) row[c] = row[kFN / 8 * kBlock + c] = 0.0;
+        return;
+    }
+    const int drains = (nrb + kFSeg - 1) / kFSeg + 1 + (max(0, nrb - kWShift) + kFSeg - 1) / kFSeg;
+    int buf = 0;
+    for (int q = 0; q < drains; ++q) {
+        const int b = (q & 1) ^ 1, seg = q >> 1;
+        const bool ok = mbar_wait(&acc_full[b], (uint32_t)seg & 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *flag = 1;
+            break;
+        }
+        tc_fence_after();
+        double* dst = row + b * (kFN / 8) * kBlock;
+#pragma unroll 1
+        for (int c = 0; c < kBlocks; c += 2) {
+            float v[16];
+            tmem_ld_16cols(tmem + ((uint32_t)(qd * 32) << 16) +
+                               (uint32_t)(b * kFN + col0 + c * 8),
+                           v);
+            if (c == kBlocks - 2) {  // the accumulator is free again
+                tc_fence_before();
+                mbar_arrive_cluster(acc_empty_lead + 8u * (uint32_t)b);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (lane == 0) bulk_wait_read_but<kWEpiBufs - 1>();  // the buffer is free again
+                __syncwarp();
+                unsigned char* sb = stage + buf * kWDrainBytes;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    reinterpret_cast<double2*>(sb + lane * 64)[k ^ ((lane >> 1) & 3)] =
+                        make_double2((double)v[8 * h + 2 * k], (double)v[8 * h + 2 * k + 1]);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    // The previous segment's operation on this block is performed.
+                    bulk_wait_but<2 * kBlocks - 1>();
+                    double* to = dst + (c + h) * kBlock;
+                    if (seg == 0)
+                        bulk_s2g(to, smem_u32(sb), kWDrainBytes);
+                    else
+                        bulk_add_s2g_f64(to, smem_u32(sb), kWDrainBytes);
+                    bulk_commit();
+                }
+                buf = buf + 1 == kWEpiBufs ? 0 : buf + 1;
+            }
+        }
+    }
+    bulk_wait_all();
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWThreads, 1)
+    fresnel_wide_kernel(FusedArgs g) {
+    using namespace sm100;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* rays_smem = tiles + kWStages * kWStage;
+    unsigned char* epi_smem = rays_smem + kFRayBufs * kFRayBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(epi_smem + kWEpiWarps * kWEpiBufs * kWDrainBytes);
+    uint64_t* empty = full + kWStages;
+    uint64_t* acc_full = empty + kWStages;
+    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* ray_full = acc_empty + 2;
+    uint64_t* ray_empty = ray_full + kFRayBufs;
+    uint64_t* mma_done = ray_empty + kFRayBufs;  // every issued MMA has completed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
+    volatile int* flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int mt = blockIdx.x, nt = blockIdx.y, sp = blockIdx.z;
+    const uint32_t half = cluster_ctarank(), peer = half ^ 1u;
+    const bool leader = half == 0;
+    const int rb0 = (int)((long long)g.ray_blocks * sp / g.splits);
+    const int rb1 = (int)((long long)g.ray_blocks * (sp + 1) / g.splits);
+    const int nrb = rb1 - rb0;
+
+    if (threadIdx.x == 0) {
+        // full and acc_empty are used in the even CTA only: they collect the
+        // arrivals of both CTAs' producer and epilogue warps.
+        for (int s = 0; s < kWStages; ++s) {
+            mbar_init(&full[s], 2 * kWProdWarps + (s == 0 ? g.stall : 0u));
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 2 * 32 * kWEpiWarps);
+        }
+        for (int b = 0; b < kFRayBufs; ++b) {
+            mbar_init(&ray_full[b], 1);
+            mbar_init(&ray_empty[b], kWProdWarps);
+        }
+        mbar_init(mma_done, 1);
+        mbar_init_fence();
+        *flag = 0;
+    }
+    if (warp == 0) tmem_alloc_pair(tmem_slot, 2 * kFN);
+    tc_fence_before();
+    cluster_sync();  // both CTAs' barriers initialised, TMEM allocated in both
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (leader && lane == 0) {
+            // Pair MMA issuer: per block hi.hi, hi.lo, lo.hi of four 256x256x16
+            // steps into either accumulator. An accumulator is issued first in its
+            // segment's last block and last in the next one, so that the other's
+            // products of both blocks run while it is drained.
+            constexpr uint32_t idesc = idesc_f16_f32(256, kFN);
+            bool good = true;
+            int end0 = min(nrb, kFSeg), end1 = min(nrb, kWShift), q0 = 0, q1 = 0;
+            bool new0 = true, new1 = true;
+            for (int i = 0; i < nrb && good; ++i) {
+                const int s = i % kWStages;
+                if (!mbar_wait_cluster(&full[s], (uint32_t)(i / kWStages) & 1u, g.wait_limit)) {
+                    *flag = 1;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t t0 = smem_u32(tiles) + (uint32_t)s * kWStage;
+                const uint32_t as[3] = {t0, t0, t0 + kPA};
+                const uint32_t bs[3] = {t0 + 2 * kPA, t0 + 3 * kPA, t0 + 2 * kPA};
+                const int first = (new0 && i > 0) || i + 1 == end1;
+                for (int h = first, t = 0; t < 2; ++t, h ^= 1) {
+                    const bool fresh = h ? new1 : new0;
+                    const int use = h ? q1 : q0;
+                    if (fresh && use >= 1 &&
+                        !mbar_wait_cluster(&acc_empty[h], (uint32_t)(use - 1) & 1u, g.wait_limit)) {
+                        *flag = 1;
+                        good = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t d = tmem + (uint32_t)(h * kFN);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)  // k < 2: A's real parts
+                            umma_f16_pair(d, desc_kmajor_sw128(as[p] + 32u * k),
+                                          desc_kmajor_sw128(bs[p] + 32u * (h ? k ^ 2 : k)),
+                                          h == 0 && k >= 2 ? idesc | kNegateB : idesc,
+                                          (uint32_t)(!fresh | p | k));
+                    const bool last = i + 1 == (h ? end1 : end0);
+                    if (last) {
+                        umma_commit_pair(smem_u32(&acc_full[h]));
+                        umma_commit_pair(mapa_shared(&acc_full[h], peer));
+                    }
+                    (h ? new1 : new0) = last;
+                    (h ? q1 : q0) += last;
+                    if (last) (h ? end1 : end0) = min(nrb, i + 1 + kFSeg);
+                }
+                umma_commit_pair(smem_u32(&empty[s]));
+                umma_commit_pair(mapa_shared(&empty[s], peer));
+            }
+            // A loop that gave up on a wait may leave MMAs in flight: wait
+            // (bounded) for them before either CTA frees its accumulators.
+            umma_commit_pair(smem_u32(mma_done));
+            if (!mbar_wait(mma_done, 0, max(g.wait_limit, kMmaDrainPolls))) *flag = 1;
+        }
+        __syncwarp();
+    } else if (warp <= kWEpiWarps) {
+        wide_drain(g, warp, lane, mt, nt, sp, nrb, tmem, acc_full, mapa_shared(acc_empty, 0),
+                   epi_smem + (warp - 1) * kWEpiBufs * kWDrainBytes, flag);
+    } else if (warp <= kWEpiWarps + kWProdWarps) {
+        wide_producer(g, warp - 1 - kWEpiWarps, lane, mt, nt, half, nrb, tiles,
+                      mapa_shared(full, 0), empty, ray_full, ray_empty, rays_smem, flag);
+    } else {
+        stage_rays_role(g, lane, rb0, nrb, rays_smem, ray_full, ray_empty, flag);
+    }
+    __syncthreads();
+    if (*flag != 0 && threadIdx.x == 0) *static_cast<volatile int*>(g.err) = 1;
+    tc_fence_before();
+    cluster_sync();  // the pair MMAs and all cross-CTA arrivals are done
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_free_pair(tmem, 2 * kFN);
+    }
+}
+
 // The ray set's bounds the product needs before it starts: max |es_re|,
 // |es_im| (the f16 scaling), max |x - ox| and |z - oz| (the cross-term bound),
 // and whether every value is finite. The maxima of non-negative doubles are
@@ -774,20 +1098,28 @@ __global__ void __launch_bounds__(256) ray_bounds_kernel(const double* __restric
     if (threadIdx.x == 3) host_out[3] = (unsigned long long)__ldcg(nonfinite);
 }
 
-// `group`: x points per real / imaginary column group of a 128-point block
-// (128 for single-CTA tiles, 64 for CTA pairs).
+// acc[iz*nx + ix] (+)= scale * sum over splits of C[iz][n(ix, c)], in FP64 and
+// split order. `group`: x points per real / imaginary column group of a 128-point
+// block (128 for single-CTA tiles, 64 for CTA pairs); 256 in the wide form, whose
+// partials are in the order of wide_at.
 __global__ void reduce_kernel(const double* __restrict__ partial, int splits, int m_pad, int n_pad,
                               int group, size_t nz, size_t nx, double scale,
                               double* __restrict__ acc_re, double* __restrict__ acc_im, int first) {
     const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (idx >= nz * nx) return;
     const size_t iz = idx / nx, ix = idx - iz * nx;
-    const size_t loc = ix & 127, col = (ix >> 7) * kFN + 2 * group * (loc / group) + loc % group;
+    const bool wide = group == 256;
+    const size_t loc = ix & 127;
+    const size_t col = wide ? (ix >> 8) * 512 + (ix & 255)
+                            : (ix >> 7) * kFN + 2 * group * (loc / group) + loc % group;
+    const size_t im_off = wide ? 256 / 8 * 256 : group;
     double re = 0.0, im = 0.0;
+#pragma unroll 8  // loads ahead of the ordered sums (148 splits: 61 -> 44 us after the product)
     for (int s = 0; s < splits; ++s) {
-        const double* row = partial + ((size_t)s * m_pad + iz) * n_pad + col;
-        re += row[0];
-        im += row[group];
+        const size_t r = (size_t)s * m_pad + iz;
+        const double* e = partial + (wide ? wide_at(r, col, n_pad) : r * n_pad + col);
+        re += e[0];
+        im += e[im_off];
     }
     re *= scale;
     im *= scale;
@@ -818,8 +1150,17 @@ FresnelShape fresnel_shape(size_t n, size_t nx, size_t nz, int num_sms, bool all
     sh.pair = allow_pair && nz > 128;
     sh.m_pad = round_up(std::max<size_t>(nz, 1), sh.pair ? 256 : 128);
     sh.n_pad = round_up(std::max<size_t>(2 * nx, 1), kFN);
+    // The wide form where its product is faster by more than its partials, twice
+    // the splits of one tile, cost the sum (20 us): 0.9 of the time per padded pair
+    // (5.30 and 4.78 ms on 2^20 rays x 512^2 points), from 1e10 pairs on (sums and
+    // all, narrow and wide: 82 and 89 us at 20000 x 256^2, 139 and 142 at 60000,
+    // 306 and 290 at 200000).
+    const size_t wide_pad = round_up(std::max<size_t>(2 * nx, 1), 2 * kFN);
+    sh.wide = sh.pair && 0.9 * (double)wide_pad < (double)sh.n_pad &&
+              (double)n * (double)sh.m_pad * (double)(wide_pad / 2) >= 1e10;
+    if (sh.wide) sh.n_pad = wide_pad;
     sh.ray_blocks = (int)((n + kFRays - 1) / kFRays);
-    sh.tiles = (sh.m_pad / 128) * (sh.n_pad / kFN);
+    sh.tiles = (sh.m_pad / 128) * (sh.n_pad / (sh.wide ? 2 * kFN : kFN));
     // K splits: about one CTA per SM over the output tiles, each split at
     // least ten ray blocks (half a segment) long. 30011 rays x 133 x 101 points:
     // product 113 us with 23 splits of 40 blocks, 80 with 46 of 20, 53 with 74;
@@ -865,7 +1206,10 @@ Status fresnel_enqueue(const FresnelIn& in, FresnelWorkspace& ws, cudaStream_t s
     XK_TRY(ws.partial.ensure((size_t)sh.splits * sh.m_pad * sh.n_pad * sizeof(double)));
     // Set on every call: the attribute belongs to the current device's
     // context, and a process may use several devices.
-    if (sh.pair)
+    if (sh.wide)
+        XK_CUDA_TRY(cudaFuncSetAttribute(fresnel_wide_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmem));
+    else if (sh.pair)
         XK_CUDA_TRY(cudaFuncSetAttribute(fresnel_pair_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmem));
     else
@@ -896,10 +1240,13 @@ Status fresnel_enqueue(const FresnelIn& in, FresnelWorkspace& ws, cudaStream_t s
     fa.wait_limit = ws.wait_limit;
     fa.stall = ws.stall_once;
     ws.stall_once = 0;  // armed for one execution
-    const dim3 grid((unsigned)(sh.m_pad / 128), (unsigned)(sh.n_pad / kFN), (unsigned)sh.splits);
+    const dim3 grid((unsigned)(sh.m_pad / 128), (unsigned)(sh.tiles / (sh.m_pad / 128)),
+                    (unsigned)sh.splits);
     const bool timed = rep->ev_gemm[0] && rep->ev_gemm[1];
     if (timed) XK_CUDA_TRY(cudaEventRecord(rep->ev_gemm[0], stream));
-    if (sh.pair)  // grid.x is even: m_pad is a multiple of 256
+    if (sh.wide)  // grid.x is even: m_pad is a multiple of 256
+        fresnel_wide_kernel<<<grid, kWThreads, kWSmem, stream>>>(fa);
+    else if (sh.pair)  // grid.x is even: m_pad is a multiple of 256
         fresnel_pair_kernel<<<grid, kPThreads, kPSmem, stream>>>(fa);
     else
         fresnel_fused_kernel<<<grid, kFThreads, kFSmem, stream>>>(fa);
@@ -907,7 +1254,7 @@ Status fresnel_enqueue(const FresnelIn& in, FresnelWorkspace& ws, cudaStream_t s
     if (timed) XK_CUDA_TRY(cudaEventRecord(rep->ev_gemm[1], stream));
     reduce_kernel<<<grid_1d(m, 256), 256, 0, stream>>>(ws.partial.as<double>(), sh.splits,
                                                         (int)sh.m_pad, (int)sh.n_pad,
-                                                        sh.pair ? 64 : 128, nz, nx,
+                                                        sh.wide ? 256 : (sh.pair ? 64 : 128), nz, nx,
                                                         in.max_amp, in.out_re, in.out_im, 1);
     XK_CUDA_TRY(cudaGetLastError());
     rep->kernels += 2;

@@ -900,7 +900,7 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     // Form, and rows along the outer or the inner axis: whichever costs less
     // (then whichever leaves the smaller first-order phase).
     bool found = false;
-    double best_area = 0.0, best_e = 0.0;
+    double best_cost = 0.0, best_e = 0.0;
     for (int form = 0; form < 4; ++form) {
         const bool swap = form & 1, wide = form & 2;
         const int am = swap ? inner : outer, an = swap ? outer : inner;
@@ -934,12 +934,17 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         const int tile_n = wide ? Form<true>::kTileN : Form<false>::kTileN;
         const size_t mt = blocks_of(nm, kTileM), nt = blocks_of(nn, tile_n);
         if (mt * nt > kGridMaxTiles) continue;
-        // Cost: the padded area, at 0.85 for the wide form (6.3 to 7.5 ms on 512 x
-        // 512 points, 0.48 to 0.55 on 256 x 256): it is taken unless it pads more.
-        const double area = (double)mt * kTileM * (double)nt * tile_n * (wide ? 0.85 : 1.0);
-        if (found && !(area < best_area || (area == best_area && e < best_e))) continue;
+        // Product: 36e12 pairs/s of the padded screen in the narrow form (2^20 rays x
+        // 512^2 points, one column). Wide: 0.85 of its time (6.3 to 7.5 ms there,
+        // kernels alone) and 18 us more for twice the partials per tile (first to
+        // last kernel, narrow and wide: 101 and 115 us at 10^4 rays x 256^2, 135 and
+        // 141 at 3 10^4, 253 and 244 at 10^5; 289 and 265 at 3 10^4 x 512^2).
+        const double area = (double)mt * kTileM * (double)nt * tile_n;
+        const double cost = area * columns * (double)n / 36e12 * (wide ? 0.85 : 1.0) +
+                            (wide ? 18e-6 : 0.0);
+        if (found && !(cost < best_cost || (cost == best_cost && e < best_e))) continue;
         found = true;
-        best_area = area;
+        best_cost = cost;
         best_e = e;
         g->m_axis = am;
         g->n_axis = an;
@@ -956,13 +961,11 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         g->amp = std::max(sm, sn) + mq > 2.384185791015625e-7;
     }
     if (!found) return false;
-    // Measured rates: the product 36e12 pairs/s of the padded screen (2^20 rays
-    // x 512^2 points, one column), the general path 1.6e12 pairs/s (1.2e12 with
-    // two columns) after 0.2 ms of sorting tiles and rays that the product does
-    // without (0.34 ms in all against 0.10 on 1024 rays x 40 x 51 points).
-    const double t_product = best_area * columns * (double)n / 36e12;
+    // Measured rates of the general path: 1.6e12 pairs/s (1.2e12 with two columns)
+    // after 0.2 ms of sorting tiles and rays that the product does without (0.34 ms
+    // in all against 0.10 on 1024 rays x 40 x 51 points).
     const double t_general = 2e-4 + (double)m * (double)n / (columns == 1 ? 1.6e12 : 1.2e12);
-    if (t_product > t_general) return false;
+    if (best_cost > t_general) return false;
     const double d0 = std::sqrt((r.pc[0] - r.rc[0]) * (r.pc[0] - r.rc[0]) +
                                 (r.pc[1] - r.rc[1]) * (r.pc[1] - r.rc[1]) +
                                 (r.pc[2] - r.rc[2]) * (r.pc[2] - r.rc[2]));

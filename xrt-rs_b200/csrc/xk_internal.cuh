@@ -204,8 +204,9 @@ struct FresnelIn {
 
 struct FresnelShape {
     size_t m_pad = 0, n_pad = 0;  // padded rows of A (screen z) and B (2 x screen x)
-    size_t tiles = 0;             // 128 x 256 output tiles (one per CTA)
+    size_t tiles = 0;             // 128 x 256 (wide: 128 x 512) output tiles, one per CTA
     bool pair = false;            // CTA pairs (256 x 256 tiles, one MMA over two SMs)
+    bool wide = false;            // pairs on 256 x points (256 x 512 tiles)
     int ray_blocks = 0;           // blocks of 32 rays (the contraction)
     int splits = 1;               // K splits per output tile
 };
