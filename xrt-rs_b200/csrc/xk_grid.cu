@@ -1028,17 +1028,24 @@ Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream) {
     return Status::Ok();
 }
 
-Status grid_reserve(const GridPlan& g, GridWorkspace& ws) {
+void grid_sizes(const GridPlan& g, size_t* recs, size_t* partial) {
     const size_t tiles = (size_t)g.m_tiles * g.n_tiles;
-    XK_TRY(ws.recs.ensure(tiles * g.chunk_rays * 64));
-    XK_TRY(ws.partial.ensure((size_t)g.splits * g.m_tiles * kTileM * g.n_tiles * g.columns *
-                             (g.wide ? 2 : 1) * kFN * sizeof(float)));
+    *recs = std::max(*recs, tiles * g.chunk_rays * 64);
+    *partial = std::max(*partial, (size_t)g.splits * g.m_tiles * kTileM * g.n_tiles * g.columns *
+                                      (g.wide ? 2 : 1) * kFN * sizeof(float));
+}
+
+Status grid_reserve(size_t recs, size_t partial, GridWorkspace& ws) {
+    XK_TRY(ws.recs.ensure(recs));
+    XK_TRY(ws.partial.ensure(partial));
     return Status::Ok();
 }
 
 Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wait_limit,
                     bool stall, cudaStream_t stream, int* kernels) {
-    XK_TRY(grid_reserve(g, ws));
+    size_t rec_bytes = 0, partial_bytes = 0;
+    grid_sizes(g, &rec_bytes, &partial_bytes);
+    XK_TRY(grid_reserve(rec_bytes, partial_bytes, ws));
     const double* rays[12];
     std::memcpy(rays, &g.rays, sizeof(rays));
     const double* axes_m = g.axes;

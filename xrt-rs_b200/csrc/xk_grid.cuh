@@ -77,7 +77,9 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
 // Gathers the axes into g.axes.
 Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream);
 
-Status grid_reserve(const GridPlan& g, GridWorkspace& ws);
+// Raises `recs` and `partial` [bytes] to what the product needs; allocates them.
+void grid_sizes(const GridPlan& g, size_t* recs, size_t* partial);
+Status grid_reserve(size_t recs, size_t partial, GridWorkspace& ws);
 
 // Enqueues the product (allocates nothing beyond grid_reserve). `err`: error
 // word the kernels can write (device or pinned). `stall`: test hook, the first
