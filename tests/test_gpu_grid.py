@@ -97,6 +97,18 @@ def test_wide_tiles(grid_ctx, oracle, n_outer, n_inner, n, pol):
     assert st["one_polarization"] == (pol == 1)
 
 
+# Screens near enough that a full tile's mixed phase is past the first order: tiles
+# use 32 to 256 of their rows and 32 to 128 of their columns, with remainders.
+@pytest.mark.parametrize("n_outer,n_inner,n,dist,energy", [
+    (385, 300, 4000, 350.0, 12000.0), (130, 97, 4000, 420.0, 12000.0),
+    (64, 200, 3000, 300.0, 12000.0), (300, 33, 3000, 330.0, 12000.0),
+    (96, 96, 2000, 350.0, 9000.0), (387, 119, 60000, 436.0, 11756.0)])
+def test_tiles_in_part(grid_ctx, oracle, n_outer, n_inner, n, dist, energy):
+    rays = synth.gaussian_aperture(n, 0.1, energy, 2e4, seed=n_inner)
+    pix = grid(np.linspace(-0.5, 0.5, n_outer), np.linspace(-0.4, 0.4, n_inner), dist, "xyz")
+    check(grid_ctx, oracle, rays, pix)
+
+
 def test_mostly_padding_takes_the_general_kernel(grid_ctx, oracle):
     """A screen that fills a 32nd of its tile, with many rays."""
     rays = synth.gaussian_aperture(1_500_000, 0.1, 10000.0, 3e4, seed=14)

@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
     // Tile extents, one warp per tile.
     const int warp = t0 >> 5, warps = step >> 5;
     for (int axis = 0; axis < 2; ++axis)
-        for (int k = 0; k < 2; ++k) {
-            const int count = axis ? len : m / len, size = 128 << k;
+        for (int k = 0; k < 4; ++k) {
+            const int count = axis ? len : m / len, size = kGridSpan << k;
             for (int t = warp; t * size < count; t += warps) {
                 double half = 0.0;
                 for (int c = 0; c < 3; ++c) {
@@ -155,12 +155,13 @@ __global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
 // One block per tile: the axis coordinates of its points and their mid-range.
 __global__ void __launch_bounds__(kTileM) grid_axes_kernel(const double* __restrict__ src_m,
                                                            size_t stride_m, int nm, int m_tiles,
+                                                           int span_m,
                                                            const double* __restrict__ src_n,
-                                                           size_t stride_n, int nn, int tile_n,
+                                                           size_t stride_n, int nn, int span_n,
                                                            double* __restrict__ axes) {
     const bool is_m = (int)blockIdx.x < m_tiles;
     const int t = is_m ? blockIdx.x : blockIdx.x - m_tiles;
-    const int size = is_m ? kTileM : tile_n, count = is_m ? nm : nn;
+    const int size = is_m ? span_m : span_n, count = is_m ? nm : nn;
     const int q = t * size + threadIdx.x;
     double lo = INFINITY, hi = -INFINITY;
     if ((int)threadIdx.x < size && q < count) {
@@ -245,6 +246,7 @@ struct ProductArgs {
     size_t pad;
     int ray_blocks, splits, seg;
     int m_tiles, n_tiles;
+    int span_m, span_n;  // rows and columns of a tile in use
     const double *cm, *cn, *refs;
     size_t nm, nn;
     double h0;
@@ -254,6 +256,17 @@ struct ProductArgs {
     int* err;
     uint32_t wait_limit, stall;
 };
+
+// Offset from the tile's reference of row `row` of row tile t, of column `col` of
+// column tile t; 0 outside the rows and columns in use.
+__device__ __forceinline__ double row_offset(const ProductArgs& g, int t, int row) {
+    const size_t i = (size_t)t * g.span_m + row;
+    return row < g.span_m && i < g.nm ? g.cm[i] - g.refs[t] : 0.0;
+}
+__device__ __forceinline__ double col_offset(const ProductArgs& g, int t, int col) {
+    const size_t i = (size_t)t * g.span_n + col;
+    return col < g.span_n && i < g.nn ? g.cn[i] - g.refs[g.m_tiles + t] : 0.0;
+}
 
 __device__ __forceinline__ uint32_t neg2(uint32_t v) { return v ^ 0x80008000u; }
 
@@ -350,19 +363,12 @@ __device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int 
     constexpr int NE = ZZ ? 1 : 2;   // pair-rows per thread
     constexpr int NCH = ZZ ? 2 : 1;  // chunks per thread
     PairRow row[NE];
-    const double ref_m = g.refs[mt >> 1], ref_n = g.refs[g.m_tiles + nt];
+    const int cta_row = (mt & 1) * 128;
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
-        const size_t im = (size_t)mt * 128 + (ZZ ? 64 + r : r + 32 * e);
-        const double ux = im < g.nm ? g.cm[im] - ref_m : 0.0;
-        double uy;
-        if (ZZ) {
-            const size_t iy = (size_t)mt * 128 + 96 + r;
-            uy = iy < g.nm ? g.cm[iy] - ref_m : 0.0;
-        } else {
-            const size_t in = (size_t)nt * 128 + 64 * half + r + 32 * e;
-            uy = in < g.nn ? g.cn[in] - ref_n : 0.0;
-        }
+        const double ux = row_offset(g, mt >> 1, cta_row + (ZZ ? 64 + r : r + 32 * e));
+        const double uy = ZZ ? row_offset(g, mt >> 1, cta_row + 96 + r)
+                             : col_offset(g, nt, 64 * half + r + 32 * e);
         row[e].set(ux, uy, g.h0);
     }
     for (int i = 0; i < nrb; ++i) {
@@ -459,13 +465,10 @@ __device__ __forceinline__ void grid_producer_wide(const ProductArgs& g, int w, 
     const int sub = (lane >> 3) & 1, oct = w & 3;
     const int row0 = 64 * (w >> 2) + (lane & 7) + ((lane & 16) >> 1);  // + 16 e
     PairRow row[4];
-    const double ref_m = g.refs[mt >> 1], ref_n = g.refs[g.m_tiles + nt];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const size_t im = (size_t)mt * 128 + row0 + 16 * e;
-        const size_t in = (size_t)nt * 256 + 128 * half + row0 + 16 * e;
-        row[e].set(im < g.nm ? g.cm[im] - ref_m : 0.0, in < g.nn ? g.cn[in] - ref_n : 0.0, g.h0);
-    }
+    for (int e = 0; e < 4; ++e)
+        row[e].set(row_offset(g, mt >> 1, (mt & 1) * 128 + row0 + 16 * e),
+                   col_offset(g, nt, 128 * half + row0 + 16 * e), g.h0);
     // This thread's 8 bytes of the real and the imaginary 16-byte word of row 0.
     const uint32_t at_re = sw128(row0, oct) + 8 * sub, at_im = sw128(row0, 4 + oct) + 8 * sub;
     for (int i = 0; i < nrb; ++i) {
@@ -794,20 +797,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
 // Threads run along the columns, which are consecutive in the partials.
 __global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restrict__ partial,
                                                           int splits, int m_pad, int n_pad,
-                                                          int columns, bool wide, size_t nm,
+                                                          int columns, bool wide, int span_m, int span_n, size_t nm,
                                                           size_t nn, bool rows_outer, double scale,
                                                           double2 pes, double2 pep, FieldDev out) {
     const size_t idx = blockIdx.x * (size_t)256 + threadIdx.x;
     if (idx >= nm * nn) return;
     const size_t im = idx / nn, in = idx - im * nn;
-    // Column of the real part; the imaginary part's is 256 (wide) or 64 further.
-    const size_t at = wide ? (in >> 8) * 512 + (in & 255)
-                           : (in >> 7) * 256 + 128 * ((in >> 6) & 1) + (in & 63);
+    // Row and real part's column in the partials; the imaginary part's column is 256
+    // (wide) or 64 further.
+    const size_t mt = im / span_m, nt = in / span_n, ln = in - nt * span_n;
+    const size_t row = mt * kTileM + (im - mt * span_m);
+    const size_t at = wide ? nt * 512 + ln : nt * 256 + 128 * (ln >> 6) + (ln & 63);
     const int im_off = (wide ? 256 : 64) / 16 * 512;
     double re[2] = {0.0, 0.0}, ie[2] = {0.0, 0.0};
     for (int c = 0; c < columns; ++c)
         for (int s = 0; s < splits; ++s) {
-            const float* e = partial + partial_at((size_t)s * m_pad + im,
+            const float* e = partial + partial_at((size_t)s * m_pad + row,
                                                   (size_t)c * (n_pad / columns) + at, n_pad);
             re[c] += e[0];
             ie[c] += e[im_off];
@@ -901,12 +906,18 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     // (then whichever leaves the smaller first-order phase).
     bool found = false;
     double best_cost = 0.0, best_e = 0.0;
-    for (int form = 0; form < 4; ++form) {
-        const bool swap = form & 1, wide = form & 2;
+    // Tiles may use fewer rows (256 >> fm) or columns (of 128 >> fn; or 256) than they
+    // have: E falls with either, at the price of the rest, which is still below the
+    // general kernel's down to 1/16 of a tile (2^18 rays x 256^2 points +-1 mm at 1 m:
+    // 11.7 -> 1.9 ms at 10 keV, 12.1 -> 4.0 at 20, 12.4 -> 8.0 at 30).
+    for (int form = 0; form < 32; ++form) {
+        const bool swap = form & 1;
+        const int fm = (form >> 1) & 3, fn = (form >> 3) & 3;
+        const bool wide = fn == 3;
         const int am = swap ? inner : outer, an = swap ? outer : inner;
         const size_t nm = swap ? len : rows, nn = swap ? rows : len;
-        const double em = bits_to_double(probe.extent[swap ? 1 : 0][1]);  // 256-point tiles
-        const double en = bits_to_double(probe.extent[swap ? 0 : 1][wide]);  // 128 or 256
+        const double em = bits_to_double(probe.extent[swap ? 1 : 0][3 - fm]);
+        const double en = bits_to_double(probe.extent[swap ? 0 : 1][wide ? 3 : 2 - fn]);
         // |dS| = |u| |(p - r) + (p0 - r)| with |p0 - r| <= |p - r|max - |u|max
         // when the tile lies inside the screen's range.
         const double pm = largest(del[am]), pn = largest(del[an]);
@@ -932,7 +943,8 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
               mq * mq <= 1e-7))
             continue;
         const int tile_n = wide ? Form<true>::kTileN : Form<false>::kTileN;
-        const size_t mt = blocks_of(nm, kTileM), nt = blocks_of(nn, tile_n);
+        const int span_m = kTileM >> fm, span_n = wide ? tile_n : tile_n >> fn;
+        const size_t mt = blocks_of(nm, span_m), nt = blocks_of(nn, span_n);
         if (mt * nt > kGridMaxTiles) continue;
         // Product: 36e12 pairs/s of the padded screen in the narrow form (2^20 rays x
         // 512^2 points, one column). Wide: 0.85 of its time (6.3 to 7.5 ms there,
@@ -953,6 +965,8 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         g->nm = nm;
         g->nn = nn;
         g->wide = wide;
+        g->span_m = span_m;
+        g->span_n = span_n;
         g->m_tiles = (int)mt;
         g->n_tiles = (int)nt;
         g->e_bound = e;
@@ -1022,8 +1036,8 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
 Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream) {
     const size_t sm = g.rows_outer ? g.inner_len : 1, sn = g.rows_outer ? 1 : g.inner_len;
     grid_axes_kernel<<<g.m_tiles + g.n_tiles, kTileM, 0, stream>>>(
-        coord_host(g.pix, g.m_axis), sm, (int)g.nm, g.m_tiles, coord_host(g.pix, g.n_axis), sn,
-        (int)g.nn, g.wide ? 256 : 128, g.axes);
+        coord_host(g.pix, g.m_axis), sm, (int)g.nm, g.m_tiles, g.span_m, coord_host(g.pix, g.n_axis), sn,
+        (int)g.nn, g.span_n, g.axes);
     XK_CUDA_TRY(cudaGetLastError());
     return Status::Ok();
 }
@@ -1055,6 +1069,8 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
     p.seg = g.seg;
     p.m_tiles = g.m_tiles;
     p.n_tiles = g.n_tiles;
+    p.span_m = g.span_m;
+    p.span_n = g.span_n;
     p.cm = axes_m;
     p.cn = axes_m + g.nm;
     p.refs = axes_m + g.nm + g.nn;
@@ -1115,7 +1131,7 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         *kernels += 2;
     }
     grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
-        p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.nm, g.nn, g.rows_outer,
+        p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.span_m, g.span_n, g.nm, g.nn, g.rows_outer,
         g.k / (4.0 * 3.14159265358979323846) / g.inv_scale, make_double2(g.pes[0], g.pes[1]),
         make_double2(g.pep[0], g.pep[1]), g.out);
     XK_CUDA_TRY(cudaGetLastError());

@@ -11,12 +11,15 @@ namespace xk {
 // most one that depends on i alone (the outer axis), the rest constant, bit
 // for bit. extent[axis][k]: largest half-extent of a tile of 128 << k
 // consecutive points of the axis (0 outer, 1 inner), as the bits of a double.
+constexpr int kGridSpan = 32;  // fewest rows or columns of a tile in use
+
 struct GridProbe {
     int len;         // inner length; 0 if there is no such order
     int bad;         // a point breaks the order
     int inner;       // coordinate index (0 x, 1 y, 2 z) of the inner axis
     int outer_mask;  // coordinates that vary with i
-    unsigned long long extent[2][2];
+    // Largest half extent (bits of a double) of kGridSpan << k points, outer and inner.
+    unsigned long long extent[2][4];
 };
 
 // Ranges of a solve's inputs (from the planner's summary).
@@ -38,6 +41,7 @@ struct GridPlan {
     size_t nm = 0, nn = 0;                   // rows, columns (screen points along the axes)
     size_t inner_len = 0;
     bool wide = false;                       // 256 columns per tile instead of 128
+    int span_m = 0, span_n = 0;              // rows and columns of a tile in use
     int m_tiles = 0, n_tiles = 0, columns = 1;  // tiles of 256 rows and 128 or 256 columns; amplitude columns
     int ray_blocks = 0, splits = 1, seg = 0;
     size_t n = 0, chunk_rays = 0;            // rays, rays per product launch
