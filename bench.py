@@ -54,9 +54,9 @@ SFU_OPS_PER_PAIR = 4
 # 512^2 workload from an ncu capture of the full-size launch, by the number of
 # amplitude columns summed (two-column kernel: key False).
 DRAM_BYTES_CONFIG1 = {False: 502.3e6, True: 270.7e6}
-# The same for one fresnel_pair_kernel launch on 2^20 rays x 512^2: the four
-# ray columns read once (the FP64 split partials stay in L2).
-FRESNEL_DRAM_BYTES_CONFIG = 33.8e6
+# The same for one fresnel_wide_kernel launch on 2^20 rays x 512^2: the four ray
+# columns read once (35 MB), the FP64 reduce-adds written through from L2.
+FRESNEL_DRAM_BYTES_CONFIG = 4.23e9
 
 
 def parse():
@@ -522,13 +522,16 @@ def run_fresnel(args):
     peak, peak_source = tensor_peak()
     gemm = float(np.mean(gemm_ms))
     achieved = algo_flops / (gemm / 1e3) / 1e12
-    # Screens of more than 128 rows run on CTA pairs (stats sweep = 1).
-    fr_kernel = "fresnel_pair_kernel" if st["sweep"] == 1 else "fresnel_fused_kernel"
-    # DRAM bytes (read + write) of one fresnel_pair_kernel launch on the
-    # 2^20-ray 512x512 workload, from a single-pass ncu capture of full-size
-    # launches; other sizes report null.
+    # Screens of more than 128 rows run on CTA pairs (stats sweep = 1), large
+    # products on 256-point tiles (fewer tiles than 128-point ones).
+    wide = st["sweep"] == 1 and st["n_tiles"] < 2 * -(-g // 256) * -(-g // 128)
+    fr_kernel = ("fresnel_wide_kernel" if wide else
+                 "fresnel_pair_kernel" if st["sweep"] == 1 else "fresnel_fused_kernel")
+    # DRAM bytes (read + write) of one fresnel_wide_kernel launch on the
+    # 2^20-ray 512x512 workload, from a single-pass ncu capture of a full-size
+    # launch; other sizes report null.
     fr_traffic = (FRESNEL_DRAM_BYTES_CONFIG
-                  if (args.rays == 1 << 20 and args.grid == 512 and st["sweep"] == 1) else None)
+                  if (args.rays == 1 << 20 and args.grid == 512 and wide) else None)
     cpu = None
     if not args.no_cpu:
         row = xrt_rs.FresnelScreen(-0.5, 0.5, g, 0.0, 0.0, 1)

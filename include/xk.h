@@ -190,7 +190,8 @@ const char* xk_route_reason(int reason);
  *                    and nothing stays in flight; cleared after that execution
  *   "fresnel_pair"   XK_PATH_SEPARABLE: 1 (default) computes screens of more
  *                    than 128 rows on CTA pairs (one tcgen05 MMA over two SMs,
- *                    256 x 256 tiles); 0 keeps one CTA per 128 x 256 tile */
+ *                    256 x 256 tiles, 256 x 512 from 1e10 pairs on); 0 keeps
+ *                    one CTA per 128 x 256 tile */
 int xk_set_option(xk_ctx* ctx, const char* name, double value);
 
 typedef struct xk_tune_result {
