@@ -87,21 +87,30 @@ __device__ __forceinline__ const double* coord(const PixDev& p, int c) {
     return c == 0 ? p.x : (c == 1 ? p.y : p.z);
 }
 
-__global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
-                                                         const double* __restrict__ first_change,
-                                                         GridProbe* __restrict__ out,
-                                                         unsigned* __restrict__ ticket,
-                                                         GridProbe* __restrict__ host_out) {
-    const double lend = *first_change;
+// As summary_kernel, up to N screens per launch (nine screens of a batch: 122 us one
+// after another, 15 in one launch; a single one is bound by its latency).
+template <int N>
+struct ProbeBatch {
+    ProbeArgs s[N];
+};
+
+template <int N>
+__global__ void __launch_bounds__(256)
+    grid_probe_kernel(const __grid_constant__ ProbeBatch<N> batch) {
+    const ProbeArgs& A = solve_of_block(batch.s);
+    const PixDev& p = A.pix;
+    const int m = A.m, block = (int)blockIdx.x - A.first;
+    GridProbe* const out = A.probe;
+    const double lend = *A.first_change;
     if (!(lend >= 2.0 && lend <= 0.5 * m)) return;  // len stays 0
     const int len = (int)lend;
     if (m % len != 0) return;
     const int inner = p.x[1] != p.x[0] ? 0 : (p.y[1] != p.y[0] ? 1 : 2);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (block == 0 && threadIdx.x == 0) {
         out->len = len;
         out->inner = inner;
     }
-    const int t0 = blockIdx.x * 256 + threadIdx.x, step = gridDim.x * 256;
+    const int t0 = block * 256 + threadIdx.x, step = A.blocks * 256;
     int bad = 0, mask = 0;
     for (int q = t0; q < m; q += step) {
         const int i = q / len, l = q - i * len;
@@ -120,12 +129,15 @@ __global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
         if (bad) atomicOr(&out->bad, 1);
         if (mask) atomicOr(&out->outer_mask, mask);
     }
-    // Tile extents, one warp per tile.
+    // Half extents of every tile of every size, one warp per tile. Sizes and axes
+    // share the warps' turns, so that a small screen takes one of them.
     const int warp = t0 >> 5, warps = step >> 5;
+    int base = 0;  // tiles of the sizes and axes before
     for (int axis = 0; axis < 2; ++axis)
         for (int k = 0; k < 4; ++k) {
             const int count = axis ? len : m / len, size = kGridSpan << k;
-            for (int t = warp; t * size < count; t += warps) {
+            const int tiles = (count + size - 1) / size;
+            for (int t = (warp + warps - base % warps) % warps; t < tiles; t += warps) {
                 double half = 0.0;
                 for (int c = 0; c < 3; ++c) {
                     if ((c == inner) != (axis == 1)) continue;
@@ -145,10 +157,11 @@ __global__ void __launch_bounds__(256) grid_probe_kernel(PixDev p, int m,
                 if (lane == 0)
                     atomicMax(&out->extent[axis][k], (unsigned long long)__double_as_longlong(half));
             }
+            base += tiles;
         }
     static_assert(sizeof(GridProbe) % 8 == 0, "copied by 8-byte words");
-    if (last_block(ticket) && threadIdx.x < sizeof(GridProbe) / 8)
-        reinterpret_cast<unsigned long long*>(host_out)[threadIdx.x] =
+    if (last_block(A.ticket, A.blocks) && threadIdx.x < sizeof(GridProbe) / 8)
+        reinterpret_cast<unsigned long long*>(A.host_probe)[threadIdx.x] =
             __ldcg(reinterpret_cast<const unsigned long long*>(out) + threadIdx.x);
 }
 
@@ -861,12 +874,13 @@ double bits_to_double(unsigned long long b) {
 
 }  // namespace
 
-Status grid_probe_enqueue(const PixDev& pix, int m, const double* first_change, GridProbe* probe,
-                          unsigned* ticket, GridProbe* host_probe, cudaStream_t stream) {
-    const int blocks = (int)std::min<size_t>(blocks_of((size_t)m, 1024), 296);
-    grid_probe_kernel<<<blocks, 256, 0, stream>>>(pix, m, first_change, probe, ticket, host_probe);
-    XK_CUDA_TRY(cudaGetLastError());
-    return Status::Ok();
+Status grid_probe_enqueue(std::vector<ProbeArgs>& screens, cudaStream_t stream, int* kernels) {
+    for (ProbeArgs& a : screens)
+        a.blocks = (int)std::min<size_t>(blocks_of((size_t)a.m, 1024), 296);
+    if (screens.size() == 1)
+        return launch_solves<1, ProbeBatch<1>>(grid_probe_kernel<1>, screens, stream, kernels);
+    return launch_solves<kSolvesPerLaunch, ProbeBatch<kSolvesPerLaunch>>(
+        grid_probe_kernel<kSolvesPerLaunch>, screens, stream, kernels);
 }
 
 bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, int columns,

@@ -2,6 +2,9 @@
 // product (xk_grid.cu).
 #pragma once
 
+#include <climits>
+#include <vector>
+
 #include "xk_internal.cuh"
 
 namespace xk {
@@ -67,11 +70,41 @@ constexpr size_t kGridMinRays = 1024, kGridMinPoints = 1025;
 // Doubles `axes` of a plan for m screen points may need.
 inline size_t grid_axes_doubles(size_t m) { return 2 * (m + 2) + 4; }
 
-// Checks the screen's order. `first_change`: the candidate for the inner length
-// (device). `probe` is zeroed by an earlier kernel on the stream, `host_probe`
-// (pinned) by the caller; the kernel writes both. `ticket`: see last_block.
-Status grid_probe_enqueue(const PixDev& pix, int m, const double* first_change, GridProbe* probe,
-                          unsigned* ticket, GridProbe* host_probe, cudaStream_t stream);
+// Launches `kernel` over the solves' blocks, N solves at a time.
+template <int N, class Batch, class Args>
+Status launch_solves(void (*kernel)(Batch), std::vector<Args>& solves, cudaStream_t stream,
+                     int* kernels) {
+    for (size_t i0 = 0; i0 < solves.size(); i0 += N) {
+        Batch b{};
+        int blocks = 0;
+        for (int i = 0; i < N; ++i) {
+            b.s[i].first = INT_MAX;
+            if (i0 + i >= solves.size()) continue;
+            b.s[i] = solves[i0 + i];
+            b.s[i].first = blocks;
+            blocks += b.s[i].blocks;
+        }
+        kernel<<<blocks, 256, 0, stream>>>(b);
+        XK_CUDA_TRY(cudaGetLastError());
+        ++*kernels;
+    }
+    return Status::Ok();
+}
+
+// Checks the order of one screen. `first_change`: the candidate for the inner
+// length (device). `probe` is zeroed by an earlier kernel on the stream,
+// `host_probe` (pinned) by the caller; the kernel writes both. `ticket`: see
+// last_block.
+struct ProbeArgs {
+    PixDev pix;
+    int m;
+    int first, blocks;  // of the grid's blocks; set by the launch
+    const double* first_change;
+    GridProbe* probe;
+    unsigned* ticket;
+    GridProbe* host_probe;
+};
+Status grid_probe_enqueue(std::vector<ProbeArgs>& screens, cudaStream_t stream, int* kernels);
 
 // Decides whether the product takes the solve and fills `g` (without device
 // pointers); `columns` amplitude columns; `tolerance` as requested.

@@ -122,17 +122,28 @@ struct HostBuf {
 // Whole block: true in the block that arrives last. What the blocks wrote
 // before is visible to it (read it with __ldcg). `ticket` starts at zero and is
 // left at zero, so it needs clearing only once.
-__device__ __forceinline__ bool last_block(unsigned* ticket) {
+__device__ __forceinline__ bool last_block(unsigned* ticket, unsigned blocks) {
     __shared__ bool last;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        last = atomicAdd(ticket, 1u) == blocks - 1;
         if (last) *ticket = 0;
     }
     __syncthreads();
     __threadfence();
     return last;
+}
+__device__ __forceinline__ bool last_block(unsigned* ticket) { return last_block(ticket, gridDim.x); }
+
+// Solves per launch of a kernel that serves many, and the one a block belongs to
+// (their blocks lie one after another; unused entries begin past the grid).
+constexpr int kSolvesPerLaunch = 16;
+template <class Args, int N>
+__device__ __forceinline__ const Args& solve_of_block(const Args (&s)[N]) {
+    int i = 0;
+    while (i + 1 < N && (int)blockIdx.x >= s[i + 1].first) ++i;
+    return s[i];
 }
 #endif
 

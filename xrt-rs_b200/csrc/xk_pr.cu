@@ -117,19 +117,40 @@ __device__ __forceinline__ double op_combine(int op, double a, double b) {
 // points 0 and 1 share changes: the inner length if the screen is rectangular
 // (infinite if points 0 and 1 differ in none or several coordinates). Clears
 // `probe` for the check of that order. The last block combines the rows into row
-// gridDim.x and into pinned host memory, which the host reads after its next
+// `blocks` and into pinned host memory, which the host reads after its next
 // synchronisation (a copy of a few hundred bytes costs more than the kernel).
-__global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p, int m,
-                                                     double* __restrict__ block_out,
-                                                     GridProbe* __restrict__ probe,
-                                                     unsigned* __restrict__ ticket,
-                                                     double* __restrict__ host_out) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *probe = GridProbe{};
+// A launch serves up to N solves: one of a batch's solves fills few SMs and takes
+// its latency whatever its size (16 uneven solves: 291 us one after another, 60 in
+// one launch).
+struct SummaryArgs {
+    RaysDev rays;
+    PixDev pix;
+    int n, m;
+    int first, blocks;  // of the grid's blocks
+    double* block_out;
+    GridProbe* probe;
+    unsigned* ticket;
+    double* host_out;
+};
+template <int N>
+struct SummaryBatch {
+    SummaryArgs s[N];
+};
+
+template <int N>
+__global__ void __launch_bounds__(256)
+    summary_kernel(const __grid_constant__ SummaryBatch<N> batch) {
+    const SummaryArgs& A = solve_of_block(batch.s);
+    const RaysDev& r = A.rays;
+    const PixDev& p = A.pix;
+    const int n = A.n, m = A.m, block = (int)blockIdx.x - A.first;
+    double* const block_out = A.block_out;
+    if (block == 0 && threadIdx.x == 0) *A.probe = GridProbe{};
     double f[kSumFields];
 #pragma unroll
     for (int i = 0; i < kSumFields; ++i)
         f[i] = sum_op(i) == OP_SUM ? 0.0 : (sum_op(i) == OP_MIN ? INFINITY : -INFINITY);
-    const int stride = gridDim.x * blockDim.x;
+    const int stride = A.blocks * 256;
     const double a0r = r.es_re[0], a0i = r.es_im[0], b0r = r.ep_re[0], b0i = r.ep_im[0];
     const double a0n = sqrt(a0r * a0r + a0i * a0i), b0n = sqrt(b0r * b0r + b0i * b0i);
     const double x0 = r.x[0], y0 = r.y[0], z0 = r.z[0];
@@ -137,7 +158,7 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
     const int one = m > 1 ? 1 : 0;
     const bool in0 = p.x[one] != q0, in1 = p.y[one] != q1, in2 = p.z[one] != q2;
     const bool ordered = (int)in0 + (int)in1 + (int)in2 == 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    for (int i = block * 256 + threadIdx.x; i < n; i += stride) {
         double x = r.x[i], y = r.y[i], z = r.z[i], e = r.energy[i];
         double a = r.nx[i], b = r.ny[i], c = r.nz[i];
         f[0] += x; f[1] += y; f[2] += z;
@@ -169,7 +190,7 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
             f[39] += z;
         }
     }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride) {
+    for (int i = block * 256 + threadIdx.x; i < m; i += stride) {
         double x = p.x[i], y = p.y[i], z = p.z[i];
         f[17] += x; f[18] += y; f[19] += z;
         f[20] = fmin(f[20], x); f[21] = fmin(f[21], y); f[22] = fmin(f[22], z);
@@ -193,12 +214,12 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
         double v = sm[0][i];
         const int op = sum_op(i);
         for (int w = 1; w < 8; ++w) v = op_combine(op, v, sm[w][i]);
-        block_out[blockIdx.x * kSumFields + i] = v;
+        block_out[block * kSumFields + i] = v;
     }
-    if (!last_block(ticket)) return;
+    if (!last_block(A.ticket, A.blocks)) return;
     constexpr int kParts = 6;  // threads per field
     __shared__ double sp[kParts][kSumFields];
-    const int rows = gridDim.x, i = threadIdx.x % kSumFields, part = threadIdx.x / kSumFields;
+    const int rows = A.blocks, i = threadIdx.x % kSumFields, part = threadIdx.x / kSumFields;
     const int op = sum_op(i);
     if (part < kParts) {
         double v = op == OP_SUM ? 0.0 : (op == OP_MIN ? INFINITY : -INFINITY);
@@ -212,7 +233,7 @@ __global__ void __launch_bounds__(256) summary_kernel(RaysDev r, int n, PixDev p
         double v = sp[0][i];
         for (int w = 1; w < kParts; ++w) v = op_combine(op, v, sp[w][i]);
         block_out[rows * kSumFields + i] = v;
-        host_out[i] = v;
+        A.host_out[i] = v;
     }
 }
 
@@ -1814,22 +1835,26 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
 
     // --- A. summaries ------------------------------------------------------
     bool any = false;
+    std::vector<SummaryArgs> sums;
+    std::vector<ProbeArgs> probes;
     for (int s = 0; s < count; ++s) {
         if (plans[s].routed) continue;
         any = true;
         const int parts = sum_parts(in[s].n, in[s].m, sum_blocks);
-        summary_kernel<<<parts, 256, 0, stream>>>(in[s].rays, (int)in[s].n, in[s].pix,
-                                                  (int)in[s].m, bufs[s].sum, bufs[s].probe,
-                                                  tickets + 4 * s, h_sum + s * kSumFields);
-        XK_CUDA_TRY(cudaGetLastError());
+        sums.push_back({in[s].rays, in[s].pix, (int)in[s].n, (int)in[s].m, 0, parts, bufs[s].sum,
+                        bufs[s].probe, tickets + 4 * s, h_sum + s * kSumFields});
         if (grid_candidate(opt, in[s].n, in[s].m)) {
             h_probe[s] = GridProbe{};
-            XK_TRY(grid_probe_enqueue(in[s].pix, (int)in[s].m, bufs[s].sum + parts * kSumFields + 33,
-                                      bufs[s].probe, tickets + 4 * s + 1, h_probe + s, stream));
-            ++nk;
+            probes.push_back({in[s].pix, (int)in[s].m, 0, 0, bufs[s].sum + parts * kSumFields + 33,
+                              bufs[s].probe, tickets + 4 * s + 1, h_probe + s});
         }
-        ++nk;
     }
+    if (sums.size() == 1)
+        XK_TRY((launch_solves<1, SummaryBatch<1>>(summary_kernel<1>, sums, stream, &nk)));
+    else
+        XK_TRY((launch_solves<kSolvesPerLaunch, SummaryBatch<kSolvesPerLaunch>>(
+            summary_kernel<kSolvesPerLaunch>, sums, stream, &nk)));
+    XK_TRY(grid_probe_enqueue(probes, stream, &nk));
     if (!any) {
         if (kernels) *kernels += nk;
         return Status::Ok();
