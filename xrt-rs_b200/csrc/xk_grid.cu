@@ -68,8 +68,8 @@ static_assert(kGSmem <= 227 * 1024, "shared memory");
 // and the imaginary part; a part is drained while the other's products run.
 // 2^20 rays x 512^2 points: 7.5 ms narrow, 6.3 ms wide (first calls; 8.5 and
 // 7.1 ms in a row, the chip at its power limit and 1.55 GHz). In the wide form
-// the tensor pipe is busy 72 % of the time (narrow 43 %) and shared memory 77 %
-// (products 35, record loads 24, stores 18 %).
+// the tensor pipe is busy 72 % of the time (narrow 43 %) and shared memory 75 %
+// (products 35, record loads 22, stores 18 %).
 template <bool WIDE>
 struct Form {
     static constexpr int kTileN = WIDE ? 256 : 128;
@@ -810,8 +810,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
 // Threads run along the columns, which are consecutive in the partials.
 __global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restrict__ partial,
                                                           int splits, int m_pad, int n_pad,
-                                                          int columns, bool wide, int span_m, int span_n, size_t nm,
-                                                          size_t nn, bool rows_outer, double scale,
+                                                          int columns, bool wide, int span_m,
+                                                          int span_n, size_t nm, size_t nn,
+                                                          bool rows_outer, double scale,
                                                           double2 pes, double2 pep, FieldDev out) {
     const size_t idx = blockIdx.x * (size_t)256 + threadIdx.x;
     if (idx >= nm * nn) return;
@@ -1145,7 +1146,8 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         *kernels += 2;
     }
     grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
-        p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.span_m, g.span_n, g.nm, g.nn, g.rows_outer,
+        p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.span_m, g.span_n, g.nm, g.nn,
+        g.rows_outer,
         g.k / (4.0 * 3.14159265358979323846) / g.inv_scale, make_double2(g.pes[0], g.pes[1]),
         make_double2(g.pep[0], g.pep[1]), g.out);
     XK_CUDA_TRY(cudaGetLastError());
