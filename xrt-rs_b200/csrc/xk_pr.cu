@@ -7,8 +7,9 @@
 //     |p - r| = |q| - u.rho + Delta,
 //     Delta   = (|rho_perp|^2 - 2 v.rho) / (|p - r| + |q| - u.rho),
 // with v = q - |q| u (|v| <= tile radius) and rho_perp = rho - (u.rho) u.
-// The denominator equals 2(|q| - u.rho) + Delta, and Delta/|q| is far below
-// FP32 resolution, so the kernel uses 2(|q| - u.rho).
+// The denominator equals 2(|q| - u.rho) + Delta. The kernel uses 2(|q| - u.rho),
+// which changes the phase by k Delta^2 / (2|q|): half the tolerance at most, by
+// the planner's cap of the residual phase (pair_budget).
 //   * exp(i k |q|)      per screen point and chunk: reference path length and
 //                       its turn count in FP64, sin/cos of the reduced turn,
 //   * exp(-i k u.rho)   per ray and item, FP64 argument reduction folded
@@ -1548,6 +1549,14 @@ bool grid_candidate(const PrOptions& o, size_t n, size_t m) {
            n >= kGridMinRays && m >= kGridMinPoints;
 }
 
+// Largest residual phase of a pair [rad]: the caller's budget, and B with
+// B^2 / (2 k d) = tolerance / 2 (the term left out of the reciprocal). The second
+// is the smaller one only where k d is below 8e8 at the default settings, 15 mm at
+// 10 keV: 1 mm behind an aperture the budget alone left 1.3e-4 of the field.
+double pair_budget(const PrOptions& o, double k, double d) {
+    return std::min(effective_phase_budget(o), std::sqrt(o.tolerance * k * d));
+}
+
 // Blocks of a solve's summary: at least four elements per thread, because below
 // that the reduction of the fields and the host's pass over the blocks' results
 // cost more than reading the inputs (10^4 rays: 18 us and 95 KB with 296
@@ -2054,7 +2063,7 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             return std::sqrt(sq);
         };
         double cell[3];
-        const double budget = effective_phase_budget(o);
+        const double budget = pair_budget(o, k, I.d_lo);
         double h_hi = 2.0 * std::max(ext[0], std::max(ext[1], ext[2])) + 1e-300;
         double h_lo = 0.0;
         if (phase_bound(k, a_max, cell_radius(h_hi, cell), I.d_lo) <= budget) {
