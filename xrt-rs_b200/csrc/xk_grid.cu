@@ -203,8 +203,9 @@ __global__ void __launch_bounds__(kTileM) grid_axes_kernel(const double* __restr
 
 // ---- ray records ------------------------------------------------------------------
 
-// Per ray and tile (64 bytes; a / b: row / column axis):
-//   {La hi, Lb hi, La lo, Lb lo}   L = 2 h A turns / mm
+// Per ray and tile (64 bytes; a / b: row / column axis; lengths times
+// GridPlan::unit):
+//   {La hi, Lb hi, La lo, Lb lo}   L = 2 h A turns
 //   {2A, 2B, h - h0, -q}           q = turns of the second-order term per dS^2
 //   {R, W re, W im, -m}            R = frac(k D), W = amplitude at p0, scaled
 //   {sa, sb, W2 re, W2 im}         amplitude slopes; second column
@@ -214,7 +215,9 @@ struct RecordArgs {
     const double* refs;  // tile references: m_tiles, then n_tiles
     int m_tiles, n_tiles;
     size_t n, pad;       // rays of this launch, rounded up to whole blocks
-    double c0, h0, kt, kt_lo, scale;
+    double c0;
+    double unit;         // GridPlan::unit; what follows is in such lengths
+    double h0, kt, kt_lo, scale;
 };
 
 __global__ void __launch_bounds__(256) grid_records_kernel(RecordArgs g, float4* __restrict__ out) {
@@ -227,8 +230,14 @@ __global__ void __launch_bounds__(256) grid_records_kernel(RecordArgs g, float4*
         return;
     }
     double al, bl, cl;
-    const double a = dd_diff(g.refs[mt], g.ra[j], &al), b = dd_diff(g.refs[g.m_tiles + nt], g.rb[j], &bl),
-                 c = dd_diff(g.c0, g.rc[j], &cl);
+    double a = dd_diff(g.refs[mt], g.ra[j], &al), b = dd_diff(g.refs[g.m_tiles + nt], g.rb[j], &bl),
+           c = dd_diff(g.c0, g.rc[j], &cl);
+    a *= g.unit;  // a power of two: exact
+    b *= g.unit;
+    c *= g.unit;
+    al *= g.unit;
+    bl *= g.unit;
+    cl *= g.unit;
     double d, unused;
     const double turns = dd_turns<true>(g.kt, g.kt_lo, a, b, c, &d, &unused,
                                         2.0 * (a * al + b * bl + c * cl));
@@ -262,7 +271,7 @@ struct ProductArgs {
     int span_m, span_n;  // rows and columns of a tile in use
     const double *cm, *cn, *refs;
     size_t nm, nn;
-    double h0;
+    double unit, h0;  // GridPlan::unit; turns per squared such length
     float* partial;  // [splits][m_pad][n_pad], in the order of partial_at
     int m_pad, n_pad;
     bool first;      // the splits' first segments store
@@ -270,15 +279,16 @@ struct ProductArgs {
     uint32_t wait_limit, stall;
 };
 
-// Offset from the tile's reference of row `row` of row tile t, of column `col` of
-// column tile t; 0 outside the rows and columns in use.
+// Offset from the tile's reference (in GridPlan::unit) of row `row` of row tile t,
+// of column `col` of column tile t; 0 outside the rows and columns in use.
 __device__ __forceinline__ double row_offset(const ProductArgs& g, int t, int row) {
     const size_t i = (size_t)t * g.span_m + row;
-    return row < g.span_m && i < g.nm ? g.cm[i] - g.refs[t] : 0.0;
+    return row < g.span_m && i < g.nm ? (g.cm[i] - g.refs[t]) * g.unit : 0.0;
 }
 __device__ __forceinline__ double col_offset(const ProductArgs& g, int t, int col) {
     const size_t i = (size_t)t * g.span_n + col;
-    return col < g.span_n && i < g.nn ? g.cn[i] - g.refs[g.m_tiles + t] : 0.0;
+    return col < g.span_n && i < g.nn ? (g.cn[i] - g.refs[g.m_tiles + t]) * g.unit
+                                         : 0.0;
 }
 
 __device__ __forceinline__ uint32_t neg2(uint32_t v) { return v ^ 0x80008000u; }
@@ -939,8 +949,6 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         const double ds = em * (2.0 * pm - em), dt = en * (2.0 * pn - en);
         const double e = r.k * ds * dt / (4.0 * dlo * dlo * dlo);
         const double big = std::max(ds, dt);
-        // The first-order factors dS and 4 pi q dT are f16 numbers.
-        if (!(big <= 3e4)) continue;
         // Second-order part of exp(iE): E^2/2 at the far corner of a tile and
         // of the ray box; its mean over the pairs is some fifty times smaller.
         if (!(0.5 * e * e <= 2.0 * tolerance)) continue;
@@ -985,6 +993,15 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         g->m_tiles = (int)mt;
         g->n_tiles = (int)nt;
         g->e_bound = e;
+        // The first-order factors dS and 4 pi q dT (whose product is E) and their
+        // products with phasors of up to 1 and kGridScale are f16 numbers: normal
+        // from 6e-5, finite to 65504. In mm dS and the other factor, k dT / (4 D^3),
+        // may lie anywhere (1 mm from an aperture the second passes 65504 times
+        // over, 50 m from one it is below 6e-5). With the largest dS within 1 .. 4
+        // the other operand is at most kGridScale E, and what either loses below 6e-5 is
+        // 3e-8 of its own largest value or of kGridScale.
+        const int half_exp = ds > 0.0 ? (int)std::floor(0.5 * std::ilogb(ds)) : 0;
+        g->unit = std::ldexp(1.0, -std::clamp(half_exp, -100, 100));
         // Below 2^-22 the change of the amplitude along a tile is lost in the
         // split phasors' own rounding.
         g->amp = std::max(sm, sn) + mq > 2.384185791015625e-7;
@@ -1091,7 +1108,8 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
     p.refs = axes_m + g.nm + g.nn;
     p.nm = g.nm;
     p.nn = g.nn;
-    p.h0 = g.h0;
+    p.unit = g.unit;
+    p.h0 = g.h0 / (g.unit * g.unit);
     p.partial = ws.partial.as<float>();
     p.m_pad = g.m_tiles * kTileM;
     p.n_pad = g.n_tiles * g.columns * (g.wide ? 2 : 1) * kFN;
@@ -1129,10 +1147,11 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         a.n = cnt;
         a.pad = pad;
         a.c0 = g.c0;
-        a.h0 = g.h0;
-        a.kt = g.kt;
-        a.kt_lo = g.kt_lo;
-        a.scale = g.inv_scale;
+        a.unit = g.unit;
+        a.h0 = p.h0;
+        a.kt = g.kt / g.unit;
+        a.kt_lo = g.kt_lo / g.unit;
+        a.scale = g.inv_scale * g.unit;
         grid_records_kernel<<<dim3((unsigned)blocks_of(pad, 256),
                                    (unsigned)(g.m_tiles * g.n_tiles)), 256, 0, stream>>>(
             a, ws.recs.as<float4>());

@@ -12,7 +12,7 @@ namespace xk {
 // What the device finds out about the order of a solve's screen points: point
 // i * len + l has one coordinate that depends on l alone (the inner axis), at
 // most one that depends on i alone (the outer axis), the rest constant, bit
-// for bit. extent[axis][k]: largest half-extent of a tile of 128 << k
+// for bit. extent[axis][k]: largest half-extent of a tile of kGridSpan << k
 // consecutive points of the axis (0 outer, 1 inner), as the bits of a double.
 constexpr int kGridSpan = 32;  // fewest rows or columns of a tile in use
 
@@ -50,6 +50,7 @@ struct GridPlan {
     size_t n = 0, chunk_rays = 0;            // rays, rays per product launch
     bool amp = false;                        // amplitude varies along a tile
     double c0 = 0.0, h0 = 0.0, k = 0.0, kt = 0.0, kt_lo = 0.0;
+    double unit = 1.0;  // the kernels' lengths are mm times this power of two
     double inv_scale = 0.0, e_bound = 0.0;
     RaysDev rays{};
     PixDev pix{};
