@@ -77,6 +77,7 @@ struct Form {
     static constexpr int kProdWarps = WIDE ? 8 : 12;
     static constexpr int kThreads = 32 + kFEpiThreads + 32 * kProdWarps + 32;
 };
+constexpr double kGridShare = 0.1;  // of the tolerance: the dropped orders of exp(iE)
 constexpr double kGridScale = 1024.0;  // largest |W|: lo parts stay normal f16 numbers
 constexpr size_t kGridRecBytes = (size_t)512 << 20;  // ray records of one launch
 constexpr size_t kGridMaxTiles = 4096;               // at least 2048 rays per launch fit then
@@ -129,16 +130,19 @@ __global__ void __launch_bounds__(256)
         if (bad) atomicOr(&out->bad, 1);
         if (mask) atomicOr(&out->outer_mask, mask);
     }
-    // Half extents of every tile of every size, one warp per tile. Sizes and axes
-    // share the warps' turns, so that a small screen takes one of them.
+    // Half extents of every tile of every size, one warp per tile (the sizes below
+    // 32 with those of 32). Sizes and axes share the warps' turns, so that a small
+    // screen takes one of them.
     const int warp = t0 >> 5, warps = step >> 5;
+    constexpr int kWarpSize = 2;  // kGridSpan << kWarpSize points: one per lane
+    static_assert(kGridSpan << kWarpSize == 32, "one point per lane");
     int base = 0;  // tiles of the sizes and axes before
     for (int axis = 0; axis < 2; ++axis)
-        for (int k = 0; k < 4; ++k) {
+        for (int k = kWarpSize; k < kGridSizes; ++k) {
             const int count = axis ? len : m / len, size = kGridSpan << k;
             const int tiles = (count + size - 1) / size;
             for (int t = (warp + warps - base % warps) % warps; t < tiles; t += warps) {
-                double half = 0.0;
+                double half = 0.0, part[kWarpSize] = {};  // whole tile; the sizes below 32
                 for (int c = 0; c < 3; ++c) {
                     if ((c == inner) != (axis == 1)) continue;
                     const double* a = coord(p, c);
@@ -148,14 +152,27 @@ __global__ void __launch_bounds__(256)
                         lo = fmin(lo, w);
                         hi = fmax(hi, w);
                     }
-                    for (int o = 16; o > 0; o >>= 1) {
-                        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-                        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+#pragma unroll
+                    for (int b = 0; b < 5; ++b) {
+                        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, 1 << b));
+                        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, 1 << b));
+#pragma unroll
+                        for (int p = 0; p < kWarpSize; ++p)  // -inf where a group has no point
+                            if (2 << b == kGridSpan << p) part[p] = fmax(part[p], 0.5 * (hi - lo));
                     }
                     half = fmax(half, 0.5 * (hi - lo));
                 }
                 if (lane == 0)
                     atomicMax(&out->extent[axis][k], (unsigned long long)__double_as_longlong(half));
+                if (k > kWarpSize) continue;
+#pragma unroll
+                for (int p = 0; p < kWarpSize; ++p) {
+                    for (int o = 16; o > 0; o >>= 1)
+                        part[p] = fmax(part[p], __shfl_xor_sync(0xffffffffu, part[p], o));
+                    if (lane == 0)
+                        atomicMax(&out->extent[axis][p],
+                                  (unsigned long long)__double_as_longlong(part[p]));
+                }
             }
             base += tiles;
         }
@@ -932,36 +949,44 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     bool found = false;
     double best_cost = 0.0, best_e = 0.0;
     // Tiles may use fewer rows (256 >> fm) or columns (of 128 >> fn; or 256) than they
-    // have: E falls with either, at the price of the rest, which is still below the
-    // general kernel's down to 1/16 of a tile (2^18 rays x 256^2 points +-1 mm at 1 m:
-    // 11.7 -> 1.9 ms at 10 keV, 12.1 -> 4.0 at 20, 12.4 -> 8.0 at 30).
-    for (int form = 0; form < 32; ++form) {
+    // have: E falls with either, at the price of the rest. For many rays that is below
+    // the general kernel's down to 1/16 of a tile (2^18 rays x 256^2 points +-1 mm at
+    // 1 m: 10.3 -> 4.0 ms at 10 keV, 12.0 -> 7.9 at 20, general at 30), for a few
+    // thousand, where the general kernel's sorting counts, down to 1/128 (3000 rays x
+    // 64 x 200 points at 0.3 m: 0.83 -> 0.48 ms).
+    const double d2 = dlo * dlo, d3 = d2 * dlo, d5 = d3 * d2;
+    for (int form = 0; form < 2 * kGridSizes * kGridSizes; ++form) {
         const bool swap = form & 1;
-        const int fm = (form >> 1) & 3, fn = (form >> 3) & 3;
-        const bool wide = fn == 3;
+        const int fm = (form >> 1) % kGridSizes, fn = (form >> 1) / kGridSizes;
+        const bool wide = fn == kGridSizes - 1;
         const int am = swap ? inner : outer, an = swap ? outer : inner;
         const size_t nm = swap ? len : rows, nn = swap ? rows : len;
-        const double em = bits_to_double(probe.extent[swap ? 1 : 0][3 - fm]);
-        const double en = bits_to_double(probe.extent[swap ? 0 : 1][wide ? 3 : 2 - fn]);
+        const double em = bits_to_double(probe.extent[swap ? 1 : 0][kGridSizes - 1 - fm]);
+        const double en = bits_to_double(
+            probe.extent[swap ? 0 : 1][wide ? kGridSizes - 1 : kGridSizes - 2 - fn]);
         // |dS| = |u| |(p - r) + (p0 - r)| with |p0 - r| <= |p - r|max - |u|max
         // when the tile lies inside the screen's range.
         const double pm = largest(del[am]), pn = largest(del[an]);
         const double ds = em * (2.0 * pm - em), dt = en * (2.0 * pn - en);
-        const double e = r.k * ds * dt / (4.0 * dlo * dlo * dlo);
+        const double e = r.k * ds * dt / (4.0 * d3);
         const double big = std::max(ds, dt);
-        // Second-order part of exp(iE): E^2/2 at the far corner of a tile and
-        // of the ray box; its mean over the pairs is some fifty times smaller.
-        if (!(0.5 * e * e <= 2.0 * tolerance)) continue;
-        if (!(big / (dlo * dlo) <= 1e-2)) continue;
+        // What 1 + iE leaves out of exp(i phase): E^2 / 2, and the next order of the
+        // mixed phase, 3/4 E (dS + dT) / D^2. Both at the far corner of a tile and of
+        // the ray box: on a screen beside the rays' axis nearly every ray has that E,
+        // and a focus on a tile's corner then has that error (rays of +-0.05 mm, 5.9 mm
+        // off both axes at 1 m: 1.5e-4 at E = 0.019). A tenth of the tolerance is
+        // about the general kernel's error on coherent fields.
+        if (!(0.5 * e * e + 0.75 * e * (ds + dt) / d2 <= kGridShare * tolerance)) continue;
+        if (!(big / d2 <= 1e-2)) continue;
         // Linear phase: an exact FP32 product up to 2^21 turns.
         if (!(kt / dlo * std::max(em * pm, en * pn) < 1.9e6)) continue;
         // FP32 terms: u^2 (h - h0) and the dropped third order of the root.
         if (!(0.5 * kt * (1.0 / dlo - 1.0 / dhi) * std::max(em * em, en * en) <= 24.0)) continue;
-        if (!(kt * big * big * big / (16.0 * std::pow(dlo, 5)) <= 1e-7)) continue;
+        if (!(kt * big * big * big / (16.0 * d5) <= 1e-7)) continue;
         // Amplitude: first order along each axis, mixed terms dropped.
         const double sm = largest({r.nlo[am], r.nhi[am]}) * em / (dlo * omin);
         const double sn = largest({r.nlo[an], r.nhi[an]}) * en / (dlo * omin);
-        const double mq = 0.5 * (1.0 + largest(nd) / omin) * big / (dlo * dlo);
+        const double mq = 0.5 * (1.0 + largest(nd) / omin) * big / d2;
         if (!(sm <= 0.25 && sn <= 0.25 && sm * sn <= 1e-6 && (sm + sn) * mq <= 1e-6 &&
               mq * mq <= 1e-7))
             continue;

@@ -14,7 +14,8 @@ namespace xk {
 // most one that depends on i alone (the outer axis), the rest constant, bit
 // for bit. extent[axis][k]: largest half-extent of a tile of kGridSpan << k
 // consecutive points of the axis (0 outer, 1 inner), as the bits of a double.
-constexpr int kGridSpan = 32;  // fewest rows or columns of a tile in use
+constexpr int kGridSpan = 8;   // fewest rows or columns of a tile in use
+constexpr int kGridSizes = 6;  // tile sizes, kGridSpan << 0 .. 5 (256)
 
 struct GridProbe {
     int len;         // inner length; 0 if there is no such order
@@ -22,7 +23,7 @@ struct GridProbe {
     int inner;       // coordinate index (0 x, 1 y, 2 z) of the inner axis
     int outer_mask;  // coordinates that vary with i
     // Largest half extent (bits of a double) of kGridSpan << k points, outer and inner.
-    unsigned long long extent[2][4];
+    unsigned long long extent[2][kGridSizes];
 };
 
 // Ranges of a solve's inputs (from the planner's summary).
