@@ -234,7 +234,8 @@ struct RecordArgs {
     size_t n, pad;       // rays of this launch, rounded up to whole blocks
     double c0;
     double unit;         // GridPlan::unit; what follows is in such lengths
-    double h0, kt, kt_lo, scale;
+    double h0, kt, kt_lo;
+    double scale[2];     // of either amplitude column
 };
 
 __global__ void __launch_bounds__(256) grid_records_kernel(RecordArgs g, float4* __restrict__ out) {
@@ -262,18 +263,19 @@ __global__ void __launch_bounds__(256) grid_records_kernel(RecordArgs g, float4*
     const double na = g.na[j], nb = g.nb[j], nc = g.nc[j];
     const double nu = (na * a + nb * b + nc * c) * inv;
     const double obl = g.nl[j] + nu;
-    const double w = obl * inv * g.scale;
+    const double w = obl * inv, w1 = w * g.scale[0];
     const double la = 2.0 * h * a, lb = 2.0 * h * b;
     const float lah = (float)la, lbh = (float)lb;
     o[0] = make_float4(lah, lbh, (float)(la - (double)lah), (float)(lb - (double)lbh));
     o[1] = make_float4((float)(2.0 * a), (float)(2.0 * b), (float)(h - g.h0),
                        (float)(-0.25 * h * inv * inv));
-    o[2] = make_float4((float)(turns - rint(turns)), (float)(g.w_re[j] * w), (float)(g.w_im[j] * w),
+    o[2] = make_float4((float)(turns - rint(turns)), (float)(g.w_re[j] * w1), (float)(g.w_im[j] * w1),
                        (float)(-0.5 * (1.0 + nu / obl) * inv * inv));
     float4 e = make_float4((float)(na * inv / obl), (float)(nb * inv / obl), 0.f, 0.f);
     if (g.w2_re) {
-        e.z = (float)(g.w2_re[j] * w);
-        e.w = (float)(g.w2_im[j] * w);
+        const double w2 = w * g.scale[1];
+        e.z = (float)(g.w2_re[j] * w2);
+        e.w = (float)(g.w2_im[j] * w2);
     }
     o[3] = e;
 }
@@ -833,13 +835,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
 }
 
 // Field of every screen point: the splits' sums in split order, times `scale`
-// (i k / (4 pi) over the f16 scaling). One column: (Es, Ep) = (pes, pep) A.
+// (i k / (4 pi) over the column's f16 scaling). One column: (Es, Ep) = (pes, pep) A.
 // Threads run along the columns, which are consecutive in the partials.
 __global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restrict__ partial,
                                                           int splits, int m_pad, int n_pad,
                                                           int columns, bool wide, int span_m,
                                                           int span_n, size_t nm, size_t nn,
-                                                          bool rows_outer, double scale,
+                                                          bool rows_outer, double2 scale,
                                                           double2 pes, double2 pep, FieldDev out) {
     const size_t idx = blockIdx.x * (size_t)256 + threadIdx.x;
     if (idx >= nm * nn) return;
@@ -860,9 +862,9 @@ __global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restric
         }
     // times i
     for (int c = 0; c < 2; ++c) {
-        const double t = re[c];
-        re[c] = -ie[c] * scale;
-        ie[c] = t * scale;
+        const double t = re[c], f = c ? scale.y : scale.x;
+        re[c] = -ie[c] * f;
+        ie[c] = t * f;
     }
     const size_t o = rows_outer ? idx : in * nm + im;
     if (columns == 1) {
@@ -913,7 +915,7 @@ Status grid_probe_enqueue(std::vector<ProbeArgs>& screens, cudaStream_t stream, 
 
 bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, int columns,
                double tolerance, int num_sms, GridPlan* g) {
-    if (probe.len < 2 || probe.bad || !(r.max_amp > 0.0)) return false;
+    if (probe.len < 2 || probe.bad || !(r.max_amp[0] > 0.0 || r.max_amp[1] > 0.0)) return false;
     const int inner = probe.inner;
     const int mask = probe.outer_mask;
     if (mask != 1 && mask != 2 && mask != 4) return false;
@@ -1050,8 +1052,15 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     g->inner_len = len;
     g->columns = columns;
     g->n = n;
-    g->inv_scale = kGridScale / (1.4142135623730951 * r.max_amp * omax / dlo);
-    if (!std::isfinite(g->inv_scale) || !std::isfinite(g->h0)) return false;
+    // Either column by its own largest amplitude: one scale for both left a column
+    // 1e-7 times the other's with 3e-4 of error, one 1e-10 times with none of its bits.
+    for (int c = 0; c < columns; ++c) {
+        g->inv_scale[c] = r.max_amp[c] > 0.0
+                              ? kGridScale / (1.4142135623730951 * r.max_amp[c] * omax / dlo)
+                              : 1.0;
+        if (!std::isfinite(g->inv_scale[c])) return false;
+    }
+    if (!std::isfinite(g->h0)) return false;
     const size_t tiles = (size_t)g->m_tiles * g->n_tiles;
     const size_t fit = std::max<size_t>(kGridRecBytes / (tiles * 64) / kFRays, 64) * kFRays;
     g->chunk_rays = std::min(blocks_of(n, kFRays) * kFRays, fit);
@@ -1176,7 +1185,7 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         a.h0 = p.h0;
         a.kt = g.kt / g.unit;
         a.kt_lo = g.kt_lo / g.unit;
-        a.scale = g.inv_scale * g.unit;
+        for (int c = 0; c < 2; ++c) a.scale[c] = g.inv_scale[c] * g.unit;
         grid_records_kernel<<<dim3((unsigned)blocks_of(pad, 256),
                                    (unsigned)(g.m_tiles * g.n_tiles)), 256, 0, stream>>>(
             a, ws.recs.as<float4>());
@@ -1189,10 +1198,10 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         p.stall = 0;
         *kernels += 2;
     }
+    const double amp = g.k / (4.0 * 3.14159265358979323846);
     grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
         p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.span_m, g.span_n, g.nm, g.nn,
-        g.rows_outer,
-        g.k / (4.0 * 3.14159265358979323846) / g.inv_scale, make_double2(g.pes[0], g.pes[1]),
+        g.rows_outer, make_double2(amp / g.inv_scale[0], amp / g.inv_scale[1]), make_double2(g.pes[0], g.pes[1]),
         make_double2(g.pep[0], g.pep[1]), g.out);
     XK_CUDA_TRY(cudaGetLastError());
     *kernels += 1;

@@ -34,7 +34,7 @@ struct GridRanges {
     double nl_lo, nl_hi;
     double rc[3], pc[3];    // centroids
     double spread2;         // mean squared ray distance from the centroid
-    double max_amp;         // largest amplitude component
+    double max_amp[2];      // largest component of either amplitude column summed
     double k;
 };
 
@@ -52,7 +52,7 @@ struct GridPlan {
     bool amp = false;                        // amplitude varies along a tile
     double c0 = 0.0, h0 = 0.0, k = 0.0, kt = 0.0, kt_lo = 0.0;
     double unit = 1.0;  // the kernels' lengths are mm times this power of two
-    double inv_scale = 0.0, e_bound = 0.0;
+    double inv_scale[2] = {1.0, 1.0}, e_bound = 0.0;
     RaysDev rays{};
     PixDev pix{};
     FieldDev out{};

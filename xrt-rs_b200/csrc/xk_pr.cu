@@ -57,7 +57,7 @@ namespace xk {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kSumFields = 40;
+constexpr int kSumFields = 41;
 // |e| bound under which the packed sweep's series reciprocal is used.
 constexpr double kSeriesRcpBound = 2e-3;
 // Fold the base phase when the estimated chunks per ray group reach this.
@@ -96,7 +96,7 @@ __host__ __device__ constexpr int sum_op(int i) {
         case 14: case 15: case 16:
         case 23: case 24: case 25:
         case 27:                       // polarization deviation
-        case 32:                       // largest amplitude component
+        case 32: case 40:              // largest component of es, of ep
         case 35:
             return OP_MAX;
         default:  // 0-2 ray and 17-19 screen position sums, 26 non-finite probe, 28-31
@@ -113,8 +113,8 @@ __device__ __forceinline__ double op_combine(int op, double a, double b) {
 // sums every input value times zero: 0 when all are finite, NaN otherwise
 // (fmin / fmax skip NaN, so the boxes alone would not show it). Fields 27-31
 // test whether all rays share ray 0's polarization: the largest relative
-// |es_j ep_0 - ep_j es_0|, and ray 0's (es, ep); field 32 is the largest
-// amplitude component. Field 33 is the first point at which a coordinate that
+// |es_j ep_0 - ep_j es_0|, and ray 0's (es, ep); fields 32 and 40 are the largest
+// components of es and of ep. Field 33 is the first point at which a coordinate that
 // points 0 and 1 share changes: the inner length if the screen is rectangular
 // (infinite if points 0 and 1 differ in none or several coordinates). Clears
 // `probe` for the check of that order. The last block combines the rows into row
@@ -180,7 +180,8 @@ __global__ void __launch_bounds__(256)
         const double nrm = sqrt(ar * ar + ai * ai) * b0n + sqrt(br * br + bi * bi) * a0n;
         const double dn = sqrt(dr * dr + di * di);
         f[27] = fmax(f[27], nrm > 0.0 ? dn / nrm : (dn > 0.0 ? INFINITY : 0.0));
-        f[32] = fmax(f[32], fmax(fmax(fabs(ar), fabs(ai)), fmax(fabs(br), fabs(bi))));
+        f[32] = fmax(f[32], fmax(fabs(ar), fabs(ai)));
+        f[40] = fmax(f[40], fmax(fabs(br), fabs(bi)));
         if (i == 0) {
             f[28] += ar;
             f[29] += ai;
@@ -1749,7 +1750,9 @@ Status try_grid(const PrSolveIn& in, const GridProbe& probe, const HostSolveInfo
     r.spread2 = std::max(0.0, f[36] / (double)in.n - off2);
     r.nl_lo = f[34];
     r.nl_hi = f[35];
-    r.max_amp = f[32];
+    const int first = P->one_pol && P->dev.amp_src ? 1 : 0;  // amplitude column summed first
+    r.max_amp[0] = first ? f[40] : f[32];
+    r.max_amp[1] = P->one_pol ? 0.0 : f[40];
     r.k = I.k;
     GridPlan& g = P->grid_plan;
     if (!grid_plan(probe, r, in.n, in.m, P->one_pol ? 1 : 2, o.tolerance, num_sms, &g))
@@ -1758,7 +1761,6 @@ Status try_grid(const PrSolveIn& in, const GridProbe& probe, const HostSolveInfo
     g.pix = in.pix;
     g.out = in.out;
     const double* amps[2][2] = {{in.rays.es_re, in.rays.es_im}, {in.rays.ep_re, in.rays.ep_im}};
-    const int first = P->one_pol && P->dev.amp_src ? 1 : 0;
     for (int c = 0; c < g.columns; ++c)
         for (int k = 0; k < 2; ++k) g.amps[c][k] = amps[first + c][k];
     for (int k = 0; k < 2; ++k) {
@@ -1884,7 +1886,8 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
             P.route_reason = 7;
             continue;
         }
-        if (f[32] > kF32AmpMax || (f[32] > 0.0 && f[32] < kF32AmpMin)) {
+        const double most = std::max(f[32], f[40]);
+        if (most > kF32AmpMax || (most > 0.0 && most < kF32AmpMin)) {
             P.routed = true;
             P.route_reason = 8;
             continue;
