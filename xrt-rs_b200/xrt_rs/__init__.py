@@ -126,13 +126,22 @@ def _ptr(a):
     return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
-def _columns(cls, arrays):
-    """A struct of pointers to the arrays (numpy arrays or device tensors), filled
-    in one step: one ctypes cast per column costs more than a small launch."""
-    ptrs = [int(a.data_ptr()) if hasattr(a, "data_ptr") else a.ctypes.data for a in arrays]
-    if ctypes.sizeof(cls) != 8 * len(ptrs):
-        raise ValueError(f"expected {ctypes.sizeof(cls) // 8} arrays, got {len(ptrs)}")
-    return cls.from_buffer_copy(struct.pack(f"{len(ptrs)}Q", *ptrs))
+def _pointers(cls, ptrs):
+    """A struct of pointers (null where none is given), filled in one step: one ctypes
+    cast per column costs more than a small launch."""
+    size = ctypes.sizeof(cls) // 8
+    if len(ptrs) > size:
+        raise TypeError("too many initializers")
+    return cls.from_buffer_copy(struct.pack(f"{size}Q", *ptrs, *[0] * (size - len(ptrs))))
+
+
+def _host_columns(cls, arrays):
+    return _pointers(cls, [a.ctypes.data for a in arrays])
+
+
+def _device_columns(cls, tensors):
+    # Nothing but data_ptr(): a host array's address must not reach a kernel.
+    return _pointers(cls, [int(t.data_ptr()) for t in tensors])
 
 
 def _check_lengths(pairs):
@@ -168,9 +177,9 @@ def diffraction_integral(rays, pixels, path="f64", ctx=None, return_stats=False)
     out = [np.zeros(m, dtype=np.float64) for _ in range(4)]
     ctx = _require_ctx(ctx)
     lib = _lib.load()
-    xr = _columns(_lib.XkRays, r)
-    xp = _columns(_lib.XkPixels, p)
-    xf = _columns(_lib.XkField, out)
+    xr = _host_columns(_lib.XkRays, r)
+    xp = _host_columns(_lib.XkPixels, p)
+    xf = _host_columns(_lib.XkField, out)
     st = _lib.XkStats()
     rc = lib.xk_diffraction_integral(ctx.handle, ctypes.byref(xr), n, ctypes.byref(xp), m,
                                      ctypes.byref(xf), path_code, ctypes.byref(st))
@@ -209,9 +218,9 @@ def diffraction_integral_device(rays, pixels, out, path="f32pr", ctx=None, strea
         out = [out[k] for k in FIELD_FIELDS]
     n = int(rays[0].numel()) if hasattr(rays[0], "numel") else len(rays[0])
     m = int(pixels[0].numel()) if hasattr(pixels[0], "numel") else len(pixels[0])
-    xr = _columns(_lib.XkRays, rays)
-    xp = _columns(_lib.XkPixels, pixels)
-    xf = _columns(_lib.XkField, out)
+    xr = _device_columns(_lib.XkRays, rays)
+    xp = _device_columns(_lib.XkPixels, pixels)
+    xf = _device_columns(_lib.XkField, out)
     st = _lib.XkStats()
     s = ctypes.c_void_p(int(stream)) if stream is not None else None
     rc = lib.xk_diffraction_integral_device(ctx.handle, ctypes.byref(xr), n, ctypes.byref(xp), m,
