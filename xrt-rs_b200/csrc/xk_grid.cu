@@ -80,6 +80,10 @@ struct Form {
 constexpr double kGridShare = 0.1;  // of the tolerance: the dropped orders of exp(iE)
 constexpr double kGridScale = 1024.0;  // largest |W|: lo parts stay normal f16 numbers
 constexpr size_t kGridRecBytes = (size_t)512 << 20;  // ray records of one launch
+constexpr size_t kGridPartialBytes = (size_t)1 << 30;  // of the splits' partials
+// FP32 additions into one partial: of random phasors N lose 1.8e-8 sqrt(N) of the sum
+// (4e-7 here, below what one-block segments lose in the tensor cores; 3.3e-6 at 32768).
+constexpr int kGridMaxAdds = 512;
 constexpr size_t kGridMaxTiles = 4096;               // at least 2048 rays per launch fit then
 
 // ---- order of the screen points -------------------------------------------------
@@ -293,7 +297,6 @@ struct ProductArgs {
     double unit, h0;  // GridPlan::unit; turns per squared such length
     float* partial;  // [splits][m_pad][n_pad], in the order of partial_at
     int m_pad, n_pad;
-    bool first;      // the splits' first segments store
     int* err;
     uint32_t wait_limit, stall;
 };
@@ -600,7 +603,7 @@ __device__ __forceinline__ void grid_drain(const ProductArgs& g, int warp, int l
     int drains = (nrb + g.seg - 1) / g.seg;
     if (WIDE) drains += 1 + (max(0, nrb - max(1, g.seg / 2)) + g.seg - 1) / g.seg;
     if (nrb == 0) {
-        for (int c = lane; g.first && c < F::kAcc * kBlocks * kBlock; c += 32) row[c] = 0.f;
+        for (int c = lane; c < F::kAcc * kBlocks * kBlock; c += 32) row[c] = 0.f;
         return;
     }
     int buf = 0;
@@ -639,7 +642,7 @@ __device__ __forceinline__ void grid_drain(const ProductArgs& g, int warp, int l
                     // The previous segment's operation on this block is performed.
                     bulk_wait_but<F::kAcc * kBlocks - 1>();
                     float* to = dst + (c + h) * kBlock;
-                    if (seg == 0 && g.first)
+                    if (seg == 0)
                         bulk_s2g(to, smem_u32(sb), kDrainBytes);
                     else
                         bulk_add_s2g_f32(to, smem_u32(sb), kDrainBytes);
@@ -836,13 +839,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
 
 // Field of every screen point: the splits' sums in split order, times `scale`
 // (i k / (4 pi) over the column's f16 scaling). One column: (Es, Ep) = (pes, pep) A.
-// Threads run along the columns, which are consecutive in the partials.
+// `add`: to what earlier launches' rays left there. Threads run along the columns,
+// which are consecutive in the partials.
 __global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restrict__ partial,
                                                           int splits, int m_pad, int n_pad,
                                                           int columns, bool wide, int span_m,
                                                           int span_n, size_t nm, size_t nn,
                                                           bool rows_outer, double2 scale,
-                                                          double2 pes, double2 pep, FieldDev out) {
+                                                          double2 pes, double2 pep, bool add,
+                                                          FieldDev out) {
     const size_t idx = blockIdx.x * (size_t)256 + threadIdx.x;
     if (idx >= nm * nn) return;
     const size_t im = idx / nn, in = idx - im * nn;
@@ -867,17 +872,23 @@ __global__ void __launch_bounds__(256) grid_reduce_kernel(const float* __restric
         ie[c] = t * f;
     }
     const size_t o = rows_outer ? idx : in * nm + im;
+    double f[4] = {re[0], ie[0], re[1], ie[1]};
     if (columns == 1) {
-        out.es_re[o] = pes.x * re[0] - pes.y * ie[0];
-        out.es_im[o] = pes.x * ie[0] + pes.y * re[0];
-        out.ep_re[o] = pep.x * re[0] - pep.y * ie[0];
-        out.ep_im[o] = pep.x * ie[0] + pep.y * re[0];
-    } else {
-        out.es_re[o] = re[0];
-        out.es_im[o] = ie[0];
-        out.ep_re[o] = re[1];
-        out.ep_im[o] = ie[1];
+        f[0] = pes.x * re[0] - pes.y * ie[0];
+        f[1] = pes.x * ie[0] + pes.y * re[0];
+        f[2] = pep.x * re[0] - pep.y * ie[0];
+        f[3] = pep.x * ie[0] + pep.y * re[0];
     }
+    if (add) {
+        f[0] += out.es_re[o];
+        f[1] += out.es_im[o];
+        f[2] += out.ep_re[o];
+        f[3] += out.ep_im[o];
+    }
+    out.es_re[o] = f[0];
+    out.es_im[o] = f[1];
+    out.ep_re[o] = f[2];
+    out.ep_im[o] = f[3];
 }
 
 // ---- host ------------------------------------------------------------------------------
@@ -895,6 +906,12 @@ double largest(Range a) { return std::max(std::fabs(a.lo), std::fabs(a.hi)); }
 size_t blocks_of(size_t n, size_t size) { return (n + size - 1) / size; }
 
 const double* coord_host(const PixDev& p, int c) { return c == 0 ? p.x : (c == 1 ? p.y : p.z); }
+
+// Bytes of one split's partial.
+size_t partial_plane(const GridPlan& g) {
+    return (size_t)g.m_tiles * kTileM * g.n_tiles * g.columns * (g.wide ? 2 : 1) * kFN *
+           sizeof(float);
+}
 
 double bits_to_double(unsigned long long b) {
     double d;
@@ -1061,25 +1078,6 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         if (!std::isfinite(g->inv_scale[c])) return false;
     }
     if (!std::isfinite(g->h0)) return false;
-    const size_t tiles = (size_t)g->m_tiles * g->n_tiles;
-    const size_t fit = std::max<size_t>(kGridRecBytes / (tiles * 64) / kFRays, 64) * kFRays;
-    g->chunk_rays = std::min(blocks_of(n, kFRays) * kFRays, fit);
-    g->ray_blocks = (int)blocks_of(n, kFRays);
-    // Ray splits: whole waves of CTA pairs, a split at least ten blocks long.
-    const size_t units = std::max(1, num_sms / 2), work = tiles * columns;
-    const size_t most = std::max<size_t>(1, g->chunk_rays / kFRays / 10);
-    size_t s = work >= units ? 1 : units / work;
-    if (work > units) {
-        double best = 1e300;
-        for (size_t t = 1; t <= 8; ++t) {
-            const double cost = (double)blocks_of(work * t, units) / t + 0.01 * t;
-            if (cost < best) {
-                best = cost;
-                s = t;
-            }
-        }
-    }
-    g->splits = (int)std::max<size_t>(1, std::min(s, most));
     // Blocks per segment. The tensor cores truncate when they accumulate, 16 MMAs
     // per block: on top of 3.5e-7 (sine and cosine of both factors) the error
     // against 64 bits is 4.7e-7, 6.5e-7, 8.3e-7 and 2.4e-6 of the field at 1, 2,
@@ -1096,6 +1094,33 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         r.k * (r.spread2 + 0.6 * side * std::sqrt(r.spread2)) / (2.0 * d0);
     if (phase < 7.0) return false;
     g->seg = phase < 12.0 ? 1 : phase < 24.0 ? 3 : 10;
+    // Rays per launch: what their records' memory allows, and what `cap` splits can sum
+    // in kGridMaxAdds segments each (a launch is added to the field in FP64).
+    const size_t tiles = (size_t)g->m_tiles * g->n_tiles;
+    const size_t cap = std::max<size_t>(1, kGridPartialBytes / partial_plane(*g));
+    const size_t segs = (size_t)kGridMaxAdds * g->seg;  // blocks per split
+    const size_t fit = std::max<size_t>(kGridRecBytes / (tiles * 64) / kFRays, 64);
+    g->ray_blocks = (int)blocks_of(n, kFRays);
+    const size_t blocks = std::min<size_t>((size_t)g->ray_blocks, std::min(fit, cap * segs));
+    g->chunk_rays = blocks * kFRays;
+    // Ray splits: whole waves of CTA pairs, a split at least ten blocks and at most
+    // kGridMaxAdds segments long.
+    const size_t units = std::max(1, num_sms / 2), work = tiles * columns;
+    const size_t least = blocks_of(blocks, segs);
+    const size_t most = std::min(cap, std::max(least, blocks / 10));
+    size_t s = std::max<size_t>(1, units / work);
+    if (work > units || s < least) {
+        double best = 1e300;
+        for (size_t t = least; t < least + std::max<size_t>(8, units / work); ++t) {
+            const double waves = (double)blocks_of(work * t, units) * units / (double)(work * t);
+            const double cost = waves + 0.01 * (double)(t - least) * std::min(1.0, (double)units / work);
+            if (cost < best) {
+                best = cost;
+                s = t;
+            }
+        }
+    }
+    g->splits = (int)std::min(s, most);
     return true;
 }
 
@@ -1111,8 +1136,7 @@ Status grid_axes_enqueue(const GridPlan& g, cudaStream_t stream) {
 void grid_sizes(const GridPlan& g, size_t* recs, size_t* partial) {
     const size_t tiles = (size_t)g.m_tiles * g.n_tiles;
     *recs = std::max(*recs, tiles * g.chunk_rays * 64);
-    *partial = std::max(*partial, (size_t)g.splits * g.m_tiles * kTileM * g.n_tiles * g.columns *
-                                      (g.wide ? 2 : 1) * kFN * sizeof(float));
+    *partial = std::max(*partial, g.splits * partial_plane(g));
 }
 
 Status grid_reserve(size_t recs, size_t partial, GridWorkspace& ws) {
@@ -1159,6 +1183,7 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
     XK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem));
     const dim3 grid((unsigned)(2 * g.m_tiles), (unsigned)(g.n_tiles * g.columns),
                     (unsigned)g.splits);
+    const double amp = g.k / (4.0 * 3.14159265358979323846);
     for (size_t j0 = 0; j0 < g.n; j0 += g.chunk_rays) {
         const size_t cnt = std::min(g.chunk_rays, g.n - j0), pad = blocks_of(cnt, kFRays) * kFRays;
         RecordArgs a{};
@@ -1192,19 +1217,16 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         XK_CUDA_TRY(cudaGetLastError());
         p.pad = pad;
         p.ray_blocks = (int)(pad / kFRays);
-        p.first = j0 == 0;
         kern<<<grid, threads, kGSmem, stream>>>(p);
         XK_CUDA_TRY(cudaGetLastError());
         p.stall = 0;
-        *kernels += 2;
+        grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
+            p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.span_m, g.span_n, g.nm,
+            g.nn, g.rows_outer, make_double2(amp / g.inv_scale[0], amp / g.inv_scale[1]),
+            make_double2(g.pes[0], g.pes[1]), make_double2(g.pep[0], g.pep[1]), j0 > 0, g.out);
+        XK_CUDA_TRY(cudaGetLastError());
+        *kernels += 3;
     }
-    const double amp = g.k / (4.0 * 3.14159265358979323846);
-    grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
-        p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.span_m, g.span_n, g.nm, g.nn,
-        g.rows_outer, make_double2(amp / g.inv_scale[0], amp / g.inv_scale[1]), make_double2(g.pes[0], g.pes[1]),
-        make_double2(g.pep[0], g.pep[1]), g.out);
-    XK_CUDA_TRY(cudaGetLastError());
-    *kernels += 1;
     return Status::Ok();
 }
 
