@@ -147,6 +147,10 @@ __global__ void __launch_bounds__(256)
     const int n = A.n, m = A.m, block = (int)blockIdx.x - A.first;
     double* const block_out = A.block_out;
     if (block == 0 && threadIdx.x == 0) *A.probe = GridProbe{};
+    // Fields 32 and 40 as floats, rounded up: as doubles they cost the registers of the
+    // second block per SM (2^18 rays x 256^2 points: 33 us so, 40 as doubles, 30.5 with
+    // one double for both).
+    float amp[2] = {0.f, 0.f};
     double f[kSumFields];
 #pragma unroll
     for (int i = 0; i < kSumFields; ++i)
@@ -180,8 +184,8 @@ __global__ void __launch_bounds__(256)
         const double nrm = sqrt(ar * ar + ai * ai) * b0n + sqrt(br * br + bi * bi) * a0n;
         const double dn = sqrt(dr * dr + di * di);
         f[27] = fmax(f[27], nrm > 0.0 ? dn / nrm : (dn > 0.0 ? INFINITY : 0.0));
-        f[32] = fmax(f[32], fmax(fabs(ar), fabs(ai)));
-        f[40] = fmax(f[40], fmax(fabs(br), fabs(bi)));
+        amp[0] = fmaxf(amp[0], __double2float_ru(fmax(fabs(ar), fabs(ai))));
+        amp[1] = fmaxf(amp[1], __double2float_ru(fmax(fabs(br), fabs(bi))));
         if (i == 0) {
             f[28] += ar;
             f[29] += ai;
@@ -205,6 +209,13 @@ __global__ void __launch_bounds__(256)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < kSumFields; ++i) {
+        if (i == 32 || i == 40) {
+            float v = amp[i == 40];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
+            if (lane == 0) sm[warp][i] = v;
+            continue;
+        }
         double v = f[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = op_combine(sum_op(i), v, __shfl_xor_sync(kFull, v, o));
