@@ -181,13 +181,6 @@ xk::Status create_batch(xk_ctx* ctx, const xk_solve* solves, size_t n, int path,
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 
     XK_TRY(xk::pr_reserve_exec(b->ws, (int)n, ctx->num_sms));
-    // The products' scratch at once, at its largest: growing it solve by solve
-    // mapped new memory each time (planning a process's first batch of 64 uneven
-    // solves took 0.27 s, 0.05 so).
-    size_t rec_bytes = 0, partial_bytes = 0;
-    for (const xk::PrPlan& P : b->plans)
-        if (!P.routed && P.grid) xk::grid_sizes(P.grid_plan, &rec_bytes, &partial_bytes);
-    XK_TRY(xk::grid_reserve(rec_bytes, partial_bytes, b->ws.grid));
     if ((flags & XK_BATCH_NO_GRAPH) == 0) {
         XK_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         xk::Status st = enqueue_batch(b);
