@@ -312,14 +312,14 @@ __global__ void pixel_keys_kernel(PixDev p, int m, Frame fr, uint64_t* __restric
 // One warp per tile: slot table, slot-ordered coordinates, bounding-box
 // centre; the largest radius of any tile, its largest extents across and along
 // the frame's long axis u0 (amax_bits[0..2]) and the sum of the tiles' extents
-// across (amax_bits[3], a double), which the last block writes to pinned host
-// memory.
+// across (amax_bits[3], in units of 1 / sum_scale: an integer, so that it does not
+// depend on the order of the tiles), which the last block writes to pinned host memory.
 // Centres are snapped to multiples of `quantum` as the chunk centres are, so
 // that differences between points, tile and chunk centres are exact. rel, ns:
 // each slot's offset from the centre (PrSolve::tile_rel); n2 = 2 n for solves
 // of one normal.
 __global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, double quantum,
-                            double inv_quantum, double3 n2,
+                            double inv_quantum, double sum_scale, double3 n2,
                             const int* __restrict__ sorted_idx, double4* __restrict__ rel,
                             float* __restrict__ ns, int* __restrict__ tile_perm, double* __restrict__ tpx,
                             double* __restrict__ tpy, double* __restrict__ tpz,
@@ -384,12 +384,14 @@ __global__ void tile_kernel(PixDev p, int m, int n_tiles, Frame fr, double quant
             atomicMax(amax_bits, (unsigned long long)__double_as_longlong(rad));
             atomicMax(amax_bits + 1, (unsigned long long)__double_as_longlong(across));
             atomicMax(amax_bits + 2, (unsigned long long)__double_as_longlong(along));
-            atomicAdd(reinterpret_cast<double*>(amax_bits + 3), across);
+            atomicAdd(amax_bits + 3, (unsigned long long)rint(across * sum_scale));
         }
     }
-    if (last_block(ticket) && threadIdx.x < 4)
+    if (last_block(ticket) && threadIdx.x < 4) {
+        const unsigned long long v = __ldcg(amax_bits + threadIdx.x);
         host_out[threadIdx.x] =
-            __longlong_as_double((long long)__ldcg(amax_bits + threadIdx.x));
+            threadIdx.x < 3 ? __longlong_as_double((long long)v) : (double)v / sum_scale;
+    }
 }
 
 struct CellGrid {
@@ -2055,8 +2057,13 @@ Status pr_plan(const PrSolveIn* in, int count, PrWorkspace& ws, cudaStream_t str
         XK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws.cub_tmp.ptr, tmp, B.pk_in, B.pk_out, B.pi_in,
                                                     B.pi_out, m, pf.scale[2] > 0.0 ? 0 : 21, 53,
                                                     stream));
+        // No tile reaches further than the screen's diagonal, below 2 units of 2^e; 2^22
+        // tiles (2^30 points) of 2^41 fit in 64 bits.
+        double diag = 0.0;
+        for (int a = 0; a < 3; ++a) diag = std::hypot(diag, I.phi[a] - I.plo[a]);
+        const double sum_scale = diag > 0.0 ? std::ldexp(1.0, 40 - std::ilogb(diag)) : 1.0;
         tile_kernel<<<(n_tiles[s] * 32 + 255) / 256, 256, 0, stream>>>(
-            in[s].pix, m, n_tiles[s], pf, I.quantum, 1.0 / I.quantum,
+            in[s].pix, m, n_tiles[s], pf, I.quantum, 1.0 / I.quantum, sum_scale,
             make_double3(2.0 * I.f[11], 2.0 * I.f[12], 2.0 * I.f[13]), B.pi_out, B.rel, B.ns,
             B.tile_perm, B.tpx, B.tpy, B.tpz, B.tile_center,
             B.amax, tickets + 4 * s + 2, h_amax + 4 * s);
