@@ -231,9 +231,12 @@ __device__ __forceinline__ void stage_rays_role(const FusedArgs& g, int lane, in
             er = __ldg(g.er + j);
             ei = __ldg(g.ei + j);
         }
-        if (i >= kFRayBufs &&
-            !mbar_wait(&ray_empty[rb], (uint32_t)(i / kFRayBufs - 1) & 1u, g.wait_limit))
+        const bool ok = i < kFRayBufs || mbar_wait(&ray_empty[rb],
+                                                   (uint32_t)(i / kFRayBufs - 1) & 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
             *flag = 1;
+            return;
+        }
         float xh, xl, xf, zh, zl, zf;
         split_coord(x - g.ox, g.a_turns, &xh, &xl, &xf);
         split_coord(z - g.oz, g.a_turns, &zh, &zl, &zf);
@@ -374,8 +377,11 @@ __global__ void __launch_bounds__(kFThreads, 1) fresnel_fused_kernel(FusedArgs g
         for (int i = 0; i < nrb; ++i) {
             const int s = i % kFStages, rb = i % kFRayBufs;
             bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kFRayBufs) & 1u, g.wait_limit);
-            ok = mbar_wait(&empty[s], ((uint32_t)(i / kFStages) & 1u) ^ 1u, g.wait_limit) && ok;
-            if (!ok) *flag = 1;
+            ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kFStages) & 1u) ^ 1u, g.wait_limit);
+            if (!__all_sync(0xffffffffu, ok)) {
+                *flag = 1;
+                break;
+            }
             unsigned char* base = tiles + (size_t)s * kFStage;
             const float4* sr = reinterpret_cast<const float4*>(rays_smem + rb * kFRayBytes);
 #pragma unroll 1
@@ -522,8 +528,11 @@ __device__ __forceinline__ void pair_producer(const FusedArgs& g, int c0, int r,
     for (int i = 0; i < nrb; ++i) {
         const int s = i % kPStages, rb = i % kFRayBufs;
         bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kFRayBufs) & 1u, g.wait_limit);
-        ok = mbar_wait(&empty[s], ((uint32_t)(i / kPStages) & 1u) ^ 1u, g.wait_limit) && ok;
-        if (!ok) *flag = 1;
+        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kPStages) & 1u) ^ 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *flag = 1;
+            return;
+        }
         unsigned char* base = tiles + (size_t)s * kPStage;
         unsigned char* bhi = base + 2 * kPA;
         unsigned char* blo = bhi + kPB;
@@ -795,8 +804,11 @@ __device__ __forceinline__ void wide_producer(const FusedArgs& g, int w, int lan
     for (int i = 0; i < nrb; ++i) {
         const int s = i % kWStages, rb = i % kFRayBufs;
         bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kFRayBufs) & 1u, g.wait_limit);
-        ok = mbar_wait(&empty[s], ((uint32_t)(i / kWStages) & 1u) ^ 1u, g.wait_limit) && ok;
-        if (!ok) *flag = 1;
+        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kWStages) & 1u) ^ 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *flag = 1;
+            return;
+        }
         unsigned char* base = tiles + (size_t)s * kWStage;
         const float4* sr =
             reinterpret_cast<const float4*>(rays_smem + rb * kFRayBytes) + 2 * (8 * oct + 4 * sub);
