@@ -921,7 +921,7 @@ __device__ __forceinline__ void prep_stage(PrRawRay* buf, int len, int lane, con
 }
 
 // Adds the lane's FP32 partials into its two-float accumulators and clears
-// them (at most kPrStage rays apart, and at item ends).
+// them (after every stage, that is at most kPrStage rays of one chunk).
 // One-polarization kernels (POL) carry components 0 and 1 only.
 template <bool POL, bool UNIFORM, class WS>
 __device__ __forceinline__ void fold_acc(ScalarState<UNIFORM>& ls, WS& ws, int lane) {
@@ -1147,7 +1147,6 @@ __device__ bool process_item(const PrSolve& sv, long long local, WarpPipe& wp,
     using State = typename std::conditional<FAST, PackedState<UNIFORM>, ScalarState<UNIFORM>>::type;
     State st;
     clear_acc(st);
-    int since_fold = 0;  // rays summed in FP32 since the last fold
     int cur_chunk = -1;
     int geo_first = -64;  // FOLD: first of the 32 chunks whose geometry is in `ws`
     int pos = r0;
@@ -1228,13 +1227,10 @@ __device__ bool process_item(const PrSolve& sv, long long local, WarpPipe& wp,
         }
         __syncwarp();
         sweep_stage<UNIFORM, FOLD, POL, LIN>(wp.buf[b], len, lane, st, ws);
-        // FP32 partials run over at most one full stage of rays, of one chunk or
-        // (folded) of several short ones.
-        since_fold += len;
-        if (since_fold + nlen > kPrStage || nlen == 0 || (!FOLD && nc != c)) {
-            fold_acc<POL>(st, ws, lane);
-            since_fold = 0;
-        }
+        // FP32 partials hold one stage of one chunk. (Over several short chunks they
+        // saved 8 % between mirrors, 2.6 % on the near-field screen, and cost a tenth of
+        // the error between mirrors: 3.7e-7 instead of 3.3e-7.)
+        fold_acc<POL>(st, ws, lane);
         // Order this stage's generic-proxy accesses before the next bulk
         // copy into the same buffer.
         fence_proxy_async();
@@ -1410,10 +1406,11 @@ struct DepthCells {
 
 // Residual phase bounds [rad] such cells are sized for. The ball bound kept the
 // true phases of these solves, and so their errors, below what the budget
-// allows; these bounds keep the errors where they were. Deep tiles: 6 rad in the
-// mean tile, 60 in the widest (mirror to mirror, 6e4 rays x 5e4 points: 35.8 ms
-// and 2.9e-7 with the ball bound, 9.7 ms and 3.5e-7 so, 7.4 ms and 4.3e-7 at 10
-// and 100, 6.3 ms and 4.9e-7 at 20 and 100). Flat tiles: a share of the budget.
+// allows; these bounds keep the errors near that. Deep tiles: 6 rad in the
+// mean tile, 60 in the widest: ten pairs of mirrors, 4 to 19 keV and 3 to 8.5 m apart,
+// take 0.08 to 0.6 of the ball bound's time at 3.3e-7 to 4.7e-7 instead of 2.7e-7 to
+// 3.0e-7 (6e4 rays x 5e4 points at 3 m: 35.8 ms and 2.7e-7 with the ball bound, 10.0 ms
+// and 3.3e-7 so). Flat tiles: a share of the budget.
 constexpr double kDeepTileBudget = 6.0, kDeepWideBudget = 60.0;
 constexpr double kDepthShare = 0.3;
 
