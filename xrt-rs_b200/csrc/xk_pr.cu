@@ -1578,13 +1578,18 @@ int sum_parts(size_t n, size_t m, int sum_blocks) {
 
 int sum_blocks_for(int num_sms) { return std::min(512, std::max(1, 2 * num_sms)); }
 
+// Items per resident warp: the caller's or an autotuned setting.
+long long items_per_warp(int n, int m, const PrOptions& opt) {
+    long long ipw = opt.items_per_warp;
+    if (opt.tune && opt.tune->use) opt.tune->find_ipw((size_t)n, (size_t)m, &ipw);
+    return ipw;
+}
+
 // Ray groups per tile: enough items to keep every resident warp busy, at
 // least four stages of rays per item, partial slots within 1 GiB.
 int plan_groups_large(int n, int m, int n_tiles, int num_sms, const PrOptions& opt) {
     if (opt.groups > 0) return std::min(opt.groups, kMaxGroups);
-    long long ipw = opt.items_per_warp;
-    if (opt.tune && opt.tune->use) opt.tune->find_ipw((size_t)n, (size_t)m, &ipw);
-    long long want = (long long)num_sms * 12 * ipw;
+    long long want = (long long)num_sms * 12 * items_per_warp(n, m, opt);
     int g = (int)std::max<long long>(1, (want + n_tiles - 1) / n_tiles);
     g = std::min(g, std::max(1, n / (4 * kPrStage)));
     long long cap = (1LL << 30) / (32LL * n_tiles * kPrTile);
@@ -1595,11 +1600,14 @@ int plan_groups_large(int n, int m, int n_tiles, int num_sms, const PrOptions& o
 // The same, and where that leaves less than four items per resident warp (a
 // line of 256 points is one tile: 44 items on 1776 warps with 10^4 rays), the
 // count that minimises rounds of items x (rays per item + the item's fixed
-// cost), items as small as kPrMinItem rays.
+// cost), items as small as kPrMinItem rays. A number of items per warp that is not the
+// default stands as it is.
 int plan_groups(int n, int m, int n_tiles, int num_sms, const PrOptions& opt) {
     const int base = plan_groups_large(n, m, n_tiles, num_sms, opt);
     const long long warps = (long long)num_sms * 12;
-    if (opt.groups > 0 || (long long)base * n_tiles >= 4 * warps) return base;
+    if (opt.groups > 0 || items_per_warp(n, m, opt) != PrOptions{}.items_per_warp ||
+        (long long)base * n_tiles >= 4 * warps)
+        return base;
     constexpr double kItemCost = 60.0;  // set-up, flush and pipeline fill of an item, in rays
     const long long cap = (1LL << 30) / (32LL * n_tiles * kPrTile);
     const int most = (int)std::min<long long>(std::min(n / kPrMinItem, kMaxGroups), cap);
