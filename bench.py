@@ -900,20 +900,7 @@ def main():
         b = np.concatenate([out64[0] + 1j * out64[1], out64[2] + 1j * out64[3]])
         ia = np.abs(a[:m]) ** 2 + np.abs(a[m:]) ** 2
         ib = np.abs(b[:m]) ** 2 + np.abs(b[m:]) ** 2
-        # The same FP64 path with the option set (it selects the same kernel).
-        ctx.set_option("f64_reduction", 1)
-        solve("f64")
-        torch.cuda.synchronize()
-        flush.zero_()
-        e0.record(stream)
-        solve("f64")
-        e1.record(stream)
-        e1.synchronize()
-        ms64r = e0.elapsed_time(e1)
-        ctx.set_option("f64_reduction", 0)
         fp64 = {"value": pairs / (ms64 / 1e3) / 1e9, "unit": UNIT, "ms_per_step": ms64,
-                "reduced_phase_option": {"value": pairs / (ms64r / 1e3) / 1e9, "unit": UNIT,
-                                         "ms_per_step": ms64r},
                 "speedup_f32pr_vs_f64": (pairs / (ms / 1e3)) / (pairs / (ms64 / 1e3)),
                 "rel_l2_field_f32pr_vs_f64": float(np.linalg.norm(a - b) / np.linalg.norm(b)),
                 "rel_l2_intensity_f32pr_vs_f64": float(np.linalg.norm(ia - ib) / np.linalg.norm(ib))}

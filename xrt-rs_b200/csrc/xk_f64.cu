@@ -156,7 +156,7 @@ __device__ __forceinline__ void pairs_f64(const RayRec64& r, const double (&px)[
         p2[i] = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
         nd[i] = fma(r.nz, dz, fma(r.ny, dy, r.nx * dx));
         phase[i] = __dmul_rn(r.k, sqrt_and_rcp(p2[i], &inv[i]));
-        // 2^-198 <= p2 < 2^777 (path > 1e-30, no under- or overflow above)
+        // 2^-198 <= p2 < 2^817 (path > 1e-30, no under- or overflow above)
         // and |phase| < 2^50; NaN and infinities fall outside.
         fast = fast &&
                (unsigned)(__double2hiint(p2[i]) - 0x33900000) < 0x73000000u - 0x33900000u &&
