@@ -9,9 +9,9 @@
 //     E         = -k dS dT / (4 D^3) (1 + O((dS + dT) / D^2)).
 // The first three terms make a phase that is a row phase plus a column phase,
 // so the tile is a complex matrix product over the rays, and
-// exp(i E) = 1 + i E + O(E^2) adds one more product with the same ray index as
-// contraction, because E is a row factor dS times a column factor dT. The
-// planner takes the product only where the dropped terms stay far below the
+// exp(i E) = 1 + i E - E^2 / 2 + O(E^3) adds one or two more products with the same
+// ray index as contraction, because E is a row factor dS times a column factor dT.
+// The planner takes the product only where the dropped terms stay far below the
 // requested tolerance (grid_plan). The amplitude (nl + n.(p - r)/|p - r|) /
 // |p - r| varies along a tile by 1e-7 to 1e-2; its ray part at p0 goes to the
 // columns, its first-order change to each side as a factor.
@@ -47,17 +47,15 @@ using namespace phasor;
 
 constexpr int kTileM = 256;
 constexpr uint32_t kGA = 128 * 128;  // 128 rows x 128 B: one f16 tile of a CTA
-constexpr int kGStages = 2;
-constexpr uint32_t kGStage = 6 * kGA;  // hi, lo, first order of A (128 rows) and of B (128 rows)
-constexpr uint32_t kGRayBytes = kFRays * 64;
-constexpr int kGRayBufs = 3;
+constexpr uint32_t kGTiles = 12 * kGA;  // the stages' tiles, in every form
+constexpr uint32_t kGRays = 3 * kFRays * 64;  // staged ray records
 constexpr int kGEpiBufs = 3;  // staging buffers per epilogue warp
 constexpr uint32_t kDrainBytes = 32 * 16 * 4;  // 32 rows x 16 columns of a partial
-constexpr size_t kGSmem = 1024 + (size_t)kGStages * kGStage + kGRayBufs * kGRayBytes +
-                          4 * kGEpiBufs * kDrainBytes + 256;
+constexpr size_t kGSmem = 1024 + kGTiles + kGRays + 4 * kGEpiBufs * kDrainBytes + 256;
 static_assert(kGSmem <= 227 * 1024, "shared memory");
 
-// The product's two forms, the same bytes per stage of 32 rays.
+// The product's three forms. The first two have two stages of 32 rays, each of six
+// tiles: hi, lo and first order of A (128 rows) and of B (128 rows).
 // Narrow: 128 columns per tile. A row of either operand holds its rays' (re, im)
 // words, and B has a real-part and an imaginary-part row per column; the two
 // accumulators of 256 TMEM columns alternate between segments.
@@ -70,14 +68,29 @@ static_assert(kGSmem <= 227 * 1024, "shared memory");
 // 7.1 ms in a row, the chip at its power limit and 1.55 GHz). In the wide form
 // the tensor pipe is busy 72 % of the time (narrow 43 %) and shared memory 75 %
 // (products 35, record loads 22, stores 18 %).
-template <bool WIDE>
+// Second: the wide form with the product A_2 B_2 of the second order, X dS^2 times
+// -W (4 pi q dT)^2 / 2, in three stages of 16 rays: a row of a tile holds 16 real and 16
+// imaginary hi parts, then the lo parts; of another, first, then second orders. For the
+// screens on which E is past first order on whole tiles. 20 MMAs per accumulator and 32
+// rays instead of 16: 8.7 ms on 2^20 rays x 512^2 points at 0.5 m, where the wide form
+// would take 7.1. First order alone, on tiles small enough for it, took 4.0 and 7.9 ms on
+// 2^18 rays x 256^2 points +-1 mm at 1 m, 10 and 20 keV; so 1.07 and 3.6.
+template <int FORM>
 struct Form {
-    static constexpr int kTileN = WIDE ? 256 : 128;
-    static constexpr int kAcc = WIDE ? 2 : 1;       // accumulators of a segment
-    static constexpr int kProdWarps = WIDE ? 8 : 12;
+    static constexpr bool kWide = FORM != kFormNarrow, kSecond = FORM == kFormSecond;
+    static constexpr int kTileN = kWide ? 256 : 128;
+    static constexpr int kAcc = kWide ? 2 : 1;  // accumulators of a segment
+    static constexpr int kProdWarps = kWide ? 8 : 12;
     static constexpr int kThreads = 32 + kFEpiThreads + 32 * kProdWarps + 32;
+    static constexpr int kRays = kSecond ? 16 : kFRays;  // of a stage
+    static constexpr int kStages = kSecond ? 3 : 2;
+    static constexpr int kRayBufs = kSecond ? 6 : 3;
+    static constexpr uint32_t kStage = kGTiles / kStages, kRayBytes = kRays * 64;
+    static_assert(kRayBufs * kRayBytes == kGRays, "ray buffers");
 };
 constexpr double kGridShare = 0.1;  // of the tolerance: the dropped orders of exp(iE)
+constexpr double kGridMostE = 300.0;  // largest E per tolerance
+constexpr double kSecondCost = 1.1;   // of the narrow form's time per padded pair
 constexpr double kGridScale = 1024.0;  // largest |W|: lo parts stay normal f16 numbers
 constexpr size_t kGridRecBytes = (size_t)512 << 20;  // ray records of one launch
 constexpr size_t kGridPartialBytes = (size_t)1 << 30;  // of the splits' partials
@@ -134,19 +147,16 @@ __global__ void __launch_bounds__(256)
         if (bad) atomicOr(&out->bad, 1);
         if (mask) atomicOr(&out->outer_mask, mask);
     }
-    // Half extents of every tile of every size, one warp per tile (the sizes below
-    // 32 with those of 32). Sizes and axes share the warps' turns, so that a small
-    // screen takes one of them.
+    // Half extents of every tile of every size, one warp per tile. Sizes and axes
+    // share the warps' turns, so that a small screen takes one of them.
     const int warp = t0 >> 5, warps = step >> 5;
-    constexpr int kWarpSize = 2;  // kGridSpan << kWarpSize points: one per lane
-    static_assert(kGridSpan << kWarpSize == 32, "one point per lane");
     int base = 0;  // tiles of the sizes and axes before
     for (int axis = 0; axis < 2; ++axis)
-        for (int k = kWarpSize; k < kGridSizes; ++k) {
+        for (int k = 0; k < kGridSizes; ++k) {
             const int count = axis ? len : m / len, size = kGridSpan << k;
             const int tiles = (count + size - 1) / size;
             for (int t = (warp + warps - base % warps) % warps; t < tiles; t += warps) {
-                double half = 0.0, part[kWarpSize] = {};  // whole tile; the sizes below 32
+                double half = 0.0;
                 for (int c = 0; c < 3; ++c) {
                     if ((c == inner) != (axis == 1)) continue;
                     const double* a = coord(p, c);
@@ -156,27 +166,14 @@ __global__ void __launch_bounds__(256)
                         lo = fmin(lo, w);
                         hi = fmax(hi, w);
                     }
-#pragma unroll
-                    for (int b = 0; b < 5; ++b) {
-                        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, 1 << b));
-                        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, 1 << b));
-#pragma unroll
-                        for (int p = 0; p < kWarpSize; ++p)  // -inf where a group has no point
-                            if (2 << b == kGridSpan << p) part[p] = fmax(part[p], 0.5 * (hi - lo));
+                    for (int o = 16; o > 0; o >>= 1) {
+                        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
                     }
                     half = fmax(half, 0.5 * (hi - lo));
                 }
                 if (lane == 0)
                     atomicMax(&out->extent[axis][k], (unsigned long long)__double_as_longlong(half));
-                if (k > kWarpSize) continue;
-#pragma unroll
-                for (int p = 0; p < kWarpSize; ++p) {
-                    for (int o = 16; o > 0; o >>= 1)
-                        part[p] = fmax(part[p], __shfl_xor_sync(0xffffffffu, part[p], o));
-                    if (lane == 0)
-                        atomicMax(&out->extent[axis][p],
-                                  (unsigned long long)__double_as_longlong(part[p]));
-                }
             }
             base += tiles;
         }
@@ -273,8 +270,8 @@ __global__ void __launch_bounds__(256) grid_records_kernel(RecordArgs g, float4*
     o[0] = make_float4(lah, lbh, (float)(la - (double)lah), (float)(lb - (double)lbh));
     o[1] = make_float4((float)(2.0 * a), (float)(2.0 * b), (float)(h - g.h0),
                        (float)(-0.25 * h * inv * inv));
-    o[2] = make_float4((float)(turns - rint(turns)), (float)(g.w_re[j] * w1), (float)(g.w_im[j] * w1),
-                       (float)(-0.5 * (1.0 + nu / obl) * inv * inv));
+    o[2] = make_float4((float)(turns - rint(turns)), (float)(g.w_re[j] * w1),
+                       (float)(g.w_im[j] * w1), (float)(-0.5 * (1.0 + nu / obl) * inv * inv));
     float4 e = make_float4((float)(na * inv / obl), (float)(nb * inv / obl), 0.f, 0.f);
     if (g.w2_re) {
         const double w2 = w * g.scale[1];
@@ -378,15 +375,16 @@ struct PairRow {
     }
 };
 
-// (c, s) of two rays -> f16 hi, lo and hi times the factors (e0, e1).
-__device__ __forceinline__ void split_pair(const float (&c)[2], const float (&s)[2], float e0,
-                                           float e1, uint32_t* h, uint32_t* l, uint32_t* e,
-                                           int re, int im) {
+// (c, s) of two rays -> f16 hi, lo and hi times the factors (e0, e1); returns these.
+__device__ __forceinline__ uint32_t split_pair(const float (&c)[2], const float (&s)[2], float e0,
+                                               float e1, uint32_t* h, uint32_t* l, uint32_t* e,
+                                               int re, int im) {
     split16x2(c[0], c[1], &h[re], &l[re]);
     split16x2(s[0], s[1], &h[im], &l[im]);
     const uint32_t f = pack16x2(e0, e1);
     e[re] = mul2(h[re], f);
     e[im] = mul2(h[im], f);
+    return f;
 }
 
 // Producer warps of a CTA of the pair, narrow form. A warp fills 16-byte chunks
@@ -405,6 +403,7 @@ __device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int 
                                               uint64_t* ray_empty, unsigned char* rays_smem,
                                               volatile int* flag) {
     using namespace sm100;
+    using F = Form<kFormNarrow>;
     constexpr int NE = ZZ ? 1 : 2;   // pair-rows per thread
     constexpr int NCH = ZZ ? 2 : 1;  // chunks per thread
     PairRow row[NE];
@@ -417,15 +416,15 @@ __device__ __forceinline__ void grid_producer(const ProductArgs& g, int c0, int 
         row[e].set(ux, uy, g.h0);
     }
     for (int i = 0; i < nrb; ++i) {
-        const int s = i % kGStages, rb = i % kGRayBufs;
-        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kGRayBufs) & 1u, g.wait_limit);
-        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kGStages) & 1u) ^ 1u, g.wait_limit);
+        const int s = i % F::kStages, rb = i % F::kRayBufs;
+        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / F::kRayBufs) & 1u, g.wait_limit);
+        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / F::kStages) & 1u) ^ 1u, g.wait_limit);
         if (!__all_sync(0xffffffffu, ok)) {
             *flag = 1;
             return;
         }
-        unsigned char* base = tiles + (size_t)s * kGStage;
-        const float4* sr = reinterpret_cast<const float4*>(rays_smem + rb * kGRayBytes);
+        unsigned char* base = tiles + (size_t)s * F::kStage;
+        const float4* sr = reinterpret_cast<const float4*>(rays_smem + rb * F::kRayBytes);
 #pragma unroll
         for (int ch = 0; ch < NCH; ++ch) {
             const int c = c0 + ch;
@@ -506,6 +505,7 @@ __device__ __forceinline__ void grid_producer_wide(const ProductArgs& g, int w, 
                                                    uint64_t* ray_empty, unsigned char* rays_smem,
                                                    volatile int* flag) {
     using namespace sm100;
+    using F = Form<kFormWide>;
     constexpr int NE = 2;  // pair-rows at a time (1: 6.68, 2: 6.50, 4: 7.85 ms)
     const int sub = (lane >> 3) & 1, oct = w & 3;
     const int row0 = 64 * (w >> 2) + (lane & 7) + ((lane & 16) >> 1);  // + 16 e
@@ -517,16 +517,16 @@ __device__ __forceinline__ void grid_producer_wide(const ProductArgs& g, int w, 
     // This thread's 8 bytes of the real and the imaginary 16-byte word of row 0.
     const uint32_t at_re = sw128(row0, oct) + 8 * sub, at_im = sw128(row0, 4 + oct) + 8 * sub;
     for (int i = 0; i < nrb; ++i) {
-        const int s = i % kGStages, rb = i % kGRayBufs;
-        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / kGRayBufs) & 1u, g.wait_limit);
-        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / kGStages) & 1u) ^ 1u, g.wait_limit);
+        const int s = i % F::kStages, rb = i % F::kRayBufs;
+        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / F::kRayBufs) & 1u, g.wait_limit);
+        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / F::kStages) & 1u) ^ 1u, g.wait_limit);
         if (!__all_sync(0xffffffffu, ok)) {
             *flag = 1;
             return;
         }
-        unsigned char* base = tiles + (size_t)s * kGStage;
-        const float4* sr =
-            reinterpret_cast<const float4*>(rays_smem + rb * kGRayBytes) + 4 * (8 * oct + 4 * sub);
+        unsigned char* base = tiles + (size_t)s * F::kStage;
+        const float4* sr = reinterpret_cast<const float4*>(rays_smem + rb * F::kRayBytes) +
+                           4 * (8 * oct + 4 * sub);
 #pragma unroll
         for (int e0 = 0; e0 < 4; e0 += NE) {
             uint32_t ah[NE][4], al[NE][4], ae[NE][4];  // re, re, im, im
@@ -578,6 +578,96 @@ __device__ __forceinline__ void grid_producer_wide(const ProductArgs& g, int w, 
     }
 }
 
+// Producer warps of the second-order form, as grid_producer_wide's: warp w takes rays
+// 8 (w % 2) .. + 7 of the stage for the pair-rows 32 (w / 2) .. + 31.
+template <bool AMP>
+__device__ __forceinline__ void grid_producer_second(const ProductArgs& g, int w, int lane, int mt,
+                                                     int nt, int col, uint32_t half, int nrb,
+                                                     unsigned char* tiles, uint32_t full_lead,
+                                                     uint64_t* empty, uint64_t* ray_full,
+                                                     uint64_t* ray_empty,
+                                                     unsigned char* rays_smem,
+                                                     volatile int* flag) {
+    using namespace sm100;
+    using F = Form<kFormSecond>;
+    constexpr int NE = 2;
+    const int sub = (lane >> 3) & 1, oct = w & 1;
+    const int row0 = 32 * (w >> 1) + (lane & 7) + ((lane & 16) >> 1);  // + 16 e
+    PairRow row[NE];
+#pragma unroll
+    for (int e = 0; e < NE; ++e)
+        row[e].set(row_offset(g, mt >> 1, (mt & 1) * 128 + row0 + 16 * e),
+                   col_offset(g, nt, 128 * half + row0 + 16 * e), g.h0);
+    // This thread's 8 bytes of row 0's real and imaginary 16-byte words, in the first
+    // (hi, first order) and the second (lo, second order) half of the row.
+    uint32_t at[2][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) at[k >> 1][k & 1] = sw128(row0, 2 * k + oct) + 8 * sub;
+    for (int i = 0; i < nrb; ++i) {
+        const int s = i % F::kStages, rb = i % F::kRayBufs;
+        bool ok = mbar_wait(&ray_full[rb], (uint32_t)(i / F::kRayBufs) & 1u, g.wait_limit);
+        ok = ok && mbar_wait(&empty[s], ((uint32_t)(i / F::kStages) & 1u) ^ 1u, g.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *flag = 1;
+            return;
+        }
+        unsigned char* base = tiles + (size_t)s * F::kStage;
+        const float4* sr = reinterpret_cast<const float4*>(rays_smem + rb * F::kRayBytes) +
+                           4 * (8 * oct + 4 * sub);
+        // Words re, re, im, im of hi, lo, first and second order.
+        uint32_t a[4][NE][4], b[4][NE][4];
+#pragma unroll
+        for (int pr = 0; pr < 2; ++pr) {
+            float cx[NE][2], sx[NE][2], cy[NE][2], sy[NE][2], ex[NE][2], ey[NE][2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float4* rec = sr + 4 * (2 * pr + u);
+                const float4 v0 = rec[0], v1 = rec[1], v2 = rec[2];
+                float4 v3 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (AMP || col) v3 = rec[3];
+#pragma unroll
+                for (int e = 0; e < NE; ++e)
+                    row[e].template ray<false, AMP>(v0, v1, v2, v3, col, cx[e][u], sx[e][u],
+                                                    cy[e][u], sy[e][u], ex[e][u], ey[e][u]);
+            }
+            constexpr uint32_t kMinusHalf2 = 0xb800b800u;
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+                const uint32_t fx = split_pair(cx[e], sx[e], ex[e][0], ex[e][1], a[0][e], a[1][e],
+                                               a[2][e], pr, 2 + pr);
+                const uint32_t fy = mul2(split_pair(cy[e], sy[e], ey[e][0], ey[e][1], b[0][e],
+                                                    b[1][e], b[2][e], pr, 2 + pr),
+                                         kMinusHalf2);
+#pragma unroll
+                for (int k = pr; k < 4; k += 2) {
+                    a[3][e][k] = mul2(a[2][e][k], fx);
+                    b[3][e][k] = mul2(b[2][e][k], fy);
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+                const uint32_t(&v)[4] = t < 2 ? a[2 * t][e] : b[2 * (t - 2)][e];
+                const uint32_t(&w2)[4] = t < 2 ? a[2 * t + 1][e] : b[2 * (t - 2) + 1][e];
+                unsigned char* o = base + t * kGA + 16 * 128 * e;
+                *reinterpret_cast<uint2*>(o + at[0][0]) = make_uint2(v[0], v[1]);
+                *reinterpret_cast<uint2*>(o + at[0][1]) = make_uint2(v[2], v[3]);
+                *reinterpret_cast<uint2*>(o + at[1][0]) = make_uint2(w2[0], w2[1]);
+                *reinterpret_cast<uint2*>(o + at[1][1]) = make_uint2(w2[2], w2[3]);
+            }
+        // Make the generic-proxy stores visible to the tensor cores, then one
+        // arrival per warp on the even CTA's stage barrier.
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive_cluster(full_lead + 8u * (uint32_t)s);
+            mbar_arrive(&ray_empty[rb]);
+        }
+    }
+}
+
 // Epilogue role (warps 1..4): adds each finished accumulator segment to this
 // CTA's 128 rows of the split's partial. The partial is stored in contiguous
 // blocks of 32 rows x 16 columns (partial_at), so that 16 columns of a warp's 32
@@ -588,20 +678,22 @@ __device__ __forceinline__ void grid_producer_wide(const ProductArgs& g, int w, 
 // segments of one block and 7.8 ms with ten, now 16.8 and 7.5 ms, narrow form.)
 // Each block's operations complete before its next segment's start, so the
 // partial is s0 + s1 + ... in segment order.
-template <bool WIDE>
+template <int FORM>
 __device__ __forceinline__ void grid_drain(const ProductArgs& g, int warp, int lane, int mt,
-                                           int sp, int nrb, uint32_t tmem, uint64_t* acc_full,
+                                           int sp, int nrb, int seg_len, uint32_t tmem,
+                                           uint64_t* acc_full,
                                            uint32_t acc_empty_lead, unsigned char* stage,
                                            volatile int* flag) {
     using namespace sm100;
-    using F = Form<WIDE>;
+    using F = Form<FORM>;
+    constexpr bool WIDE = F::kWide;
     constexpr int kBlocks = kFN / 16, kBlock = 512;  // blocks per accumulator, floats
     const int qd = warp & 3;
     float* row = g.partial + (((size_t)sp * (g.m_pad / 32) + (size_t)mt * 4 + qd) * (g.n_pad / 16) +
                               (size_t)blockIdx.y * F::kAcc * kBlocks) * kBlock;
     // Segments of the accumulators, as the MMA issuer counts them.
-    int drains = (nrb + g.seg - 1) / g.seg;
-    if (WIDE) drains += 1 + (max(0, nrb - max(1, g.seg / 2)) + g.seg - 1) / g.seg;
+    int drains = (nrb + seg_len - 1) / seg_len;
+    if (WIDE) drains += 1 + (max(0, nrb - max(1, seg_len / 2)) + seg_len - 1) / seg_len;
     if (nrb == 0) {
         for (int c = lane; c < F::kAcc * kBlocks * kBlock; c += 32) row[c] = 0.f;
         return;
@@ -662,23 +754,24 @@ __device__ __forceinline__ size_t partial_at(size_t im, size_t x, int n_pad) {
     return ((im >> 5) * (size_t)(n_pad >> 4) + (x >> 4)) * 512 + r * 16 + k;
 }
 
-template <bool AMP, bool WIDE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads, 1)
+template <bool AMP, int FORM>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<FORM>::kThreads, 1)
     grid_product_kernel(ProductArgs g) {
     using namespace sm100;
-    using F = Form<WIDE>;
+    using F = Form<FORM>;
+    constexpr bool WIDE = F::kWide;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    unsigned char* rays_smem = tiles + kGStages * kGStage;
-    unsigned char* epi_smem = rays_smem + kGRayBufs * kGRayBytes;
+    unsigned char* rays_smem = tiles + kGTiles;
+    unsigned char* epi_smem = rays_smem + kGRays;
     uint64_t* full = reinterpret_cast<uint64_t*>(epi_smem + 4 * kGEpiBufs * kDrainBytes);
-    uint64_t* empty = full + kGStages;
-    uint64_t* acc_full = empty + kGStages;
+    uint64_t* empty = full + F::kStages;
+    uint64_t* acc_full = empty + F::kStages;
     uint64_t* acc_empty = acc_full + 2;
     uint64_t* ray_full = acc_empty + 2;
-    uint64_t* ray_empty = ray_full + kGRayBufs;
-    uint64_t* mma_done = ray_empty + kGRayBufs;  // every issued MMA has completed
+    uint64_t* ray_empty = ray_full + F::kRayBufs;
+    uint64_t* mma_done = ray_empty + F::kRayBufs;  // every issued MMA has completed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
     volatile int* flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -689,12 +782,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
     const bool leader = half == 0;
     const int rb0 = (int)((long long)g.ray_blocks * sp / g.splits);
     const int rb1 = (int)((long long)g.ray_blocks * (sp + 1) / g.splits);
-    const int nrb = rb1 - rb0;
+    // Stages of the split and of a segment.
+    constexpr int kPerBlock = kFRays / F::kRays;
+    const int nrb = (rb1 - rb0) * kPerBlock, seg = g.seg * kPerBlock;
 
     if (threadIdx.x == 0) {
         // full and acc_empty are used in the even CTA only: they collect the
         // arrivals of both CTAs' producer and epilogue warps.
-        for (int s = 0; s < kGStages; ++s) {
+        for (int s = 0; s < F::kStages; ++s) {
             mbar_init(&full[s], 2 * F::kProdWarps + (s == 0 ? g.stall : 0u));
             mbar_init(&empty[s], 1);
         }
@@ -702,7 +797,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 2 * kFEpiThreads);
         }
-        for (int b = 0; b < kGRayBufs; ++b) {
+        for (int b = 0; b < F::kRayBufs; ++b) {
             mbar_init(&ray_full[b], 1);
             mbar_init(&ray_empty[b], F::kProdWarps);
         }
@@ -735,18 +830,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
             // own half a segment earlier. A part is issued first in its segment's
             // last stage and last in the next stage, so that the other part's
             // products of both stages run while it is drained.
-            int end0 = min(nrb, g.seg), end1 = min(nrb, max(1, g.seg / 2)), q0 = 0, q1 = 0;
+            int end0 = min(nrb, seg), end1 = min(nrb, max(1, seg / 2)), q0 = 0, q1 = 0;
             bool new0 = true, new1 = true;
             for (int i = 0; i < nrb && good; ++i) {
-                const int s = i % kGStages;
-                if (!mbar_wait_cluster(&full[s], (uint32_t)(i / kGStages) & 1u, g.wait_limit)) {
+                const int s = i % F::kStages;
+                if (!mbar_wait_cluster(&full[s], (uint32_t)(i / F::kStages) & 1u, g.wait_limit)) {
                     *flag = 1;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t t0 = smem_u32(tiles) + (uint32_t)s * kGStage;
-                const uint32_t as[4] = {t0 + 2 * kGA, t0, t0, t0 + kGA};
-                const uint32_t bs[4] = {t0 + 5 * kGA, t0 + 3 * kGA, t0 + 4 * kGA, t0 + 3 * kGA};
+                // First order, (second order,) hi hi, hi lo, lo hi.
+                const uint32_t t0 = smem_u32(tiles) + (uint32_t)s * F::kStage;
+                constexpr int P = F::kSecond ? 5 : 4, K = F::kSecond ? 2 : 4;
+                uint32_t as[5], bs[5];
+                if (F::kSecond) {
+                    const uint32_t a1 = t0 + kGA, b0 = t0 + 2 * kGA, b1 = t0 + 3 * kGA;
+                    as[0] = a1, as[1] = a1 + 64, as[2] = t0, as[3] = t0, as[4] = t0 + 64;
+                    bs[0] = b1, bs[1] = b1 + 64, bs[2] = b0, bs[3] = b0 + 64, bs[4] = b0;
+                } else {
+                    as[0] = t0 + 2 * kGA, as[1] = t0, as[2] = t0, as[3] = t0 + kGA;
+                    bs[0] = t0 + 5 * kGA, bs[1] = t0 + 3 * kGA, bs[2] = t0 + 4 * kGA;
+                    bs[3] = t0 + 3 * kGA;
+                }
                 const int first = WIDE && ((new0 && i > 0) || i + 1 == end1);
                 for (int h = first, t = 0; t < F::kAcc; ++t, h ^= 1) {
                     const bool fresh = h ? new1 : new0;
@@ -755,19 +860,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
                     if (!good) break;
                     const uint32_t d = tmem + (uint32_t)(b * kFN);
 #pragma unroll
-                    for (int p = 0; p < 4; ++p)
+                    for (int p = 0; p < P; ++p)
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            // Wide: A's real (k < 2) or imaginary parts meet B's
+                        for (int k = 0; k < K; ++k) {
+                            // Wide: A's real (k < K / 2) or imaginary parts meet B's
                             // of the same kind, subtracted for the imaginary
                             // ones, or (h) of the other kind; of i E W (p == 0),
                             // stored as E W, the other way round.
-                            const int x = k >> 1;
+                            const int x = k / (K / 2);
                             const bool swap = WIDE && (h ^ (p == 0));
                             const bool neg =
                                 WIDE && (p == 0 ? (h == 0 || x == 1) : (h == 0 && x == 1));
                             umma_f16_pair(d, desc_kmajor_sw128(as[p] + 32u * k),
-                                          desc_kmajor_sw128(bs[p] + 32u * (swap ? k ^ 2 : k)),
+                                          desc_kmajor_sw128(bs[p] + 32u * (swap ? k ^ (K / 2) : k)),
                                           neg ? idesc | kNegateB : idesc,
                                           (uint32_t)(!fresh | p | k));
                         }
@@ -778,7 +883,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
                     }
                     (h ? new1 : new0) = last;
                     (h ? q1 : q0) += last;
-                    (h ? end1 : end0) = last ? min(nrb, i + 1 + g.seg) : (h ? end1 : end0);
+                    (h ? end1 : end0) = last ? min(nrb, i + 1 + seg) : (h ? end1 : end0);
                 }
                 umma_commit_pair(smem_u32(&empty[s]));
                 umma_commit_pair(mapa_shared(&empty[s], peer));
@@ -790,12 +895,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
         }
         __syncwarp();
     } else if (warp <= 4) {
-        grid_drain<WIDE>(g, warp, lane, mt, sp, nrb, tmem, acc_full, mapa_shared(acc_empty, 0),
+        grid_drain<FORM>(g, warp, lane, mt, sp, nrb, seg, tmem, acc_full, mapa_shared(acc_empty, 0),
                          epi_smem + (warp - 1) * kGEpiBufs * kDrainBytes, flag);
     } else if (warp < 5 + F::kProdWarps) {
         const int w = warp - 5;
         const uint32_t full_lead = mapa_shared(full, 0);
-        if constexpr (WIDE)
+        if constexpr (F::kSecond)
+            grid_producer_second<AMP>(g, w, lane, mt, nt, col, half, nrb, tiles, full_lead, empty,
+                                      ray_full, ray_empty, rays_smem, flag);
+        else if constexpr (WIDE)
             grid_producer_wide<AMP>(g, w, lane, mt, nt, col, half, nrb, tiles, full_lead, empty,
                                     ray_full, ray_empty, rays_smem, flag);
         else if (w < 8)
@@ -810,20 +918,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Form<WIDE>::kThreads
             g.recs + ((size_t)((mt >> 1) * g.n_tiles + nt) * g.pad + (size_t)rb0 * kFRays) * 4;
         int i = 0;
         for (; i < nrb; ++i) {
-            const int rb = i % kGRayBufs;
-            if (i >= kGRayBufs &&
-                !mbar_wait(&ray_empty[rb], (uint32_t)(i / kGRayBufs - 1) & 1u, g.wait_limit)) {
+            const int rb = i % F::kRayBufs;
+            if (i >= F::kRayBufs &&
+                !mbar_wait(&ray_empty[rb], (uint32_t)(i / F::kRayBufs - 1) & 1u, g.wait_limit)) {
                 *flag = 1;
                 break;
             }
-            mbar_arrive_expect_tx(&ray_full[rb], kGRayBytes);
-            bulk_g2s(rays_smem + rb * kGRayBytes, src + (size_t)i * kFRays * 4, kGRayBytes,
+            mbar_arrive_expect_tx(&ray_full[rb], F::kRayBytes);
+            bulk_g2s(rays_smem + rb * F::kRayBytes, src + (size_t)i * F::kRays * 4, F::kRayBytes,
                      &ray_full[rb]);
         }
         // No copy may still be writing into this CTA's shared memory when it
         // exits: the last ones land whether or not a producer waits for them.
-        for (int k = max(0, i - kGRayBufs); k < i; ++k)
-            if (!mbar_wait(&ray_full[k % kGRayBufs], (uint32_t)(k / kGRayBufs) & 1u,
+        for (int k = max(0, i - F::kRayBufs); k < i; ++k)
+            if (!mbar_wait(&ray_full[k % F::kRayBufs], (uint32_t)(k / F::kRayBufs) & 1u,
                            max(g.wait_limit, kMmaDrainPolls)))
                 *flag = 1;
     }
@@ -909,8 +1017,8 @@ const double* coord_host(const PixDev& p, int c) { return c == 0 ? p.x : (c == 1
 
 // Bytes of one split's partial.
 size_t partial_plane(const GridPlan& g) {
-    return (size_t)g.m_tiles * kTileM * g.n_tiles * g.columns * (g.wide ? 2 : 1) * kFN *
-           sizeof(float);
+    return (size_t)g.m_tiles * kTileM * g.n_tiles * g.columns *
+           (g.form == kFormNarrow ? 1 : 2) * kFN * sizeof(float);
 }
 
 double bits_to_double(unsigned long long b) {
@@ -964,38 +1072,49 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     const double omin = std::min(std::fabs(obl.lo), std::fabs(obl.hi)), omax = largest(obl);
 
     // Form, and rows along the outer or the inner axis: whichever costs less
-    // (then whichever leaves the smaller first-order phase).
+    // (then whichever leaves the smaller mixed phase).
     bool found = false;
     double best_cost = 0.0, best_e = 0.0;
-    // Tiles may use fewer rows (256 >> fm) or columns (of 128 >> fn; or 256) than they
-    // have: E falls with either, at the price of the rest. For many rays that is below
-    // the general kernel's down to 1/16 of a tile (2^18 rays x 256^2 points +-1 mm at
-    // 1 m: 10.3 -> 4.0 ms at 10 keV, 12.0 -> 7.9 at 20, general at 30), for a few
-    // thousand, where the general kernel's sorting counts, down to 1/128 (3000 rays x
-    // 64 x 200 points at 0.3 m: 0.83 -> 0.48 ms).
+    // Tiles may use fewer rows (256 >> fm) or columns (of 128 >> fn, or 256; with the
+    // second order 256 >> fn - 4) than they have: E falls with either, at the price of
+    // the rest, which is still below the general kernel's down to 1/16 of a tile (2^18
+    // rays x 256^2 points +-1 mm at 1 m: 10.3 -> 1.07 ms at 10 keV, 12.0 -> 3.6 at 20,
+    // 12.3 -> 3.6 at 30).
     const double d2 = dlo * dlo, d3 = d2 * dlo, d5 = d3 * d2;
-    for (int form = 0; form < 2 * kGridSizes * kGridSizes; ++form) {
-        const bool swap = form & 1;
-        const int fm = (form >> 1) % kGridSizes, fn = (form >> 1) / kGridSizes;
-        const bool wide = fn == kGridSizes - 1;
+    constexpr int kSpans = 2 * kGridSizes;
+    for (int i = 0; i < 2 * kGridSizes * kSpans; ++i) {
+        const bool swap = i & 1;
+        const int fm = (i >> 1) % kGridSizes, fn = (i >> 1) / kGridSizes;
+        const int form = fn < kGridSizes - 1 ? kFormNarrow
+                                             : (fn == kGridSizes - 1 ? kFormWide : kFormSecond);
         const int am = swap ? inner : outer, an = swap ? outer : inner;
         const size_t nm = swap ? len : rows, nn = swap ? rows : len;
-        const double em = bits_to_double(probe.extent[swap ? 1 : 0][kGridSizes - 1 - fm]);
-        const double en = bits_to_double(
-            probe.extent[swap ? 0 : 1][wide ? kGridSizes - 1 : kGridSizes - 2 - fn]);
+        const int tile_n = form == kFormNarrow ? Form<kFormNarrow>::kTileN
+                                               : Form<kFormWide>::kTileN;
+        const int zm = kGridSizes - 1 - fm;  // sizes of the rows and columns in use
+        const int zn = form == kFormNarrow ? kGridSizes - 2 - fn
+                                           : (form == kFormWide ? kGridSizes - 1 : kSpans - 1 - fn);
+        const int span_m = kGridSpan << zm, span_n = kGridSpan << zn;
+        const size_t mt = blocks_of(nm, span_m), nt = blocks_of(nn, span_n);
+        if (mt * nt > kGridMaxTiles) continue;
+        const double em = bits_to_double(probe.extent[swap ? 1 : 0][zm]);
+        const double en = bits_to_double(probe.extent[swap ? 0 : 1][zn]);
         // |dS| = |u| |(p - r) + (p0 - r)| with |p0 - r| <= |p - r|max - |u|max
         // when the tile lies inside the screen's range.
         const double pm = largest(del[am]), pn = largest(del[an]);
         const double ds = em * (2.0 * pm - em), dt = en * (2.0 * pn - en);
         const double e = r.k * ds * dt / (4.0 * d3);
         const double big = std::max(ds, dt);
-        // What 1 + iE leaves out of exp(i phase): E^2 / 2, and the next order of the
-        // mixed phase, 3/4 E (dS + dT) / D^2. Both at the far corner of a tile and of
-        // the ray box: on a screen beside the rays' axis nearly every ray has that E,
-        // and a focus on a tile's corner then has that error (rays of +-0.05 mm, 5.9 mm
-        // off both axes at 1 m: 1.5e-4 at E = 0.019). A tenth of the tolerance is
-        // about the general kernel's error on coherent fields.
-        if (!(0.5 * e * e + 0.75 * e * (ds + dt) / d2 <= kGridShare * tolerance)) continue;
+        // What 1 + iE (- E^2 / 2) leaves out of exp(i phase): E^2 / 2 (E^3 / 6), and the
+        // next order of the mixed phase, 3/4 E (dS + dT) / D^2. Both at the far corner of
+        // a tile and of the ray box: on a screen beside the rays' axis nearly every ray
+        // has that E, and a focus on a tile's corner then has that error (rays of +-0.05
+        // mm, 5.9 mm off both axes at 1 m, 1 + iE: 1.5e-4 at E = 0.019). A tenth of the
+        // tolerance is about the general kernel's error on coherent fields.
+        const double left = form == kFormSecond ? e * e * e / 6.0 : 0.5 * e * e;
+        if (!(left + 0.75 * e * (ds + dt) / d2 <= kGridShare * tolerance)) continue;
+        // The first-order operands' roundings, 3.5e-4 E of a pair, random over the rays.
+        if (!(e <= kGridMostE * tolerance)) continue;
         if (!(big / d2 <= 1e-2)) continue;
         // Linear phase: an exact FP32 product up to 2^21 turns.
         if (!(kt / dlo * std::max(em * pm, en * pn) < 1.9e6)) continue;
@@ -1009,18 +1128,16 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         if (!(sm <= 0.25 && sn <= 0.25 && sm * sn <= 1e-6 && (sm + sn) * mq <= 1e-6 &&
               mq * mq <= 1e-7))
             continue;
-        const int tile_n = wide ? Form<true>::kTileN : Form<false>::kTileN;
-        const int span_m = kTileM >> fm, span_n = wide ? tile_n : tile_n >> fn;
-        const size_t mt = blocks_of(nm, span_m), nt = blocks_of(nn, span_n);
-        if (mt * nt > kGridMaxTiles) continue;
         // Product: 36e12 pairs/s of the padded screen in the narrow form (2^20 rays x
         // 512^2 points, one column). Wide: 0.85 of its time (6.3 to 7.5 ms there,
         // kernels alone) and 18 us more for twice the partials per tile (first to
         // last kernel, narrow and wide: 101 and 115 us at 10^4 rays x 256^2, 135 and
-        // 141 at 3 10^4, 253 and 244 at 10^5; 289 and 265 at 3 10^4 x 512^2).
+        // 141 at 3 10^4, 253 and 244 at 10^5; 289 and 265 at 3 10^4 x 512^2). With the
+        // second order 1.1 of the narrow form's (8.6 ms there at 0.5 m), and the same 18 us.
         const double area = (double)mt * kTileM * (double)nt * tile_n;
-        const double cost = area * columns * (double)n / 36e12 * (wide ? 0.85 : 1.0) +
-                            (wide ? 18e-6 : 0.0);
+        const double rel = form == kFormNarrow ? 1.0 : (form == kFormWide ? 0.85 : kSecondCost);
+        const double cost = area * columns * (double)n / 36e12 * rel +
+                            (form == kFormNarrow ? 0.0 : 18e-6);
         if (found && !(cost < best_cost || (cost == best_cost && e < best_e))) continue;
         found = true;
         best_cost = cost;
@@ -1031,7 +1148,7 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         g->rows_outer = swap == 0;
         g->nm = nm;
         g->nn = nn;
-        g->wide = wide;
+        g->form = form;
         g->span_m = span_m;
         g->span_n = span_n;
         g->m_tiles = (int)mt;
@@ -1093,7 +1210,9 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
     const double phase =
         r.k * (r.spread2 + 0.6 * side * std::sqrt(r.spread2)) / (2.0 * d0);
     if (phase < 7.0) return false;
-    g->seg = phase < 12.0 ? 1 : phase < 24.0 ? 3 : 10;
+    // The second order makes it 20 MMAs per block.
+    const bool second = g->form == kFormSecond;
+    g->seg = phase < 12.0 ? 1 : phase < 24.0 ? (second ? 2 : 3) : (second ? 8 : 10);
     // Rays per launch: what their records' memory allows, and what `cap` splits can sum
     // in kGridMaxAdds segments each (a launch is added to the field in FP64).
     const size_t tiles = (size_t)g->m_tiles * g->n_tiles;
@@ -1113,7 +1232,8 @@ bool grid_plan(const GridProbe& probe, const GridRanges& r, size_t n, size_t m, 
         double best = 1e300;
         for (size_t t = least; t < least + std::max<size_t>(8, units / work); ++t) {
             const double waves = (double)blocks_of(work * t, units) * units / (double)(work * t);
-            const double cost = waves + 0.01 * (double)(t - least) * std::min(1.0, (double)units / work);
+            const double cost =
+                waves + 0.01 * (double)(t - least) * std::min(1.0, (double)units / work);
             if (cost < best) {
                 best = cost;
                 s = t;
@@ -1170,15 +1290,18 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
     p.h0 = g.h0 / (g.unit * g.unit);
     p.partial = ws.partial.as<float>();
     p.m_pad = g.m_tiles * kTileM;
-    p.n_pad = g.n_tiles * g.columns * (g.wide ? 2 : 1) * kFN;
+    p.n_pad = g.n_tiles * g.columns * (g.form == kFormNarrow ? 1 : 2) * kFN;
     p.err = err;
     p.wait_limit = wait_limit;
     p.stall = stall ? 1 : 0;
-    const auto kern = g.wide ? (g.amp ? grid_product_kernel<true, true>
-                                      : grid_product_kernel<false, true>)
-                             : (g.amp ? grid_product_kernel<true, false>
-                                      : grid_product_kernel<false, false>);
-    const int threads = g.wide ? Form<true>::kThreads : Form<false>::kThreads;
+    void (*const kernels_of[3][2])(ProductArgs) = {
+        {grid_product_kernel<false, kFormNarrow>, grid_product_kernel<true, kFormNarrow>},
+        {grid_product_kernel<false, kFormWide>, grid_product_kernel<true, kFormWide>},
+        {grid_product_kernel<false, kFormSecond>, grid_product_kernel<true, kFormSecond>}};
+    const auto kern = kernels_of[g.form][g.amp ? 1 : 0];
+    static_assert(Form<kFormSecond>::kThreads == Form<kFormWide>::kThreads, "threads");
+    const int threads = g.form == kFormNarrow ? Form<kFormNarrow>::kThreads
+                                              : Form<kFormWide>::kThreads;
     // Set on every call: the attribute belongs to the current device's context.
     XK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem));
     const dim3 grid((unsigned)(2 * g.m_tiles), (unsigned)(g.n_tiles * g.columns),
@@ -1221,8 +1344,8 @@ Status grid_enqueue(const GridPlan& g, GridWorkspace& ws, int* err, uint32_t wai
         XK_CUDA_TRY(cudaGetLastError());
         p.stall = 0;
         grid_reduce_kernel<<<(unsigned)blocks_of(g.nm * g.nn, 256), 256, 0, stream>>>(
-            p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.wide, g.span_m, g.span_n, g.nm,
-            g.nn, g.rows_outer, make_double2(amp / g.inv_scale[0], amp / g.inv_scale[1]),
+            p.partial, g.splits, p.m_pad, p.n_pad, g.columns, g.form != kFormNarrow, g.span_m,
+            g.span_n, g.nm, g.nn, g.rows_outer, make_double2(amp / g.inv_scale[0], amp / g.inv_scale[1]),
             make_double2(g.pes[0], g.pes[1]), make_double2(g.pep[0], g.pep[1]), j0 > 0, g.out);
         XK_CUDA_TRY(cudaGetLastError());
         *kernels += 3;

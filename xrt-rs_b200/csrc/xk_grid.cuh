@@ -14,8 +14,11 @@ namespace xk {
 // most one that depends on i alone (the outer axis), the rest constant, bit
 // for bit. extent[axis][k]: largest half-extent of a tile of kGridSpan << k
 // consecutive points of the axis (0 outer, 1 inner), as the bits of a double.
-constexpr int kGridSpan = 8;   // fewest rows or columns of a tile in use
-constexpr int kGridSizes = 6;  // tile sizes, kGridSpan << 0 .. 5 (256)
+constexpr int kGridSpan = 32;  // fewest rows or columns of a tile in use
+constexpr int kGridSizes = 4;  // tile sizes, kGridSpan << 0 .. 3 (256)
+
+// The product's forms: 128 columns per tile, 256, and 256 with the second order.
+enum GridForm { kFormNarrow, kFormWide, kFormSecond };
 
 struct GridProbe {
     int len;         // inner length; 0 if there is no such order
@@ -44,7 +47,7 @@ struct GridPlan {
     bool rows_outer = true;                  // rows are the outer screen axis
     size_t nm = 0, nn = 0;                   // rows, columns (screen points along the axes)
     size_t inner_len = 0;
-    bool wide = false;                       // 256 columns per tile instead of 128
+    int form = kFormNarrow;                  // GridForm
     int span_m = 0, span_n = 0;              // rows and columns of a tile in use
     int m_tiles = 0, n_tiles = 0, columns = 1;  // tiles of 256 rows and 128 or 256 columns; amplitude columns
     int ray_blocks = 0, splits = 1, seg = 0;
