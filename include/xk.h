@@ -104,15 +104,16 @@ typedef struct xk_stats {
     int n_tiles;             /* screen tiles (F32PR) */
     int n_chunks;            /* ray chunks (F32PR) */
     long long n_items;       /* work items (F32PR) */
-    double phase_bound_rad;  /* planner's bound on the FP32 residual phase */
+    double phase_bound_rad;  /* planner's bound on the FP32 residual phase (sweep 3: pi, its
+                                phases are reduced to half a turn) */
     double h2d_bytes, d2h_bytes;
     double main_kernel_ms;   /* device time of the pair kernel alone (CUDA events) */
     int groups;              /* ray groups per tile (F32PR) */
     int routed_reason;       /* 0 = not routed; see xk_route_reason() */
     int sweep;               /* F32PR sweep used: 0 SFU reciprocal, 1 packed + quadratic series,
                                 2 packed + linear series, 3 rectangular screen as a tensor-core
-                                product (n_tiles, groups and n_chunks: its 256 x 128 tiles, ray
-                                splits and 32-ray blocks); XK_PATH_SEPARABLE (Fresnel): 1 CTA-pair
+                                product (n_tiles, groups and n_chunks: its 256 x 128 or 256 x 256
+                                tiles, ray splits and 32-ray blocks); XK_PATH_SEPARABLE (Fresnel): 1 CTA-pair
                                 tiles, 0 one CTA per tile; -1 none */
     int one_polarization;    /* F32PR: 1 if every ray had ray 0's polarization, so the kernel
                                 summed one amplitude column and Ep = (ep_0 / es_0) Es */
