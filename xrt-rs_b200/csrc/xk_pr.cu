@@ -1432,9 +1432,12 @@ bool depth_cells(double k, double d, double g, double a_across, double a_mean, d
             sq += 0.25 * c->cell[ax] * c->cell[ax];
         }
         const double across = std::sqrt(sq);
+        // At least half of b_most stays for the length along the beam. (Across the
+        // whole of it the length came out as zero, which is no cell at all: counted as
+        // one, it put rays of any depth into the same chunk.)
+        if (!(across * g <= 0.5 * b_most)) return INFINITY;
         const double along =
             std::min(0.5 * ext[2], std::min(b_most - across * g, 0.3 * across / std::max(g, 1e-9)));
-        if (!(along >= 0.0)) return INFINITY;
         c->cell[2] = 2.0 * along;
         const double b = across + along * g, den = d - 2.0 * (b + along);
         if (!(den > 0.0)) return INFINITY;
@@ -1458,7 +1461,8 @@ bool depth_cells(double k, double d, double g, double a_across, double a_mean, d
     eval(lo);
     double cells = 1.0, before = 1.0;
     for (int ax = 0; ax < 3; ++ax) {
-        const double cnt = c->cell[ax] > 0 ? std::floor(ext[ax] / c->cell[ax]) + 1.0 : 1.0;
+        const double cnt = c->cell[ax] > 0 ? std::floor(ext[ax] / c->cell[ax]) + 1.0
+                                           : (ext[ax] > 0 ? INFINITY : 1.0);
         if (!(cnt <= 2097151.0)) return false;
         c->n[ax] = (long long)cnt;
         cells *= cnt;
